@@ -852,6 +852,13 @@ def bench_cok(args, rank, world, local):
         dist.destroy_process_group()
 
 
+def shared_solve(W, np_, v, precision):
+    """Whether variant v of a key runs the FP64 solves that share factorisations."""
+    if precision:
+        return v == getattr(W, "VARIANT_SHARE", -1)
+    return (np_ == 32 and v == W.VARIANT_FOLD) or (np_ == 64 and v in (getattr(W, "VARIANT_WIDE", -1), W.VARIANT_DEFAULT))
+
+
 def bucket_kernel(W, b, cov_type, precision, ordinary):
     """Name of the solve kernel that ran bucket b (0..4) for this key."""
     if b == 4:
@@ -859,9 +866,11 @@ def bucket_kernel(W, b, cov_type, precision, ordinary):
     np_ = [8, 16, 32, 64][b]
     v = W.solve_variant(np_, cov_type, precision) if hasattr(W, "solve_variant") else 1
     kind = "ordinary" if ordinary else "simple"
+    if shared_solve(W, np_, v, precision):
+        cb, th = (3, 512) if np_ == 32 else (7, 256)
+        return f"k_solve_share<CB={cb}, {kind}, {th}> (FP64 tensor, factorisations shared by neighbouring cells)"
     if np_ == 64 and v in (getattr(W, "VARIANT_WIDE", -1), W.VARIANT_DEFAULT):
-        th, pr = (256, "FP64 plain") if precision == 0 else (256, "FP32 refined")
-        return f"k_solve_wide{64 if precision == 0 else 32}<{kind}, {th}> ({pr}, one warp per system, rolled phases)"
+        return f"k_solve_wide32<{kind}, 256> (FP32 refined, one warp per system, rolled phases)"
     if precision == 0:
         th = 384 if (np_ <= 32 and v == W.VARIANT_FOLD) else 256
         return f"k_solve_fold64<NP={np_}, {kind}, {th}> (FP64 plain, NP/2 lanes per system)"
@@ -883,10 +892,12 @@ def solve_roofline(W, stats_list, cov_type, precision, ordinary, pk):
     ms = float(np.mean([s[f"bucket_ms_{b}"] for s in stats_list]))
     flops = last[f"bucket_flops_{b}"]
     tf = flops / (ms / 1e3) / 1e12 if ms > 0 else 0.0
-    peak = pk["fp32"] if precision else pk["fp64"]
+    np_ = [8, 16, 32, 64, 65][b]
+    fp32 = precision and not (b < 4 and shared_solve(W, np_, W.solve_variant(np_, cov_type, precision), precision))
+    peak = pk["fp32"] if fp32 else pk["fp64"]
     return {"kernel": bucket_kernel(W, b, cov_type, precision, ordinary), "kernel_ms": ms,
             "algorithmic_flops": flops, "achieved_tflops": tf, "peak_tflops": peak, "frac": tf / peak,
-            "bound": "fp32" if precision else "fp64"}
+            "bound": "fp32" if fp32 else "fp64"}
 
 
 def bench_other_configs(args, W, dev, stream, pk):

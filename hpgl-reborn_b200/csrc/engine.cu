@@ -637,22 +637,26 @@ static void run_solves(Engine &E, const Plan &pl, const DevPoints &P, const DevS
     // FP32-refined systems that fail the four-rows-per-lane kernel's check go
     // first to the two-rows-per-lane kernel (classic refinement), and what
     // that does not converge to the FP64 kernel
-    int *esc_cnt = E.buf<int>("esc_cnt", 2 * kBuckets);
+    int *esc_cnt = E.buf<int>("esc_cnt", 3 * kBuckets);
     int *ref_cnt = esc_cnt + kBuckets;
+    int *left_cnt = ref_cnt + kBuckets; // cells the sharing solves leave to the one-system kernel
     int2 *esc_cells = precision ? E.buf<int2>("esc_cells", (size_t)g.n_cells) : nullptr;
     int2 *ref_cells = nullptr;
     int variant[kBuckets];
-    bool any_quad = false;
+    bool any_quad = false, any_share = false;
     for (int b = 0; b < kBuckets; ++b)
     {
         variant[b] = b < 4 ? solve_variant(kBucketNP[b], pl.f.m.type, precision) : kVariantFold;
         any_quad = any_quad || (precision && b < 4 && kBucketNP[b] <= 32 &&
                                 (is_quad_variant(variant[b]) || tune_wanted(kBucketNP[b], pl.f.m.type, precision)));
     }
+    for (int b = 0; b < 4 && g.n_cells >= 64 * E.n_sm(); ++b)
+        any_share = any_share || is_share_variant(kBucketNP[b], precision, variant[b]) ||
+                    tune_wanted(kBucketNP[b], pl.f.m.type, precision);
     if (any_quad) ref_cells = E.buf<int2>("ref_cells", (size_t)g.n_cells);
-    launch_prepare(g, d_mask, all_cells, S.nb_n, d_status, bucket_cnt, bucket_off, tile_cnt, tile_mom, cells, moments,
-                   st);
-    HB_CK(cudaMemsetAsync(esc_cnt, 0, sizeof(int) * 2 * kBuckets, st));
+    launch_prepare(g, any_share ? solve_share_tile(g) : CellTile{0, 0, 0}, d_mask, all_cells, S.nb_n, d_status,
+                   bucket_cnt, bucket_off, tile_cnt, tile_mom, cells, moments, st);
+    HB_CK(cudaMemsetAsync(esc_cnt, 0, sizeof(int) * 3 * kBuckets, st));
     HB_CK(cudaGetLastError());
     E.stats.launches += 3;
     int cnt[kBuckets];
@@ -661,6 +665,8 @@ static void run_solves(Engine &E, const Plan &pl, const DevPoints &P, const DevS
     HB_CK(cudaMemcpyAsync(mom, moments, sizeof(mom), cudaMemcpyDeviceToHost, st));
     HB_CK(cudaStreamSynchronize(st));
     E.mark(STAGE_PREPARE, st);
+    // one list for every sharing bucket (they run one after another)
+    int2 *left_cells = any_share ? E.buf<int2>("left_cells", (size_t)std::max(1, std::max(cnt[2], cnt[3]))) : nullptr;
     int off = 0;
     const double c0 = pl.f.c0();
     const double rhs = ordinary ? 2.0 : 1.0;
@@ -680,11 +686,12 @@ static void run_solves(Engine &E, const Plan &pl, const DevPoints &P, const DevS
             {
                 HB_CK(cudaMemsetAsync(esc_cnt + b, 0, sizeof(int), st));
                 HB_CK(cudaMemsetAsync(ref_cnt + b, 0, sizeof(int), st));
+                HB_CK(cudaMemsetAsync(left_cnt + b, 0, sizeof(int), st));
                 HB_CK(cudaEventRecord(E.ev_[10 + 2 * b], st));
                 HB_CK(launch_solve_bucket(np, precision, v, ordinary, g, bcells, bucket_cnt + b, cnt[b], S.nb_rec,
                                           S.nb_n, ind_value, S.pair64, S.pair32, mean, c0, steps, tol, out,
                                           quad ? ref_cells + first : (esc_cells ? esc_cells + first : nullptr),
-                                          quad ? ref_cnt + b : esc_cnt + b, E.n_sm(), st));
+                                          quad ? ref_cnt + b : esc_cnt + b, left_cells, left_cnt + b, E.n_sm(), st));
                 HB_CK(cudaEventRecord(E.ev_[11 + 2 * b], st));
                 E.stats.launches += 1;
             }
@@ -696,6 +703,7 @@ static void run_solves(Engine &E, const Plan &pl, const DevPoints &P, const DevS
         tune_record(np, pl.f.m.type, precision, ms);
         HB_CK(cudaMemsetAsync(esc_cnt + b, 0, sizeof(int), st));
         HB_CK(cudaMemsetAsync(ref_cnt + b, 0, sizeof(int), st));
+        HB_CK(cudaMemsetAsync(left_cnt + b, 0, sizeof(int), st));
         variant[b] = solve_variant(np, pl.f.m.type, precision);
     };
     for (int b = 0; b < kBuckets; ++b)
@@ -711,9 +719,16 @@ static void run_solves(Engine &E, const Plan &pl, const DevPoints &P, const DevS
             if (b < 4)
             {
                 int2 *first_esc = quad ? ref_cells + off : (esc_cells ? esc_cells + off : nullptr);
+                // A warp of the sharing solve takes eight cells in a row, about 20 us of
+                // dependent steps; below 64 cells an SM the one-system kernel, one cell a
+                // warp, is through sooner (9,472 systems of 32: 24 us against 25).
+                const bool share =
+                    is_share_variant(kBucketNP[b], precision, variant[b]) && cnt[b] >= 64 * E.n_sm();
                 HB_CK(launch_solve_bucket(kBucketNP[b], precision, variant[b], ordinary, g, bcells, bucket_cnt + b,
                                           cnt[b], S.nb_rec, S.nb_n, ind_value, S.pair64, S.pair32, mean, c0, steps,
-                                          tol, out, first_esc, quad ? ref_cnt + b : esc_cnt + b, E.n_sm(), st));
+                                          tol, out, first_esc, quad ? ref_cnt + b : esc_cnt + b,
+                                          share ? left_cells : nullptr, left_cnt + b, E.n_sm(), st));
+                if (share) E.stats.launches += 1;
             }
             else
             {
@@ -741,16 +756,17 @@ static void run_solves(Engine &E, const Plan &pl, const DevPoints &P, const DevS
             HB_CK(launch_solve_bucket(kBucketNP[b], 1, kVariantFold, ordinary, g, ref_cells + esc_off[b], ref_cnt + b,
                                       std::min(cnt[b], E.n_sm() * 8), S.nb_rec, S.nb_n, ind_value, S.pair64,
                                       S.pair32, mean, c0, steps, tol, out, esc_cells + esc_off[b], esc_cnt + b,
-                                      E.n_sm(), st));
+                                      nullptr, nullptr, E.n_sm(), st));
             E.stats.launches += 1;
         }
         // FP64 re-solve of escalated systems, one persistent launch per bucket
         for (int b = 0; b < 4; ++b)
         {
-            if (cnt[b] == 0) continue;
+            if (cnt[b] == 0 || is_share_variant(kBucketNP[b], precision, variant[b])) continue;
             HB_CK(launch_solve_bucket(kBucketNP[b], 0, kVariantDefault, ordinary, g, esc_cells + esc_off[b],
                                       esc_cnt + b, std::min(cnt[b], E.n_sm() * 8), S.nb_rec, S.nb_n, ind_value,
-                                      S.pair64, S.pair32, mean, c0, 0, tol, out, nullptr, nullptr, E.n_sm(), st));
+                                      S.pair64, S.pair32, mean, c0, 0, tol, out, nullptr, nullptr, nullptr, nullptr,
+                                      E.n_sm(), st));
             E.stats.launches += 1;
         }
         int esc[2 * kBuckets];

@@ -50,6 +50,31 @@ struct Geom
     long long pair_center;   // index of offset (0,0,0) in the pair block
 };
 
+// Order of the solve work lists: tiles of 2^lx x 2^ly x 2^lz cells one after
+// another (cut at the grid's end), x fastest inside a tile and between tiles.
+struct CellTile
+{
+    int lx, ly, lz;
+};
+// the t-th cell in that order
+__host__ __device__ __forceinline__ unsigned tile_cell(const Geom &g, const CellTile &o, unsigned t)
+{
+    const unsigned nx = g.nx, ny = g.ny, plane = nx * ny;
+    const unsigned z0 = t / (plane << o.lz) << o.lz;
+    t -= z0 * plane;
+    const unsigned hz = z0 + (1u << o.lz) <= (unsigned)g.nz ? 1u << o.lz : g.nz - z0;
+    const unsigned strip = nx * hz;
+    const unsigned y0 = t / (strip << o.ly) << o.ly;
+    t -= y0 * strip;
+    const unsigned hy = y0 + (1u << o.ly) <= ny ? 1u << o.ly : ny - y0;
+    const unsigned col = hy * hz;
+    const unsigned x0 = t / (col << o.lx) << o.lx;
+    t -= x0 * col;
+    const unsigned wx = x0 + (1u << o.lx) <= nx ? 1u << o.lx : nx - x0;
+    const unsigned y = t / wx % hy, z = t / wx / hy;
+    return x0 + t % wx + nx * (y0 + y) + plane * (z0 + z);
+}
+
 __host__ __device__ __forceinline__ long long key_index(const Geom &g, int dx, int dy, int dz)
 {
     return ((long long)(dz + g.khz) * g.kny + (dy + g.khy)) * g.knx + (dx + g.khx);

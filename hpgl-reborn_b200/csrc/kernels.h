@@ -101,16 +101,20 @@ cudaError_t launch_resolve_ties_fast(const Geom &g, const int *tie_cells, const 
 
 // solves (solve.cu, misc.cu)
 // Solve-kernel variants (the launch shapes the tuning table chooses between,
-// tune.cpp). n <= 32: kVariantFold (two rows per lane: FP32-refined 512-thread
-// blocks with in-kernel classic refinement, FP64 384-thread blocks),
-// kVariantFoldNarrow (the same with 256-thread blocks and up to 255
-// registers); FP32-refined also kVariantQuad (four rows per lane, 384-thread
-// blocks, solve_quad.cu) and kVariantQuadNarrow (256-thread blocks), and for
-// n 17-32 kVariantTile (four rows per lane reading a union matrix the block
-// shares, solve_tile.cu; 384-thread blocks, one per SM) and kVariantTileNarrow
-// (192-thread blocks, two per SM). n 33-64: kVariantWide (one warp per system,
+// tune.cpp). n <= 32: kVariantFold (FP32-refined: two rows per lane, 512-thread
+// blocks, in-kernel classic refinement; FP64: two rows per lane, 384-thread
+// blocks, up to n 16, and for n 17-32 the sharing solve, solve_share.cu, with
+// solve_mma.cu for what cannot share), kVariantFoldNarrow (two rows per lane,
+// 256-thread blocks and up to 255 registers); FP32-refined also kVariantQuad
+// (four rows per lane, 384-thread blocks, solve_quad.cu) and kVariantQuadNarrow
+// (256-thread blocks), and for n 17-32 kVariantTile (four rows per lane reading
+// a union matrix the block shares, solve_tile.cu; 384-thread blocks, one per
+// SM) and kVariantTileNarrow (192-thread blocks, two per SM). n 33-64:
+// kVariantWide (FP64: the sharing solve; FP32-refined: one warp per system,
 // rows shifted in registers, rolled factorisation phases, solve_wide.cu) and
 // kVariantFold (one warp per system, fully unrolled, 256-thread blocks).
+// kVariantShare: FP32-refined keys of n 17-64 solved by the FP64 sharing solve,
+// which is faster than any FP32 kernel and needs no refinement.
 enum SolveVariant : int
 {
     kVariantDefault = 0,
@@ -121,12 +125,18 @@ enum SolveVariant : int
     kVariantTile = 5,
     kVariantTileNarrow = 6,
     kVariantWide = 7,
+    kVariantShare = 8,
 };
-constexpr int kVariantCount = 8;
+constexpr int kVariantCount = 9;
 // the four-rows-per-lane FP32 kernels queue failing systems for classic refinement
 inline bool is_quad_variant(int v)
 {
     return v == kVariantQuad || v == kVariantQuadNarrow || v == kVariantTile || v == kVariantTileNarrow;
+}
+// whether a bucket's variant shares factorisations between cells (solve_share.cu)
+inline bool is_share_variant(int np, int precision, int v)
+{
+    return precision ? v == kVariantShare : (np == 32 && v == kVariantFold) || (np == 64 && v == kVariantWide);
 }
 // the variant that runs for a (bucket, covariance type, precision) key
 int solve_variant(int np, int cov_type, int precision);
@@ -140,11 +150,15 @@ int set_solve_variant(int np, int cov_type, int precision, int variant);
 constexpr int kTuneMinItems = 20000;
 bool tune_wanted(int np, int cov_type, int precision);
 void tune_record(int np, int cov_type, int precision, const double *ms_per_variant);
+// the tile order of the work lists that the sharing solves want (solve_share.cu)
+CellTile solve_share_tile(const Geom &g);
+// left_cells / left_count (a list of its own, the count zeroed by the caller):
+// needed by the sharing variants, whose `cells` are in solve_share_tile's order
 cudaError_t launch_solve_bucket(int np, int precision, int variant, bool ordinary, const Geom &g, const int2 *cells,
                                 const int *n_items, int max_items, const int2 *nb_rec, const int *nb_n, int ind_value,
                                 const double *pair64, const float *pair32, double mean, double c0, int steps,
-                                double tol, const SolveOut &out, int2 *esc_cells, int *esc_count, int n_sm,
-                                cudaStream_t st);
+                                double tol, const SolveOut &out, int2 *esc_cells, int *esc_count, int2 *left_cells,
+                                int *left_count, int n_sm, cudaStream_t st);
 size_t large_scratch_doubles(int k, int blocks);
 cudaError_t launch_solve_large(const Geom &g, const int2 *cells, const int *n_items, int blocks, const int2 *nb_rec,
                                const int *nb_n, int ind_value, const double *pair64, bool ordinary, double mean,
@@ -156,8 +170,8 @@ void launch_build_pair(const Geom &g, const DevModel &m, int truncated, const do
 // tiles of the stable bucket partition; tile_cnt holds kBuckets ints and tile_mom
 // 3 kBuckets values per tile
 long long prepare_tiles(long long n_cells);
-void launch_prepare(const Geom &g, const uint8_t *mask, int all_cells, const int *nb_n, signed char *status,
-                    int *bucket_cnt, int *bucket_off, int *tile_cnt, unsigned long long *tile_mom, int2 *cells,
+void launch_prepare(const Geom &g, const CellTile &order, const uint8_t *mask, int all_cells, const int *nb_n,
+                    signed char *status, int *bucket_cnt, int *bucket_off, int *tile_cnt, unsigned long long *tile_mom, int2 *cells,
                     unsigned long long *moments, cudaStream_t st);
 void launch_finalize_cont(const Geom &g, const float *in_data, signed char *status, int simple, float mean_f,
                           const float *cell_mean, float *out_data, uint8_t *out_mask, double *est64, double *var,

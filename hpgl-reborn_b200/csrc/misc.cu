@@ -79,9 +79,9 @@ __device__ __forceinline__ int bucket_of(int n)
 // Per-cell status before the solve: -1 informed (continuous kriging only),
 // 1 no neighbours, 3 pending (to be solved).
 // Per-cell status and the solve work lists, as a stable partition by bucket:
-// the list of every bucket holds its cells in ascending cell order, so the
-// solver's blocks, which take contiguous runs of a list, work on neighbouring
-// cells. Three passes over tiles of kTile cells: counts (and the moments of n
+// the list of every bucket holds its cells in the order `order` (tiles of a
+// few cells each), so the solver's blocks, which take contiguous runs of a
+// list, work on neighbouring cells. Three passes over tiles of kTile cells: counts (and the moments of n
 // per bucket, for the flop count), a one-block scan, and the ordered fill.
 constexpr int kTileThreads = 256, kTileIters = 8, kTile = kTileThreads * kTileIters;
 
@@ -97,7 +97,7 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
 // status: -1 informed (not kriged), 1 no neighbours, 3 queued for a solve.
 // tile_cnt[q * T + tile] = cells of bucket q in the tile; tile_mom[(3q + e) * T + tile]
 // = sum of n^(e+1) over them.
-__global__ void __launch_bounds__(kTileThreads) k_prepare(const Geom g, const uint8_t *__restrict__ mask, int all_cells,
+__global__ void __launch_bounds__(kTileThreads) k_prepare(const Geom g, const CellTile order, const uint8_t *__restrict__ mask, int all_cells,
                                                           const int *__restrict__ nb_n, signed char *__restrict__ status,
                                                           int *__restrict__ tile_cnt,
                                                           unsigned long long *__restrict__ tile_mom)
@@ -113,10 +113,11 @@ __global__ void __launch_bounds__(kTileThreads) k_prepare(const Geom g, const ui
     for (int q = 0; q < kBuckets * 3; ++q) mom[q] = 0;
     for (int it = 0; it < kTileIters; ++it)
     {
-        const long long c = base + it * kTileThreads + threadIdx.x;
+        const long long t = base + it * kTileThreads + threadIdx.x;
         int b = -1, n = 0;
-        if (c < g.n_cells)
+        if (t < g.n_cells)
         {
+            const unsigned c = tile_cell(g, order, (unsigned)t);
             if (!all_cells && mask[c])
                 status[c] = -1;
             else
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(1024) k_prepare_scan(int T, int *__restrict__ 
     }
 }
 
-__global__ void __launch_bounds__(kTileThreads) k_bucket_fill(const Geom g, const signed char *__restrict__ status,
+__global__ void __launch_bounds__(kTileThreads) k_bucket_fill(const Geom g, const CellTile order, const signed char *__restrict__ status,
                                                               const int *__restrict__ nb_n,
                                                               const int *__restrict__ tile_off,
                                                               const int *__restrict__ bucket_off,
@@ -253,9 +254,10 @@ __global__ void __launch_bounds__(kTileThreads) k_bucket_fill(const Geom g, cons
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
     for (int it = 0; it < kTileIters; ++it)
     {
-        const long long c = base + it * kTileThreads + threadIdx.x;
+        const long long t = base + it * kTileThreads + threadIdx.x;
+        const unsigned c = t < g.n_cells ? tile_cell(g, order, (unsigned)t) : 0u;
         int b = -1, n = 0;
-        if (c < g.n_cells && status[c] == 3)
+        if (t < g.n_cells && status[c] == 3)
         {
             n = nb_n[c];
             b = bucket_of(n);
@@ -286,14 +288,14 @@ __global__ void __launch_bounds__(kTileThreads) k_bucket_fill(const Geom g, cons
     }
 }
 
-void launch_prepare(const Geom &g, const uint8_t *mask, int all_cells, const int *nb_n, signed char *status,
-                    int *bucket_cnt, int *bucket_off, int *tile_cnt, unsigned long long *tile_mom, int2 *cells,
+void launch_prepare(const Geom &g, const CellTile &order, const uint8_t *mask, int all_cells, const int *nb_n,
+                    signed char *status, int *bucket_cnt, int *bucket_off, int *tile_cnt, unsigned long long *tile_mom, int2 *cells,
                     unsigned long long *moments, cudaStream_t st)
 {
     const int T = (int)prepare_tiles(g.n_cells);
-    k_prepare<<<T, kTileThreads, 0, st>>>(g, mask, all_cells, nb_n, status, tile_cnt, tile_mom);
+    k_prepare<<<T, kTileThreads, 0, st>>>(g, order, mask, all_cells, nb_n, status, tile_cnt, tile_mom);
     k_prepare_scan<<<1, 1024, 0, st>>>(T, tile_cnt, tile_mom, bucket_cnt, bucket_off, moments);
-    k_bucket_fill<<<T, kTileThreads, 0, st>>>(g, status, nb_n, tile_cnt, bucket_off, cells);
+    k_bucket_fill<<<T, kTileThreads, 0, st>>>(g, order, status, nb_n, tile_cnt, bucket_off, cells);
 }
 
 // ------------------------------------------------------------- finalize

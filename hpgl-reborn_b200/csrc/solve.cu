@@ -1040,8 +1040,11 @@ static cudaError_t launch_np(int precision, int variant, bool ordinary, const Ge
             if (variant == kVariantFoldNarrow)
                 return ordinary ? launch_one<NP, double, true, false, 256>(HB_ARGS)
                                 : launch_one<NP, double, false, false, 256>(HB_ARGS);
-            return ordinary ? launch_one<NP, double, true, false, 384>(HB_ARGS)
-                            : launch_one<NP, double, false, false, 384>(HB_ARGS);
+            if constexpr (NP == 32)
+                return launch_solve_mma(NP, ordinary, g, cells, n_items, max_items, nb_rec, ind_value, P, n_sm, st);
+            else
+                return ordinary ? launch_one<NP, double, true, false, 384>(HB_ARGS)
+                                : launch_one<NP, double, false, false, 384>(HB_ARGS);
         }
         if constexpr (NP == 32)
         {
@@ -1058,7 +1061,10 @@ static cudaError_t launch_np(int precision, int variant, bool ordinary, const Ge
     }
     else
     {
-        if (variant != kVariantFold) return launch_solve_wide(precision, ordinary, HB_ARGS);
+        if (variant != kVariantFold)
+            return precision ? launch_solve_wide(ordinary, HB_ARGS)
+                             : launch_solve_mma(NP, ordinary, g, cells, n_items, max_items, nb_rec, ind_value, P, n_sm,
+                                                st);
         if (precision == 0)
             return ordinary ? launch_one<NP, double, true, false, 256>(HB_ARGS)
                             : launch_one<NP, double, false, false, 256>(HB_ARGS);
@@ -1071,6 +1077,7 @@ static cudaError_t launch_np(int precision, int variant, bool ordinary, const Ge
 bool solve_variant_valid(int np, int precision, int variant)
 {
     if (variant == kVariantDefault) return true;
+    if (variant == kVariantShare) return precision == 1 && np >= 32;
     if (np > 32) return variant == kVariantFold || variant == kVariantWide;
     if (precision == 1)
         return (variant >= kVariantFold && variant <= kVariantQuadNarrow) ||
@@ -1081,8 +1088,8 @@ bool solve_variant_valid(int np, int precision, int variant)
 cudaError_t launch_solve_bucket(int np, int precision, int variant, bool ordinary, const Geom &g, const int2 *cells,
                                 const int *n_items, int max_items, const int2 *nb_rec, const int *nb_n, int ind_value,
                                 const double *pair64, const float *pair32, double mean, double c0, int steps,
-                                double tol, const SolveOut &out, int2 *esc_cells, int *esc_count, int n_sm,
-                                cudaStream_t st)
+                                double tol, const SolveOut &out, int2 *esc_cells, int *esc_count, int2 *left_cells,
+                                int *left_count, int n_sm, cudaStream_t st)
 {
     (void)nb_n;
     SolveParams P;
@@ -1095,6 +1102,15 @@ cudaError_t launch_solve_bucket(int np, int precision, int variant, bool ordinar
     P.out = out;
     P.esc_cells = esc_cells;
     P.esc_count = esc_count;
+    if (left_cells && is_share_variant(np, precision, variant))
+    {
+        const cudaError_t e = launch_solve_share(np, ordinary, g, cells, n_items, max_items, nb_rec, ind_value, P,
+                                                 solve_share_tile(g), left_cells, left_count, n_sm, st);
+        if (e != cudaSuccess) return e;
+        return launch_solve_mma(np, ordinary, g, left_cells, left_count, max_items, nb_rec, ind_value, P, n_sm, st);
+    }
+    if (variant == kVariantShare)
+        return launch_solve_mma(np, ordinary, g, cells, n_items, max_items, nb_rec, ind_value, P, n_sm, st);
 #define HB_NARGS precision, variant, ordinary, g, cells, n_items, max_items, nb_rec, ind_value, pair32, P, n_sm, st
     switch (np)
     {

@@ -94,13 +94,22 @@ namespace hb
 cudaError_t launch_solve_tile(int np, bool ordinary, int threads, const Geom &g, const int2 *cells, const int *n_items,
                               int max_items, const int2 *nb_rec, int ind_value, const float *pair32,
                               const SolveParams &P, int n_sm, cudaStream_t st);
-// FP32-refined (precision 1) and FP64-plain solves of 33 to 64 neighbours,
-// one warp per system (solve_wide.cu)
-cudaError_t launch_solve_wide(int precision, bool ordinary, const Geom &g, const int2 *cells, const int *n_items,
+// FP32-refined solves of 33 to 64 neighbours, one warp per system (solve_wide.cu)
+cudaError_t launch_solve_wide(bool ordinary, const Geom &g, const int2 *cells, const int *n_items,
                               int max_items, const int2 *nb_rec, int ind_value, const float *pair32,
                               const SolveParams &P, int n_sm, cudaStream_t st);
 // (threads per block: 384 or 256)
 cudaError_t launch_solve_quad(int np, bool ordinary, int threads, const Geom &g, const int2 *cells,
                               const int *n_items, int max_items, const int2 *nb_rec, int ind_value,
                               const float *pair32, const SolveParams &P, int n_sm, cudaStream_t st);
+// FP64 solves of 17 to 64 neighbours on the FP64 tensor instruction, one
+// system per warp (solve_mma.cu)
+cudaError_t launch_solve_mma(int np, bool ordinary, const Geom &g, const int2 *cells, const int *n_items,
+                             int max_items, const int2 *nb_rec, int ind_value, const SolveParams &P, int n_sm,
+                             cudaStream_t st);
+// the same, one factorisation shared by neighbouring cells (solve_share.cu);
+// cells that cannot share are queued in left_cells for launch_solve_mma
+cudaError_t launch_solve_share(int np, bool ordinary, const Geom &g, const int2 *cells, const int *n_items,
+                               int max_items, const int2 *nb_rec, int ind_value, const SolveParams &P,
+                               const CellTile &tile, int2 *left_cells, int *left_count, int n_sm, cudaStream_t st);
 } // namespace hb

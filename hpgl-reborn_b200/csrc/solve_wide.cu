@@ -19,13 +19,11 @@
 // the instruction caches, and its warps waited on instruction fetch ten times
 // as long as on anything else.
 //
-// k_solve_wide64: FP64 plain, forward substitution only (the forms are
-// (L^-1 u) . (L^-1 w)). k_solve_wide32: FP32 factorisation (two steps a body
-// as a rank-2 update, the rows as float2 pairs shifted by two, so that the
-// update runs as packed FP32x2 FMAs) and substitutions,
-// the bilinear forms corrected with the FP64 dual-weighted residual from the
-// lower triangle (as the other FP32-refined kernels do); a system whose check
-// fails is queued for the FP64 kernel.
+// k_solve_wide32: FP32 factorisation (two steps a body as a rank-2 update, the
+// rows as float2 pairs shifted by two, so that the update runs as packed
+// FP32x2 FMAs) and substitutions, the bilinear forms corrected with the FP64
+// dual-weighted residual from the lower triangle (as the other FP32-refined
+// kernels do); a system whose check fails is queued for the FP64 kernel.
 #include "engine.cuh"
 #include "kernels.h"
 #include "solve_common.cuh"
@@ -40,10 +38,10 @@ constexpr int kWidePhase = 8; // factorisation steps per rolled phase
 
 // Broadcast buffer: 63 column entries, the diagonal at [63], R right-hand
 // sides from [64]; padded to 16 bytes.
-template <typename T, int R>
+template <int R>
 __host__ __device__ constexpr int wide_ldw()
 {
-    return ((kWideNP + R) * (int)sizeof(T) + 15) / 16 * 16 / (int)sizeof(T);
+    return ((kWideNP + R) * (int)sizeof(float) + 15) / 16 * 16 / (int)sizeof(float);
 }
 
 // Start of column j in the packed column-major lower triangle
@@ -52,148 +50,21 @@ __host__ __device__ constexpr int wide_col(int j)
     return kWideNP * j - j * (j - 1) / 2;
 }
 
-template <typename T, int R, bool BACK>
+template <int R>
 struct WideSmem
 {
-    static constexpr int LDW = wide_ldw<T, R>();
-    // two broadcast buffers in turn; FP32 (BACK) broadcasts two columns a body
-    static constexpr size_t w_bytes = (size_t)(BACK ? 4 : 2) * LDW * sizeof(T);
+    static constexpr int LDW = wide_ldw<R>();
+    // two broadcast buffers in turn, two columns a body
+    static constexpr size_t w_bytes = (size_t)4 * LDW * sizeof(float);
     static constexpr size_t lin_off = w_bytes;
-    // (FP32) the factor's columns before scaling, for the back substitution
+    // the factor's columns before scaling, for the back substitution
     static constexpr size_t lc_off = lin_off + kWideNP * sizeof(int);
-    static constexpr size_t lc_bytes = BACK ? (size_t)kWideNP * (kWideNP + 1) / 2 * sizeof(float) : 0;
-    // (FP32) the R solution vectors in double, for the correction's row sums
+    static constexpr size_t lc_bytes = (size_t)kWideNP * (kWideNP + 1) / 2 * sizeof(float);
+    // the R solution vectors in double, for the correction's row sums
     static constexpr size_t x_off = (lc_off + lc_bytes + 15) / 16 * 16;
-    static constexpr size_t raw = x_off + (BACK ? (size_t)R * kWideNP * sizeof(double) : 0);
+    static constexpr size_t raw = x_off + (size_t)R * kWideNP * sizeof(double);
     static constexpr size_t bytes = (raw + 15) / 16 * 16;
 };
-
-__device__ __forceinline__ float wide_rsqrt(float d) { return rsqrtf(d); }
-__device__ __forceinline__ double wide_rsqrt(double d) { return rsqrt(d); }
-
-// One shift-update of the lane's rows by column j (entries in W):
-// r[k] = r[k + 1] - s W[k] for k < L - 1 (L <= N), read 16 bytes at a time.
-template <int L, typename T, int N>
-__device__ __forceinline__ void wide_shift(T (&r)[N], T s, const T *W)
-{
-    if constexpr (L > 1)
-    {
-        constexpr int V = 16 / (int)sizeof(T);
-        static_for<0, (L - 1 + V - 1) / V>([&](auto CC) {
-            constexpr int c = decltype(CC)::value;
-            T w[V];
-            if constexpr (V == 4)
-            {
-                const float4 v = reinterpret_cast<const float4 *>(W)[c];
-                w[0] = v.x;
-                w[1] = v.y;
-                w[2] = v.z;
-                w[3] = v.w;
-            }
-            else
-            {
-                const double2 v = reinterpret_cast<const double2 *>(W)[c];
-                w[0] = v.x;
-                w[1] = v.y;
-            }
-#pragma unroll
-            for (int e = 0; e < V; ++e)
-            {
-                const int k = V * c + e;
-                if (k < L - 1) r[k] = r[k + 1] - s * w[e];
-            }
-        });
-    }
-}
-
-// Right-looking Cholesky of the warp's system with the forward substitution
-// of R right-hand sides riding in the broadcast rows. On return ya / yb hold
-// the forward solutions of rows a and b, inv_a / inv_b their 1 / L(r, r);
-// with KEEP the factor's columns before scaling are left in LC
-// (LC[wide_col(j) + r - j] = L(r, j) sqrt(A(j, j)) for r >= j).
-template <typename T, int R, bool KEEP>
-__device__ __forceinline__ bool wide_factor(T (&ra)[32], T (&rbv)[kWideNP], T (&rhs_a)[R], T (&rhs_b)[R],
-                                            T (&ya)[R], T (&yb)[R], T &inv_a, T &inv_b, int t, T *Wbuf, float *LC)
-{
-    constexpr int NP = kWideNP;
-    constexpr int LDW = wide_ldw<T, R>();
-    const int b = NP - 1 - t;
-    bool fail = false;
-    static_for<0, NP / kWidePhase>([&](auto PC) {
-        constexpr int p = decltype(PC)::value;
-        constexpr int LA = 32 - kWidePhase * p > 0 ? 32 - kWidePhase * p : 0;
-        constexpr int LB = NP - kWidePhase * p;
-#pragma unroll 1
-        for (int jj = 0; jj < kWidePhase; ++jj)
-        {
-            const int j = kWidePhase * p + jj;
-            T *W = Wbuf + (j & 1) * LDW;
-            if constexpr (LA > 0)
-            {
-                if (t > j) W[t - j - 1] = ra[0];
-                if (t == j)
-                {
-                    W[NP - 1] = ra[0];
-#pragma unroll
-                    for (int q = 0; q < R; ++q) W[NP + q] = rhs_a[q];
-                }
-                if constexpr (KEEP)
-                {
-                    if (t >= j) LC[wide_col(j) + t - j] = (float)ra[0];
-                }
-            }
-            if (b > j) W[b - j - 1] = rbv[0];
-            if (b == j)
-            {
-                W[NP - 1] = rbv[0];
-#pragma unroll
-                for (int q = 0; q < R; ++q) W[NP + q] = rhs_b[q];
-            }
-            if constexpr (KEEP)
-            {
-                if (b >= j) LC[wide_col(j) + b - j] = (float)rbv[0];
-            }
-            __syncwarp();
-            const T d = W[NP - 1];
-            fail |= !(d > T(0));
-            const T inv_s = wide_rsqrt(d);
-            const T inv2 = inv_s * inv_s;
-            const T s_b = rbv[0] * inv2;
-            T wr[R];
-#pragma unroll
-            for (int q = 0; q < R; ++q) wr[q] = W[NP + q];
-            if constexpr (LA > 0)
-            {
-                const T s_a = ra[0] * inv2;
-                wide_shift<LA>(ra, s_a, W);
-                if (t > j)
-                {
-#pragma unroll
-                    for (int q = 0; q < R; ++q) rhs_a[q] -= s_a * wr[q];
-                }
-                if (t == j)
-                {
-                    inv_a = inv_s;
-#pragma unroll
-                    for (int q = 0; q < R; ++q) ya[q] = rhs_a[q] * inv_s;
-                }
-            }
-            wide_shift<LB>(rbv, s_b, W);
-            if (b > j)
-            {
-#pragma unroll
-                for (int q = 0; q < R; ++q) rhs_b[q] -= s_b * wr[q];
-            }
-            if (b == j)
-            {
-                inv_b = inv_s;
-#pragma unroll
-                for (int q = 0; q < R; ++q) yb[q] = rhs_b[q] * inv_s;
-            }
-        }
-    });
-    return fail;
-}
 
 // FP32: r[m] = r[m + 1] - s0 (V[2m + 2], V[2m + 3]) - s1 (U[2m + 2], U[2m + 3])
 // for pairs m < L - 1 (L <= N): two steps' updates of the lane's row, shifted
@@ -240,7 +111,7 @@ __device__ __forceinline__ bool wide_factor2(float2 (&ra)[16], float2 (&rb)[32],
                                              float &inv_b, int t, float *Wbuf, float *LC)
 {
     constexpr int NP = kWideNP;
-    constexpr int LDW = wide_ldw<float, R>();
+    constexpr int LDW = wide_ldw<R>();
     const int b = NP - 1 - t;
     bool fail = false;
     static_for<0, NP / PH>([&](auto PC) {
@@ -409,95 +280,6 @@ struct WideItems
     }
 };
 
-// FP64 plain, forward substitution only.
-template <bool ORDINARY, int TH>
-__global__ void __launch_bounds__(TH, 1)
-    k_solve_wide64(const Geom g, const int2 *__restrict__ cells, const int *__restrict__ n_items_ptr,
-                   const int2 *__restrict__ nb_rec, int ind_value, SolveParams P)
-{
-    constexpr int NP = kWideNP;
-    constexpr int QB = ORDINARY ? 2 : 1;
-    constexpr int R = QB + 1;
-    constexpr int V = R - 1;
-    typedef WideSmem<double, R, false> SM;
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int t = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int b = NP - 1 - t;
-    unsigned char *gb = smem + SM::bytes * warp;
-    double *Wbuf = reinterpret_cast<double *>(gb);
-    int *LIN = reinterpret_cast<int *>(gb + SM::lin_off);
-    const double *p64c = P.pair64 + P.pc;
-
-    const int n_items = *n_items_ptr;
-    const int per_block = (n_items + gridDim.x - 1) / gridDim.x;
-    WideItems it;
-    it.item = blockIdx.x * per_block + warp;
-    it.end = min(n_items, blockIdx.x * per_block + per_block);
-    it.stride = TH / 32;
-    it.load(g, cells, nb_rec, t);
-    while (it.item < it.end)
-    {
-        const int my_cell = it.w.x, my_n = it.w.y;
-        const bool live_a = t < my_n, live_b = b < my_n;
-        const int lin_a = it.rec_a.x, lin_b = it.rec_b.x;
-        const double vc_a = centred_value(live_a, __int_as_float(it.rec_a.y), ind_value, P.mf);
-        const double vc_b = centred_value(live_b, __int_as_float(it.rec_b.y), ind_value, P.mf);
-        it.item += it.stride;
-        it.load(g, cells, nb_rec, t);
-        LIN[t] = live_a ? lin_a : 0;
-        LIN[b] = live_b ? lin_b : 0;
-        __syncwarp();
-
-        // ---- assembly (lower triangles of rows a and b; padding rows identity)
-        double ra[32], rbv[NP];
-        const double *base_a = p64c + lin_a, *base_b = p64c + lin_b;
-#pragma unroll
-        for (int c = 0; c < 32; ++c)
-        {
-            double a = 0.0;
-            if (live_a && c <= t) a = __ldg(base_a - LIN[c]);
-            if (!live_a && c == t) a = 1.0;
-            ra[c] = a;
-        }
-#pragma unroll
-        for (int c = 0; c < NP; ++c)
-        {
-            double a = 0.0;
-            if (live_b && c <= b) a = __ldg(base_b - LIN[c]);
-            if (!live_b && c == b) a = 1.0;
-            rbv[c] = a;
-        }
-        double rhs_a[R], rhs_b[R], ya[R], yb[R];
-        rhs_a[0] = live_a ? __ldg(base_a) : 0.0;
-        rhs_b[0] = live_b ? __ldg(base_b) : 0.0;
-        if constexpr (ORDINARY)
-        {
-            rhs_a[1] = live_a ? 1.0 : 0.0;
-            rhs_b[1] = live_b ? 1.0 : 0.0;
-        }
-        rhs_a[V] = vc_a;
-        rhs_b[V] = vc_b;
-#pragma unroll
-        for (int q = 0; q < R; ++q) ya[q] = yb[q] = 0.0;
-        double inv_a = 0.0, inv_b = 0.0;
-        const bool fail = wide_factor<double, R, false>(ra, rbv, rhs_a, rhs_b, ya, yb, inv_a, inv_b, t, Wbuf,
-                                                         nullptr);
-
-        // ---- forms (L^-1 u) . (L^-1 w); q: 0 = b, 1 = ones (OK), V = v - mean
-        const double s_vb = wide_sum(ya[V] * ya[0] + yb[V] * yb[0]);
-        const double s_bb = wide_sum(ya[0] * ya[0] + yb[0] * yb[0]);
-        double s_1b = 0.0, s_v1 = 0.0, s_11 = 0.0;
-        if constexpr (ORDINARY)
-        {
-            s_1b = wide_sum(ya[1] * ya[0] + yb[1] * yb[0]);
-            s_v1 = wide_sum(ya[V] * ya[1] + yb[V] * yb[1]);
-            s_11 = wide_sum(ya[1] * ya[1] + yb[1] * yb[1]);
-        }
-        if (t == 0) write_solution<ORDINARY>(P, my_cell, fail, s_vb, s_bb, s_1b, s_v1, s_11);
-        __syncwarp();
-    }
-}
-
 // FP32 factorisation and substitutions, bilinear forms corrected in FP64.
 template <bool ORDINARY, int TH>
 __global__ void __launch_bounds__(TH, 1)
@@ -508,7 +290,7 @@ __global__ void __launch_bounds__(TH, 1)
     constexpr int QB = ORDINARY ? 2 : 1;
     constexpr int R = QB + 1;
     constexpr int V = R - 1;
-    typedef WideSmem<float, R, true> SM;
+    typedef WideSmem<R> SM;
     extern __shared__ __align__(16) unsigned char smem[];
     const int t = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int b = NP - 1 - t;
@@ -720,43 +502,30 @@ __global__ void __launch_bounds__(TH, 1)
     }
 }
 
-// Threads per block: 256 (up to 255 registers; the FP64 rows take 192). FP32
-// in 384-thread blocks (168 registers) spilled in the factorisation's body and
-// ran 6 % slower (213 against 200 ms on the clustered 512x512x64 grid).
-template <bool ORD, bool F64>
+// Threads per block: 256 (up to 255 registers). 384-thread blocks (168
+// registers) spilled in the factorisation's body and ran 6 % slower (213
+// against 200 ms on the clustered 512x512x64 grid).
+template <bool ORD>
 static cudaError_t launch_wide_one(const Geom &g, const int2 *cells, const int *n_items, int max_items,
                                    const int2 *nb_rec, int ind_value, const float *pair32, const SolveParams &P,
                                    int n_sm, cudaStream_t st)
 {
-    constexpr int R = ORD ? 3 : 2;
     constexpr int TH = 256;
-    const size_t smem = (F64 ? WideSmem<double, R, false>::bytes : WideSmem<float, R, true>::bytes) * (TH / 32);
+    const size_t smem = WideSmem<ORD ? 3 : 2>::bytes * (TH / 32);
     int blocks = 0;
-    if constexpr (F64)
-    {
-        auto kern = k_solve_wide64<ORD, TH>;
-        cudaError_t e = launch_kernel(kern, TH, smem, max_items, TH / 32, n_sm, blocks);
-        if (e != cudaSuccess) return e;
-        kern<<<(unsigned)blocks, TH, smem, st>>>(g, cells, n_items, nb_rec, ind_value, P);
-    }
-    else
-    {
-        auto kern = k_solve_wide32<ORD, TH>;
-        cudaError_t e = launch_kernel(kern, TH, smem, max_items, TH / 32, n_sm, blocks);
-        if (e != cudaSuccess) return e;
-        kern<<<(unsigned)blocks, TH, smem, st>>>(g, cells, n_items, nb_rec, ind_value, pair32, P);
-    }
+    auto kern = k_solve_wide32<ORD, TH>;
+    cudaError_t e = launch_kernel(kern, TH, smem, max_items, TH / 32, n_sm, blocks);
+    if (e != cudaSuccess) return e;
+    kern<<<(unsigned)blocks, TH, smem, st>>>(g, cells, n_items, nb_rec, ind_value, pair32, P);
     return cudaGetLastError();
 }
 
-cudaError_t launch_solve_wide(int precision, bool ordinary, const Geom &g, const int2 *cells, const int *n_items,
-                              int max_items, const int2 *nb_rec, int ind_value, const float *pair32,
-                              const SolveParams &P, int n_sm, cudaStream_t st)
+cudaError_t launch_solve_wide(bool ordinary, const Geom &g, const int2 *cells, const int *n_items, int max_items,
+                              const int2 *nb_rec, int ind_value, const float *pair32, const SolveParams &P, int n_sm,
+                              cudaStream_t st)
 {
 #define HB_ARGS g, cells, n_items, max_items, nb_rec, ind_value, pair32, P, n_sm, st
-    if (precision == 0)
-        return ordinary ? launch_wide_one<true, true>(HB_ARGS) : launch_wide_one<false, true>(HB_ARGS);
-    return ordinary ? launch_wide_one<true, false>(HB_ARGS) : launch_wide_one<false, false>(HB_ARGS);
+    return ordinary ? launch_wide_one<true>(HB_ARGS) : launch_wide_one<false>(HB_ARGS);
 #undef HB_ARGS
 }
 } // namespace hb

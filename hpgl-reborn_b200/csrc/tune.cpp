@@ -61,7 +61,7 @@ bool key_ok(int b, int cov_type, int precision)
 }
 
 const char *kVariantNames[kVariantCount] = {"default", "fold", "quad", "fold_narrow", "quad_narrow", "tile",
-                                            "tile_narrow", "wide"};
+                                            "tile_narrow", "wide", "share"};
 } // namespace
 
 int solve_variant(int np, int cov_type, int precision)

@@ -320,11 +320,12 @@ int hpgl_b200_last_stats(double *out, int cap);
  * HPGL_B200_FP64_PLAIN or HPGL_B200_FP32_REFINED. Variants:
  *   HPGL_B200_VARIANT_DEFAULT      the built-in pick of the key
  *   HPGL_B200_VARIANT_FOLD         two rows per lane (FP32: 512-thread blocks,
- *                                  classic refinement in the kernel; FP64:
- *                                  384-thread blocks; bucket 64: one warp per
- *                                  system, 256-thread blocks)
- *   HPGL_B200_VARIANT_FOLD_NARROW  bucket_np <= 32: FOLD in 256-thread blocks
- *                                  (up to 255 registers a thread)
+ *                                  classic refinement in the kernel; FP64,
+ *                                  buckets 8 and 16: 384-thread blocks; bucket
+ *                                  64: one warp per system, 256-thread blocks);
+ *                                  FP64, bucket 32: the sharing solve (SHARE)
+ *   HPGL_B200_VARIANT_FOLD_NARROW  bucket_np <= 32: two rows per lane, 256-thread
+ *                                  blocks (up to 255 registers a thread)
  *   HPGL_B200_VARIANT_QUAD         FP32_REFINED, bucket_np <= 32: four rows
  *                                  per lane, 384-thread blocks; failing systems
  *                                  go on to FOLD's refinement, then to FP64
@@ -335,11 +336,16 @@ int hpgl_b200_last_stats(double *out, int cap);
  *                                  consecutive cells it solves at once
  *   HPGL_B200_VARIANT_TILE_NARROW  TILE in 192-thread blocks, two a
  *                                  multiprocessor, 24 cells at once
- *   HPGL_B200_VARIANT_WIDE         bucket_np == 64 (the built-in pick): one
- *                                  warp per system, the factorisation's steps
- *                                  rolled in phases of eight over rows kept
- *                                  shifted in registers (FOLD is the same
- *                                  layout fully unrolled)
+ *   HPGL_B200_VARIANT_WIDE         bucket_np == 64 (the built-in pick): FP64 the
+ *                                  sharing solve (SHARE); FP32 one warp per
+ *                                  system, the factorisation's steps rolled in
+ *                                  phases of eight over rows kept shifted in
+ *                                  registers
+ *   HPGL_B200_VARIANT_SHARE        FP32_REFINED, bucket_np >= 32: solved in FP64
+ *                                  instead, neighbouring cells sharing the
+ *                                  factorisation of their common neighbours'
+ *                                  block on the FP64 tensor instruction (faster
+ *                                  than any of the FP32 variants)
  * hpgl_b200_solve_variant sets a key and returns its previous setting, or
  * HPGL_B200_EINVAL for an invalid key or a variant the key cannot run;
  * hpgl_b200_solve_variant_get returns the variant a key runs now. Results of
@@ -352,6 +358,7 @@ int hpgl_b200_last_stats(double *out, int cap);
 #define HPGL_B200_VARIANT_TILE 5
 #define HPGL_B200_VARIANT_TILE_NARROW 6
 #define HPGL_B200_VARIANT_WIDE 7
+#define HPGL_B200_VARIANT_SHARE 8
 int hpgl_b200_solve_variant(int bucket_np, int cov_type, int precision, int variant);
 int hpgl_b200_solve_variant_get(int bucket_np, int cov_type, int precision);
 /* The tuner behind those keys (no counterpart in the reference).
