@@ -402,11 +402,14 @@ struct DevSearch
     int template_cells = 0;
 };
 
+// sqrt(h2), rounded up past its own error
+static double root_up(double h2) { return std::sqrt(h2) * (1.0 + 1e-15); }
+
 // Search for one flavour; `all_cells` selects every cell (IK) or only the
 // uninformed ones. Table slots are suffixed with `tag` so several flavours can
 // coexist (IK categories run one after another and reuse them).
 static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const uint8_t *d_mask, int all_cells,
-                            cudaStream_t st, bool want_pids = false, bool exact_search = false)
+                            cudaStream_t st, bool want_pids = false, bool exact_search = false, bool ordered = false)
 {
     const Geom &g = pl.g;
     DevSearch S;
@@ -443,15 +446,16 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
     SurrDev sd = {};
     if (use_sd)
     {
-        std::memcpy(stg + off_h2, pl.sg.h2_rank.data(), nh * 8);
-        double *h2r = E.buf<double>("h2_rank", nh);
-        HB_CK(cudaMemcpyAsync(h2r, stg + off_h2, nh * 8, cudaMemcpyHostToDevice, st));
+        double *roots = reinterpret_cast<double *>(stg + off_h2);
+        for (size_t i = 0; i < nh; ++i) roots[i] = root_up(pl.sg.h2_rank[i]);
+        double *h_rank = E.buf<double>("h_rank", nh);
+        HB_CK(cudaMemcpyAsync(h_rank, roots, nh * 8, cudaMemcpyHostToDevice, st));
         sd.on = 1;
         for (int i = 0; i < 9; ++i) sd.T[i] = pl.sg.T[i];
         for (int a = 0; a < 3; ++a) sd.step[a] = pl.sg.step[a];
         sd.e3 = pl.sg.e3;
-        sd.h2_cut = pl.sg.h2_cut;
-        sd.h2_rank = h2r;
+        sd.h_cut = root_up(pl.sg.h2_cut);
+        sd.h_rank = h_rank;
     }
     long long pn = (long long)g.pnx * g.pny * (2 * g.phz + 1);
     S.pair64 = E.buf<double>("pair64", (size_t)pn);
@@ -466,26 +470,32 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
     S.bin_flag = E.buf<uint8_t>("bin_flag", g.n_bins);
     int *bin_pts = E.buf<int>("bin_pts", std::max(P.m, 1));
     int *tmpl_bins = E.buf<int>("tmpl_bins", g.n_bins);
-    // 0 total, 1 max_cand, 2 tmpl bins, 3 ties, 4 tmpl cells, 5 exact cells, 6 max_cand of the template bins
-    int *scal = E.buf<int>("scalars", 8);
+    // 0 total, 1 max_cand, 2 tmpl bins, 3 ties, 4 tmpl cells, 5 exact cells, 6 max_cand of the template
+    // bins, 7 the largest bin above kBinSortMax, 8 ties of template-path cells selected by rank
+    constexpr int kScalars = 9;
+    int *scal = E.buf<int>("scalars", kScalars);
     int *tmp = E.buf<int>("scan_tmp2", (size_t)scan_tmp_ints(g.n_bins) + 4);
     HB_CK(cudaMemsetAsync(bin_cnt, 0, sizeof(int) * g.n_bins, st));
     HB_CK(cudaMemsetAsync(bin_fill, 0, sizeof(int) * g.n_bins, st));
-    HB_CK(cudaMemsetAsync(scal, 0, sizeof(int) * 8, st));
+    HB_CK(cudaMemsetAsync(scal, 0, sizeof(int) * kScalars, st));
     launch_bin_count(P.pts_xyz, P.n_pts, g, bin_cnt, st);
     HB_CK(cudaMemcpyAsync(bin_start, bin_cnt, sizeof(int) * g.n_bins, cudaMemcpyDeviceToDevice, st));
     exclusive_scan(bin_start, g.n_bins, tmp, scal + 0, st);
-    launch_bin_fill(P.pts_xyz, P.n_pts, g, bin_start, bin_fill, bin_pts, st);
-    launch_bin_sort(g, bin_start, bin_cnt, bin_pts, S.bin_flag, st);
-    launch_bin_region(g, S.bin_flag, bin_cnt, scal + 1, scal + 2, tmpl_bins, scal + 6, st);
+    int *bin_tmp = E.buf<int>("bin_tmp", std::max(P.m, 1));
+    launch_bin_fill(P.pts_xyz, P.n_pts, g, bin_start, bin_fill, bin_tmp, st);
+    launch_bin_sort(g, bin_start, bin_cnt, bin_tmp, bin_pts, S.bin_flag, st);
+    launch_bin_region(g, S.bin_flag, bin_cnt, scal + 1, scal + 2, tmpl_bins, scal + 6, scal + 7, st);
     HB_CK(cudaGetLastError());
-    int host_scal[8];
+    int host_scal[kScalars];
     HB_CK(cudaMemcpyAsync(host_scal, scal, sizeof(host_scal), cudaMemcpyDeviceToHost, st));
     HB_CK(cudaStreamSynchronize(st));
     E.mark(STAGE_BINS, st);
     int max_cand = host_scal[1];
     const int n_tmpl_bins = host_scal[2];
     const int max_cand_tmpl = host_scal[6];
+    // neighbours in candidate order serve where only the set matters, and where that
+    // order is the points' own (a bin left unsorted has none that repeats)
+    ordered = ordered || want_pids || host_scal[7] > 0;
     // Template-path bins (sugarbox_neighbour_lookup.h:171-197: the first k informed
     // cells of the sorted template, in its order) as a selection: the informed
     // cells of the 27 bins around a cell keyed by their offset's position in the
@@ -493,51 +503,80 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
     // search; the template scan over the informed-cell bitmap beyond its limits.
     int n_tmpl = 0;
     int4 *tmpl = E.buf<int4>("tmpl", std::max<long>(pl.tmpl_count, 1));
-    bool tmpl_select = false;
+    bool tmpl_select = false, tmpl_tile = false, tmpl_scan = false, rank_keys = false;
+    // one cell a lane where the order of the neighbours is free
+    const int tile_limit = search_tile_limit(g.k, E.max_smem() - 1024);
     uint16_t *keypos16 = nullptr;
     SurrDev sdp = {};
     int cand_cap_t = 0, warps_t = 8;
     if (n_tmpl_bins > 0 && pl.tmpl_count > 0)
     {
         const std::vector<Offset> tv = build_template(pl.f, pl.kt);
-        if (g.k <= 64 && tv.size() <= 0xFFFE)
+        std::vector<uint16_t> kp;
+        Surrogate sgp;
+        // Templates past the 16-bit positions: by covariance rank inside the radius box,
+        // and the cells whose k-th slot a tie straddles by the template scan (on the
+        // clustered 512x512x64 grid, 111,537 offsets: 49 ms for every template-path
+        // cell's scan)
+        rank_keys = tv.size() > 0xFFFE && use_sd && !ordered && tile_limit > 0;
+        if (rank_keys)
         {
+            tmpl_tile = true;
             cand_cap_t = std::max(4, (max_cand_tmpl + 3) / 4 * 4);
-            while (warps_t > 1 && search_fast_smem_bytes(cand_cap_t, g.k, warps_t) > (size_t)E.max_smem()) --warps_t;
-            tmpl_select = cand_cap_t <= 65536 && search_fast_smem_bytes(cand_cap_t, g.k, warps_t) <= (size_t)E.max_smem();
         }
-        if (tmpl_select)
+        else if (g.k <= 64 && tv.size() <= 0xFFFE)
         {
-            std::vector<uint16_t> kp(nk, (uint16_t)0xFFFF);
-            for (size_t i = 0; i < tv.size(); ++i) kp[key_index(g, tv[i].dx, tv[i].dy, tv[i].dz)] = (uint16_t)i;
+            build_surrogate_template(pl.f, tv, sgp);
+            sdp.on = sgp.ok && !exact_search ? 1 : 0;
+            cand_cap_t = std::max(4, (max_cand_tmpl + 3) / 4 * 4);
+            tmpl_tile = sdp.on && !ordered && tile_limit > 0;
+            if (!tmpl_tile)
+            {
+                while (warps_t > 1 && search_fast_smem_bytes(cand_cap_t, g.k, warps_t) > (size_t)E.max_smem()) --warps_t;
+                tmpl_select =
+                    cand_cap_t <= 65536 && search_fast_smem_bytes(cand_cap_t, g.k, warps_t) <= (size_t)E.max_smem();
+            }
+        }
+        if (tmpl_select || tmpl_tile)
+        {
+            kp.assign(nk, (uint16_t)0xFFFF);
+            for (size_t i = 0; i < tv.size(); ++i)
+            {
+                const size_t at = (size_t)key_index(g, tv[i].dx, tv[i].dy, tv[i].dz);
+                kp[at] = rank_keys ? (uint16_t)pl.kt.rank[at] : (uint16_t)i;
+            }
             keypos16 = E.buf<uint16_t>("keypos16", nk);
             HB_CK(cudaMemcpyAsync(keypos16, kp.data(), nk * 2, cudaMemcpyHostToDevice, st));
-            Surrogate sgp;
-            build_surrogate_template(pl.f, tv, sgp);
-            double *h2p = E.buf<double>("h2_pos", sgp.h2_rank.size());
-            HB_CK(cudaMemcpyAsync(h2p, sgp.h2_rank.data(), sgp.h2_rank.size() * 8, cudaMemcpyHostToDevice, st));
-            sdp.on = sgp.ok && !exact_search ? 1 : 0;
-            for (int i = 0; i < 9; ++i) sdp.T[i] = sgp.T[i];
-            for (int a = 0; a < 3; ++a) sdp.step[a] = sgp.step[a];
-            sdp.e3 = sgp.e3;
-            sdp.h2_cut = sgp.h2_cut;
-            sdp.h2_rank = h2p;
-            HB_CK(cudaStreamSynchronize(st)); // kp and sgp are temporaries
+            if (rank_keys)
+                sdp = sd;
+            else
+            {
+                for (double &h : sgp.h2_rank) h = root_up(h);
+                double *h2p = E.buf<double>("h_pos", sgp.h2_rank.size());
+                HB_CK(cudaMemcpyAsync(h2p, sgp.h2_rank.data(), sgp.h2_rank.size() * 8, cudaMemcpyHostToDevice, st));
+                for (int i = 0; i < 9; ++i) sdp.T[i] = sgp.T[i];
+                for (int a = 0; a < 3; ++a) sdp.step[a] = sgp.step[a];
+                sdp.e3 = sgp.e3;
+                sdp.h_cut = root_up(sgp.h2_cut);
+                sdp.h_rank = h2p;
+            }
         }
-        else
+        std::vector<int4> t4;
+        tmpl_scan = !tmpl_select && (!tmpl_tile || max_cand_tmpl > tile_limit);
+        if (tmpl_scan || rank_keys)
         {
             // the template probes a bitmap of the grid padded by the radiuses; its
             // linear offsets are 32-bit
             const long long PX = g.nx + 2LL * g.rx, PY = g.ny + 2LL * g.ry;
             if ((long long)g.rz * PY * PX + (long long)g.ry * PX + g.rx > 2147483647LL)
                 throw CudaFail{-4, "grid too large for the template search path at these radiuses"};
-            std::vector<int4> t4(tv.size());
+            t4.resize(tv.size());
             for (size_t i = 0; i < tv.size(); ++i)
                 t4[i] = make_int4(tv[i].dx, tv[i].dy, tv[i].dz, template_padded_offset(g, tv[i].dx, tv[i].dy, tv[i].dz));
             HB_CK(cudaMemcpyAsync(tmpl, t4.data(), t4.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
-            HB_CK(cudaStreamSynchronize(st)); // t4 is a temporary
             n_tmpl = (int)tv.size();
         }
+        HB_CK(cudaStreamSynchronize(st)); // kp, sgp and t4 are temporaries
     }
 
     // search
@@ -557,22 +596,39 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
     int *tie_cells = E.buf<int>("tie_cells", (size_t)g.n_cells);
     HB_CK(cudaMemsetAsync(S.nb_n, 0, sizeof(int) * g.n_cells, st));
     HB_CK(cudaEventRecord(E.ev_[8], st));
-    if (fast)
+    const bool tile = fast && sd.on && !ordered && cand_cap <= tile_limit;
+    if (tile)
+        HB_CK(launch_search_tile(g, d_mask, all_cells, bin_start, bin_cnt, S.bin_flag, bin_pts, P.pts_xyz, P.pts_val,
+                                 keytab16, sd, 0, g.n_bins, cand_cap, E.max_smem() - 1024, S.nb_rec, S.nb_n, tie_cells, scal + 3,
+                                 scal + 4, scal + 5, st));
+    else if (fast)
         HB_CK(launch_search_fast(g, d_mask, all_cells, bin_start, bin_cnt, S.bin_flag, bin_pts, P.pts_xyz, P.pts_val,
-                                 keytab16, sd, 0, P.pid_of_node, cand_cap, warps, S.nb_pid,
+                                 keytab16, sd, 0, ordered, P.pid_of_node, cand_cap, warps, S.nb_pid,
                                  S.nb_rec, S.nb_n, tie_cells, scal + 3, scal + 4, scal + 5, st));
     else
         HB_CK(launch_search(g, d_mask, all_cells, bin_start, bin_cnt, S.bin_flag, bin_pts, P.pts_xyz, P.pts_val,
                             keytab(), pl.rank_bits, tmpl, n_tmpl, P.pid_of_node, cand_cap, warps,
                             S.nb_pid, S.nb_rec, S.nb_n, tie_cells, scal + 3, scal + 4, st));
-    if (n_tmpl_bins > 0 && tmpl_select)
+    uint32_t *bits = tmpl_scan || rank_keys
+                         ? E.buf<uint32_t>("mask_bits", (size_t)(template_padded_cells(g) + 31) / 32)
+                         : nullptr;
+    if (tmpl_tile)
+    {
+        int *ties_t = rank_keys ? E.buf<int>("tmpl_ties", (size_t)g.n_cells) : tie_cells;
+        HB_CK(launch_search_tile(g, d_mask, all_cells, bin_start, bin_cnt, S.bin_flag, bin_pts, P.pts_xyz, P.pts_val,
+                                 keypos16, sdp, 1, n_tmpl_bins, cand_cap_t, E.max_smem() - 1024, S.nb_rec, S.nb_n, ties_t,
+                                 scal + (rank_keys ? 8 : 3), scal + 4, scal + 5, st));
+        if (rank_keys)
+            HB_CK(launch_search_template_list(g, d_mask, bits, ties_t, scal + 8, P.pts_val, tmpl, n_tmpl,
+                                              P.pid_of_node, S.nb_pid, S.nb_rec, S.nb_n, E.n_sm(), st));
+    }
+    else if (tmpl_select)
         HB_CK(launch_search_fast(g, d_mask, all_cells, bin_start, bin_cnt, S.bin_flag, bin_pts, P.pts_xyz, P.pts_val,
-                                 keypos16, sdp, 1, P.pid_of_node, cand_cap_t, warps_t, S.nb_pid, S.nb_rec, S.nb_n,
+                                 keypos16, sdp, 1, ordered, P.pid_of_node, cand_cap_t, warps_t, S.nb_pid, S.nb_rec, S.nb_n,
                                  tie_cells, scal + 3, scal + 4, scal + 5, st));
-    else if (n_tmpl_bins > 0)
-        HB_CK(launch_search_template(g, d_mask, E.buf<uint32_t>("mask_bits", (size_t)(template_padded_cells(g) + 31) / 32), all_cells,
-                                     tmpl_bins, n_tmpl_bins, P.pts_val, tmpl, n_tmpl, P.pid_of_node, S.nb_pid,
-                                     S.nb_rec, S.nb_n, scal + 4, E.n_sm(), st));
+    if (tmpl_scan)
+        HB_CK(launch_search_template(g, d_mask, bits, all_cells, tmpl_bins, n_tmpl_bins, bin_cnt, tmpl_tile ? tile_limit : -1, P.pts_val, tmpl,
+                                     n_tmpl, P.pid_of_node, S.nb_pid, S.nb_rec, S.nb_n, scal + 4, E.n_sm(), st));
     HB_CK(cudaEventRecord(E.ev_[9], st));
     HB_CK(cudaMemcpyAsync(host_scal, scal, sizeof(host_scal), cudaMemcpyDeviceToHost, st));
     HB_CK(cudaStreamSynchronize(st));
@@ -587,7 +643,8 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
         E.stats.search_kernel_ms += ms;
     }
     // flag, scan tiles (+add), emit, pair table, bin count, bin scan, fill, sort, region, search
-    E.stats.launches += 10 + (g.n_cells > 1024 ? 2 : 0) + (n_tmpl_bins > 0 ? (tmpl_select ? 1 : 2) : 0);
+    E.stats.launches += 10 + (g.n_cells > 1024 ? 2 : 0) + (tmpl_select || tmpl_tile ? 1 : 0) +
+                        (tmpl_scan ? 2 : 0) + (rank_keys ? 2 : 0);
 
     // tie groups straddling the k-th slot: std::sort's choice, replayed
     if (S.ties > 0)
@@ -1899,7 +1956,8 @@ int cokriging(const int *dims, const float *pdata, const unsigned char *pmask, c
             pl.g.limit = INT_MAX; // no bin takes the template path
             try
             {
-                DevSearch S = run_search(E, pl, P, d_pm, 0, st);
+                // cokriging's float sums run in the neighbours' order
+                DevSearch S = run_search(E, pl, P, d_pm, 0, st, false, false, true);
                 if (S.ties != 0) throw CudaFail{-2, "cokriging search: equal template keys"};
                 nb_rec = S.nb_rec;
                 nb_n = S.nb_n;
@@ -1944,7 +2002,7 @@ int cokriging(const int *dims, const float *pdata, const unsigned char *pmask, c
             if (n_t > 0)
             {
                 HB_CK(launch_search_template(g, d_pm, E.buf<uint32_t>("mask_bits", (size_t)(template_padded_cells(g) + 31) / 32),
-                                             0, tmpl_bins, g.n_bins, P.pts_val, tmpl, (int)t4.size(), P.pid_of_node,
+                                             0, tmpl_bins, g.n_bins, nullptr, -1, P.pts_val, tmpl, (int)t4.size(), P.pid_of_node,
                                              nullptr, nb_rec, nb_n, tcount, E.n_sm(), st));
                 E.stats.launches += 2;
             }

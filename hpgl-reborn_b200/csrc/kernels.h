@@ -44,21 +44,31 @@ void launch_bin_count(const unsigned long long *pts_xyz, const int *n_pts, const
                       cudaStream_t st);
 void launch_bin_fill(const unsigned long long *pts_xyz, const int *n_pts, const Geom &g, const int *bin_start,
                      int *bin_fill, int *bin_pts, cudaStream_t st);
-void launch_bin_sort(const Geom &g, const int *bin_start, const int *bin_cnt, int *bin_pts, uint8_t *bin_flag,
-                     cudaStream_t st);
+// bin_tmp (as filled) -> bin_pts (ascending in each bin; bins above both the
+// limit and kBinSortMax points as filled)
+constexpr int kBinSortMax = 1024;
+void launch_bin_sort(const Geom &g, const int *bin_start, const int *bin_cnt, const int *bin_tmp, int *bin_pts,
+                     uint8_t *bin_flag, cudaStream_t st);
 // max_cand / max_cand_tmpl: the largest 27-bin candidate count of the cluster-
-// path / template-path bins
+// path / template-path bins; max_bin: the largest bin when above kBinSortMax
 void launch_bin_region(const Geom &g, uint8_t *bin_flag, const int *bin_cnt, int *max_cand, int *n_tmpl_bins,
-                       int *tmpl_bins, int *max_cand_tmpl, cudaStream_t st);
+                       int *tmpl_bins, int *max_cand_tmpl, int *max_bin, cudaStream_t st);
 // Template-path search over a bitmap of the grid padded by the radiuses:
 // `bits` is scratch of (template_padded_cells + 31) / 32 words; template entries
-// carry template_padded_offset(dx, dy, dz) in .w.
+// carry template_padded_offset(dx, dy, dz) in .w. With min_cand >= 0 only bins of
+// more candidates than that are searched.
 long long template_padded_cells(const Geom &g);
 int template_padded_offset(const Geom &g, int dx, int dy, int dz);
 cudaError_t launch_search_template(const Geom &g, const uint8_t *mask, uint32_t *bits, int all_cells,
-                                   const int *tmpl_bins, int n_tmpl_bins, const float *pts_vf, const int4 *tmpl,
-                                   int n_tmpl, const int *pid_of_node, int *nb_pid, int2 *nb_rec, int *nb_n,
-                                   int *n_template_cells, int n_sm, cudaStream_t st);
+                                   const int *tmpl_bins, int n_tmpl_bins, const int *bin_cnt, int min_cand,
+                                   const float *pts_vf, const int4 *tmpl, int n_tmpl, const int *pid_of_node,
+                                   int *nb_pid, int2 *nb_rec, int *nb_n, int *n_template_cells, int n_sm,
+                                   cudaStream_t st);
+// the scan of the *n_list cells in `list` alone
+cudaError_t launch_search_template_list(const Geom &g, const uint8_t *mask, uint32_t *bits, const int *list,
+                                        const int *n_list, const float *pts_vf, const int4 *tmpl, int n_tmpl,
+                                        const int *pid_of_node, int *nb_pid, int2 *nb_rec, int *nb_n, int n_sm,
+                                        cudaStream_t st);
 size_t search_smem_bytes(int cand_cap, int k, int warps);
 cudaError_t launch_search(const Geom &g, const uint8_t *mask, int all_cells, const int *bin_start,
                           const int *bin_cnt, const uint8_t *bin_flag, const int *bin_pts,
@@ -74,20 +84,31 @@ struct SurrDev
     float T[9];
     float step[3];
     double e3;
-    double h2_cut;
-    const double *h2_rank;
+    double h_cut;         // square root of the largest h2 of a kept offset, rounded up
+    const double *h_rank; // and of each rank's largest h2
 };
 
 size_t search_fast_smem_bytes(int cand_cap, int k, int warps);
 // exact_cells (may be null) counts cells the float prefilter left to the exact
-// path. template_bins = 0 searches the cluster-path bins; 1 the template-path
+// path. `ordered` writes each cell's neighbours in key order; without it they
+// stand in candidate order (the same set, cheaper). template_bins = 0 searches the cluster-path bins; 1 the template-path
 // bins, keytab16 then holding template positions (n_template_cells counts them)
 cudaError_t launch_search_fast(const Geom &g, const uint8_t *mask, int all_cells, const int *bin_start,
                                const int *bin_cnt, const uint8_t *bin_flag, const int *bin_pts,
                                const unsigned long long *pts_xyz, const float *pts_vf, const uint16_t *keytab16,
-                               const SurrDev &sd, int template_bins, const int *pid_of_node, int cand_cap,
-                               int warps, int *nb_pid, int2 *nb_rec, int *nb_n, int *tie_cells, int *tie_count,
+                               const SurrDev &sd, int template_bins, bool ordered, const int *pid_of_node,
+                               int cand_cap, int warps, int *nb_pid, int2 *nb_rec, int *nb_n, int *tie_cells, int *tie_count,
                                int *n_template_cells, int *exact_cells, cudaStream_t st);
+// The same selection with the prefilter on, one cell a lane, neighbours in
+// candidate order (search_tile.cu): the bins with at most search_tile_limit
+// candidates. n_bins: how many bins there are of the kind searched.
+int search_tile_limit(int k, int max_smem);
+cudaError_t launch_search_tile(const Geom &g, const uint8_t *mask, int all_cells, const int *bin_start,
+                               const int *bin_cnt, const uint8_t *bin_flag, const int *bin_pts,
+                               const unsigned long long *pts_xyz, const float *pts_vf, const uint16_t *keytab16,
+                               const SurrDev &sd, int template_bins, int n_bins, int cand_cap, int max_smem, int2 *nb_rec,
+                               int *nb_n, int *tie_cells, int *tie_count, int *n_template_cells, int *exact_cells,
+                               cudaStream_t st);
 void launch_resolve_ties(const Geom &g, const int *tie_cells, const int *tie_count, int first, int chunk,
                          const int *bin_start, const int *bin_cnt, const int *bin_pts,
                          const unsigned long long *pts_xyz, const float *pts_vf, const uint32_t *keytab,

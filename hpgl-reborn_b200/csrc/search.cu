@@ -24,7 +24,9 @@
 #include "engine.cuh"
 #include "gnu_introsort.h"
 #include "kernels.h"
+#include "search_common.cuh"
 
+#include <algorithm>
 #include <cstdint>
 
 namespace hb
@@ -194,29 +196,37 @@ __global__ void k_bin_fill(const unsigned long long *__restrict__ pts_xyz, const
     }
 }
 
-// Restores ascending point order inside each non-exceeded bin (insertion sort;
-// bins hold at most `limit` points) and records per-bin flags:
+// Restores ascending point order inside each bin (the fill's atomics leave it
+// open) and records per-bin flags:
 //   bit 0: exceeded (count > limit)
-__global__ void k_bin_sort(Geom g, const int *__restrict__ bin_start, const int *__restrict__ bin_cnt,
-                           int *__restrict__ bin_pts, uint8_t *__restrict__ bin_flag)
+// A warp per bin places every point by the number of smaller ones. (One thread
+// per bin with an insertion sort took 1.6 to 2.0 ms on the clustered 512x512x64
+// grid, whose fullest bins hold some 200 points.) Exceeded bins of more than
+// kBinSortMax points stay as they are: the searches then order the neighbours.
+__global__ void __launch_bounds__(256) k_bin_sort(Geom g, const int *__restrict__ bin_start,
+                                                  const int *__restrict__ bin_cnt, const int *__restrict__ bin_tmp,
+                                                  int *__restrict__ bin_pts, uint8_t *__restrict__ bin_flag)
 {
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < g.n_bins; b += gridDim.x * blockDim.x)
+    const int lane = threadIdx.x & 31;
+    for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < g.n_bins; b += gridDim.x * blockDim.x >> 5)
     {
-        int c = bin_cnt[b];
-        bool exceeded = c > g.limit;
-        bin_flag[b] = exceeded ? 1 : 0;
-        if (exceeded) continue;
-        int *a = bin_pts + bin_start[b];
-        for (int i = 1; i < c; ++i)
+        const int c = bin_cnt[b];
+        const bool exceeded = c > g.limit;
+        if (lane == 0) bin_flag[b] = exceeded ? 1 : 0;
+        const int *a = bin_tmp + bin_start[b];
+        int *out = bin_pts + bin_start[b];
+        const bool sort = !exceeded || c <= kBinSortMax;
+        for (int i = lane; i < c; i += 32)
         {
-            int v = a[i];
-            int j = i - 1;
-            while (j >= 0 && a[j] > v)
+            const int v = a[i];
+            int at = i;
+            if (sort)
             {
-                a[j + 1] = a[j];
-                --j;
+                at = 0;
+#pragma unroll 8
+                for (int j = 0; j < c; ++j) at += __ldg(a + j) < v;
             }
-            a[j + 1] = v;
+            out[at] = v;
         }
     }
 }
@@ -224,13 +234,15 @@ __global__ void k_bin_sort(Geom g, const int *__restrict__ bin_start, const int 
 // bit 1: the cells of this bin take the template path
 __global__ void k_bin_region(Geom g, uint8_t *__restrict__ bin_flag, const int *__restrict__ bin_cnt,
                              int *__restrict__ max_cand, int *__restrict__ n_template_bins,
-                             int *__restrict__ template_bins, int *__restrict__ max_cand_tmpl)
+                             int *__restrict__ template_bins, int *__restrict__ max_cand_tmpl,
+                             int *__restrict__ max_bin)
 {
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < g.n_bins; b += gridDim.x * blockDim.x)
     {
         int cx = b % g.bx, cy = (b / g.bx) % g.by, cz = b / (g.bx * g.by);
         bool tmpl = false;
         int cand = 0;
+        if (bin_cnt[b] > kBinSortMax) atomicMax(max_bin, bin_cnt[b]);
         for (int k = cz - 1; k <= cz + 1; ++k)
             for (int j = cy - 1; j <= cy + 1; ++j)
                 for (int i = cx - 1; i <= cx + 1; ++i)
@@ -258,12 +270,6 @@ struct SearchSmem
     // then per warp: keys[C_cap] u32, hist[256] u32, sel[k_cap] u64
 };
 
-__device__ __forceinline__ unsigned lanemask_lt()
-{
-    unsigned m;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-    return m;
-}
 
 // Selects, for the cell at (x, y, z), the up-to-k candidates with the
 // smallest keys. Returns the number selected (written to `out` as point ids,
@@ -432,6 +438,52 @@ __global__ void k_mask_bits_padded(const Geom g, const uint8_t *__restrict__ mas
 // reaching out of the grid land on padding). A warp tests 4 x 32 offsets per
 // round: the entries and bits of all four steps are loaded before the first is
 // consumed, then the steps are taken in order (the same first-k as the serial walk).
+__device__ void template_cell(const Geom &g, const uint32_t *__restrict__ bits, int hx, int hy, int hz, int x, int y,
+                              int z, long long cell, int lane, const float *__restrict__ pts_vf,
+                              const int4 *__restrict__ tmpl, int n_tmpl, const int *__restrict__ pid_of_node,
+                              int *__restrict__ nb_pid, int2 *__restrict__ nb_rec, int *__restrict__ nb_n)
+{
+    constexpr int U = 4;
+    const int k = g.k;
+    const long long PX = g.nx + 2LL * hx, PY = g.ny + 2LL * hy;
+    const long long qc = ((long long)(z + hz) * PY + (y + hy)) * PX + (x + hx);
+    int found = 0;
+    for (int base = 0; base < n_tmpl && found < k; base += 32 * U)
+    {
+        bool ok[U];
+        int t_of[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+        {
+            const int t = base + 32 * u + lane;
+            t_of[u] = t;
+            ok[u] = false;
+            if (t < n_tmpl)
+            {
+                const long long q = qc + tmpl[t].w;
+                ok[u] = (bits[q >> 5] >> (q & 31)) & 1u;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+        {
+            if (found >= k) break; // warp-uniform
+            const unsigned bl = __ballot_sync(0xffffffffu, ok[u]);
+            const int slot = found + __popc(bl & lanemask_lt());
+            if (ok[u] && slot < k)
+            {
+                const int4 o = tmpl[t_of[u]];
+                const long long node = ((long long)(z + o.z) * g.ny + (y + o.y)) * g.nx + (x + o.x);
+                const int p = pid_of_node[node];
+                if (nb_pid) nb_pid[cell * k + slot] = p;
+                if (nb_rec) nb_rec[cell * k + slot] = make_int2(pair_lin(g, o.x, o.y, o.z), __float_as_int(pts_vf[p]));
+            }
+            found += __popc(bl);
+        }
+    }
+    if (lane == 0) nb_n[cell] = min(found, k);
+}
+
 __device__ void template_cells(const Geom &g, const uint32_t *__restrict__ bits, int hx, int hy, int hz,
                                const uint8_t *__restrict__ mask, int all_cells, int x0, int y0, int z0, int wx,
                                int wy, int n_cells_bin, int warp, int nwarps, int lane,
@@ -439,9 +491,6 @@ __device__ void template_cells(const Geom &g, const uint32_t *__restrict__ bits,
                                const int *__restrict__ pid_of_node, int *__restrict__ nb_pid,
                                int2 *__restrict__ nb_rec, int *__restrict__ nb_n, int *__restrict__ n_template_cells)
 {
-    constexpr int U = 4;
-    const int k = g.k;
-    const long long PX = g.nx + 2LL * hx, PY = g.ny + 2LL * hy;
     int counted = 0;
     for (int c = warp; c < n_cells_bin; c += nwarps)
     {
@@ -449,42 +498,7 @@ __device__ void template_cells(const Geom &g, const uint32_t *__restrict__ bits,
         long long cell = ((long long)z * g.ny + y) * g.nx + x;
         if (!all_cells && mask[cell]) continue;
         ++counted;
-        const long long qc = ((long long)(z + hz) * PY + (y + hy)) * PX + (x + hx);
-        int found = 0;
-        for (int base = 0; base < n_tmpl && found < k; base += 32 * U)
-        {
-            bool ok[U];
-            int t_of[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-            {
-                const int t = base + 32 * u + lane;
-                t_of[u] = t;
-                ok[u] = false;
-                if (t < n_tmpl)
-                {
-                    const long long q = qc + tmpl[t].w;
-                    ok[u] = (bits[q >> 5] >> (q & 31)) & 1u;
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-            {
-                if (found >= k) break; // warp-uniform
-                const unsigned bl = __ballot_sync(0xffffffffu, ok[u]);
-                const int slot = found + __popc(bl & lanemask_lt());
-                if (ok[u] && slot < k)
-                {
-                    const int4 o = tmpl[t_of[u]];
-                    const long long node = ((long long)(z + o.z) * g.ny + (y + o.y)) * g.nx + (x + o.x);
-                    const int p = pid_of_node[node];
-                    if (nb_pid) nb_pid[cell * k + slot] = p;
-                    if (nb_rec) nb_rec[cell * k + slot] = make_int2(pair_lin(g, o.x, o.y, o.z), __float_as_int(pts_vf[p]));
-                }
-                found += __popc(bl);
-            }
-        }
-        if (lane == 0) nb_n[cell] = min(found, k);
+        template_cell(g, bits, hx, hy, hz, x, y, z, cell, lane, pts_vf, tmpl, n_tmpl, pid_of_node, nb_pid, nb_rec, nb_n);
     }
     if (lane == 0 && counted) atomicAdd(n_template_cells, counted);
 }
@@ -641,7 +655,93 @@ __device__ __forceinline__ int warp_count_le(const uint32_t *keys, int C, uint32
     return c;
 }
 
-template <int E>
+// Writes the kept candidates of a cell. With ORDERED, v is sorted ascending
+// (element i in v[i / 32] of lane i % 32) and the first n_sel go out in that
+// order; else v holds them anywhere (0 elsewhere) and they go out as they stand,
+// in candidate order.
+template <int E, bool ORDERED>
+__device__ __forceinline__ void emit_selected(const uint32_t (&v)[E], int n_sel, int lane, const int *cplin,
+                                              const int *cpid, const float *cval, int plin_c, int *out_pid,
+                                              int2 *out_rec)
+{
+    int done = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+    {
+        int i = e * 32 + lane;
+        bool in = i < n_sel;
+        if (!ORDERED)
+        {
+            in = v[e] != 0u;
+            const unsigned bl = __ballot_sync(0xffffffffu, in);
+            i = done + __popc(bl & lanemask_lt());
+            done += __popc(bl);
+        }
+        if (in)
+        {
+            const int pos = (int)((v[e] - 1u) & 0xFFFFu);
+            if (out_pid) out_pid[i] = cpid[pos];
+            if (out_rec) out_rec[i] = make_int2(cplin[pos] - plin_c, __float_as_int(cval[pos]));
+        }
+    }
+}
+
+// The k smallest of the warp's nk non-zero keys in v (unique; 0 is no key, a
+// key is its rank << 16 | position, plus one): kth and nxt receive the k-th and
+// the (k+1)-th smallest (nxt 0 when nk <= k; kth the largest when nk < k). v
+// keeps the k smallest in place, or, with ORDERED, sorted. In place, the few keys
+// above the k-th are taken out one by one, largest first, each by a warp maximum
+// (a step on the benchmark keeps 37 keys for 32); from kSelectSteps surplus keys
+// on, and with ORDERED, the whole set is sorted (21 exchange stages for 64 keys).
+constexpr int kSelectSteps = 20;
+template <int E, bool ORDERED>
+__device__ __forceinline__ void select_smallest(uint32_t (&v)[E], int nk, int k, int lane, uint32_t &kth,
+                                                uint32_t &nxt)
+{
+    nxt = 0u;
+    kth = 0u;
+    if (nk == 0) return;
+    if (!ORDERED && nk - k < kSelectSteps)
+    {
+        uint32_t top = 0u;
+        for (int it = nk; it >= k; --it)
+        {
+            uint32_t m = v[0];
+#pragma unroll
+            for (int e = 1; e < E; ++e) m = max(m, v[e]);
+            top = __reduce_max_sync(0xffffffffu, m);
+            if (it <= k) break;
+            nxt = top;
+#pragma unroll
+            for (int e = 0; e < E; ++e)
+                if (v[e] == top) v[e] = 0u;
+        }
+        if (nk < k)
+        {
+            uint32_t m = v[0];
+#pragma unroll
+            for (int e = 1; e < E; ++e) m = max(m, v[e]);
+            top = __reduce_max_sync(0xffffffffu, m);
+        }
+        kth = top;
+        return;
+    }
+    uint32_t t[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) t[e] = v[e] - 1u; // no key: the largest
+    warp_bitonic_sort<E>(t, lane);
+    const int i = min(nk, k) - 1;
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+    {
+        if (e == (i >> 5)) kth = __shfl_sync(0xffffffffu, t[e], i & 31) + 1u;
+        if (nk > k && e == (k >> 5)) nxt = __shfl_sync(0xffffffffu, t[e], k & 31) + 1u;
+    }
+#pragma unroll
+    for (int e = 0; e < E; ++e) v[e] = ORDERED ? t[e] + 1u : (v[e] <= kth ? v[e] : 0u);
+}
+
+template <int E, bool ORDERED>
 __device__ __forceinline__ int select_fast(const Geom &g, int C, const int *cklin, const int *cplin, const int *cpid,
                            const float *cval, int kc0, int klin_c, int plin_c,
                            const uint16_t *__restrict__ keytab, uint32_t *keys, uint32_t *sel, int lane,
@@ -720,148 +820,126 @@ __device__ __forceinline__ int select_fast(const Geom &g, int C, const int *ckli
     for (int e = 0; e < E; ++e)
     {
         const int i = e * 32 + lane;
-        v[e] = i < cnt ? sel[i] : 0xFFFFFFFFu;
+        v[e] = i < cnt ? sel[i] + 1u : 0u;
     }
-    warp_bitonic_sort<E>(v, lane);
-    // sorted element i sits in v[i / 32] of lane i % 32
     const int n_sel = cnt < k ? cnt : k;
     if (n_sel <= 0) return 0;
-    const uint32_t kth = __shfl_sync(0xffffffffu, v[(n_sel - 1) >> 5], (n_sel - 1) & 31);
-    if (cnt > k)
-    {
-        const uint32_t nxt = __shfl_sync(0xffffffffu, v[k >> 5], k & 31);
-        if ((nxt >> 16) == (kth >> 16))
-        {
-            kguess = (int)(kth >> 16);
-            return -1;
-        }
-    }
-    kguess = (int)(kth >> 16);
-#pragma unroll
-    for (int e = 0; e < E; ++e)
-    {
-        const int i = e * 32 + lane;
-        if (i < n_sel)
-        {
-            const int pos = (int)(v[e] & 0xFFFFu);
-            if (out_pid) out_pid[i] = cpid[pos];
-            if (out_rec) out_rec[i] = make_int2(cplin[pos] - plin_c, __float_as_int(cval[pos]));
-        }
-    }
+    uint32_t kth, nxt;
+    select_smallest<E, ORDERED>(v, cnt, k, lane, kth, nxt);
+    kguess = (int)((kth - 1u) >> 16);
+    if (cnt > k && (int)((nxt - 1u) >> 16) == kguess) return -1;
+    emit_selected<E, ORDERED>(v, n_sel, lane, cplin, cpid, cval, plin_c, out_pid, out_rec);
     return n_sel;
 }
 
 // Float prefilter of select_fast. One sweep forms every candidate's squared
 // transformed distance h2f in float (no table reads) and keeps those with
-// h2f <= Tg; only these (at most CAP) read their exact ranks, which are sorted
-// as in select_fast. A candidate left out has h2f > Tg, so its true h2 exceeds
-// lo = (sqrt(Tg / (1 + 4u)) - e3)^2 (three roundings in h2f, e3 the bound on the
-// coordinate error). With the ranks non-decreasing in h2, lo above the largest
-// h2 carrying the k-th kept rank (or above every kept offset's h2 when fewer
-// than k are kept) means every candidate left out ranks strictly after the
-// k-th, so the outcome equals the exact path's. Returns n_sel, -1 for a tie group straddling
-// the k-th slot, or -2 when the prefilter cannot decide (the caller then runs
-// select_fast). On success or -1, H receives that bound.
-template <int E>
+// h2f <= Tg, Tg >= rt^2 (1 + 1e-6); only these (at most CAP) read their exact
+// ranks. A candidate left out has h2f > Tg, so its true distance exceeds
+// sqrt(Tg / (1 + 4u)) - e3 > rt - e3 (three roundings in h2f, e3 the bound on the
+// coordinate error). With the ranks non-decreasing in h2, rt - e3 above the
+// largest distance carrying the k-th kept rank (or above every kept offset's
+// when fewer than k are kept) means every candidate left out ranks strictly after
+// the k-th, so the outcome equals the exact path's. rt is a guess: with more than
+// CAP survivors, fewer than k, or the k-th too near rt, the sweep repeats with
+// another, a few times at most. The sublist `sub` (n_sub entries) holds every
+// candidate within r_sub of the cell. Returns n_sel, -1 for a tie group
+// straddling the k-th slot, or -2 when the prefilter cannot decide (the caller
+// then runs select_fast). On success or -1, H receives that largest distance.
+template <int E, bool ORDERED>
 __device__ __forceinline__ int select_surr(const Geom &g, const SurrDev &sd, int C, const float4 *ctp, const int *cklin,
                            const int *cplin, const int *cpid, const float *cval, int kc0, int klin_c, int plin_c,
                            const uint16_t *__restrict__ keytab, uint32_t *sel, int lane, float tcx, float tcy,
-                           float tcz, float Tg, const uint32_t *sub, int n_sub, double &H, int &kguess,
+                           float tcz, double rt, const uint32_t *sub, int n_sub, float r_sub, double &H, int &kguess,
                            int *out_pid, int2 *out_rec)
 {
     constexpr int CAP = 32 * E;
+    constexpr int kTries = 6;
     const int k = g.k;
-    int cnt = 0;
-    __syncwarp(); // the previous cell's reads of sel are done
-    // candidates scanned: the sublist `sub` (n_sub entries) when given, else all C
-    const int n_scan = sub ? n_sub : C;
-    for (int base = 0; base < n_scan; base += 32)
+    const double r_all = sd.h_cut * (1.0 + 1e-9) + 3.0 * sd.e3; // a radius that decides every candidate
+    float lo = 0.0f; // a radius known to keep fewer than k
+    for (int tries = 0; tries < kTries; ++tries)
     {
-        const int j = base + lane;
-        bool in = false;
-        int i = 0;
-        if (j < n_scan)
+        if (rt > r_all) rt = r_all;
+        const float Tg = __double2float_ru(rt * rt * (1.0 + 1e-6));
+        const float rf = (float)rt;
+        const bool use_sub = rf * (1.0f + 1e-6f) <= r_sub;
+        const int n_scan = use_sub ? n_sub : C;
+        int cnt = 0, base = 0;
+        __syncwarp(); // earlier reads of sel are done
+        for (; base < n_scan && cnt <= CAP; base += 32)
         {
-            i = sub ? (int)sub[j] : j;
-            const float4 t = ctp[i];
-            const float qx = t.x - tcx, qy = t.y - tcy, qz = t.z - tcz;
-            in = fmaf(qz, qz, fmaf(qy, qy, qx * qx)) <= Tg;
-        }
-        const unsigned bl = __ballot_sync(0xffffffffu, in);
-        if (in)
-        {
+            const int j = base + lane;
+            bool in = false;
+            int i = 0;
+            if (j < n_scan)
+            {
+                i = use_sub ? (int)sub[j] : j;
+                const float4 t = ctp[i];
+                const float qx = t.x - tcx, qy = t.y - tcy, qz = t.z - tcz;
+                in = fmaf(qz, qz, fmaf(qy, qy, qx * qx)) <= Tg;
+            }
+            const unsigned bl = __ballot_sync(0xffffffffu, in);
             const int slot = cnt + __popc(bl & lanemask_lt());
-            if (slot < CAP) sel[slot] = (uint32_t)i;
+            if (in && slot < CAP) sel[slot] = (uint32_t)i;
+            cnt += __popc(bl);
         }
-        cnt += __popc(bl);
-        if (cnt > CAP) return -2;
-    }
-    __syncwarp();
-    uint32_t v[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e)
-    {
-        const int i = e * 32 + lane;
-        v[e] = 0xFFFFFFFFu;
-        if (i < cnt)
+        if (cnt > CAP)
         {
-            const uint32_t pos = sel[i];
-            const uint32_t r16 = keytab[kc0 + cklin[pos] - klin_c];
-            if (r16 != 0xFFFFu) v[e] = (r16 << 16) | pos;
+            // the whole sweep would have found about cnt n_scan / base of them
+            const float est = (float)cnt * (float)n_scan / (float)min(base, n_scan);
+            const float f = cbrtf(0.5f * (float)(k + CAP) / est);
+            rt = fmaxf(rf * fminf(f, 0.95f), 0.5f * (lo + rf));
+            continue;
         }
-    }
-    __syncwarp();
-    warp_bitonic_sort<E>(v, lane);
-    int nk = 0;
-#pragma unroll
-    for (int e = 0; e < E; ++e) nk += __popc(__ballot_sync(0xffffffffu, v[e] != 0xFFFFFFFFu));
-    uint32_t kth = 0;
-    if (nk >= k)
-    {
-        kth = __shfl_sync(0xffffffffu, v[(k - 1) >> 5], (k - 1) & 31);
-        H = sd.h2_rank[kth >> 16];
-    }
-    else
-        H = sd.h2_cut;
-    const double s = sqrt((double)Tg / (1.0 + 4.0 / 16777216.0)) - sd.e3;
-    const double lo = s > 0.0 ? s * s * (1.0 - 1e-12) : 0.0;
-    if (!(lo > H)) return -2;
-    const int n_sel = nk < k ? nk : k;
-    if (nk > k)
-    {
-        const uint32_t nxt = __shfl_sync(0xffffffffu, v[k >> 5], k & 31);
-        if ((nxt >> 16) == (kth >> 16))
+        if (cnt < k && rt < r_all)
         {
-            kguess = (int)(kth >> 16);
-            return -1;
+            lo = rf;
+            rt = rt * (double)fminf(1.1f * cbrtf((float)k / fmaxf((float)cnt, 0.25f)) + 0.02f, 4.0f) + sd.e3;
+            continue;
         }
-    }
-    if (n_sel > 0) kguess = (int)(__shfl_sync(0xffffffffu, v[(n_sel - 1) >> 5], (n_sel - 1) & 31) >> 16);
+        __syncwarp();
+        uint32_t v[E];
+        int nk = 0;
 #pragma unroll
-    for (int e = 0; e < E; ++e)
-    {
-        const int i = e * 32 + lane;
-        if (i < n_sel)
+        for (int e = 0; e < E; ++e)
         {
-            const int pos = (int)(v[e] & 0xFFFFu);
-            if (out_pid) out_pid[i] = cpid[pos];
-            if (out_rec) out_rec[i] = make_int2(cplin[pos] - plin_c, __float_as_int(cval[pos]));
+            const int i = e * 32 + lane;
+            v[e] = 0u;
+            if (i < cnt)
+            {
+                const uint32_t pos = sel[i];
+                const uint32_t r16 = keytab[kc0 + cklin[pos] - klin_c];
+                if (r16 != 0xFFFFu) v[e] = ((r16 << 16) | pos) + 1u;
+            }
+            nk += __popc(__ballot_sync(0xffffffffu, v[e] != 0u));
         }
+        if (nk < k && rt < r_all)
+        {
+            lo = rf;
+            rt = r_all; // some survivors rank nowhere: the kept offsets end near here
+            continue;
+        }
+        uint32_t kth, nxt;
+        select_smallest<E, ORDERED>(v, nk, k, lane, kth, nxt);
+        H = nk >= k ? sd.h_rank[(kth - 1u) >> 16] : sd.h_cut;
+        if (!((rt - sd.e3) * (1.0 - 1e-12) > H))
+        {
+            lo = rf;
+            rt = H * (1.0 + 1e-9) + 2.0 * sd.e3;
+            continue;
+        }
+        const int n_sel = nk < k ? nk : k;
+        if (n_sel > 0) kguess = (int)((kth - 1u) >> 16);
+        if (nk > k && (int)((nxt - 1u) >> 16) == kguess) return -1;
+        emit_selected<E, ORDERED>(v, n_sel, lane, cplin, cpid, cval, plin_c, out_pid, out_rec);
+        return n_sel;
     }
-    return n_sel;
+    return -2;
 }
 
-// transformed coordinates of an offset from the bin corner, in float
-__device__ __forceinline__ float4 surr_coords(const SurrDev &sd, int x, int y, int z)
-{
-    const float fx = (float)x, fy = (float)y, fz = (float)z;
-    return make_float4(fmaf(sd.T[2], fz, fmaf(sd.T[1], fy, sd.T[0] * fx)),
-                       fmaf(sd.T[5], fz, fmaf(sd.T[4], fy, sd.T[3] * fx)),
-                       fmaf(sd.T[8], fz, fmaf(sd.T[7], fy, sd.T[6] * fx)), 0.0f);
-}
-
-template <int E>
-__global__ void __launch_bounds__(256) k_search_fast(
+template <int E, bool ORDERED>
+__global__ void __launch_bounds__(256, E == 2 ? 4 : 2) k_search_fast(
     const Geom g, const uint8_t *__restrict__ mask, int all_cells, const int *__restrict__ bin_start,
     const int *__restrict__ bin_cnt, const uint8_t *__restrict__ bin_flag, const int *__restrict__ bin_pts,
     const unsigned long long *__restrict__ pts_xyz, const float *__restrict__ pts_vf,
@@ -940,18 +1018,18 @@ __global__ void __launch_bounds__(256) k_search_fast(
     const int run_len = (n_cells_bin + nwarps - 1) / nwarps;
     const int c0 = warp * run_len, c1 = min(c0 + run_len, n_cells_bin);
     int kguess = -1;
-    bool have_h = false;
-    double h_prev = 0.0;
-    float path = 0.0f;
+    // The k-th distance of the previous cell plus the path walked since bounds
+    // this cell's (`rt`); the first cell of a run guesses from the candidates'
+    // density (27 bins hold C of them).
+    double rt = cbrt(1.5 * (double)k * 27.0 * (double)g.rx * g.ry * g.rz / (4.18879 * (double)max(C, 1))) *
+                cbrt((double)sd.step[0] * sd.step[1] * sd.step[2]);
     int n_exact = 0, n_done = 0;
     // Chunks of kChunk consecutive cells share a sublist of the candidates within
     // R of the chunk's centre (transformed coordinates), kept in `keys`. A cell scans
-    // it instead of all C when sqrt(Tg) + |cell - centre| + slack <= R: every
-    // candidate left out of the sublist is then farther than sqrt(Tg) from the cell
-    // (true distance), so it lies beyond the prefilter's threshold like any other
-    // candidate the prefilter drops. select_fast reuses `keys`, invalidating the sublist.
-    // (Search stage on the 256x256x128 benchmark by chunk length: 4: 9.38 ms, 6: 9.12,
-    // 8: 9.14-9.20, 12: 9.66, 16: 10.31, 24: 11.57.)
+    // it instead of all C when rt + |cell - centre| + slack <= R: every candidate left
+    // out of the sublist is then farther than sqrt(Tg) from the cell (true distance),
+    // so it lies beyond the prefilter's threshold like any other candidate the
+    // prefilter drops. select_fast reuses `keys`, invalidating the sublist.
     constexpr int kChunk = 8;
     int ch_left = 0, n_sub = 0;
     bool sl_ok = false;
@@ -965,16 +1043,47 @@ __global__ void __launch_bounds__(256) k_search_fast(
         sy = row - sz * wy;
         if (sz & 1) sy = wy - 1 - sy;
     };
+    // the walk's position, advanced a unit step at a time
+    int cxr = 0, cyr = 0, czr = 0, in_x = 0, in_y = 0;
+    if (c0 < c1)
+    {
+        snake(c0, cxr, cyr, czr);
+        in_x = c0 % wx;
+        in_y = c0 / wx % wy;
+    }
+    int dir_x = (c0 / wx) & 1 ? -1 : 1, dir_y = (c0 / wx / wy) & 1 ? -1 : 1;
     for (int c = c0; c < c1; ++c)
     {
-        if (c > c0) path += (c % wx) ? sd.step[0] : ((c / wx) % wy ? sd.step[1] : sd.step[2]);
-        int cxr, cyr, czr;
-        snake(c, cxr, cyr, czr);
+        if (c > c0)
+        {
+            if (++in_x < wx)
+            {
+                cxr += dir_x;
+                rt += sd.step[0];
+            }
+            else
+            {
+                in_x = 0;
+                dir_x = -dir_x;
+                if (++in_y < wy)
+                {
+                    cyr += dir_y;
+                    rt += sd.step[1];
+                }
+                else
+                {
+                    in_y = 0;
+                    dir_y = -dir_y;
+                    ++czr;
+                    rt += sd.step[2];
+                }
+            }
+        }
         if (ch_left == 0)
         {
             ch_left = min(kChunk, c1 - c);
             sl_ok = false;
-            if (sd.on && have_h)
+            if (sd.on)
             {
                 // centre and radius of the chunk's cells in transformed coordinates
                 int sx, sy, sz;
@@ -982,7 +1091,7 @@ __global__ void __launch_bounds__(256) k_search_fast(
                 const float4 q = surr_coords(sd, sx, sy, sz);
                 float lo_x = q.x, hi_x = q.x, lo_y = q.y, hi_y = q.y, lo_z = q.z, hi_z = q.z;
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1)
+                for (int o = 4; o > 0; o >>= 1) // lanes past the chunk repeat its last cell
                 {
                     lo_x = fminf(lo_x, __shfl_xor_sync(0xffffffffu, lo_x, o));
                     hi_x = fmaxf(hi_x, __shfl_xor_sync(0xffffffffu, hi_x, o));
@@ -991,12 +1100,19 @@ __global__ void __launch_bounds__(256) k_search_fast(
                     lo_z = fminf(lo_z, __shfl_xor_sync(0xffffffffu, lo_z, o));
                     hi_z = fmaxf(hi_z, __shfl_xor_sync(0xffffffffu, hi_z, o));
                 }
+                // every lane the first group's
+                lo_x = __shfl_sync(0xffffffffu, lo_x, 0);
+                hi_x = __shfl_sync(0xffffffffu, hi_x, 0);
+                lo_y = __shfl_sync(0xffffffffu, lo_y, 0);
+                hi_y = __shfl_sync(0xffffffffu, hi_y, 0);
+                lo_z = __shfl_sync(0xffffffffu, lo_z, 0);
+                hi_z = __shfl_sync(0xffffffffu, hi_z, 0);
                 ccx = 0.5f * (lo_x + hi_x);
                 ccy = 0.5f * (lo_y + hi_y);
                 ccz = 0.5f * (lo_z + hi_z);
                 const float ex = hi_x - ccx, ey = hi_y - ccy, ez = hi_z - ccz;
                 const float rho = sqrtf(ex * ex + ey * ey + ez * ez);
-                Rcov = (float)sqrt(h_prev) + 2.0f * rho + 1.5f;
+                Rcov = (float)rt + 2.0f * rho + 1.5f;
                 const float R2 = Rcov * Rcov;
                 __syncwarp();
                 n_sub = 0;
@@ -1027,37 +1143,32 @@ __global__ void __launch_bounds__(256) k_search_fast(
         int2 *o_rec = nb_rec ? nb_rec + cell * k : nullptr;
         int n = -2;
         double h = 0.0;
-        if (sd.on && have_h)
+        if (sd.on)
         {
-            const double rt = sqrt(h_prev) + (double)path + 2.0 * sd.e3;
-            const float Tg = __double2float_ru(rt * rt * (1.0 + 1e-6));
             const float4 tc = surr_coords(sd, cxr, cyr, czr);
-            bool use_sub = false;
+            float r_sub = -1.0f;
             if (sl_ok)
             {
-                const float dx = tc.x - ccx, dy = tc.y - ccy, dz = tc.z - ccz;
-                const float dc = sqrtf(fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
                 // R excludes candidates at float distance > R from the centre: true
                 // distance > R - e3 - rounding; the cell is within dc + e3 of the
-                // centre; slack covers both errors and the roundings of dc and sqrt(Tg)
-                use_sub = sqrtf(Tg) * (1.0f + 1e-6f) + dc * (1.0f + 1e-6f) + slack + 1e-5f * Rcov <= Rcov;
+                // centre; slack covers both errors and the roundings of dc and rt
+                const float dx = tc.x - ccx, dy = tc.y - ccy, dz = tc.z - ccz;
+                const float dc = sqrtf(fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
+                r_sub = Rcov * (1.0f - 1e-5f) - dc * (1.0f + 1e-6f) - slack;
             }
-            n = select_surr<E>(g, sd, C, ctp, cklin, cplin, cpid, cval, kc0, klin_c, plin_c, keytab16, sel, lane,
-                               tc.x, tc.y, tc.z, Tg, use_sub ? keys : nullptr, n_sub, h, kguess, o_pid, o_rec);
+            n = select_surr<E, ORDERED>(g, sd, C, ctp, cklin, cplin, cpid, cval, kc0, klin_c, plin_c, keytab16, sel,
+                                        lane, tc.x, tc.y, tc.z, rt + 2.0 * sd.e3, keys, n_sub, r_sub, h, kguess, o_pid,
+                                        o_rec);
         }
         if (n == -2)
         {
-            n = select_fast<E>(g, C, cklin, cplin, cpid, cval, kc0, klin_c, plin_c, keytab16, keys, sel, lane,
-                               kguess, o_pid, o_rec);
+            n = select_fast<E, ORDERED>(g, C, cklin, cplin, cpid, cval, kc0, klin_c, plin_c, keytab16, keys, sel, lane,
+                                        kguess, o_pid, o_rec);
             sl_ok = false; // keys[] now holds select_fast's keys
             n_exact += sd.on;
-            h = (sd.on && kguess >= 0) ? sd.h2_rank[kguess] : 0.0;
-            have_h = sd.on && kguess >= 0 && n != 0;
+            h = (sd.on && kguess >= 0 && n != 0) ? sd.h_rank[kguess] : rt;
         }
-        else
-            have_h = n != 0;
-        h_prev = h;
-        path = 0.0f;
+        rt = h;
         ++n_done;
         if (lane == 0)
         {
@@ -1084,30 +1195,21 @@ size_t search_fast_smem_bytes(int cand_cap, int k, int warps)
 cudaError_t launch_search_fast(const Geom &g, const uint8_t *mask, int all_cells, const int *bin_start,
                                const int *bin_cnt, const uint8_t *bin_flag, const int *bin_pts,
                                const unsigned long long *pts_xyz, const float *pts_vf, const uint16_t *keytab16,
-                               const SurrDev &sd, int template_bins, const int *pid_of_node, int cand_cap,
-                               int warps, int *nb_pid, int2 *nb_rec, int *nb_n, int *tie_cells, int *tie_count,
+                               const SurrDev &sd, int template_bins, bool ordered, const int *pid_of_node,
+                               int cand_cap, int warps, int *nb_pid, int2 *nb_rec, int *nb_n, int *tie_cells, int *tie_count,
                                int *n_template_cells, int *exact_cells, cudaStream_t st)
 {
-    size_t smem = search_fast_smem_bytes(cand_cap, g.k, warps);
-    if (g.k <= 32)
-    {
-        cudaError_t e = cudaFuncSetAttribute(k_search_fast<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t smem = search_fast_smem_bytes(cand_cap, g.k, warps);
+    auto launch = [&](auto kern) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        k_search_fast<2><<<g.n_bins, warps * 32, smem, st>>>(g, mask, all_cells, bin_start, bin_cnt, bin_flag, bin_pts,
-                                                            pts_xyz, pts_vf, keytab16, sd, template_bins, pid_of_node,
-                                                            cand_cap, nb_pid, nb_rec, nb_n, tie_cells, tie_count,
-                                                            n_template_cells, exact_cells);
-    }
-    else
-    {
-        cudaError_t e = cudaFuncSetAttribute(k_search_fast<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        k_search_fast<4><<<g.n_bins, warps * 32, smem, st>>>(g, mask, all_cells, bin_start, bin_cnt, bin_flag, bin_pts,
-                                                            pts_xyz, pts_vf, keytab16, sd, template_bins, pid_of_node,
-                                                            cand_cap, nb_pid, nb_rec, nb_n, tie_cells, tie_count,
-                                                            n_template_cells, exact_cells);
-    }
-    return cudaGetLastError();
+        kern<<<g.n_bins, warps * 32, smem, st>>>(g, mask, all_cells, bin_start, bin_cnt, bin_flag, bin_pts, pts_xyz,
+                                                 pts_vf, keytab16, sd, template_bins, pid_of_node, cand_cap, nb_pid,
+                                                 nb_rec, nb_n, tie_cells, tie_count, n_template_cells, exact_cells);
+        return cudaGetLastError();
+    };
+    if (g.k <= 32) return ordered ? launch(k_search_fast<2, true>) : launch(k_search_fast<2, false>);
+    return ordered ? launch(k_search_fast<4, true>) : launch(k_search_fast<4, false>);
 }
 
 // One thread per tie-straddling cell: rebuild the threshold-filtered candidate
@@ -1473,17 +1575,17 @@ void launch_bin_fill(const unsigned long long *pts_xyz, const int *n_pts, const 
 {
     k_bin_fill<<<592, 256, 0, st>>>(pts_xyz, n_pts, g, bin_start, bin_fill, bin_pts);
 }
-void launch_bin_sort(const Geom &g, const int *bin_start, const int *bin_cnt, int *bin_pts, uint8_t *bin_flag,
-                     cudaStream_t st)
+void launch_bin_sort(const Geom &g, const int *bin_start, const int *bin_cnt, const int *bin_tmp, int *bin_pts,
+                     uint8_t *bin_flag, cudaStream_t st)
 {
-    int blocks = (g.n_bins + 255) / 256;
-    k_bin_sort<<<blocks, 256, 0, st>>>(g, bin_start, bin_cnt, bin_pts, bin_flag);
+    const int blocks = std::min((g.n_bins + 7) / 8, 1 << 16);
+    k_bin_sort<<<blocks, 256, 0, st>>>(g, bin_start, bin_cnt, bin_tmp, bin_pts, bin_flag);
 }
 void launch_bin_region(const Geom &g, uint8_t *bin_flag, const int *bin_cnt, int *max_cand, int *n_tmpl_bins,
-                       int *tmpl_bins, int *max_cand_tmpl, cudaStream_t st)
+                       int *tmpl_bins, int *max_cand_tmpl, int *max_bin, cudaStream_t st)
 {
     int blocks = (g.n_bins + 255) / 256;
-    k_bin_region<<<blocks, 256, 0, st>>>(g, bin_flag, bin_cnt, max_cand, n_tmpl_bins, tmpl_bins, max_cand_tmpl);
+    k_bin_region<<<blocks, 256, 0, st>>>(g, bin_flag, bin_cnt, max_cand, n_tmpl_bins, tmpl_bins, max_cand_tmpl, max_bin);
 }
 
 // Template-path cells (k_search and k_search_fast leave their bins alone): a
@@ -1492,7 +1594,7 @@ void launch_bin_region(const Geom &g, uint8_t *bin_flag, const int *bin_cnt, int
 // overflowing bin) are spread over the whole GPU.
 __global__ void __launch_bounds__(256) k_search_template(
     const Geom g, const uint32_t *__restrict__ bits, int hx, int hy, int hz, const uint8_t *__restrict__ mask,
-    int all_cells, const int *__restrict__ template_bins,
+    int all_cells, const int *__restrict__ template_bins, const int *__restrict__ bin_cnt, int min_cand,
     const float *__restrict__ pts_vf, const int4 *__restrict__ tmpl, int n_tmpl, const int *__restrict__ pid_of_node,
     int *__restrict__ nb_pid, int2 *__restrict__ nb_rec, int *__restrict__ nb_n, int *__restrict__ n_template_cells)
 {
@@ -1500,6 +1602,14 @@ __global__ void __launch_bounds__(256) k_search_template(
     const int bxi = b % g.bx, byi = (b / g.bx) % g.by, bzi = b / (g.bx * g.by);
     const int x0 = bxi * g.rx, y0 = byi * g.ry, z0 = bzi * g.rz;
     if (x0 >= g.nx || y0 >= g.ny || z0 >= g.nz) return;
+    if (min_cand >= 0)
+    {
+        int cand = 0;
+        const int q = threadIdx.x & 31, kk = bzi - 1 + q / 9, jj = byi - 1 + (q / 3) % 3, ii = bxi - 1 + q % 3;
+        if (q < 27 && ii >= 0 && jj >= 0 && kk >= 0 && ii < g.bx && jj < g.by && kk < g.bz)
+            cand = bin_cnt[(kk * g.by + jj) * g.bx + ii];
+        if (__reduce_add_sync(0xffffffffu, cand) <= min_cand) return;
+    }
     const int wx = min(x0 + g.rx, g.nx) - x0, wy = min(y0 + g.ry, g.ny) - y0, wz = min(z0 + g.rz, g.nz) - z0;
     const int lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     const int warp = blockIdx.y * nwarps + (threadIdx.x >> 5);
@@ -1519,25 +1629,55 @@ int template_padded_offset(const Geom &g, int dx, int dy, int dz)
     return (int)(((long long)dz * PY + dy) * PX + dx);
 }
 
+// the template scan of listed cells, a warp a cell
+__global__ void __launch_bounds__(256) k_search_template_list(
+    const Geom g, const uint32_t *__restrict__ bits, int hx, int hy, int hz, const int *__restrict__ list,
+    const int *__restrict__ n_list, const float *__restrict__ pts_vf, const int4 *__restrict__ tmpl, int n_tmpl,
+    const int *__restrict__ pid_of_node, int *__restrict__ nb_pid, int2 *__restrict__ nb_rec, int *__restrict__ nb_n)
+{
+    const int lane = threadIdx.x & 31, n = *n_list;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += gridDim.x * blockDim.x >> 5)
+    {
+        const int cell = list[i];
+        template_cell(g, bits, hx, hy, hz, cell % g.nx, cell / g.nx % g.ny, cell / g.nx / g.ny, cell, lane, pts_vf,
+                      tmpl, n_tmpl, pid_of_node, nb_pid, nb_rec, nb_n);
+    }
+}
+
+static void launch_mask_bits(const Geom &g, const uint8_t *mask, uint32_t *bits, int n_sm, cudaStream_t st)
+{
+    const long long n_padded = template_padded_cells(g);
+    const int blocks = (int)std::min<long long>((n_padded + 255) / 256, (long long)n_sm * 16);
+    k_mask_bits_padded<<<blocks, 256, 0, st>>>(g, mask, g.rx, g.ry, g.rz, n_padded, bits);
+}
+
+cudaError_t launch_search_template_list(const Geom &g, const uint8_t *mask, uint32_t *bits, const int *list,
+                                        const int *n_list, const float *pts_vf, const int4 *tmpl, int n_tmpl,
+                                        const int *pid_of_node, int *nb_pid, int2 *nb_rec, int *nb_n, int n_sm,
+                                        cudaStream_t st)
+{
+    launch_mask_bits(g, mask, bits, n_sm, st);
+    k_search_template_list<<<n_sm * 8, 256, 0, st>>>(g, bits, g.rx, g.ry, g.rz, list, n_list, pts_vf, tmpl, n_tmpl,
+                                                     pid_of_node, nb_pid, nb_rec, nb_n);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_search_template(const Geom &g, const uint8_t *mask, uint32_t *bits, int all_cells,
-                                   const int *tmpl_bins, int n_tmpl_bins, const float *pts_vf, const int4 *tmpl,
-                                   int n_tmpl, const int *pid_of_node, int *nb_pid, int2 *nb_rec, int *nb_n,
-                                   int *n_template_cells, int n_sm, cudaStream_t st)
+                                   const int *tmpl_bins, int n_tmpl_bins, const int *bin_cnt, int min_cand,
+                                   const float *pts_vf, const int4 *tmpl, int n_tmpl, const int *pid_of_node,
+                                   int *nb_pid, int2 *nb_rec, int *nb_n, int *n_template_cells, int n_sm,
+                                   cudaStream_t st)
 {
     if (n_tmpl_bins <= 0) return cudaSuccess;
-    {
-        const long long n_padded = template_padded_cells(g);
-        const int blocks = (int)std::min<long long>((n_padded + 255) / 256, (long long)n_sm * 16);
-        k_mask_bits_padded<<<blocks, 256, 0, st>>>(g, mask, g.rx, g.ry, g.rz, n_padded, bits);
-    }
+    launch_mask_bits(g, mask, bits, n_sm, st);
     // about four waves of 256-thread blocks, at most one warp per 32 cells of a bin
     const long long cells = (long long)g.rx * g.ry * g.rz;
     long long split = ((long long)4 * n_sm * 8 + n_tmpl_bins - 1) / n_tmpl_bins;
     split = std::min(split, std::max(1LL, cells / (8 * 32)));
     split = std::max(1LL, std::min(split, 65535LL));
     dim3 grid((unsigned)n_tmpl_bins, (unsigned)split);
-    k_search_template<<<grid, 256, 0, st>>>(g, bits, g.rx, g.ry, g.rz, mask, all_cells, tmpl_bins, pts_vf, tmpl,
-                                            n_tmpl, pid_of_node, nb_pid, nb_rec, nb_n, n_template_cells);
+    k_search_template<<<grid, 256, 0, st>>>(g, bits, g.rx, g.ry, g.rz, mask, all_cells, tmpl_bins, bin_cnt, min_cand,
+                                            pts_vf, tmpl, n_tmpl, pid_of_node, nb_pid, nb_rec, nb_n, n_template_cells);
     return cudaGetLastError();
 }
 

@@ -1,0 +1,478 @@
+// Neighbour selection, one cell a lane (the set of the reference's lookups; see
+// search.cu for the warp-per-cell forms, which order the neighbours by key).
+#include "engine.cuh"
+#include "kernels.h"
+#include "search_common.cuh"
+
+#include <algorithm>
+#include <cstdint>
+#include <cuda_runtime.h>
+
+namespace hb
+{
+// One cell by exact ranks over all C candidates, without scratch: the smallest
+// rank with k candidates up to it by bisection, then those candidates in their
+// order. Returns the neighbour count, or -1 for a tie group across the k-th slot.
+__device__ int exact_select(const Geom &g, int C, const float4 *ctp, const int2 *crec, int kofs, int plin_c,
+                            const uint16_t *__restrict__ keytab, int lane, int2 *out_rec)
+{
+    const int k = g.k;
+    auto count = [&](int top) {
+        int c = 0;
+        for (int i = lane; i < C; i += 32) c += (int)keytab[kofs + __float_as_int(ctp[i].w)] <= top;
+        return __reduce_add_sync(0xffffffffu, c);
+    };
+    int lo = -1, hi = 0xFFFE; // kept ranks stay below 0xFFFF
+    const int kept = count(hi);
+    int at = kept;
+    if (kept > k)
+        while (at != k)
+        {
+            if (hi - lo == 1) return -1;
+            const int mid = (lo + hi) >> 1;
+            const int c = count(mid);
+            if (c >= k)
+            {
+                hi = mid;
+                at = c;
+            }
+            else
+                lo = mid;
+        }
+    int done = 0;
+    for (int base = 0; base < C; base += 32)
+    {
+        const int i = base + lane;
+        const bool in = i < C && (int)keytab[kofs + __float_as_int(ctp[i < C ? i : 0].w)] <= hi;
+        const unsigned bl = __ballot_sync(0xffffffffu, in);
+        if (in) out_rec[done + __popc(bl & lanemask_lt())] = make_int2(crec[i].x - plin_c, crec[i].y);
+        done += __popc(bl);
+    }
+    return done;
+}
+
+// ---- the same selection, one cell a lane
+//
+// A warp takes a tile of 32 cells of a bin (a few cells in each direction, so
+// that their neighbourhoods nearly coincide) and lists the candidates near the
+// tile once; each lane then scans that list for its own cell, keeps the
+// candidates inside its radius, reads their exact ranks, finds the k-th by
+// counting, and decides as select_surr does, with the same bounds. A cell's work
+// is about a tenth of the warp-per-cell form's (whose every step costs a warp
+// instruction for one cell). Lanes whose radius was a bad guess repeat the scan
+// with another; what is undecided after kTileTries goes through select_fast.
+// Neighbours are written in candidate order.
+constexpr int kTileTries = 8;
+constexpr int kManyCandidates = 1024; // candidates of a bin away from data clusters
+
+struct SearchTile
+{
+    int ty, tz;  // rows and layers of a tile (32 / (ty tz) cells along x)
+    int cap;     // survivors a lane keeps
+    int sub;     // candidates near a tile, at most (beyond: all are scanned)
+    int slices;  // blocks per bin
+    int c_min, c_max; // the bins of this launch: c_min < candidates <= c_max
+};
+
+__global__ void __launch_bounds__(256) k_search_tile(
+    const Geom g, const uint8_t *__restrict__ mask, int all_cells, const int *__restrict__ bin_start,
+    const int *__restrict__ bin_cnt, const uint8_t *__restrict__ bin_flag, const int *__restrict__ bin_pts,
+    const unsigned long long *__restrict__ pts_xyz, const float *__restrict__ pts_vf,
+    const uint16_t *__restrict__ keytab, const SurrDev sd, const SearchTile tl, int template_bins, int cand_cap,
+    int2 *__restrict__ nb_rec, int *__restrict__ nb_n, int *__restrict__ tie_cells, int *__restrict__ tie_count,
+    int *__restrict__ n_template_cells, int *__restrict__ exact_cells)
+{
+    constexpr unsigned FULL = 0xffffffffu;
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int b = blockIdx.x / tl.slices, slice = blockIdx.x % tl.slices;
+    const int bxi = b % g.bx, byi = (b / g.bx) % g.by, bzi = b / (g.bx * g.by);
+    const int x0 = bxi * g.rx, y0 = byi * g.ry, z0 = bzi * g.rz;
+    if (x0 >= g.nx || y0 >= g.ny || z0 >= g.nz) return;
+    if (((bin_flag[b] >> 1) & 1) != template_bins) return;
+    const int wx = min(g.rx, g.nx - x0), wy = min(g.ry, g.ny - y0), wz = min(g.rz, g.nz - z0);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int k = g.k, cap = tl.cap, ld = blockDim.x + 1;
+
+    float4 *ctp = reinterpret_cast<float4 *>(smem);
+    int2 *crec = reinterpret_cast<int2 *>(ctp + cand_cap); // pair-table offset from the bin corner, value
+    uint32_t *lists = reinterpret_cast<uint32_t *>(crec + cand_cap); // [cap][threads + 1]
+    uint32_t *list = lists + threadIdx.x;
+    uint16_t *sub = reinterpret_cast<uint16_t *>(lists + (size_t)cap * ld) + warp * tl.sub;
+
+    __shared__ int s_off[28];
+    if (threadIdx.x < 32)
+    {
+        // candidates of the 27 bins around, in the reference's order
+        const int q = threadIdx.x;
+        const int kk = bzi - 1 + q / 9, jj = byi - 1 + (q / 3) % 3, ii = bxi - 1 + q % 3;
+        const bool in = q < 27 && ii >= 0 && jj >= 0 && kk >= 0 && ii < g.bx && jj < g.by && kk < g.bz;
+        const int cnt = in ? bin_cnt[(kk * g.by + jj) * g.bx + ii] : 0;
+        int run = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            const int v = __shfl_up_sync(FULL, run, o);
+            if (q >= o) run += v;
+        }
+        if (q < 28) s_off[q] = run - cnt;
+    }
+    __syncthreads();
+    const int C = s_off[27];
+    if (C <= tl.c_min || C > tl.c_max) return;
+    for (int q = 0; q < 27; ++q)
+    {
+        const int cnt = s_off[q + 1] - s_off[q];
+        if (cnt == 0) continue;
+        const int kk = bzi - 1 + q / 9, jj = byi - 1 + (q / 3) % 3, ii = bxi - 1 + q % 3;
+        const int s = bin_start[(kk * g.by + jj) * g.bx + ii];
+        for (int i = threadIdx.x; i < cnt; i += blockDim.x)
+        {
+            const int p = bin_pts[s + i];
+            int px, py, pz;
+            unpack_xyz(pts_xyz[p], px, py, pz);
+            const int d = s_off[q] + i;
+            // float coordinates, and the offset into the key table from the bin corner
+            float4 c = surr_coords(sd, px - x0, py - y0, pz - z0);
+            c.w = __int_as_float(((pz - z0) * g.kny + (py - y0)) * g.knx + (px - x0));
+            ctp[d] = c;
+            crec[d] = make_int2(pair_lin(g, px - x0, py - y0, pz - z0), __float_as_int(pts_vf[p]));
+        }
+    }
+    __syncthreads();
+    const int kc0 = (g.khz * g.kny + g.khy) * g.knx + g.khx;
+    const float e3 = (float)sd.e3 * (1.0f + 1e-6f) + 1e-30f;
+    const float r_all = (float)(sd.h_cut * (1.0 + 1e-5) + 4.0 * sd.e3); // decides every candidate
+    // radius that holds 1.25 k of C candidates spread over 27 bins
+    float guess = cbrtf(1.25f * (float)k * 27.0f * (float)g.rx * (float)g.ry * (float)g.rz / (4.18879f * (float)max(C, 1)) *
+                        sd.step[0] * sd.step[1] * sd.step[2]);
+
+    const int ny_s = (wy + tl.ty - 1) / tl.ty, nz_s = (wz + tl.tz - 1) / tl.tz;
+    const int parts = (wx * min(tl.ty, wy) * min(tl.tz, wz) + 31) / 32;
+    const int n_tiles = ny_s * nz_s * parts;
+    const int per = (n_tiles + tl.slices * nwarps - 1) / (tl.slices * nwarps);
+    const int t0 = (slice * nwarps + warp) * per, t1 = min(t0 + per, n_tiles);
+    int n_exact = 0, n_done = 0;
+    for (int tile = t0; tile < t1; ++tile)
+    {
+        // ---- the lane's cell: rows and layers fastest, then x
+        const int part = tile % parts, ys = tile / parts % ny_s, zs = tile / parts / ny_s;
+        const int hy = min(tl.ty, wy - ys * tl.ty), hz = min(tl.tz, wz - zs * tl.tz);
+        const int t = part * 32 + lane, col = hy * hz;
+        const int cxr = min(t / col, wx - 1), cyr = ys * tl.ty + t % col % hy, czr = zs * tl.tz + t % col / hy;
+        const long long cell = ((long long)(z0 + czr) * g.ny + (y0 + cyr)) * g.nx + (x0 + cxr);
+        bool open = t < col * wx && (all_cells || !mask[cell]);
+        if (!__any_sync(FULL, open)) continue;
+        n_done += __popc(__ballot_sync(FULL, open));
+        const float4 tc = surr_coords(sd, cxr, cyr, czr);
+        const int klin_c = (czr * g.kny + cyr) * g.knx + cxr;
+        // the tile's centre and the lane's distance from it
+        float ccx, ccy, ccz, dc;
+        {
+            const float4 c0 = make_float4(__shfl_sync(FULL, tc.x, 0), __shfl_sync(FULL, tc.y, 0),
+                                          __shfl_sync(FULL, tc.z, 0), 0.0f);
+            const float4 c1 = make_float4(__shfl_sync(FULL, tc.x, 31), __shfl_sync(FULL, tc.y, 31),
+                                          __shfl_sync(FULL, tc.z, 31), 0.0f);
+            ccx = 0.5f * (c0.x + c1.x);
+            ccy = 0.5f * (c0.y + c1.y);
+            ccz = 0.5f * (c0.z + c1.z);
+            const float dx = tc.x - ccx, dy = tc.y - ccy, dz = tc.z - ccz;
+            dc = sqrtf(fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
+        }
+        // the lane's radius: known to keep fewer than k at lo_r, more than cap at hi_r
+        float rt = fminf(guess, r_all), lo_r = 0.0f, hi_r = 0.0f, H = 0.0f;
+        float lo_c = 0.0f, hi_c = 0.0f, have = -1.0f; // have: reach of the list in `sub`
+        int n = -2, n_sub = 0;
+        bool all = false;
+        for (int tries = 0; tries < kTileTries; ++tries)
+        {
+            // ---- candidates within reach of any open lane: every candidate whose float
+            // distance from the centre exceeds R is truly farther than R - e3 - rounding
+            // from it, so farther than rt + e3 from a lane's cell at dc + e3 from it
+            float reach = open ? (rt + dc) * (1.0f + 1e-5f) + 4.0f * e3 : 0.0f;
+            reach = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(reach)));
+            if (reach > have)
+            {
+                have = reach;
+                const float R2 = reach * reach * (1.0f + 1e-5f);
+                n_sub = 0;
+                __syncwarp();
+                for (int base = 0; base < C; base += 32)
+                {
+                    const int i = base + lane;
+                    bool in = false;
+                    if (i < C)
+                    {
+                        const float4 c = ctp[i];
+                        const float dx = c.x - ccx, dy = c.y - ccy, dz = c.z - ccz;
+                        in = fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= R2;
+                    }
+                    const unsigned bl = __ballot_sync(FULL, in);
+                    const int at = n_sub + __popc(bl & lanemask_lt());
+                    if (in && at < tl.sub) sub[at] = (uint16_t)i;
+                    n_sub += __popc(bl);
+                }
+                all = n_sub > tl.sub;
+                if (all) n_sub = C;
+                __syncwarp();
+            }
+            // ---- the lane's scan
+            const float Tg = __fmul_ru(__fmul_ru(rt, rt), 1.0f + 1e-6f);
+            int cnt = open ? 0 : cap + 1;
+#pragma unroll 4
+            for (int j = 0; j < n_sub; ++j)
+            {
+                const int i = all ? j : (int)sub[j];
+                const float4 c = ctp[i];
+                const float qx = c.x - tc.x, qy = c.y - tc.y, qz = c.z - tc.z;
+                if (fmaf(qz, qz, fmaf(qy, qy, qx * qx)) <= Tg)
+                {
+                    if (cnt < cap) list[cnt * ld] = (uint32_t)i;
+                    ++cnt;
+                }
+            }
+            // ---- the lane's decision
+            if (open)
+            {
+                const bool few = cnt < k && rt < r_all;
+                if (few)
+                {
+                    lo_r = rt;
+                    lo_c = (float)cnt;
+                }
+                else if (cnt > cap)
+                {
+                    hi_r = rt;
+                    hi_c = (float)cnt;
+                }
+                if (few || cnt > cap)
+                {
+                    // between both bounds by their counts, else by the volume
+                    const float goal = 0.5f * (float)(k + cap);
+                    if (lo_r > 0.0f && hi_r > 0.0f)
+                        rt = lo_r + (hi_r - lo_r) * fminf(fmaxf((goal - lo_c) / (hi_c - lo_c), 0.1f), 0.9f);
+                    else if (few)
+                        rt = fminf(rt * fminf(cbrtf(goal / fmaxf((float)cnt, 0.25f)) + 0.01f, 2.0f) + e3, r_all);
+                    else
+                        rt = rt * fmaxf(cbrtf(goal / (float)cnt), 0.7f);
+                }
+                else
+                {
+                    int nk = 0, rmin = 0x10000, rmax = -1;
+                    for (int e = 0; e < cnt; ++e)
+                    {
+                        const uint32_t pos = list[e * ld];
+                        const int r16 = keytab[kc0 - klin_c + __float_as_int(ctp[pos].w)];
+                        if (r16 != 0xFFFF)
+                        {
+                            list[nk * ld] = ((uint32_t)r16 << 16) | pos;
+                            ++nk;
+                            rmin = min(rmin, r16);
+                            rmax = max(rmax, r16);
+                        }
+                    }
+                    if (nk < k && rt < r_all)
+                    {
+                        rt = r_all; // survivors without a rank: the kept offsets end near here
+                    }
+                    else
+                    {
+                        // smallest rank T with k survivors up to it, by interpolating counts
+                        // (clo below k up to lo, chi above k up to hi); a rank that holds the
+                        // k-th and the (k+1)-th is a tie across the last slot
+                        int T = rmax;
+                        bool tie = false;
+                        if (nk > k)
+                        {
+                            int lo = rmin - 1, hi = rmax, clo = 0, chi = nk;
+                            for (int it = 0;; ++it)
+                            {
+                                if (hi - lo == 1)
+                                {
+                                    T = hi;
+                                    tie = true;
+                                    break;
+                                }
+                                int mid = (it & 3) == 3 ? (lo + hi) >> 1
+                                                      : lo + (int)((float)(hi - lo) * ((float)(k - clo) + 0.5f) /
+                                                                   ((float)(chi - clo) + 0.5f));
+                                mid = min(max(mid, lo + 1), hi - 1);
+                                const uint32_t top = ((uint32_t)mid << 16) | 0xFFFFu;
+                                int c = 0;
+                                for (int e = 0; e < nk; ++e) c += list[e * ld] <= top;
+                                if (c == k)
+                                {
+                                    T = mid;
+                                    break;
+                                }
+                                if (c < k)
+                                {
+                                    lo = mid;
+                                    clo = c;
+                                }
+                                else
+                                {
+                                    hi = mid;
+                                    chi = c;
+                                }
+                            }
+                            // in place, the survivors up to T
+                            const uint32_t top = ((uint32_t)T << 16) | 0xFFFFu;
+                            int w = 0, last = 0;
+                            for (int e = 0; e < nk; ++e)
+                            {
+                                const uint32_t key = list[e * ld];
+                                if (key <= top)
+                                {
+                                    last = max(last, (int)(key >> 16));
+                                    list[w * ld] = key;
+                                    ++w;
+                                }
+                            }
+                            T = last;
+                        }
+                        H = __double2float_ru(nk >= k ? sd.h_rank[T] : sd.h_cut);
+                        if ((rt - e3) * (1.0f - 1e-6f) > H)
+                        {
+                            n = tie ? -1 : min(nk, k);
+                            open = false;
+                        }
+                        else
+                            rt = fminf(H * (1.0f + 4e-6f) + 3.0f * e3, r_all);
+                    }
+                }
+            }
+            if (!__any_sync(FULL, open)) break;
+        }
+        const bool mine = t < col * wx && (n != -2 || open);
+        // ---- the next tile's radius: the largest k-th distance of this one
+        {
+            const float h = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(n != -2 ? H : 0.0f)));
+            if (h > 0.0f) guess = h * 1.02f + e3;
+        }
+        // ---- write the decided cells' neighbours, a cell at a time
+        __syncwarp();
+        for (unsigned todo = __ballot_sync(FULL, mine && n >= 0); todo; todo &= todo - 1)
+        {
+            const int src = __ffs(todo) - 1;
+            const int ns = __shfl_sync(FULL, n, src);
+            const long long cs = __shfl_sync(FULL, cell, src);
+            const int pl = __shfl_sync(FULL, pair_lin(g, cxr, cyr, czr), src);
+            for (int e = lane; e < ns; e += 32)
+            {
+                const int2 rec = crec[lists[e * ld + warp * 32 + src] & 0xFFFFu];
+                nb_rec[cs * k + e] = make_int2(rec.x - pl, rec.y);
+            }
+        }
+        // ---- undecided cells: by exact ranks over every candidate
+        __syncwarp();
+        for (unsigned todo = __ballot_sync(FULL, open); todo; todo &= todo - 1)
+        {
+            const int src = __ffs(todo) - 1;
+            const int r = exact_select(g, C, ctp, crec, kc0 - __shfl_sync(FULL, klin_c, src),
+                                       __shfl_sync(FULL, pair_lin(g, cxr, cyr, czr), src), keytab, lane,
+                                       nb_rec + __shfl_sync(FULL, cell, src) * k);
+            if (lane == src) n = r;
+            ++n_exact;
+        }
+        if (mine)
+        {
+            nb_n[cell] = n < 0 ? k : n;
+            if (n < 0) tie_cells[atomicAdd(tie_count, 1)] = (int)cell;
+        }
+    }
+    if (exact_cells && lane == 0 && n_exact) atomicAdd(exact_cells, n_exact);
+    if (template_bins && n_template_cells && lane == 0 && n_done) atomicAdd(n_template_cells, n_done);
+}
+
+// survivors a lane keeps, for k neighbours
+static int tile_cap(int k) { return k + std::max(12, k * 3 / 8 + 4); }
+static size_t tile_smem(int cand_cap, int cap, int sub, int warps)
+{
+    return (size_t)cand_cap * 24 + (size_t)cap * (warps * 32 + 1) * 4 + (size_t)warps * sub * 2;
+}
+
+// Shape of k_search_tile for a search: the tile of 32 cells with the least extent
+// in transformed coordinates, room for three eighths more survivors than
+// neighbours, and the block size for the most warps on an SM; warps 0 when the candidates
+// leave no room.
+static SearchTile search_tile_shape(const Geom &g, const SurrDev &sd, int n_bins, int cand_cap, int max_smem, int &warps,
+                                    size_t &smem)
+{
+    SearchTile t{1, 1, tile_cap(g.k), cand_cap <= kManyCandidates ? 256 : 1024, 1, 0, cand_cap};
+    float best = 3.4e38f;
+    for (int ty = 1; ty <= 32; ty *= 2)
+        for (int tz = 1; ty * tz <= 32; tz *= 2)
+        {
+            if ((ty > 1 && ty > g.ry) || (tz > 1 && tz > g.rz)) continue;
+            const float ex = sd.step[0] * (float)std::min(32 / (ty * tz), g.rx), ey = sd.step[1] * ty,
+                        ez = sd.step[2] * tz;
+            const float e = ex * ex + ey * ey + ez * ez;
+            if (e < best)
+            {
+                best = e;
+                t.ty = ty;
+                t.tz = tz;
+            }
+        }
+    const long long tiles = ((long long)g.rx * g.ry * g.rz + 31) / 32;
+    // bins with many candidates leave room for few warps a block, and there may be few
+    // bins: more blocks each, down to eight tiles a block
+    const long long fill = (3552 + n_bins - 1) / n_bins;
+    t.slices = (int)std::max<long long>(
+        1, std::min(tiles / 8, std::max(tiles / (cand_cap > kManyCandidates ? 16 : 128), fill)));
+    // the block size that keeps most warps on an SM (24 at most: 80 registers a thread)
+    int most = 0;
+    warps = 0;
+    for (int w = 8; w > 0; --w)
+    {
+        const size_t need = tile_smem(cand_cap, t.cap, t.sub, w);
+        if (need > (size_t)max_smem) continue;
+        const int resident = std::min(24 / w, (int)(228 * 1024 / (need + 1024))) * w;
+        if (resident > most)
+        {
+            most = resident;
+            warps = w;
+            smem = need;
+        }
+    }
+    return t;
+}
+
+// Candidates per bin that k_search_tile takes at most, at k neighbours.
+int search_tile_limit(int k, int max_smem)
+{
+    const long long room = (long long)max_smem - (long long)tile_smem(0, tile_cap(k), 1024, 1);
+    return (int)std::max(0LL, std::min(room / 24 / 4 * 4, 65536LL));
+}
+
+cudaError_t launch_search_tile(const Geom &g, const uint8_t *mask, int all_cells, const int *bin_start,
+                               const int *bin_cnt, const uint8_t *bin_flag, const int *bin_pts,
+                               const unsigned long long *pts_xyz, const float *pts_vf, const uint16_t *keytab16,
+                               const SurrDev &sd, int template_bins, int n_bins, int cand_cap, int max_smem, int2 *nb_rec,
+                               int *nb_n, int *tie_cells, int *tie_count, int *n_template_cells, int *exact_cells,
+                               cudaStream_t st)
+{
+    cand_cap = std::min(cand_cap, search_tile_limit(g.k, max_smem));
+    if (cand_cap <= 0) return cudaErrorInvalidValue;
+    cudaError_t e = cudaFuncSetAttribute(k_search_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+    if (e != cudaSuccess) return e;
+    // the bins around data clusters in launches of their own: their candidates would
+    // take the shared memory of every other bin's block too
+    for (int c_min = -1, c_max = std::min(cand_cap, kManyCandidates);;)
+    {
+        int warps = 0;
+        size_t smem = 0;
+        SearchTile tl = search_tile_shape(g, sd, n_bins, c_max, max_smem, warps, smem);
+        if (warps <= 0) return cudaErrorInvalidValue;
+        tl.c_min = c_min;
+        tl.c_max = c_max;
+        k_search_tile<<<(unsigned)((long long)g.n_bins * tl.slices), warps * 32, smem, st>>>(
+            g, mask, all_cells, bin_start, bin_cnt, bin_flag, bin_pts, pts_xyz, pts_vf, keytab16, sd, tl, template_bins,
+            c_max, nb_rec, nb_n, tie_cells, tie_count, n_template_cells, exact_cells);
+        if (c_max == cand_cap) break;
+        c_min = c_max;
+        c_max = std::min(cand_cap, 3 * c_max);
+    }
+    return cudaGetLastError();
+}
+} // namespace hb
