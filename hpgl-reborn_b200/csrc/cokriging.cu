@@ -13,8 +13,8 @@
 // (gauss_solver.cpp:8-70), which processes the border last. The result is
 // combine()'s float accumulation (simple_cokriging_markI.cpp:83-106).
 #include "engine.cuh"
-#include "fold32.cuh"
 #include "kernels.h"
+#include "warp64.cuh"
 
 #include <algorithm>
 #include <cfloat>
@@ -87,89 +87,78 @@ __device__ __forceinline__ void cok_write(const CokArgsDev &a, int cell, int sta
     if (a.status) a.status[cell] = (signed char)status;
 }
 
-// n <= 32: two targets per warp in the folded layout
-constexpr int kCokThreads = 256;
+// n <= 32: a target per warp on the FP64 tensor instruction (warp64.cuh), b and
+// the cross covariances as its two right-hand sides. 20 warps of 96 registers an
+// SM; two targets per warp in folded rows, 8 warps an SM, took 12.3 ms for the
+// 1.82M targets of a 160x144x80 grid with 32 neighbours; this takes 7.8.
+constexpr int kCokThreads = 640;
 
-// BOUND (k < 32): the factorisation stops at the warp's largest system
-template <bool BOUND>
-__global__ void __launch_bounds__(kCokThreads, 1) k_cok_solve_fold(const CokArgsDev a)
+__global__ void __launch_bounds__(kCokThreads, 1) k_cok_solve_warp(const CokArgsDev a)
 {
-    constexpr int NP = kFold32NP, G = kFold32G;
+    constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ __align__(16) unsigned char smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const int h = lane / G, t = lane % G, rb = NP - 1 - t;
-    const unsigned gm = 0xFFFFu << (h * G);
-    unsigned char *gb = smem + kFold32SysBytes * (warp * 2 + h);
-    double *M = reinterpret_cast<double *>(gb);
-    int *LIN = reinterpret_cast<int *>(gb + kFold32MBytes);
+    const int lane = threadIdx.x & 31;
+    WarpSmem<2, false> &T = reinterpret_cast<WarpSmem<2, false> *>(smem)[threadIdx.x >> 5];
     const Geom &g = a.g;
-    const long long pc = g.pair_center;
-    const int stride = gridDim.x * nwarps * 2;
-    for (int it0 = (blockIdx.x * nwarps + warp) * 2; it0 < a.n_targets; it0 += stride)
+    const double *pair_c = a.pair64 + g.pair_center;
+    const int stride = gridDim.x * (kCokThreads / 32);
+    // the next target's record is loaded during the current solve
+    int it = blockIdx.x * (kCokThreads / 32) + (threadIdx.x >> 5);
+    int cell = 0, n = 0, ncell = 0, nn = 0;
+    int2 rec = make_int2(0, 0);
+    auto load = [&](int c, int m) { return lane < m ? a.nb_rec[(long long)c * a.k + lane] : make_int2(0, 0); };
+    if (it < a.n_targets)
     {
-        const int it = it0 + h;
-        const bool valid = it < a.n_targets;
-        const int cell = valid ? a.targets[it] : 0;
-        const int n = valid ? a.nb_n[cell] : 0;
-        const bool live_a = t < n, live_b = rb < n;
-        int lin_a = 0, lin_b = 0;
-        float va = 0.0f, vb = 0.0f;
-        double c_a = 0.0, c_b = 0.0;
-        if (live_a)
+        cell = a.targets[it];
+        n = a.nb_n[cell];
+        rec = load(cell, n);
+    }
+    if (it + stride < a.n_targets) ncell = a.targets[it + stride];
+    for (; it < a.n_targets; it += stride)
+    {
+        const int lin = rec.x;
+        double b = 0.0, c = 0.0;
+        if (lane < n)
         {
-            const int2 rec = a.nb_rec[(long long)cell * a.k + t];
-            lin_a = rec.x;
-            va = __int_as_float(rec.y);
-            c_a = __dmul_rn(a.p.coef, a.cross_tab[cross_index_of_lin(g, lin_a)]);
+            b = __ldg(pair_c + abs(lin));
+            c = __dmul_rn(a.p.coef, a.cross_tab[cross_index_of_lin(g, lin)]);
         }
-        if (live_b)
-        {
-            const int2 rec = a.nb_rec[(long long)cell * a.k + rb];
-            lin_b = rec.x;
-            vb = __int_as_float(rec.y);
-            c_b = __dmul_rn(a.p.coef, a.cross_tab[cross_index_of_lin(g, lin_b)]);
-        }
-        const float sv = valid ? (a.smask[cell] ? a.sdata[cell] : a.p.sm) : 0.0f;
-        LIN[t] = lin_a;
-        LIN[rb] = lin_b;
-        __syncwarp(gm);
-        double b_a = 0.0, b_b = 0.0, xa[2], xb[2];
-        auto load_rhs = [&](double(&rhs_a)[2], double(&rhs_b)[2]) {
-            b_a = live_a ? __ldg(a.pair64 + pc + lin_a) : 0.0;
-            b_b = live_b ? __ldg(a.pair64 + pc + lin_b) : 0.0;
-            rhs_a[0] = b_a;
-            rhs_a[1] = c_a;
-            rhs_b[0] = b_b;
-            rhs_b[1] = c_b;
-        };
-        const int nmax = BOUND ? __reduce_max_sync(0xffffffffu, n) : NP; // both targets of the warp
-        const bool fail = fold32_solve<2, true>(a.pair64 + pc, LIN, M, gm, t, live_a, live_b, lin_a, lin_b, load_rhs,
-                                                xa, xb, [] {}, [] {}, nullptr, 1.0, 1.0, nmax);
+        const float v = __int_as_float(rec.y);
+        const float sv = a.smask[cell] ? a.sdata[cell] : a.p.sm;
+        T.lin[lane] = lin;
+        T.y[0][lane] = b;
+        T.y[1][lane] = c;
+        __syncwarp();
+        const int nb = (n + 7) >> 3;
+        nn = it + stride < a.n_targets ? a.nb_n[ncell] : 0;
+        const bool fail = warp_factor<2, true, false>(T, lane, n, nb, pair_c);
+        rec = load(ncell, nn);
+        warp_back<2>(T, lane, nb);
+        const double x = lane < n ? T.y[0][lane] : 0.0, y = lane < n ? T.y[1][lane] : 0.0;
         // the border: wn = (b_n - c.x) / (s - c.y)
-        double cx_ = c_a * xa[0] + c_b * xb[0], cy_ = c_a * xa[1] + c_b * xb[1];
+        double cx = c * x, cy = c * y;
 #pragma unroll
-        for (int o = G / 2; o > 0; o >>= 1)
+        for (int o = 16; o > 0; o >>= 1)
         {
-            cx_ += __shfl_xor_sync(gm, cx_, o, G);
-            cy_ += __shfl_xor_sync(gm, cy_, o, G);
+            cx += __shfl_xor_sync(FULL, cx, o);
+            cy += __shfl_xor_sync(FULL, cy, o);
         }
-        const double piv = a.p.sec_var - cy_;
+        const double piv = a.p.sec_var - cy;
         const bool bad = fail || !(fabs(piv) >= DBL_EPSILON);
-        const double wn = bad ? 0.0 : (a.p.b_last - cx_) / piv;
+        const double wn = bad ? 0.0 : (a.p.b_last - cx) / piv;
         // combine: result accumulated in double per term, stored as float
-        const double ta = __dmul_rn((double)__fsub_rn(va, a.p.pm), __dsub_rn(xa[0], __dmul_rn(wn, xa[1])));
-        const double tb = __dmul_rn((double)__fsub_rn(vb, a.p.pm), __dsub_rn(xb[0], __dmul_rn(wn, xb[1])));
+        __syncwarp();
+        T.y[0][lane] = __dmul_rn((double)__fsub_rn(v, a.p.pm), __dsub_rn(x, __dmul_rn(wn, y)));
+        __syncwarp();
         float result = a.p.pm;
 #pragma unroll 4
-        for (int i = 0; i < NP; ++i)
-        {
-            const bool lo = i < G;
-            const double ti = __shfl_sync(gm, lo ? ta : tb, lo ? i : NP - 1 - i, G);
-            if (i < n) result = __double2float_rn(__dadd_rn((double)result, ti));
-        }
+        for (int i = 0; i < n; ++i) result = __double2float_rn(__dadd_rn((double)result, T.y[0][i]));
         result = __double2float_rn(__dadd_rn((double)result, __dmul_rn(wn, (double)__fsub_rn(sv, a.p.sm))));
-        if (valid && t == 0) cok_write(a, cell, n == 0 ? 1 : (bad ? 2 : 0), result, sv);
-        __syncwarp(gm);
+        if (lane == 0) cok_write(a, cell, n == 0 ? 1 : (bad ? 2 : 0), result, sv);
+        cell = ncell;
+        n = nn;
+        ncell = it + 2 * stride < a.n_targets ? a.targets[it + 2 * stride] : 0;
+        __syncwarp();
     }
 }
 
@@ -297,14 +286,12 @@ cudaError_t launch_cok_solve(const Geom &g, const int *targets, int n_targets, c
                  status};
     if (k <= 32)
     {
-        const int spb = kCokThreads / kFold32G;
-        const size_t smem = kFold32SysBytes * spb;
-        auto kern = k < 32 ? k_cok_solve_fold<true> : k_cok_solve_fold<false>;
+        constexpr int warps = kCokThreads / 32;
+        const size_t smem = sizeof(WarpSmem<2, false>) * warps;
         int per_sm = 0;
-        cudaError_t e = set_smem_min_carveout(kern, kCokThreads, smem, per_sm);
+        cudaError_t e = set_smem_min_carveout(k_cok_solve_warp, kCokThreads, smem, per_sm);
         if (e != cudaSuccess) return e;
-        const int blocks = std::min((n_targets + spb - 1) / spb, n_sm);
-        kern<<<blocks, kCokThreads, smem, st>>>(a);
+        k_cok_solve_warp<<<std::min((n_targets + warps - 1) / warps, n_sm), kCokThreads, smem, st>>>(a);
     }
     else
     {

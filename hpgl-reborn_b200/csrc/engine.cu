@@ -76,6 +76,7 @@ class Engine
     {
         HB_CK(cudaSetDevice(dev));
         HB_CK(cudaStreamCreateWithFlags(&own_stream_, cudaStreamNonBlocking));
+        HB_CK(cudaStreamCreateWithFlags(&aux_stream_, cudaStreamNonBlocking));
         cudaDeviceProp prop;
         HB_CK(cudaGetDeviceProperties(&prop, dev));
         n_sm_ = prop.multiProcessorCount;
@@ -100,6 +101,22 @@ class Engine
             b.cap = want;
         }
         return reinterpret_cast<T *>(b.p);
+    }
+
+    // buf, or null when the device has no room for it
+    template <typename T>
+    T *try_buf(const char *name, size_t count)
+    {
+        try
+        {
+            return buf<T>(name, count);
+        }
+        catch (const CudaFail &f)
+        {
+            if (f.code != -3) throw;
+            cudaGetLastError();
+            return nullptr;
+        }
     }
 
     // Stage timing: mark(id) records the end of stage `id` on the stream; the
@@ -185,6 +202,7 @@ class Engine
     int n_downloads = 0;
     int n_sm() const { return n_sm_; }
     int max_smem() const { return max_smem_; }
+    cudaStream_t aux_stream() const { return aux_stream_; } // copies beside the call's stream
     cudaStream_t stream(const void *user) const { return user ? (cudaStream_t)user : own_stream_; }
     static constexpr int kNumEvents = 32;
     cudaEvent_t ev_[kNumEvents];
@@ -198,7 +216,7 @@ class Engine
     unsigned char *stage2_ = nullptr;
     size_t stage2_cap_ = 0;
     int device_;
-    cudaStream_t own_stream_ = nullptr;
+    cudaStream_t own_stream_ = nullptr, aux_stream_ = nullptr;
     int n_sm_ = 148;
     int max_smem_ = 227 * 1024;
     std::map<std::string, DevBuf> bufs_;
@@ -1268,6 +1286,56 @@ static bool sgs_walk(long long size, long long seed, SgsWalk &w)
     return size % C != 0;
 }
 
+// The weights of a simulation's nodes and its levels, up to 32 neighbours:
+// chunks of nodes in level order (offs: the levels' first positions) as large as
+// kSimChunkBytes of weights allow (a million nodes of 32 neighbours: the last wave
+// of a chunk's solves is then below 1 % of it), less where the device has no
+// room; each chunk's solves in one launch, then level(weights, first, count) per level.
+// before_levels runs once, after the first chunk's solves are queued.
+constexpr size_t kSimChunkBytes = (size_t)256 << 20;
+template <typename B, typename L>
+static void run_sim_levels(Engine &E, const std::vector<SisCat> &cats, int kmax, const int *sim_cells,
+                           const int *order, const std::vector<int> &offs, int n_levels, int n_sim, bool sgs,
+                           bool ordinary, bool correlogram, cudaStream_t st, B before_levels, L level)
+{
+    SimWeights a{};
+    a.kcat = (int)cats.size();
+    a.kmax = kmax;
+    a.sim_cells = sim_cells;
+    a.order = order;
+    SisCat *d_cats = E.buf<SisCat>("sim_cats", kSisMaxCat);
+    HB_CK(cudaMemcpyAsync(d_cats, cats.data(), cats.size() * sizeof(SisCat), cudaMemcpyHostToDevice, st));
+    a.cats = d_cats;
+    const size_t rows = (size_t)a.kcat * kmax, per = rows * 8 + (size_t)a.kcat * 2 + 8;
+    size_t chunk = std::min((size_t)std::max(n_sim, 1), std::max<size_t>(4096, kSimChunkBytes / per));
+    for (;; chunk = std::max<size_t>(4096, chunk / 2))
+    {
+        a.W = E.try_buf<double>("sim_w", rows * chunk);
+        if (a.W) break;
+        if (chunk <= 4096) throw CudaFail{-3, "device memory exhausted (simulation weights)"};
+    }
+    a.n = E.buf<unsigned char>("sim_n", (size_t)a.kcat * chunk);
+    a.st = E.buf<signed char>("sim_st", (size_t)a.kcat * chunk);
+    a.var = E.buf<double>("sim_var", chunk);
+    int l = 0;
+    for (long long p0 = 0; p0 < n_sim; p0 += (long long)chunk)
+    {
+        a.first = (int)p0;
+        a.count = (int)std::min<long long>((long long)chunk, n_sim - p0);
+        HB_CK(launch_sim_weights(a, sgs, ordinary, correlogram, E.n_sm(), st));
+        E.stats.launches += 1;
+        if (p0 == 0) before_levels();
+        const int p1 = a.first + a.count;
+        for (; l < n_levels && offs[l] < p1; ++l)
+        {
+            const int from = std::max(offs[l], a.first), to = std::min(offs[l + 1], p1);
+            HB_CK(level(a, from - a.first, to - from));
+            E.stats.launches += 1;
+            if (offs[l + 1] > p1) break; // the rest of this level in the next chunk
+        }
+    }
+}
+
 int sgs_simulation(const int *dims, float *data, unsigned char *mask, const unsigned char *sim_mask,
                    const CdfTable *cdf, const float *means, const SgsArgs &a, const Options &opt)
 {
@@ -1397,7 +1465,7 @@ int sgs_simulation(const int *dims, float *data, unsigned char *mask, const unsi
         launch_build_pair(g, dev_model(pl.f.m), 1, search_vals, pair64, pair32, st);
         E.stats.launches += 1 + ((use_cdf || lvm) ? 1 : 0) + (n_sim > 0 ? 4 : 0); // + search, moments, levels x2
         std::vector<int4> t4(tv.size());
-        for (size_t i = 0; i < tv.size(); ++i) t4[i] = make_int4(tv[i].dx, tv[i].dy, tv[i].dz, 0);
+        for (size_t i = 0; i < tv.size(); ++i) t4[i] = make_int4(tv[i].dx, tv[i].dy, tv[i].dz, pair_lin(g, tv[i].dx, tv[i].dy, tv[i].dz));
         int4 *tmpl = E.buf<int4>("sgs_tmpl", std::max<size_t>(t4.size(), 1));
         if (!t4.empty())
             HB_CK(cudaMemcpyAsync(tmpl, t4.data(), t4.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
@@ -1411,10 +1479,11 @@ int sgs_simulation(const int *dims, float *data, unsigned char *mask, const unsi
         // neighbours of every simulated node
         const int k = a.max_nb;
         int *nb = E.buf<int>("sgs_nb", (size_t)std::max(n_sim, 1) * k);
+        int *nb_lin = k <= 32 ? E.buf<int>("sgs_nb_lin", (size_t)std::max(n_sim, 1) * k) : nullptr;
         int *nb_rank = E.buf<int>("sgs_nb_rank", (size_t)std::max(n_sim, 1) * k);
         int *nb_cnt = E.buf<int>("sgs_nb_cnt", (size_t)std::max(n_sim, 1));
         if (n_sim > 0)
-            launch_sgs_search(g, tmpl, (int)t4.size(), sim_cells, n_sim, rank_of, k, nb, nb_rank, nb_cnt, E.n_sm(),
+            launch_sgs_search(g, tmpl, (int)t4.size(), sim_cells, n_sim, rank_of, k, nb, nb_lin, nb_rank, nb_cnt, E.n_sm(),
                               st);
         HB_CK(cudaGetLastError());
         E.mark(STAGE_SEARCH, st);
@@ -1469,22 +1538,37 @@ int sgs_simulation(const int *dims, float *data, unsigned char *mask, const unsi
         E.stats.sgs_levels = n_levels;
         E.mark(STAGE_TIES, st);
 
-        // draws in, then one solve launch per level
-        draws_f.get();
-        E.stats.draws_ms = draws_ms;
+        // the draws come in beside the solves
         double *d_u = E.buf<double>("sgs_uniforms", (size_t)std::max(n_sim, 1));
-        if (n_sim > 0)
-        {
-            HB_CK(cudaMemcpyAsync(d_u, h_u, (size_t)n_sim * 8, cudaMemcpyHostToDevice, st));
+        auto draws_in = [&]() {
+            draws_f.get();
+            E.stats.draws_ms = draws_ms;
+            if (n_sim <= 0) return;
+            HB_CK(cudaMemcpyAsync(d_u, h_u, (size_t)n_sim * 8, cudaMemcpyHostToDevice, E.aux_stream()));
+            HB_CK(cudaEventRecord(E.ev_[20], E.aux_stream()));
+            HB_CK(cudaStreamWaitEvent(st, E.ev_[20], 0));
             E.stats.h2d += (long long)n_sim * 8;
-        }
+        };
         E.mark(STAGE_PREPARE, st);
         signed char *st_rank = E.buf<signed char>("sgs_st_rank", (size_t)std::max(n_sim, 1));
-        for (int l = 0; l < n_levels; ++l)
+        if (k <= 32 && n_sim > 0)
         {
-            HB_CK(launch_sgs_solve(g, order + offs[l], counts[l], sim_cells, nb, nb_cnt, k, pair64, d_data, d_means,
-                                   d_u, st_rank, ordinary, E.n_sm(), st));
-            E.stats.launches += 1;
+            const std::vector<SisCat> one{
+                SisCat{pair64, nb, nb_lin, nb_cnt, nullptr, g.pair_center, g.pnx, g.pny, k, 0.0f}};
+            run_sim_levels(E, one, k, sim_cells, order, offs, n_levels, n_sim, true, ordinary, false, st,
+                           draws_in, [&](const SimWeights &w, int first, int count) {
+                               return launch_sgs_level(w, first, count, d_data, d_means, d_u, st_rank, st);
+                           });
+        }
+        else
+        {
+            draws_in();
+            for (int l = 0; l < n_levels; ++l)
+            {
+                HB_CK(launch_sgs_solve(g, order + offs[l], counts[l], sim_cells, nb, nb_cnt, k, pair64, d_data,
+                                       d_means, d_u, st_rank, ordinary, E.n_sm(), st));
+                E.stats.launches += 1;
+            }
         }
         E.mark(STAGE_SOLVE, st);
         signed char *d_status =
@@ -1675,7 +1759,7 @@ int sis_simulation(const int *dims, unsigned char *data, unsigned char *mask, co
         int *nb_rank = E.buf<int>("sis_nb_rank", ns * ktot);
         HB_CK(cudaMemsetAsync(nb_rank, 0xFF, ns * ktot * 4, st)); // -1: no neighbour
         std::vector<double *> pair64(kcat);
-        std::vector<int *> nb(kcat), nb_cnt(kcat);
+        std::vector<int *> nb(kcat), nb_lin(kcat), nb_cnt(kcat);
         for (int c = 0; c < kcat; ++c)
         {
             const Plan &pl = plans[c].first;
@@ -1690,14 +1774,15 @@ int sis_simulation(const int *dims, unsigned char *data, unsigned char *mask, co
             float *p32 = E.buf<float>(("sis_pair32_" + sfx).c_str(), (size_t)pn);
             launch_build_pair(g, dev_model(pl.f.m), 1, sv, pair64[c], p32, st);
             std::vector<int4> t4(tv.size());
-            for (size_t i = 0; i < tv.size(); ++i) t4[i] = make_int4(tv[i].dx, tv[i].dy, tv[i].dz, 0);
+            for (size_t i = 0; i < tv.size(); ++i) t4[i] = make_int4(tv[i].dx, tv[i].dy, tv[i].dz, pair_lin(g, tv[i].dx, tv[i].dy, tv[i].dz));
             int4 *tmpl = E.buf<int4>(("sis_tmpl_" + sfx).c_str(), std::max<size_t>(t4.size(), 1));
             if (!t4.empty())
                 HB_CK(cudaMemcpyAsync(tmpl, t4.data(), t4.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
             nb[c] = E.buf<int>(("sis_nb_" + sfx).c_str(), ns * cats[c].max_nb);
+            nb_lin[c] = E.buf<int>(("sis_nb_lin_" + sfx).c_str(), ns * cats[c].max_nb);
             nb_cnt[c] = E.buf<int>(("sis_nb_cnt_" + sfx).c_str(), ns);
             if (n_sim > 0)
-                launch_sgs_search(g, tmpl, (int)t4.size(), sim_cells, n_sim, rank_of, cats[c].max_nb, nb[c],
+                launch_sgs_search(g, tmpl, (int)t4.size(), sim_cells, n_sim, rank_of, cats[c].max_nb, nb[c], nb_lin[c],
                                   nb_rank + koff[c], nb_cnt[c], E.n_sm(), st, -1, ktot);
             HB_CK(cudaGetLastError());
             HB_CK(cudaStreamSynchronize(st)); // the host tables of this category
@@ -1759,38 +1844,34 @@ int sis_simulation(const int *dims, unsigned char *data, unsigned char *mask, co
         E.stats.sgs_levels = n_levels;
         E.mark(STAGE_TIES, st);
 
-        draws_f.get();
-        E.stats.draws_ms = draws_ms;
         double *d_u = E.buf<double>("sgs_uniforms", ns);
-        if (n_sim > 0)
-        {
-            HB_CK(cudaMemcpyAsync(d_u, h_u, (size_t)n_sim * 8, cudaMemcpyHostToDevice, st));
+        auto draws_in = [&]() {
+            draws_f.get();
+            E.stats.draws_ms = draws_ms;
+            if (n_sim <= 0) return;
+            HB_CK(cudaMemcpyAsync(d_u, h_u, (size_t)n_sim * 8, cudaMemcpyHostToDevice, E.aux_stream()));
+            HB_CK(cudaEventRecord(E.ev_[20], E.aux_stream()));
+            HB_CK(cudaStreamWaitEvent(st, E.ev_[20], 0));
             E.stats.h2d += (long long)n_sim * 8;
-        }
+        };
         E.mark(STAGE_PREPARE, st);
-        double *probs = E.buf<double>("sis_probs", ns * kcat);
-        signed char *st_cat = E.buf<signed char>("sis_st_cat", ns * kcat);
-        int *done = E.buf<int>("sis_done", ns);
         signed char *st_rank = E.buf<signed char>("sgs_st_rank", ns);
         std::vector<SisCat> hc(kcat);
         for (int c = 0; c < kcat; ++c)
         {
             const Geom &g = plans[c].first.g;
-            hc[c] = SisCat{pair64[c], nb[c], nb_cnt[c], d_means[c], g.pair_center, g.pnx, g.pny, cats[c].max_nb,
+            hc[c] = SisCat{pair64[c], nb[c], nb_lin[c], nb_cnt[c], d_means[c], g.pair_center, g.pnx, g.pny, cats[c].max_nb,
                            (float)cats[c].marginal};
         }
         int kmax = 0;
         for (int c = 0; c < kcat; ++c) kmax = std::max(kmax, cats[c].max_nb);
-        SisCat *d_cats = E.buf<SisCat>("sis_cats", kSisMaxCat);
-        HB_CK(cudaMemcpyAsync(d_cats, hc.data(), kcat * sizeof(SisCat), cudaMemcpyHostToDevice, st));
-        HB_CK(cudaMemsetAsync(done, 0, ns * 4, st));
-        for (int l = 0; l < n_levels; ++l)
-        {
-            SisLevelArgs la{d_cats, dims[0], dims[1], order + offs[l], counts[l], kcat, ncat, sim_cells, d_data,
-                            probs, st_cat, done, d_u, st_rank, correlogram && means ? 1 : 0, kmax};
-            HB_CK(launch_sis_level(la, E.n_sm(), st));
-            E.stats.launches += 1;
-        }
+        if (n_sim > 0)
+            run_sim_levels(E, hc, kmax, sim_cells, order, offs, n_levels, n_sim, false, false,
+                           correlogram && means, st, draws_in, [&](const SimWeights &w, int first, int count) {
+                               return launch_sis_level(w, first, count, ncat, d_data, d_u, st_rank, st);
+                           });
+        else
+            draws_in();
         HB_CK(cudaGetLastError());
         E.mark(STAGE_SOLVE, st);
         signed char *d_status =

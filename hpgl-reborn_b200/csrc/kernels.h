@@ -222,17 +222,18 @@ void launch_sgs_path(const SgsWalk &w, const uint8_t *mask, const uint8_t *sim_m
 void launch_sgs_index(long long n, const int *path_cell, const int *flag, const int *scan, const uint8_t *mask,
                       int *rank_of, int *sim_cells, cudaStream_t st);
 // Template scan with the rank predicate rank_of[q] < rank (or < fixed_rank when
-// fixed_rank >= 0); nb_rank may be null.
+// fixed_rank >= 0); nb_rank may be null, and so may nb_lin, which
+// gets the neighbours' pair-table offsets (the template's .w).
 void launch_sgs_search(const Geom &g, const int4 *tmpl, int n_tmpl, const int *sim_cells, int n_sim,
-                       const int *rank_of, int k, int *nb, int *nb_rank, int *nb_cnt, int n_sm, cudaStream_t st,
+                       const int *rank_of, int k, int *nb, int *nb_lin, int *nb_rank, int *nb_cnt, int n_sm, cudaStream_t st,
                        int fixed_rank = -1, int rank_stride = 0);
-// SIS (sgs.cu): one launch per level solves every (node, kriged category)
-// system and draws each node's category when its last system is done
+// Weights of the simulated nodes, solved ahead of the levels (sim_weights.cu)
 constexpr int kSisMaxCat = 16;
 struct SisCat
 {
     const double *pair64; // the category's pair table
     const int *nb;        // its neighbour cells, k per rank
+    const int *nb_lin;    // and their pair-table offsets from the node
     const int *nb_cnt;
     const float *means;   // LVM: the category's mean per cell, or null
     long long pair_center;
@@ -240,30 +241,33 @@ struct SisCat
     int k;
     float marginal;       // the category's mean (float, as the reference stores it)
 };
-struct SisLevelArgs
+struct SimWeights
 {
-    const SisCat *cats;  // kcat entries (device)
-    int nx, ny;
-    const int *order;    // the level's ranks
-    int n_nodes;
-    int kcat, ncat;
+    const SisCat *cats;  // kcat entries (device); SGS: one
+    int kcat, kmax;      // kmax: the largest k of the categories (at most 32)
     const int *sim_cells;
-    uint8_t *data;       // categories (the draws are written here)
-    double *probs;       // per rank, kcat entries
-    signed char *st_cat; // per rank, kcat entries
-    int *done;           // per rank: systems finished (zeroed per call)
-    const double *uniforms;
-    signed char *st_rank;
-    int correlogram;     // LVM correlogram weights (corellogramed_weights_3)
-    int kmax;            // the largest k of the categories
+    const int *order;    // the nodes' ranks, level after level
+    int first, count;    // the chunk: positions first .. first + count of order
+    // by position in the chunk
+    double *W;           // [count][kcat][kmax] weights
+    unsigned char *n;    // [count][kcat] neighbour counts
+    signed char *st;     // [count][kcat] 0 kriged, 1 no neighbours, 2 singular
+    double *var;         // [count] kriging variances (SGS)
 };
-cudaError_t launch_sis_level(const SisLevelArgs &a, int n_sm, cudaStream_t st);
+cudaError_t launch_sim_weights(const SimWeights &a, bool sgs, bool ordinary, bool correlogram, int n_sm,
+                               cudaStream_t st);
+// positions first .. first + count of the chunk, all of one level
+cudaError_t launch_sgs_level(const SimWeights &a, int first, int count, float *data, const float *means,
+                             const double *uniforms, signed char *st_rank, cudaStream_t st);
+cudaError_t launch_sis_level(const SimWeights &a, int first, int count, int ncat, uint8_t *data,
+                             const double *uniforms, signed char *st_rank, cudaStream_t st);
 void launch_sgs_levels(const int *nb_rank, const int *nb_cnt, int k, int n_sim, int *levp1, int *ticket,
                        int *level_count, int level_cap, int *max_level, int *err, int n_sm, cudaStream_t st);
 void launch_sgs_moments(int n_sim, const int *nb_cnt, double *mom, int n_sm, cudaStream_t st); // mom: 3, zeroed
 void launch_sgs_level_fill(int n_sim, const int *levp1, const int *level_off, int *level_fill, int *order,
                            cudaStream_t st);
 size_t sgs_block_smem(int k);
+// one level of SGS beyond 32 neighbours, a block a node
 cudaError_t launch_sgs_solve(const Geom &g, const int *order, int n_items, const int *sim_cells, const int *nb,
                              const int *nb_cnt, int k, const double *pair64, float *data, const float *means,
                              const double *uniforms, signed char *st_rank, bool ordinary, int n_sm, cudaStream_t st);

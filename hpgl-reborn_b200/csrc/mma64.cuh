@@ -30,6 +30,22 @@ __device__ __forceinline__ void mma884(Blk &c, double a, double b)
         : "+d"(c.x), "+d"(c.y)
         : "d"(a), "d"(b));
 }
+// the product alone
+__device__ __forceinline__ Blk mma884_zero(double a, double b)
+{
+    Blk c;
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%4,%4};"
+        : "=d"(c.x), "=d"(c.y)
+        : "d"(a), "d"(b), "d"(0.0));
+    return c;
+}
+// X Y^T
+__device__ __forceinline__ Blk blk_prod_t(const Blk &x, const Blk &y)
+{
+    Blk c = mma884_zero(x.x, y.x);
+    mma884(c, x.y, y.y);
+    return c;
+}
 // C += X Y^T
 __device__ __forceinline__ void blk_mul_t(Blk &c, const Blk &x, const Blk &y)
 {
@@ -62,52 +78,62 @@ __device__ __forceinline__ bool pivot_fails(double d)
     return (unsigned)__double2hiint(d) - lo >= 0x7FF00000u - lo;
 }
 
-// doubles of shared memory that mma_diag needs per system: two copies of a row
-constexpr int kMmaRowDoubles = 16;
+// doubles of shared memory that mma_diag needs per system: two pairs of rows
+constexpr int kMmaRowDoubles = 32;
 
 // Factors the 8x8 diagonal blocks D[s] = L L^T of S systems (each warp-wide)
 // and replaces them with M = L^-1 (zero above the diagonal). The elimination
-// runs in place: row j is final at step j, and each later row r adds -m =
-// -D(r,j) / d_j times row j, whose slots hold M(j, .) left of the pivot and
-// D(j, .) right of it. Slot j of row r then starts M(r, j) = -m; it is kept as
-// -m d_j = -D(r,j), which the same multiply-add gives when row j's own slot j
-// counts twice, so column j of M waits for its factor 1/d_j, as the rows do
-// for d^-1/2, until the end. Row j travels through shared memory (row:
-// kMmaRowDoubles doubles per system, 16-byte aligned), and D(r,j) is read as
-// D(j,r). fail[s] is set (on every lane) by a pivot that is not positive, or,
-// with EPS_PIVOT, below the machine epsilon. No step branches, so the chains of
-// the S systems overlap.
+// runs in place, two pivots a step: rows j and j + 1 are final at their step,
+// and each later row r subtracts its multiples of both, whose slots hold M left
+// of the pivots and D right of them; slots j and j + 1 of row r then start
+// M(r, j) and M(r, j + 1), minus the multipliers. The two rows travel through
+// shared memory (row: kMmaRowDoubles doubles per system, 16-byte aligned), which
+// with the two reciprocals is the latency of a step (one pivot a step: twice the
+// exchanges for a quarter fewer FP64 operations; the 8.3M systems of 32 then
+// took 20.5 against 18.8 ms), and D(r, j) is read as D(j, r). The row scales
+// d^-1/2 wait for the end, where the eight pivots take one rsqrt together.
+// fail[s] is set (on every lane) by a pivot that is not positive, or, with
+// EPS_PIVOT, below the machine epsilon. No step branches, so the chains of the S
+// systems overlap.
 template <int S, bool EPS_PIVOT = false>
 __device__ __forceinline__ void mma_diag(Blk (&D)[S], double *row, int lane, bool (&fail)[S])
 {
     const int r = lane >> 2, q = lane & 3;
-    double cx[S], cy[S]; // 1 / d of the lane's columns
 #pragma unroll
-    for (int s = 0; s < S; ++s) cx[s] = cy[s] = 0.0;
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
+    for (int j = 0; j < 8; j += 2)
     {
-        double *buf = row + (j & 1) * 8;
+        double *buf = row + (j & 2) * 8;
 #pragma unroll
         for (int s = 0; s < S; ++s)
-            if (r == j) reinterpret_cast<double2 *>(buf + s * kMmaRowDoubles)[q] = make_double2(D[s].x, D[s].y);
+            if (r == j || r == j + 1)
+                reinterpret_cast<double2 *>(buf + s * kMmaRowDoubles + 8 * (r & 1))[q] = make_double2(D[s].x, D[s].y);
         __syncwarp();
 #pragma unroll
         for (int s = 0; s < S; ++s)
         {
-            const double *b = buf + s * kMmaRowDoubles;
-            const double p = b[j];
-            fail[s] |= pivot_fails<EPS_PIVOT>(p);
-            const double inv = pivot_inverse(p);
-            if (q == j / 2) (j & 1 ? cy[s] : cx[s]) = inv;
-            if (j < 7)
+            const double *b0 = buf + s * kMmaRowDoubles, *b1 = b0 + 8;
+            const double2 ab = reinterpret_cast<const double2 *>(b0)[j / 2]; // D(j, j), D(j, j + 1)
+            const double ia = pivot_inverse(ab.x);
+            const double t = ab.y * ia;
+            const double d = fma(-t, ab.y, b1[j + 1]); // the second pivot
+            fail[s] |= pivot_fails<EPS_PIVOT>(ab.x) || pivot_fails<EPS_PIVOT>(d);
+            if (j == 6)
             {
-                const double m = r > j ? b[r] * inv : 0.0;
-                double2 u = reinterpret_cast<const double2 *>(b)[q];
-                if (q == j / 2) (j & 1 ? u.y : u.x) = 2.0 * p;
-                D[s].x = fma(-m, u.x, D[s].x);
-                D[s].y = fma(-m, u.y, D[s].y);
+                // no later rows: row 7 alone
+                const double2 u0 = reinterpret_cast<const double2 *>(b0)[q];
+                const double n0 = r == 7 ? t : 0.0;
+                D[s].x = r == 7 && q == 3 ? -t : fma(-n0, u0.x, D[s].x);
+                D[s].y = fma(-n0, u0.y, D[s].y);
+                continue;
             }
+            const double id = pivot_inverse(d);
+            const double2 u0 = reinterpret_cast<const double2 *>(b0)[q], u1 = reinterpret_cast<const double2 *>(b1)[q];
+            const double m0 = b0[r] * ia;
+            const double m1 = r > j + 1 ? fma(-m0, ab.y, b1[r]) * id : 0.0;
+            const double n0 = r > j + 1 ? fma(-m1, t, m0) : (r == j + 1 ? t : 0.0);
+            const bool own = q == j / 2;
+            D[s].x = own && r > j ? -n0 : fma(-m1, u1.x, fma(-n0, u0.x, D[s].x));
+            D[s].y = own && r > j + 1 ? -m1 : fma(-m1, u1.y, fma(-n0, u0.y, D[s].y));
         }
     }
 #pragma unroll
@@ -115,8 +141,8 @@ __device__ __forceinline__ void mma_diag(Blk (&D)[S], double *row, int lane, boo
     {
         const double own = (r & 1) ? D[s].y : D[s].x; // the pivot, in lane (r, r / 2)
         const double rs = rsqrt(__shfl_sync(0xffffffffu, own, (r << 2) + (r >> 1)));
-        D[s].x = 2 * q <= r ? D[s].x * cx[s] * rs : 0.0;
-        D[s].y = 2 * q + 1 <= r ? D[s].y * cy[s] * rs : 0.0;
+        D[s].x = 2 * q < r ? D[s].x * rs : (2 * q == r ? rs : 0.0);
+        D[s].y = 2 * q + 1 < r ? D[s].y * rs : (2 * q + 1 == r ? rs : 0.0);
     }
 }
 
@@ -142,9 +168,7 @@ __device__ __forceinline__ void mma_factor(Blk (&A)[S][NB * (NB + 1) / 2], Blk (
         for (int s = 0; s < S; ++s)
         {
             A[s][blk_at(k, k)] = D[s];
-            Blk t{0.0, 0.0};
-            blk_mul_t(t, X[s][k], D[s]);
-            X[s][k] = t;
+            X[s][k] = blk_prod_t(X[s][k], D[s]);
         }
 #pragma unroll
         for (int i = k + 1; i < NB; ++i)
@@ -153,9 +177,7 @@ __device__ __forceinline__ void mma_factor(Blk (&A)[S][NB * (NB + 1) / 2], Blk (
 #pragma unroll
             for (int s = 0; s < S; ++s)
             {
-                Blk t{0.0, 0.0};
-                blk_mul_t(t, A[s][blk_at(i, k)], D[s]);
-                A[s][blk_at(i, k)] = t;
+                A[s][blk_at(i, k)] = blk_prod_t(A[s][blk_at(i, k)], D[s]);
             }
         }
 #pragma unroll
@@ -200,9 +222,7 @@ __device__ __forceinline__ void mma_factor(Blk (&A)[S][NB * (NB + 1) / 2], int n
 #pragma unroll
             for (int s = 0; s < S; ++s)
             {
-                Blk t{0.0, 0.0};
-                blk_mul_t(t, A[s][blk_at(i, k)], D[s]);
-                A[s][blk_at(i, k)] = t;
+                A[s][blk_at(i, k)] = blk_prod_t(A[s][blk_at(i, k)], D[s]);
             }
         }
 #pragma unroll
@@ -243,8 +263,19 @@ __device__ __forceinline__ void mma_load(Blk (&A)[NB * (NB + 1) / 2], const doub
     {
         if (i >= nb) break;
         const int row = 8 * i + r;
-        const bool live = row < n;
         const int rl = lin[row];
+        if (8 * i + 8 <= n) // warp-uniform: every row of the block row is live
+        {
+#pragma unroll
+            for (int k = 0; k <= i; ++k)
+            {
+                Blk &b = A[blk_at(i, k)];
+                b.x = __ldg(pair_c + abs(rl - lc[k].x));
+                b.y = __ldg(pair_c + abs(rl - lc[k].y));
+            }
+            continue;
+        }
+        const bool live = row < n;
 #pragma unroll
         for (int k = 0; k < i; ++k)
         {

@@ -16,20 +16,18 @@
 //                  order with the rank predicate, one warp per node
 //   k_sgs_levels   dependency levels: level(j) = 1 + max level of its simulated
 //                  neighbours; a single pass over the ranks in ticket order
-//   k_sgs_solve_*  one launch per level: every node of a level depends only on
-//                  lower levels, so a level is kriged and drawn in parallel
-//                  (FP64: two nodes per warp for up to 32 neighbours, one
-//                  block per node beyond)
+//   k_sim_weights, k_sgs_level (sim_weights.cu, up to 32 neighbours): every
+//                  node's weights at once, then one launch per level (its nodes
+//                  depend only on lower levels) for the sums and the draws
+//   k_sgs_solve_block  beyond: one launch per level, one block per node
 //
 // The draws are the reference's: one std::uniform_real_distribution<double>
 // draw of a std::mt19937 per simulated node, in walk order (generated on the
 // host), pushed through the inverse Gaussian CDF with the reference's float
 // mean and double variance.
 #include "engine.cuh"
-#include "fold32.cuh"
 #include "kernels.h"
-
-#include <cuda/atomic>
+#include "sim_common.cuh"
 
 #include <algorithm>
 #include <climits>
@@ -37,28 +35,6 @@
 namespace hb
 {
 // ------------------------------------------------------------------ scalar maths
-// gaussian_cdf_t (gaussian_distribution.h): Abramowitz & Stegun 26.2.17 and the
-// Odeh & Evans inverse, every operation rounded as the reference's double code
-// rounds it (no contraction); exp and log are CUDA's (within 1 ulp of glibc's).
-__device__ double sgs_gauss_inverse(double pr, double mean, double var)
-{
-    if (pr <= 0.0 || pr >= 1.0) return mean;
-    double p2 = pr > 0.5 ? __dsub_rn(1.0, pr) : pr;
-    if (p2 < 1e-150) p2 = 1e-150;
-    const double y = __dsqrt_rn(log(__ddiv_rn(1.0, __dmul_rn(p2, p2))));
-    double num = __dadd_rn(__dmul_rn(-0.453642210148e-4, y), -0.0204231210245);
-    num = __dadd_rn(__dmul_rn(num, y), -0.342242088547);
-    num = __dadd_rn(__dmul_rn(num, y), -1.0);
-    num = __dadd_rn(__dmul_rn(num, y), -0.322232431088);
-    double den = __dadd_rn(__dmul_rn(0.38560700634e-2, y), 0.103537752850);
-    den = __dadd_rn(__dmul_rn(den, y), 0.531103462366);
-    den = __dadd_rn(__dmul_rn(den, y), 0.588581570495);
-    den = __dadd_rn(__dmul_rn(den, y), 0.0993484626060);
-    double xp = __dadd_rn(y, __ddiv_rn(num, den));
-    if (pr < 0.5) xp = -xp;
-    return __dadd_rn(__dmul_rn(xp, __dsqrt_rn(var)), mean);
-}
-
 // standard normal CDF (mean 0, variance 1: sx = x exactly)
 __device__ double sgs_gauss_cdf(double x)
 {
@@ -221,7 +197,8 @@ __global__ void k_sgs_index(long long n, const int *__restrict__ path_cell, cons
 __global__ void __launch_bounds__(256) k_sgs_search(const Geom g, const int4 *__restrict__ tmpl, int n_tmpl,
                                                     const int *__restrict__ sim_cells, int n_sim,
                                                     const int *__restrict__ rank_of, int k, int fixed_rank,
-                                                    int *__restrict__ nb, int *__restrict__ nb_rank, int rank_stride,
+                                                    int *__restrict__ nb, int *__restrict__ nb_lin,
+                                                    int *__restrict__ nb_rank, int rank_stride,
                                                     int *__restrict__ nb_cnt)
 {
     const int lane = threadIdx.x & 31;
@@ -238,7 +215,7 @@ __global__ void __launch_bounds__(256) k_sgs_search(const Geom g, const int4 *__
         {
             const int t = base + lane;
             bool hit = false;
-            int q = 0, rq = 0;
+            int q = 0, rq = 0, lin = 0;
             if (t < n_tmpl)
             {
                 const int4 o = tmpl[t];
@@ -247,6 +224,7 @@ __global__ void __launch_bounds__(256) k_sgs_search(const Geom g, const int4 *__
                 {
                     q = (int)(((long long)Z * g.ny + Y) * g.nx + X);
                     rq = rank_of[q];
+                    lin = o.w;
                     hit = rq < thr;
                 }
             }
@@ -255,6 +233,7 @@ __global__ void __launch_bounds__(256) k_sgs_search(const Geom g, const int4 *__
             if (hit && slot < k)
             {
                 out[slot] = q;
+                if (nb_lin) nb_lin[r * (long long)k + slot] = lin;
                 if (out_rank) out_rank[slot] = rq;
             }
             found += __popc(m);
@@ -441,304 +420,6 @@ struct SgsSolveArgs
     int ordinary;
 };
 
-// n <= 32: two nodes per warp, sixteen lanes each, lane t holding rows t and
-// 31 - t of A (the folded lower triangle, as the kriging solves lay it out).
-// The right-looking factorisation broadcasts column j through shared memory
-// row j and carries the forward substitution of b (and, for ordinary kriging,
-// of the ones vector); the back substitution reads column i of L from the
-// lane's own shared rows. The weights then go through combine() one by one.
-constexpr int kSgsNP = kFold32NP, kSgsG = kFold32G;
-constexpr int kSgsLD = kFold32LD;
-constexpr int kSgsFoldThreads = 256;
-
-constexpr size_t kSgsSysBytes = kFold32SysBytes;
-
-// BOUND (k < 32): the factorisation stops at the warp's largest system
-template <bool ORD, bool BOUND>
-__global__ void __launch_bounds__(kSgsFoldThreads, 1) k_sgs_solve_fold(const SgsSolveArgs a)
-{
-    constexpr int NP = kSgsNP, G = kSgsG, LD = kSgsLD, QB = ORD ? 2 : 1;
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const int h = lane / G, t = lane % G, rb = NP - 1 - t;
-    const unsigned gm = 0xFFFFu << (h * G);
-    unsigned char *gb = smem + kSgsSysBytes * (warp * 2 + h);
-    double *M = reinterpret_cast<double *>(gb);
-    int *LIN = reinterpret_cast<int *>(gb + kFold32MBytes);
-    const int row_a = d_fold32_rows.row[t], row_b = d_fold32_rows.row[rb]; // the lane's rows in M
-    const Geom &g = a.g;
-    const long long pc = g.pair_center;
-    const double *pair64 = a.pair64;
-    // The next item's chain of dependent loads (rank, cell and count; its
-    // neighbours; their values) is issued in three stages during the current
-    // item's solve. Its neighbours belong to lower levels, already final.
-    const int stride = gridDim.x * nwarps * 2;
-    int nr = 0, ncell = 0, nn = 0, nqa = 0, nqb = 0;
-    float nva = 0.0f, nvb = 0.0f, nma = 0.0f, nmb = 0.0f;
-    auto stage_a = [&](int itx) {
-        nr = 0;
-        ncell = 0;
-        nn = 0;
-        if (itx < a.n_items)
-        {
-            nr = a.order[itx];
-            ncell = a.sim_cells[nr];
-            nn = a.nb_cnt[nr];
-        }
-    };
-    auto stage_b = [&]() {
-        nqa = t < nn ? a.nb[(long long)nr * a.k + t] : 0;
-        nqb = rb < nn ? a.nb[(long long)nr * a.k + rb] : 0;
-    };
-    auto stage_c = [&]() {
-        nva = t < nn ? a.data[nqa] : 0.0f;
-        nvb = rb < nn ? a.data[nqb] : 0.0f;
-        nma = (a.means && t < nn) ? a.means[nqa] : 0.0f;
-        nmb = (a.means && rb < nn) ? a.means[nqb] : 0.0f;
-    };
-    const int first = (blockIdx.x * nwarps + warp) * 2;
-    stage_a(first + h);
-    stage_b();
-    stage_c();
-    for (int it0 = first; it0 < a.n_items; it0 += stride)
-    {
-        const int it = it0 + h;
-        const bool valid = it < a.n_items;
-        const int r = nr, cell = ncell, n = nn, qa = nqa, qb = nqb;
-        const float va = nva, vb = nvb, ma = nma, mb = nmb;
-        stage_a(it + stride);
-        const int cx = cell % g.nx, cy = (int)((cell / g.nx) % g.ny), cz = (int)(cell / ((long long)g.nx * g.ny));
-        const bool live_a = t < n, live_b = rb < n;
-        int lin_a = 0, lin_b = 0;
-        if (live_a)
-            lin_a = pair_lin(g, qa % g.nx - cx, (int)((qa / g.nx) % g.ny) - cy,
-                             (int)(qa / ((long long)g.nx * g.ny)) - cz);
-        if (live_b)
-            lin_b = pair_lin(g, qb % g.nx - cx, (int)((qb / g.nx) % g.ny) - cy,
-                             (int)(qb / ((long long)g.nx * g.ny)) - cz);
-        LIN[t] = lin_a;
-        LIN[rb] = lin_b;
-        __syncwarp(gm);
-
-        // The solve of fold32_solve written out in place: measured 41.0 ms for the
-        // 8.3M systems of the 256x256x128 simulation against 46.7 ms through the
-        // shared function (same registers and loads, 6.5% more instructions).
-        // BOUND: both systems' live rows end at nmax (the warp's largest count).
-        const int nmax = BOUND ? __reduce_max_sync(0xffffffffu, n) : NP;
-        // ---- assembly (lower triangles of rows t and 31 - t; padding rows identity)
-        double ra[G], rbv[NP];
-        const double *base_a = pair64 + pc + lin_a, *base_b = pair64 + pc + lin_b;
-#pragma unroll
-        for (int c = 0; c < G; ++c)
-        {
-            double e = 0.0;
-            if (live_a && c <= t) e = __ldg(base_a - LIN[c]);
-            if (!live_a && c == t) e = 1.0;
-            ra[c] = e;
-        }
-#pragma unroll
-        for (int c = 0; c < NP; ++c)
-        {
-            double e = 0.0;
-            if (live_b && c <= rb) e = __ldg(base_b - LIN[c]);
-            if (!live_b && c == rb) e = 1.0;
-            rbv[c] = e;
-        }
-        const double b_a = live_a ? __ldg(base_a) : 0.0;
-        const double b_b = live_b ? __ldg(base_b) : 0.0;
-        stage_b();
-
-        // ---- factorisation with the forward substitution of b (and 1)
-        double rhs_a[QB], rhs_b[QB], ya[QB], yb[QB];
-        rhs_a[0] = b_a;
-        rhs_b[0] = b_b;
-        if constexpr (ORD)
-        {
-            rhs_a[1] = live_a ? 1.0 : 0.0;
-            rhs_b[1] = live_b ? 1.0 : 0.0;
-        }
-#pragma unroll
-        for (int q = 0; q < QB; ++q)
-        {
-            ya[q] = 0.0;
-            yb[q] = 0.0;
-        }
-        bool fail = false;
-        double inv_a = 0.0, inv_b = 0.0;
-#pragma unroll
-        for (int j = 0; j < NP; ++j)
-        {
-            if (BOUND && j >= nmax) break;
-            // row j of the packed matrix holds columns 2*(j/2) on
-            double *Mj = M + d_fold32_rows.row[j];
-            if (j < G)
-            {
-                if (t >= (j & ~1)) Mj[t] = ra[j];
-                if (t == j)
-                {
-#pragma unroll
-                    for (int q = 0; q < QB; ++q) Mj[NP + q] = rhs_a[q];
-                }
-            }
-            if (rb >= (j & ~1)) Mj[rb] = rbv[j];
-            if (j >= G && rb == j)
-            {
-#pragma unroll
-                for (int q = 0; q < QB; ++q) Mj[NP + q] = rhs_b[q];
-            }
-            __syncwarp(gm);
-            double mj[LD];
-            const double2 *mv = reinterpret_cast<const double2 *>(Mj);
-#pragma unroll
-            for (int q = j / 2; q < LD / 2; ++q)
-            {
-                const double2 v2 = mv[q];
-                mj[2 * q] = v2.x;
-                mj[2 * q + 1] = v2.y;
-            }
-            const double d = mj[j];
-            fail |= !(d > 0.0);
-            const double inv_s = rsqrt(d);
-            const double inv2 = inv_s * inv_s;
-            if (j < G)
-            {
-                const double sc = ra[j] * inv2;
-#pragma unroll
-                for (int c = j + 1; c < G; ++c) ra[c] -= sc * mj[c];
-                if (t > j)
-                {
-#pragma unroll
-                    for (int q = 0; q < QB; ++q) rhs_a[q] -= sc * mj[NP + q];
-                }
-                ra[j] *= inv_s;
-                if (t == j)
-                {
-                    inv_a = inv_s;
-#pragma unroll
-                    for (int q = 0; q < QB; ++q) ya[q] = rhs_a[q] * inv_s;
-                }
-            }
-            {
-                const double sc = rbv[j] * inv2;
-#pragma unroll
-                for (int c = j + 1; c < NP; ++c) rbv[c] -= sc * mj[c];
-                if (rb > j)
-                {
-#pragma unroll
-                    for (int q = 0; q < QB; ++q) rhs_b[q] -= sc * mj[NP + q];
-                }
-                rbv[j] *= inv_s;
-                if (rb == j)
-                {
-                    inv_b = inv_s;
-#pragma unroll
-                    for (int q = 0; q < QB; ++q) yb[q] = rhs_b[q] * inv_s;
-                }
-            }
-        }
-
-        stage_c();
-
-        // ---- back substitution L^T x = y; L[i][row] = M[row][i] / sqrt(d_row)
-        double xa[QB], xb[QB];
-#pragma unroll
-        for (int q = 0; q < QB; ++q)
-        {
-            xa[q] = 0.0;
-            xb[q] = 0.0;
-        }
-#pragma unroll
-        for (int i = NP - 1; i >= 0; --i)
-        {
-            if (BOUND && i >= nmax) continue;
-            double xi[QB];
-            if (i >= G)
-            {
-                if (rb == i)
-                {
-#pragma unroll
-                    for (int q = 0; q < QB; ++q) xb[q] = yb[q] * inv_b;
-                }
-#pragma unroll
-                for (int q = 0; q < QB; ++q) xi[q] = __shfl_sync(gm, xb[q], NP - 1 - i, G);
-            }
-            else
-            {
-                if (t == i)
-                {
-#pragma unroll
-                    for (int q = 0; q < QB; ++q) xa[q] = ya[q] * inv_a;
-                }
-#pragma unroll
-                for (int q = 0; q < QB; ++q) xi[q] = __shfl_sync(gm, xa[q], i, G);
-            }
-            if (t < i)
-            {
-                const double l = M[row_a + i] * inv_a;
-#pragma unroll
-                for (int q = 0; q < QB; ++q) ya[q] -= l * xi[q];
-            }
-            if (rb < i)
-            {
-                const double l = M[row_b + i] * inv_b;
-#pragma unroll
-                for (int q = 0; q < QB; ++q) yb[q] -= l * xi[q];
-            }
-        }
-
-        // ---- combine() and the variance in the reference's order
-        double sx = 0.0, sy = 0.0;
-        if constexpr (ORD)
-        {
-#pragma unroll
-            for (int i = 0; i < NP; ++i)
-            {
-                const double x0 = __shfl_sync(gm, i < G ? xa[0] : xb[0], i < G ? i : NP - 1 - i, G);
-                const double x1 = __shfl_sync(gm, i < G ? xa[1] : xb[1], i < G ? i : NP - 1 - i, G);
-                if (i < n)
-                {
-                    sx = __dadd_rn(sx, x0);
-                    sy = __dadd_rn(sy, x1);
-                }
-            }
-        }
-        const bool bad_ok = ORD && fabs(sy) < 1e-15;
-        const double mu = ORD && !bad_ok ? __ddiv_rn(__dsub_rn(sx, 1.0), sy) : 0.0;
-        // each lane forms its rows' terms; the sums run in row order
-        const double w_a = ORD ? __dsub_rn(xa[0], __dmul_rn(mu, xa[QB - 1])) : xa[0];
-        const double w_b = ORD ? __dsub_rn(xb[0], __dmul_rn(mu, xb[QB - 1])) : xb[0];
-        const double vt_a = __dmul_rn(w_a, b_a), vt_b = __dmul_rn(w_b, b_b);
-        const float et_a = __double2float_rn(__dmul_rn(w_a, (double)__fsub_rn(va, ma)));
-        const float et_b = __double2float_rn(__dmul_rn(w_b, (double)__fsub_rn(vb, mb)));
-        double var = pair64[pc];
-        float est = a.means && valid ? a.means[cell] : 0.0f;
-#pragma unroll 4
-        for (int i = 0; i < NP; ++i)
-        {
-            const bool lo = i < G;
-            const int src = lo ? i : NP - 1 - i;
-            const double vt = __shfl_sync(gm, lo ? vt_a : vt_b, src, G);
-            const float et = __shfl_sync(gm, lo ? et_a : et_b, src, G);
-            if (i < n)
-            {
-                var = __dsub_rn(var, vt);
-                est = __fadd_rn(est, et);
-            }
-        }
-        if (ORD) var = __dsub_rn(var, mu);
-        if (var < 0) var = 0;
-        if (valid && t == 0)
-        {
-            const int status = n == 0 ? 1 : ((fail || bad_ok) ? 2 : 0);
-            const double u = a.uniforms[r];
-            const double val = status == 0 ? sgs_gauss_inverse(u, (double)est, var) : sgs_gauss_inverse(u, 0.0, 1.0);
-            a.data[cell] = __double2float_rn(val);
-            a.st_rank[r] = (signed char)status;
-        }
-        __syncwarp(gm);
-    }
-}
-
 // 32 < n <= kSgsBlockMax: one block per node, the matrix in shared memory.
 constexpr int kSgsBlockThreads = 128;
 
@@ -853,180 +534,6 @@ __global__ void __launch_bounds__(kSgsBlockThreads) k_sgs_solve_block(const SgsS
     }
 }
 
-// ------------------------------------------------------------------ SIS
-// One launch per level: every (node, kriged category) system of the level
-// (sequential_indicator_simulation.cpp:77-108): the SK estimate of the
-// indicator (category == c) from the category's neighbours, accumulated in
-// double around the float mean (combine for a double result); the mean where
-// kriging fails. The last system of a node to finish draws its category
-// (sample.cpp:8-21): the first category whose running sum exceeds u times the
-// sum, p1 = 1 - p0 with two categories (median SIS).
-constexpr int kSisFoldThreads = 256;
-constexpr size_t kSisSysBytes = kFold32SysBytes + kFold32NP * 8; // plus the 32 row scales
-
-// the correlogram scale of a mean (corellogramed_weights_3, my_kriging_weights.h:407-438)
-__device__ __forceinline__ double sis_sigma(float mean)
-{
-    double m = (double)mean;
-    if (m == 0) m = __dadd_rn(m, 0.00001);
-    if (m == 1) m = __dsub_rn(m, 0.00001);
-    return __dsqrt_rn(__dmul_rn(m, __dsub_rn(1.0, m)));
-}
-
-// the draw of rank r once every category's probability is stored (read
-// through L2: other SMs wrote them); two passes, the sum then the running sum
-__device__ __forceinline__ void sis_draw(const double *probs, const signed char *st_cat, int kcat, int ncat,
-                                         double u, uint8_t *data_cell, signed char *st_out)
-{
-    const double p0 = __ldcg(probs);
-    double sum = 0.0;
-    int stv = 0;
-    for (int c = 0; c < kcat; ++c)
-    {
-        sum = __dadd_rn(sum, __ldcg(probs + c));
-        stv = max(stv, (int)__ldcg(reinterpret_cast<const unsigned char *>(st_cat) + c));
-    }
-    if (ncat == 2) sum = __dadd_rn(sum, __dsub_rn(1.0, p0)); // median SIS: p1 = 1 - p0
-    const double s = __dmul_rn(u, sum);
-    double acc = 0.0;
-    int pick = ncat - 1;
-    for (int c = 0; c < ncat; ++c)
-    {
-        acc = __dadd_rn(acc, ncat == 2 && c == 1 ? __dsub_rn(1.0, p0) : __ldcg(probs + c));
-        if (s < acc)
-        {
-            pick = c;
-            break;
-        }
-    }
-    *data_cell = (uint8_t)pick;
-    *st_out = (signed char)stv;
-}
-
-// CORR: correlogram weights (LVM): A_ij = C_ij (s_i s_j), b_i = C_ic (s_i s_c);
-// BOUND (every k < 32): the factorisation stops at the warp's largest system
-template <bool CORR, bool BOUND>
-__global__ void __launch_bounds__(kSisFoldThreads, 1) k_sis_level(const SisLevelArgs a)
-{
-    constexpr int NP = kFold32NP, G = kFold32G;
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const int h = lane / G, t = lane % G, rb = NP - 1 - t;
-    const unsigned gm = 0xFFFFu << (h * G);
-    unsigned char *gb = smem + kSisSysBytes * (warp * 2 + h);
-    double *M = reinterpret_cast<double *>(gb);
-    int *LIN = reinterpret_cast<int *>(gb + kFold32MBytes);
-    double *SIG = reinterpret_cast<double *>(gb + kFold32SysBytes); // the system's row scales
-    const int n_sys = a.n_nodes * a.kcat;
-    const int stride = gridDim.x * nwarps * 2;
-    // The next system's chain of dependent loads (rank, cell, count; its
-    // neighbours; their indicators and means) is issued in three stages during
-    // the current solve; its neighbours belong to lower levels, already final.
-    // Systems run category-major, so the SMs of a moment share a pair table.
-    int ncat_ = 0, nr = 0, ncell = 0, nn = 0, nqa = 0, nqb = 0;
-    float nda = 0.0f, ndb = 0.0f, nma = 0.0f, nmb = 0.0f, nmc = 0.0f;
-    auto stage_a = [&](int itx) {
-        ncat_ = 0;
-        nr = 0;
-        ncell = 0;
-        nn = 0;
-        if (itx < n_sys)
-        {
-            ncat_ = itx / a.n_nodes;
-            nr = a.order[itx - ncat_ * a.n_nodes];
-            ncell = a.sim_cells[nr];
-            nn = __ldg(a.cats[ncat_].nb_cnt + nr);
-        }
-    };
-    auto stage_b = [&]() {
-        const SisCat &C = a.cats[ncat_];
-        nqa = t < nn ? __ldg(C.nb + (long long)nr * C.k + t) : 0;
-        nqb = rb < nn ? __ldg(C.nb + (long long)nr * C.k + rb) : 0;
-        nmc = C.means ? C.means[ncell] : C.marginal;
-    };
-    auto stage_c = [&]() {
-        const float *means = a.cats[ncat_].means;
-        nma = t < nn && means ? means[nqa] : nmc;
-        nmb = rb < nn && means ? means[nqb] : nmc;
-        nda = t < nn && a.data[nqa] == ncat_ ? 1.0f : 0.0f;
-        ndb = rb < nn && a.data[nqb] == ncat_ ? 1.0f : 0.0f;
-    };
-    const int first = (blockIdx.x * nwarps + warp) * 2;
-    stage_a(first + h);
-    stage_b();
-    stage_c();
-    for (int it0 = first; it0 < n_sys; it0 += stride)
-    {
-        const int it = it0 + h;
-        const bool valid = it < n_sys;
-        const int cat = ncat_, r = nr, cell = ncell, n = nn, qa = nqa, qb = nqb;
-        const float ia = nda, ib = ndb, ma = nma, mb = nmb, mc = nmc;
-        stage_a(it + stride);
-        const SisCat &C = a.cats[cat];
-        const int pnx = C.pnx, pny = C.pny;
-        const double *pair_c = C.pair64 + C.pair_center;
-        const int cx = cell % a.nx, cy = (int)((cell / a.nx) % a.ny), cz = (int)(cell / ((long long)a.nx * a.ny));
-        const bool live_a = t < n, live_b = rb < n;
-        int lin_a = 0, lin_b = 0;
-        if (live_a)
-        {
-            const int qz = (int)(qa / ((long long)a.nx * a.ny)), qy = (int)((qa / a.nx) % a.ny), qx = qa % a.nx;
-            lin_a = ((qz - cz) * pny + (qy - cy)) * pnx + (qx - cx);
-        }
-        if (live_b)
-        {
-            const int qz = (int)(qb / ((long long)a.nx * a.ny)), qy = (int)((qb / a.nx) % a.ny), qx = qb % a.nx;
-            lin_b = ((qz - cz) * pny + (qy - cy)) * pnx + (qx - cx);
-        }
-        // indicator - mean, in float
-        const float da = live_a ? __fsub_rn(ia, ma) : 0.0f, db = live_b ? __fsub_rn(ib, mb) : 0.0f;
-        const double sa = CORR && live_a ? sis_sigma(ma) : 1.0, sb = CORR && live_b ? sis_sigma(mb) : 1.0;
-        LIN[t] = lin_a;
-        LIN[rb] = lin_b;
-        if (CORR)
-        {
-            SIG[t] = sa;
-            SIG[rb] = sb;
-        }
-        __syncwarp(gm);
-        const double sc = CORR ? sis_sigma(mc) : 1.0;
-        auto load_rhs = [&](double(&rhs_a)[1], double(&rhs_b)[1]) {
-            rhs_a[0] = live_a ? __ldg(pair_c + lin_a) : 0.0;
-            rhs_b[0] = live_b ? __ldg(pair_c + lin_b) : 0.0;
-            if (CORR)
-            {
-                rhs_a[0] = __dmul_rn(rhs_a[0], __dmul_rn(sa, sc));
-                rhs_b[0] = __dmul_rn(rhs_b[0], __dmul_rn(sb, sc));
-            }
-        };
-        double xa[1], xb[1];
-        const int nmax = BOUND ? __reduce_max_sync(0xffffffffu, n) : NP; // both systems of the warp
-        const bool fail = fold32_solve<1, false, CORR>(pair_c, LIN, M, gm, t, live_a, live_b, lin_a, lin_b, load_rhs,
-                                                       xa, xb, stage_b, stage_c, SIG, sa, sb, nmax);
-        const double ta = __dmul_rn(xa[0], (double)da), tb = __dmul_rn(xb[0], (double)db);
-        double prob = (double)mc;
-#pragma unroll 4
-        for (int i = 0; i < NP; ++i)
-        {
-            const bool lo = i < G;
-            const double ti = __shfl_sync(gm, lo ? ta : tb, lo ? i : NP - 1 - i, G);
-            if (i < n) prob = __dadd_rn(prob, ti);
-        }
-        if (valid && t == 0)
-        {
-            const int status = n == 0 ? 1 : (fail ? 2 : 0);
-            a.probs[(long long)r * a.kcat + cat] = status == 0 ? prob : (double)mc;
-            a.st_cat[(long long)r * a.kcat + cat] = (signed char)status;
-            // release this system's probability; the last system of the node acquires the others'
-            cuda::atomic_ref<int, cuda::thread_scope_device> done(a.done[r]);
-            if (done.fetch_add(1, cuda::memory_order_acq_rel) == a.kcat - 1)
-                sis_draw(a.probs + (long long)r * a.kcat, a.st_cat + (long long)r * a.kcat, a.kcat, a.ncat,
-                         a.uniforms[r], a.data + cell, a.st_rank + r);
-        }
-        __syncwarp(gm);
-    }
-}
-
 // ------------------------------------------------------------------ launchers
 void launch_sgs_forward(long long n, float *data, const uint8_t *mask, const float *means_in, float *means_out,
                         const float *cv, const float *cp, long long cn, cudaStream_t st)
@@ -1052,10 +559,10 @@ void launch_sgs_index(long long n, const int *path_cell, const int *flag, const 
     k_sgs_index<<<1184, 256, 0, st>>>(n, path_cell, flag, scan, mask, rank_of, sim_cells);
 }
 void launch_sgs_search(const Geom &g, const int4 *tmpl, int n_tmpl, const int *sim_cells, int n_sim,
-                       const int *rank_of, int k, int *nb, int *nb_rank, int *nb_cnt, int n_sm, cudaStream_t st,
+                       const int *rank_of, int k, int *nb, int *nb_lin, int *nb_rank, int *nb_cnt, int n_sm, cudaStream_t st,
                        int fixed_rank, int rank_stride)
 {
-    k_sgs_search<<<n_sm * 8, 256, 0, st>>>(g, tmpl, n_tmpl, sim_cells, n_sim, rank_of, k, fixed_rank, nb, nb_rank,
+    k_sgs_search<<<n_sm * 8, 256, 0, st>>>(g, tmpl, n_tmpl, sim_cells, n_sim, rank_of, k, fixed_rank, nb, nb_lin, nb_rank,
                                            rank_stride > 0 ? rank_stride : k, nb_cnt);
 }
 void launch_sgs_levels(const int *nb_rank, const int *nb_cnt, int k, int n_sim, int *levp1, int *ticket,
@@ -1073,21 +580,6 @@ void launch_sgs_level_fill(int n_sim, const int *levp1, const int *level_off, in
 {
     k_sgs_level_fill<<<1184, 256, 0, st>>>(n_sim, levp1, level_off, level_fill, order);
 }
-cudaError_t launch_sis_level(const SisLevelArgs &a, int n_sm, cudaStream_t st)
-{
-    const int n_sys = a.n_nodes * a.kcat;
-    if (n_sys <= 0) return cudaSuccess;
-    const int spb = kSisFoldThreads / kFold32G;
-    const size_t smem = kSisSysBytes * spb;
-    auto kern = a.correlogram ? (a.kmax < 32 ? k_sis_level<true, true> : k_sis_level<true, false>)
-                              : (a.kmax < 32 ? k_sis_level<false, true> : k_sis_level<false, false>);
-    int per_sm = 0;
-    cudaError_t e = set_smem_min_carveout(kern, kSisFoldThreads, smem, per_sm);
-    if (e != cudaSuccess) return e;
-    const int blocks = std::min((n_sys + spb - 1) / spb, n_sm);
-    kern<<<blocks, kSisFoldThreads, smem, st>>>(a);
-    return cudaGetLastError();
-}
 size_t sgs_block_smem(int k) { return (size_t)k * k * 8 + 3 * (size_t)k * 8 + 2 * (size_t)k * 4; }
 
 cudaError_t launch_sgs_solve(const Geom &g, const int *order, int n_items, const int *sim_cells, const int *nb,
@@ -1097,26 +589,11 @@ cudaError_t launch_sgs_solve(const Geom &g, const int *order, int n_items, const
     if (n_items <= 0) return cudaSuccess;
     SgsSolveArgs a{g, order, n_items, sim_cells, nb, nb_cnt, k, pair64, data, means, uniforms, st_rank,
                    ordinary ? 1 : 0};
-    if (k <= 32)
-    {
-        const size_t smem = kSgsSysBytes * (kSgsFoldThreads / kSgsG);
-        const int blocks = std::min((n_items + kSgsFoldThreads / kSgsG - 1) / (kSgsFoldThreads / kSgsG), n_sm);
-        auto kern = ordinary ? (k < 32 ? k_sgs_solve_fold<true, true> : k_sgs_solve_fold<true, false>)
-                             : (k < 32 ? k_sgs_solve_fold<false, true> : k_sgs_solve_fold<false, false>);
-        int per_sm = 0;
-        cudaError_t e = set_smem_min_carveout(kern, kSgsFoldThreads, smem, per_sm);
-        if (e != cudaSuccess) return e;
-        kern<<<blocks, kSgsFoldThreads, smem, st>>>(a);
-    }
-    else
-    {
-        const size_t smem = sgs_block_smem(k);
-        cudaError_t e =
-            cudaFuncSetAttribute(k_sgs_solve_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        const int blocks = std::min(n_items, n_sm * 8);
-        k_sgs_solve_block<<<blocks, kSgsBlockThreads, smem, st>>>(a);
-    }
+    const size_t smem = sgs_block_smem(k);
+    cudaError_t e = cudaFuncSetAttribute(k_sgs_solve_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    const int blocks = std::min(n_items, n_sm * 8);
+    k_sgs_solve_block<<<blocks, kSgsBlockThreads, smem, st>>>(a);
     return cudaGetLastError();
 }
 } // namespace hb

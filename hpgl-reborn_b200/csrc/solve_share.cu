@@ -283,8 +283,7 @@ __global__ void __launch_bounds__(TH, 1)
                 for (int k = 0; k < CB; ++k)
                 {
                     if (k >= cb) break;
-                    Blk t{0.0, 0.0};
-                    blk_mul_t(t, R[k], A[0][blk_at(k, k)]);
+                    Blk t = blk_prod_t(R[k], A[0][blk_at(k, k)]);
                     reinterpret_cast<double2 *>(&sh.R[rho * LD + 8 * k])[q] = make_double2(t.x, t.y);
                     t = blk_neg(t);
 #pragma unroll
