@@ -1022,47 +1022,32 @@ int cont_kriging(int kind, const int *dims, const float *in_data, const unsigned
         if (opt.variance) d_var = io.device ? opt.variance : E.buf<double>("var", (size_t)n);
         d_status = (io.device && opt.status) ? opt.status : E.buf<signed char>("status", (size_t)n);
 
-        // SK mean: calc_mean over informed cells (calc_mean.cpp:6-30), on the host
-        // data. LVM centres the values on their own means as they are compacted,
-        // so the uniform mean stays 0 there.
-        double mean = 0.0;
-        if (kind == 1)
-        {
-            if (a.auto_mean)
-            {
-                std::vector<float> hv;
-                std::vector<uint8_t> hm;
-                const float *pv = in_data;
-                const uint8_t *pm = in_mask;
-                if (io.device)
-                {
-                    hv.resize(n);
-                    hm.resize(n);
-                    HB_CK(cudaMemcpyAsync(hv.data(), in_data, n * 4, cudaMemcpyDeviceToHost, st));
-                    HB_CK(cudaMemcpyAsync(hm.data(), in_mask, n, cudaMemcpyDeviceToHost, st));
-                    HB_CK(cudaStreamSynchronize(st));
-                    pv = hv.data();
-                    pm = hm.data();
-                }
-                double sum = 0;
-                long long cnt = 0;
-                for (long long i = 0; i < n; ++i)
-                    if (pm[i])
-                    {
-                        sum += pv[i];
-                        cnt += 1;
-                    }
-                mean = cnt ? sum / cnt : 0.0;
-            }
-            else
-                mean = a.mean;
-        }
-
         HB_CK(cudaEventRecord(E.ev_[2], st));
         DevPoints P = compact_points(E, grid_geom(dims), d_mask, d_in, nullptr, st, d_means);
+        // SK mean: calc_mean over the informed cells (calc_mean.cpp:6-30), a double
+        // sum in ascending cell order. The compacted values are in that order, and
+        // they are a small part of the grid, so they are what comes to the host;
+        // the sum is taken while the search runs. (LVM centres the values on their
+        // own means as they are compacted, so its uniform mean stays 0.)
+        double mean = kind == 1 && !a.auto_mean ? a.mean : 0.0;
+        const bool auto_mean = kind == 1 && a.auto_mean && P.m > 0;
+        const float *h_val = nullptr;
+        if (auto_mean)
+        {
+            h_val = reinterpret_cast<const float *>(E.staging2((size_t)P.m * 4));
+            HB_CK(cudaMemcpyAsync(const_cast<float *>(h_val), P.pts_val, (size_t)P.m * 4, cudaMemcpyDeviceToHost, st));
+            HB_CK(cudaEventRecord(E.ev_[21], st));
+        }
         const Plan pl = plan_f.get();
         E.stats.plan_ms = plan_ms;
         DevSearch S = run_search(E, pl, P, d_mask, 0, st, false, (opt.flags & 4u) != 0);
+        if (auto_mean)
+        {
+            HB_CK(cudaEventSynchronize(E.ev_[21]));
+            double sum = 0;
+            for (int i = 0; i < P.m; ++i) sum += h_val[i];
+            mean = sum / P.m;
+        }
         HB_CK(cudaEventRecord(E.ev_[3], st));
         SolveOut so{};
         so.out_data = d_out;
@@ -1120,6 +1105,15 @@ int indicator_kriging(const int *dims, const unsigned char *in_data, const unsig
         long long n = check_dims(dims);
         const int m = (int)cats.size();
         if (m < 1) throw CudaFail{-1, "indicator_count must be positive"};
+        // A category's host tables are built while the device uploads the grid or
+        // works on the category before.
+        auto plan_of = [&](int c) {
+            return std::async(std::launch::async, [&cats, dims, c]() {
+                const IkArgs &a = cats[c];
+                return make_plan(true, a.cov_type, a.ranges, a.angles, a.sill, a.nugget, a.radiuses, a.max_nb, dims);
+            });
+        };
+        std::future<Plan> next = plan_of(0);
         Engine &E = engine_for_current_device();
         cudaStream_t st = E.stream(opt.stream);
         IoPlan io{(opt.flags & 1u) != 0, st};
@@ -1131,16 +1125,13 @@ int indicator_kriging(const int *dims, const unsigned char *in_data, const unsig
         float *d_probs = (io.device && opt.ik_probs) ? opt.ik_probs : E.buf<float>("ik_probs", (size_t)n * m);
         signed char *d_status = E.buf<signed char>("status", (size_t)n);
         HB_CK(cudaEventRecord(E.ev_[2], st));
-        Plan pl0 = make_plan(true, cats[0].cov_type, cats[0].ranges, cats[0].angles, cats[0].sill, cats[0].nugget,
-                             cats[0].radiuses, cats[0].max_nb, dims);
-        DevPoints P = compact_points(E, pl0.g, d_mask, nullptr, d_in, st);
+        DevPoints P = compact_points(E, grid_geom(dims), d_mask, nullptr, d_in, st);
         float search_ms = 0, solve_ms = 0;
         for (int c = 0; c < m; ++c)
         {
             const IkArgs &a = cats[c];
-            Plan pl = c == 0 ? pl0
-                             : make_plan(true, a.cov_type, a.ranges, a.angles, a.sill, a.nugget, a.radiuses, a.max_nb,
-                                         dims);
+            const Plan pl = next.get();
+            if (c + 1 < m) next = plan_of(c + 1);
             HB_CK(cudaEventRecord(E.ev_[5], st));
             DevSearch S = run_search(E, pl, P, d_mask, 1, st, false, (opt.flags & 4u) != 0);
             HB_CK(cudaEventRecord(E.ev_[6], st));
@@ -1441,8 +1432,15 @@ int sgs_simulation(const int *dims, float *data, unsigned char *mask, const unsi
         }
         E.mark(STAGE_COMPACT, st);
 
+        auto plan_pair = plan_f.get();
+        const Plan &pl = plan_pair.first;
+        const std::vector<Offset> &tv = plan_pair.second;
+        E.stats.plan_ms = plan_ms;
+
         // the draws: one uniform per simulated node in walk order, generated on
-        // the host while the device searches and levels
+        // the host while the device searches, levels and solves. They start once
+        // the tables are there: beside them they took the host's cores and kept
+        // the device waiting (tables 10.8 ms of a million cells, against 2.7).
         double *h_u = reinterpret_cast<double *>(E.staging2((size_t)std::max(n_sim, 1) * 8));
         double draws_ms = 0.0;
         auto draws_f = std::async(std::launch::async, [&, n_sim]() {
@@ -1451,10 +1449,6 @@ int sgs_simulation(const int *dims, float *data, unsigned char *mask, const unsi
             draws_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
         });
 
-        auto plan_pair = plan_f.get();
-        const Plan &pl = plan_pair.first;
-        const std::vector<Offset> &tv = plan_pair.second;
-        E.stats.plan_ms = plan_ms;
         const Geom &g = pl.g;
         const size_t nk = pl.kt.vals.size();
         double *search_vals = E.buf<double>("search_vals", nk);
@@ -1679,20 +1673,27 @@ int sis_simulation(const int *dims, unsigned char *data, unsigned char *mask, co
         if (!sgs_walk(n, seed, walk))
             throw CudaFail{-1, "the simulation path does not visit every node of a grid of this size"};
         if (walk.R0 < 0) throw CudaFail{-1, "seed % grid size must not be negative"};
+        // the categories' host tables, one after another, each handed over as soon
+        // as it is built: the device searches a category while the next is built
+        using SisPlan = std::pair<Plan, std::vector<Offset>>;
         double plan_ms = 0.0;
+        std::vector<std::promise<SisPlan>> plan_p(kcat);
         auto plan_f = std::async(std::launch::async, [&]() {
             const auto t0 = std::chrono::steady_clock::now();
-            std::vector<std::pair<Plan, std::vector<Offset>>> v;
             for (int c = 0; c < kcat; ++c)
-            {
-                const IkArgs &a = cats[c];
-                Plan p = make_plan(true, a.cov_type, a.ranges, a.angles, a.sill, a.nugget, a.radiuses, a.max_nb, dims,
-                                   false);
-                std::vector<Offset> tv = build_template(p.f, p.kt);
-                v.emplace_back(std::move(p), std::move(tv));
-            }
+                try
+                {
+                    const IkArgs &a = cats[c];
+                    Plan p = make_plan(true, a.cov_type, a.ranges, a.angles, a.sill, a.nugget, a.radiuses, a.max_nb,
+                                       dims, false);
+                    std::vector<Offset> tv = build_template(p.f, p.kt);
+                    plan_p[c].set_value(SisPlan(std::move(p), std::move(tv)));
+                }
+                catch (...)
+                {
+                    plan_p[c].set_exception(std::current_exception());
+                }
             plan_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-            return v;
         });
         Engine &E = engine_for_current_device();
         cudaStream_t st = E.stream(opt.stream);
@@ -1737,17 +1738,7 @@ int sis_simulation(const int *dims, unsigned char *data, unsigned char *mask, co
             E.stats.launches += 2 + scan_kernels(n);
         }
         E.mark(STAGE_COMPACT, st);
-        double *h_u = reinterpret_cast<double *>(E.staging2((size_t)std::max(n_sim, 1) * 8));
-        double draws_ms = 0.0;
-        auto draws_f = std::async(std::launch::async, [&, n_sim]() {
-            const auto t0 = std::chrono::steady_clock::now();
-            sgs_draws((unsigned long long)seed, n_sim, h_u);
-            draws_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-        });
-
         // per category: pair table, template, search (ranks into one merged row per node)
-        auto plans = plan_f.get();
-        E.stats.plan_ms = plan_ms;
         int ktot = 0;
         std::vector<int> koff(kcat);
         for (int c = 0; c < kcat; ++c)
@@ -1760,8 +1751,10 @@ int sis_simulation(const int *dims, unsigned char *data, unsigned char *mask, co
         HB_CK(cudaMemsetAsync(nb_rank, 0xFF, ns * ktot * 4, st)); // -1: no neighbour
         std::vector<double *> pair64(kcat);
         std::vector<int *> nb(kcat), nb_lin(kcat), nb_cnt(kcat);
+        std::vector<SisPlan> plans;
         for (int c = 0; c < kcat; ++c)
         {
+            plans.push_back(plan_p[c].get_future().get());
             const Plan &pl = plans[c].first;
             const std::vector<Offset> &tv = plans[c].second;
             const Geom &g = pl.g;
@@ -1785,9 +1778,20 @@ int sis_simulation(const int *dims, unsigned char *data, unsigned char *mask, co
                 launch_sgs_search(g, tmpl, (int)t4.size(), sim_cells, n_sim, rank_of, cats[c].max_nb, nb[c], nb_lin[c],
                                   nb_rank + koff[c], nb_cnt[c], E.n_sm(), st, -1, ktot);
             HB_CK(cudaGetLastError());
-            HB_CK(cudaStreamSynchronize(st)); // the host tables of this category
+            if (c + 1 < kcat) HB_CK(cudaStreamSynchronize(st)); // the host tables of this category
             E.stats.launches += 1 + (n_sim > 0 ? 1 : 0);
         }
+        plan_f.get();
+        E.stats.plan_ms = plan_ms;
+        // the draws, generated on the host once its cores are free of the tables
+        double *h_u = reinterpret_cast<double *>(E.staging2((size_t)std::max(n_sim, 1) * 8));
+        double draws_ms = 0.0;
+        auto draws_f = std::async(std::launch::async, [&, n_sim]() {
+            const auto t0 = std::chrono::steady_clock::now();
+            sgs_draws((unsigned long long)seed, n_sim, h_u);
+            draws_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+        });
+        HB_CK(cudaStreamSynchronize(st));
         E.mark(STAGE_SEARCH, st);
 
         // the solves' size moments over every category's systems
