@@ -1284,68 +1284,74 @@ struct RankLess
 };
 
 // partition_around_front (libstdc++'s unguarded partition with the pivot at lo)
-// by a warp. On the array as it stands, let L be the positions in (lo, hi) that
-// stop the left scan (not less than the pivot), ascending, and R those in
-// [lo, hi) that stop the right scan (pivot not less than them), descending.
-// The serial loop swaps a[L[m]] and a[R[m]] while L[m] < R[m]; every such L
-// lies below every such R, so the swaps are disjoint and independent, and the
-// loop returns min(L[M], R[M-1]) for the first M with L[M] >= R[M] (an exhausted
-// L counts as +inf, R[-1] as +inf). lstop / rstop hold hi - lo positions each
-// (16-bit: candidate lists stay below 65,536 entries).
+// by a warp, 32 entries from the left and 32 from the right at a time. The m-th
+// position from the left that stops the left scan (not less than the pivot), L[m],
+// and the m-th from the right that stops the right scan (pivot not less than it),
+// R[m], are swapped by the serial loop while L[m] < R[m], and it returns
+// min(L[M], R[M-1]) for the first M with L[M] >= R[M] (an exhausted L counts as
+// +inf, R[-1] as +inf). The pairs of two blocks are disjoint, so the lanes of a
+// block's left stops swap theirs at once; a block whose stops are used up is
+// followed by the next. Blocks loaded past the crossing may hold swapped entries:
+// those stop the left scan at some R[m] with m < M at the earliest, where the
+// minimum stands anyway, and stop the right scan only below L[M]. Position lo
+// stops the right scan and pairs with no left stop, so the right blocks end there.
+// ex holds 32 (entry, position) pairs of the warp.
 template <typename Less>
-__device__ int warp_partition_around_front(uint32_t *a, int lo, int hi, Less less, uint16_t *lstop, uint16_t *rstop,
-                                           int lane)
+__device__ int warp_partition_around_front(uint32_t *a, int lo, int hi, Less less, uint2 *ex, int lane)
 {
     const uint32_t pivot = a[lo];
-    int nr = 0;
-    for (int top = hi - 1; top >= lo; top -= 32)
+    int li = lo + 1, ri = hi - 1; // the next blocks
+    int pl = 0, pr = 0;           // this lane's position in the present ones
+    uint32_t vl = 0, vr = 0;
+    unsigned bl = 0, br = 0; // their unused stops
+    int last = 0x7fffffff;   // R[M-1]
+    for (;;)
     {
-        const int j = top - lane;
-        const bool st = j >= lo && !less(pivot, a[j]);
-        const unsigned bl = __ballot_sync(0xffffffffu, st);
-        if (st) rstop[nr + __popc(bl & lanemask_lt())] = (uint16_t)j;
-        nr += __popc(bl);
-    }
-    __syncwarp();
-    int nl = 0, M = -1, LM = 0x7fffffff;
-    for (int base = lo + 1; base < hi; base += 32)
-    {
-        const int i = base + lane;
-        const bool st = i < hi && !less(a[i], pivot);
-        const unsigned bl = __ballot_sync(0xffffffffu, st);
-        const int m = nl + __popc(bl & lanemask_lt());
-        const bool cross = st && (m >= nr || i >= rstop[m]);
-        if (st && !cross) lstop[m] = (uint16_t)i;
-        const unsigned cb = __ballot_sync(0xffffffffu, cross);
-        if (cb)
+        while (!bl)
         {
-            const int src = __ffs(cb) - 1;
-            M = __shfl_sync(0xffffffffu, m, src);
-            LM = __shfl_sync(0xffffffffu, i, src);
-            break;
+            if (li >= hi) return last;
+            pl = li + lane;
+            vl = pl < hi ? a[pl] : 0u;
+            bl = __ballot_sync(0xffffffffu, pl < hi && !less(vl, pivot));
+            li += 32;
         }
-        nl += __popc(bl);
+        while (!br && ri >= lo)
+        {
+            pr = ri - lane;
+            vr = pr >= lo ? a[pr] : 0u;
+            br = __ballot_sync(0xffffffffu, pr >= lo && !less(pivot, vr));
+            ri -= 32;
+        }
+        const int c = min(__popc(bl), __popc(br));
+        const int ml = __popc(bl & lanemask_lt()), mr = __popc(br & lanemask_lt());
+        if (br >> lane & 1u) ex[mr] = make_uint2(vr, (uint32_t)pr);
+        __syncwarp();
+        const bool act = (bl >> lane & 1u) && ml < c;
+        const uint2 e = ex[ml];
+        const bool ok = act && pl < (int)e.y;
+        const int v = __popc(__ballot_sync(0xffffffffu, ok));
+        if (ok)
+        {
+            a[pl] = e.x;
+            a[e.y] = vl;
+        }
+        if (v > 0) last = (int)ex[v - 1].y;
+        __syncwarp();
+        if (v < c || c == 0)
+        {
+            const unsigned first = __ballot_sync(0xffffffffu, (bl >> lane & 1u) && ml == v);
+            return min(__shfl_sync(0xffffffffu, pl, __ffs(first) - 1), last);
+        }
+        bl = __ballot_sync(0xffffffffu, (bl >> lane & 1u) && ml >= c);
+        br = __ballot_sync(0xffffffffu, (br >> lane & 1u) && mr >= c);
     }
-    if (M < 0) M = nl;
-    __syncwarp();
-    for (int m = lane; m < M; m += 32)
-    {
-        const int x = lstop[m], y = rstop[m];
-        const uint32_t t = a[x];
-        a[x] = a[y];
-        a[y] = t;
-    }
-    __syncwarp();
-    const int rm1 = M > 0 ? rstop[M - 1] : 0x7fffffff;
-    return LM < rm1 ? LM : rm1;
 }
 
 // gis::select_first_k with the partitions done by the warp (median choice,
 // heapsort fallback and the final short insertion sort by lane 0): the same
 // first-k set std::sort leaves in front.
 template <typename Less>
-__device__ void warp_select_first_k(uint32_t *a, int n, int k, Less less, uint16_t *lstop, uint16_t *rstop,
-                                    int lane)
+__device__ void warp_select_first_k(uint32_t *a, int n, int k, Less less, uint2 *ex, int lane)
 {
     const int kThreshold = 16;
     if (n <= 0 || k <= 0 || k >= n) return;
@@ -1363,7 +1369,7 @@ __device__ void warp_select_first_k(uint32_t *a, int n, int k, Less less, uint16
         const int mid = lo + (hi - lo) / 2;
         if (lane == 0) gis::median_to_front(a, (long)lo, (long)lo + 1, (long)mid, (long)hi - 1, less);
         __syncwarp();
-        const int cut = warp_partition_around_front(a, lo, hi, less, lstop, rstop, lane);
+        const int cut = warp_partition_around_front(a, lo, hi, less, ex, lane);
         if (cut == k) return;
         if (cut > k)
             hi = cut;
@@ -1374,13 +1380,25 @@ __device__ void warp_select_first_k(uint32_t *a, int n, int k, Less less, uint16
     __syncwarp();
 }
 
-// shared memory of one warp: the 27 bins' list offsets and starts, the list
-// (key and slot), the point ids, the two stop lists
-__host__ __device__ inline size_t ties_warp_bytes(int cap) { return 256 + ((size_t)cap * 12 + 15) / 16 * 16; }
+// shared memory of one warp: the 9 runs' list offsets and starts, the partition's
+// 32 pairs, the list (key and place in the unfiltered list: the point is found
+// again from the place, so that a candidate takes 4 bytes)
+__host__ __device__ inline size_t ties_warp_bytes(int cap) { return 384 + ((size_t)cap * 4 + 15) / 16 * 16; }
 
 // chunks of 32 candidates whose loads a warp has in flight at once while it
 // builds a cell's list
 constexpr int kTieChunks = 4;
+
+// the last of the 9 runs whose offset in the list is <= gi; the offsets past the
+// ninth are past every place
+__device__ __forceinline__ int run_of(const int *pre, int gi)
+{
+    int b = pre[8] <= gi ? 8 : 0;
+#pragma unroll
+    for (int st = 4; st > 0; st >>= 1)
+        if (pre[b + st] <= gi) b += st;
+    return b;
+}
 
 template <int E>
 __global__ void __launch_bounds__(128) k_resolve_ties_fast(
@@ -1391,43 +1409,44 @@ __global__ void __launch_bounds__(128) k_resolve_ties_fast(
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    int *bpre = reinterpret_cast<int *>(smem + (size_t)warp * ties_warp_bytes(cap)); // 28: list offsets
-    int *bst = bpre + 32;                                                                // 27: bin starts
-    uint32_t *arr = reinterpret_cast<uint32_t *>(bpre + 64);
-    int *pid = reinterpret_cast<int *>(arr + cap);
-    uint16_t *lstop = reinterpret_cast<uint16_t *>(pid + cap), *rstop = lstop + cap;
+    int *pre = reinterpret_cast<int *>(smem + (size_t)warp * ties_warp_bytes(cap)); // 16: list offsets
+    int *rst = pre + 16;                                                            // 9: run starts
+    uint2 *ex = reinterpret_cast<uint2 *>(pre + 32);
+    uint32_t *arr = reinterpret_cast<uint32_t *>(pre + 96);
     const int n_ties = *tie_count;
     for (int t = blockIdx.x * nwarps + warp; t < n_ties; t += gridDim.x * nwarps)
     {
         const int cell = tie_cells[t];
         const int x = cell % g.nx, y = cell % (g.nx * g.ny) / g.nx, z = cell / (g.nx * g.ny);
         const int bxi = x / g.rx, byi = y / g.ry, bzi = z / g.rz;
-        // the 27 bins (z, y, x nested) as one list: lane q < 27 holds bin q's
-        // start and count, the prefix sums give each bin's offset in the list
+        // the 27 bins (z, y, x nested) as one list: the three bins along x lie one
+        // after another in bin_pts, so lane q < 9 holds run q's start and count,
+        // and the prefix sums give each run's offset in the list
         int bs = 0, bc = 0;
-        if (lane < 27)
+        if (lane < 9)
         {
-            const int kk = bzi - 1 + lane / 9, jj = byi - 1 + (lane / 3) % 3, ii = bxi - 1 + lane % 3;
-            if (ii >= 0 && jj >= 0 && kk >= 0 && ii < g.bx && jj < g.by && kk < g.bz)
+            const int kk = bzi - 1 + lane / 3, jj = byi - 1 + lane % 3;
+            if (jj >= 0 && kk >= 0 && jj < g.by && kk < g.bz)
             {
-                const int nb = (kk * g.by + jj) * g.bx + ii;
-                bs = bin_start[nb];
-                bc = bin_cnt[nb];
+                const int row = (kk * g.by + jj) * g.bx;
+                const int i0 = max(bxi - 1, 0), i1 = min(bxi + 1, g.bx - 1);
+                bs = bin_start[row + i0];
+                bc = bin_start[row + i1] + bin_cnt[row + i1] - bs;
             }
         }
         int incl = bc;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
+        for (int o = 1; o < 16; o <<= 1)
         {
             const int tv = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += tv;
         }
-        const int total = __shfl_sync(0xffffffffu, incl, 26);
-        __syncwarp(); // the previous cell's reads of bpre / bst are done
-        if (lane < 27)
+        const int total = min(__shfl_sync(0xffffffffu, incl, 8), cap); // cap bounds every candidate list
+        __syncwarp(); // the previous cell's reads are done
+        if (lane < 16)
         {
-            bpre[lane] = incl - bc;
-            bst[lane] = bs;
+            pre[lane] = lane < 9 ? incl - bc : 0x7fffffff;
+            rst[lane] = bs;
         }
         __syncwarp();
         // kTieChunks chunks of 32 list entries at a time: their three dependent
@@ -1446,11 +1465,8 @@ __global__ void __launch_bounds__(128) k_resolve_ties_fast(
                 p[u] = -1;
                 if (gi < total)
                 {
-                    int b = 0; // the last bin whose offset is <= gi
-#pragma unroll
-                    for (int st = 16; st > 0; st >>= 1)
-                        if (b + st <= 26 && bpre[b + st] <= gi) b += st;
-                    p[u] = bin_pts[bst[b] + gi - bpre[b]];
+                    const int b = run_of(pre, gi);
+                    p[u] = bin_pts[rst[b] + gi - pre[b]];
                 }
             }
 #pragma unroll
@@ -1471,18 +1487,12 @@ __global__ void __launch_bounds__(128) k_resolve_ties_fast(
             {
                 const bool keep = key[u] != 0xFFFFu;
                 const unsigned bl = __ballot_sync(0xffffffffu, keep);
-                const int slot = n + __popc(bl & lanemask_lt());
-                if (keep && slot < cap)
-                {
-                    arr[slot] = (key[u] << 16) | (uint32_t)slot;
-                    pid[slot] = p[u];
-                }
+                if (keep) arr[n + __popc(bl & lanemask_lt())] = (key[u] << 16) | (uint32_t)(base + 32 * u + lane);
                 n += __popc(bl);
             }
         }
-        if (n > cap) n = cap; // cannot happen: cap bounds every candidate list
         __syncwarp();
-        warp_select_first_k(arr, n, g.k, RankLess(), lstop, rstop, lane);
+        warp_select_first_k(arr, n, g.k, RankLess(), ex, lane);
         const int m = n < g.k ? n : g.k;
         uint32_t v[E];
 #pragma unroll
@@ -1499,8 +1509,9 @@ __global__ void __launch_bounds__(128) k_resolve_ties_fast(
             const int i = e * 32 + lane;
             if (i < m)
             {
-                const int j = (int)(v[e] & 0xFFFFu);
-                const int p = pid[j];
+                const int gi = (int)(v[e] & 0xFFFFu);
+                const int b = run_of(pre, gi);
+                const int p = bin_pts[rst[b] + gi - pre[b]];
                 if (nb_pid) nb_pid[base + i] = p;
                 if (nb_rec)
                 {
