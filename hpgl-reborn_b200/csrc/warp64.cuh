@@ -1,6 +1,6 @@
 // FP64 solves of up to 32 symmetric positive definite systems of covariances
-// with explicit solutions, one system per warp (the simulation and cokriging
-// kernels): the factorisation and forward substitution of mma64.cuh, the factor's
+// with explicit solutions, one system per warp (the simulation, cokriging and
+// leave-one-out kernels): the factorisation and forward substitution of mma64.cuh, the factor's
 // blocks kept in shared memory, and the back substitution from there.
 //
 // Measured against it on the 8.3M systems of the 256x256x128 simulation: four
@@ -27,17 +27,15 @@ struct __align__(16) WarpSmem
 // offset of the 16-byte chunk of (r, 2q) in a block
 __device__ __forceinline__ int blk_chunk(int r, int q) { return 4 * r + (q ^ ((r >> 1) & 3)); }
 
-// The factorisation of the warp's system of n unknowns (nb = ceil(n / 8) block
-// rows) with the forward substitution of its Q right-hand sides, T.y in place.
-// T.lin, T.y (and T.sig) must be visible. Returns whether a pivot failed.
+// The factorisation of the warp's system A of nb block rows with the forward
+// substitution of its Q right-hand sides, T.y in place (it must be visible).
+// Returns whether a pivot failed.
 template <int Q, bool EPS_PIVOT, bool SCALE>
-__device__ __forceinline__ bool warp_factor(WarpSmem<Q, SCALE> &T, int lane, int n, int nb,
-                                            const double *__restrict__ pair_c)
+__device__ __forceinline__ bool warp_eliminate(WarpSmem<Q, SCALE> &T, int lane, int nb, Blk (&A)[1][kWarpBlocks])
 {
     constexpr int NB = kWarpNB;
     const int r = lane >> 2, q = lane & 3;
-    Blk A[1][kWarpBlocks], X[1][NB];
-    mma_load<NB>(A[0], pair_c, T.lin, n, nb, lane);
+    Blk X[1][NB];
 #pragma unroll
     for (int k = 0; k < NB; ++k)
     {
@@ -46,24 +44,6 @@ __device__ __forceinline__ bool warp_factor(WarpSmem<Q, SCALE> &T, int lane, int
         {
             const double2 v = reinterpret_cast<const double2 *>(&T.y[r][8 * k])[q];
             X[0][k] = Blk{v.x, v.y};
-        }
-    }
-    if constexpr (SCALE)
-    {
-        // A[i][c] = pair * (sig_i * sig_c) for live entries (padding rows: sig 1)
-#pragma unroll
-        for (int i = 0; i < NB; ++i)
-        {
-            if (i >= nb) break;
-            const double si = T.sig[8 * i + r];
-#pragma unroll
-            for (int k = 0; k <= i; ++k)
-            {
-                const double2 sc = reinterpret_cast<const double2 *>(&T.sig[8 * k])[q];
-                Blk &b = A[0][blk_at(i, k)];
-                b.x = __dmul_rn(b.x, __dmul_rn(si, sc.x));
-                b.y = __dmul_rn(b.y, __dmul_rn(si, sc.y));
-            }
         }
     }
     bool fail[1] = {false};
@@ -82,6 +62,37 @@ __device__ __forceinline__ bool warp_factor(WarpSmem<Q, SCALE> &T, int lane, int
     }
     __syncwarp();
     return fail[0];
+}
+
+// The same for the system of n unknowns read from a pair table (nb = ceil(n / 8));
+// T.lin (and T.sig) must be visible too.
+template <int Q, bool EPS_PIVOT, bool SCALE>
+__device__ __forceinline__ bool warp_factor(WarpSmem<Q, SCALE> &T, int lane, int n, int nb,
+                                            const double *__restrict__ pair_c)
+{
+    constexpr int NB = kWarpNB;
+    const int r = lane >> 2, q = lane & 3;
+    Blk A[1][kWarpBlocks];
+    mma_load<NB>(A[0], pair_c, T.lin, n, nb, lane);
+    if constexpr (SCALE)
+    {
+        // A[i][c] = pair * (sig_i * sig_c) for live entries (padding rows: sig 1)
+#pragma unroll
+        for (int i = 0; i < NB; ++i)
+        {
+            if (i >= nb) break;
+            const double si = T.sig[8 * i + r];
+#pragma unroll
+            for (int k = 0; k <= i; ++k)
+            {
+                const double2 sc = reinterpret_cast<const double2 *>(&T.sig[8 * k])[q];
+                Blk &b = A[0][blk_at(i, k)];
+                b.x = __dmul_rn(b.x, __dmul_rn(si, sc.x));
+                b.y = __dmul_rn(b.y, __dmul_rn(si, sc.y));
+            }
+        }
+    }
+    return warp_eliminate<Q, EPS_PIVOT, SCALE>(T, lane, nb, A);
 }
 
 // The back substitution of the warp's own system, L^T x = y, T.y in place: lane

@@ -138,6 +138,7 @@ EXPORTS = [
     "hpgl_b200_find_neighbours", "hpgl_b200_last_stats", "hpgl_b200_host_alloc", "hpgl_b200_host_free",
     "hpgl_b200_transform", "hpgl_b200_template", "hpgl_b200_covariance", "hpgl_b200_version",
     "hpgl_b200_sk_weights_noalloc", "hpgl_b200_loo_ok", "hpgl_b200_loo_ok_adjoint",
+    "hpgl_b200_loo_ok_device", "hpgl_b200_loo_ok_adjoint_device",
     "hpgl_b200_solve_variant", "hpgl_b200_solve_variant_get", "hpgl_b200_tune_mode", "hpgl_b200_tune_load",
     "hpgl_b200_tune_save", "hpgl_b200_tune_reset",
 ]
@@ -279,6 +280,11 @@ def _load():
     lib.hpgl_b200_loo_ok.argtypes = loo_common + [vp, vp, vp]
     lib.hpgl_b200_loo_ok_adjoint.restype = C.c_int
     lib.hpgl_b200_loo_ok_adjoint.argtypes = loo_common + [vp, vp, vp, vp]
+    loo_device = loo_common[:9] + [vp, C.c_double, vp, vp]
+    lib.hpgl_b200_loo_ok_device.restype = C.c_int
+    lib.hpgl_b200_loo_ok_device.argtypes = loo_device + [vp, vp, vp]
+    lib.hpgl_b200_loo_ok_adjoint_device.restype = C.c_int
+    lib.hpgl_b200_loo_ok_adjoint_device.argtypes = loo_device + [vp, vp, vp, vp]
     return lib
 
 

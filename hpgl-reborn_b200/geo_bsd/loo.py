@@ -102,11 +102,24 @@ def loo_geometry(prop, grid, radiuses: Sequence[int], max_neighbours: int, cov_m
                        nodes=nodes)
 
 
-def _loo_args(geom: LooGeometry, M, r0: float, sill: float, nugget: float, values):
-    m9 = (C.c_double * 9)(*[float(v) for v in M.detach().reshape(-1).cpu().tolist()])
-    return (geom.pts_xyz.data_ptr(), values.data_ptr(), int(values.numel()), geom.targets.data_ptr(),
-            geom.nb_idx.data_ptr(), geom.nb_cnt.data_ptr(), int(geom.targets.numel()), geom.k, geom.cov_type,
-            m9, float(r0), float(sill), float(nugget))
+def _loo_call(name: str, geom: LooGeometry, M, r0: float, sill, nugget, values, stream, outputs):
+    """hpgl_b200_<name> on `stream`. A variogram that lies on the values' device is
+    read there by the kernel (reading it here would wait for the device three times
+    a call); any other is passed as host numbers."""
+    points = (geom.pts_xyz.data_ptr(), values.data_ptr(), int(values.numel()), geom.targets.data_ptr(),
+              geom.nb_idx.data_ptr(), geom.nb_cnt.data_ptr(), int(geom.targets.numel()), geom.k, geom.cov_type)
+    tail = [t.data_ptr() for t in outputs] + [stream.cuda_stream]
+    par = (M, sill, nugget)
+    if all(torch.is_tensor(t) and t.device == values.device and t.dtype == torch.float64 for t in par):
+        par = tuple(t.detach().contiguous() for t in par)
+        for t in par:
+            t.record_stream(stream)
+        rc = getattr(W._hpgl_so, name + "_device")(*points, par[0].data_ptr(), float(r0), par[1].data_ptr(),
+                                                    par[2].data_ptr(), *tail)
+    else:
+        m9 = (C.c_double * 9)(*[float(v) for v in M.detach().reshape(-1).cpu().tolist()])
+        rc = getattr(W._hpgl_so, name)(*points, m9, float(r0), float(sill), float(nugget), *tail)
+    W.check(rc, name)
 
 
 class LooKriging(torch.autograd.Function):
@@ -119,10 +132,8 @@ class LooKriging(torch.autograd.Function):
         values = values.detach().contiguous()
         zhat = torch.empty(geom.targets.numel(), dtype=torch.float64, device=values.device)
         status = torch.empty(geom.targets.numel(), dtype=torch.int8, device=values.device)
-        stream = torch.cuda.current_stream(values.device).cuda_stream
-        rc = W._hpgl_so.hpgl_b200_loo_ok(*_loo_args(geom, M, r0, float(sill), float(nugget), values),
-                                         zhat.data_ptr(), status.data_ptr(), stream)
-        W.check(rc, "hpgl_b200_loo_ok")
+        _loo_call("hpgl_b200_loo_ok", geom, M, r0, sill, nugget, values, torch.cuda.current_stream(values.device),
+                  (zhat, status))
         ctx.save_for_backward(M.detach(), torch.as_tensor(sill).detach(), torch.as_tensor(nugget).detach(), values)
         ctx.geom, ctx.r0 = geom, r0
         ctx.mark_non_differentiable(status)
@@ -135,10 +146,8 @@ class LooKriging(torch.autograd.Function):
         g = g_zhat.detach().to(torch.float64).contiguous()
         grad_values = torch.zeros_like(values)
         grad_params = torch.zeros(11, dtype=torch.float64, device=values.device)
-        stream = torch.cuda.current_stream(values.device).cuda_stream
-        rc = W._hpgl_so.hpgl_b200_loo_ok_adjoint(*_loo_args(geom, M, ctx.r0, float(sill), float(nugget), values),
-                                                 g.data_ptr(), grad_values.data_ptr(), grad_params.data_ptr(), stream)
-        W.check(rc, "hpgl_b200_loo_ok_adjoint")
+        _loo_call("hpgl_b200_loo_ok_adjoint", geom, M, ctx.r0, sill, nugget, values,
+                  torch.cuda.current_stream(values.device), (g, grad_values, grad_params))
         gM = grad_params[:9].reshape(3, 3).to(M.device)
         return gM, grad_params[9], grad_params[10], grad_values, None, None
 

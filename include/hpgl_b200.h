@@ -422,6 +422,16 @@ int hpgl_b200_loo_ok_adjoint(const int *pts_xyz, const double *values, int n_pts
                              const int *nb_idx, const int *nb_cnt, int n_targets, int k, int cov_type,
                              const double *M, double r0, double sill, double nugget, const double *grad_zhat,
                              double *grad_values, double *grad_params, void *stream);
+/* The same with M, sill and nugget in device memory: nothing is read on the host,
+ * so the calls only queue work. The arrays are read when the kernel runs. */
+int hpgl_b200_loo_ok_device(const int *pts_xyz, const double *values, int n_pts, const int *targets,
+                            const int *nb_idx, const int *nb_cnt, int n_targets, int k, int cov_type,
+                            const double *M, double r0, const double *sill, const double *nugget, double *zhat,
+                            signed char *status, void *stream);
+int hpgl_b200_loo_ok_adjoint_device(const int *pts_xyz, const double *values, int n_pts, const int *targets,
+                                    const int *nb_idx, const int *nb_cnt, int n_targets, int k, int cov_type,
+                                    const double *M, double r0, const double *sill, const double *nugget,
+                                    const double *grad_zhat, double *grad_values, double *grad_params, void *stream);
 
 /* Page-locked host buffers for fast copies (cudaHostAlloc / cudaFreeHost). */
 void *hpgl_b200_host_alloc(size_t bytes);
