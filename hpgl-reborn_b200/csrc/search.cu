@@ -1389,17 +1389,6 @@ __host__ __device__ inline size_t ties_warp_bytes(int cap) { return 384 + ((size
 // builds a cell's list
 constexpr int kTieChunks = 4;
 
-// the last of the 9 runs whose offset in the list is <= gi; the offsets past the
-// ninth are past every place
-__device__ __forceinline__ int run_of(const int *pre, int gi)
-{
-    int b = pre[8] <= gi ? 8 : 0;
-#pragma unroll
-    for (int st = 4; st > 0; st >>= 1)
-        if (pre[b + st] <= gi) b += st;
-    return b;
-}
-
 template <int E>
 __global__ void __launch_bounds__(128) k_resolve_ties_fast(
     const Geom g, const int *__restrict__ tie_cells, const int *__restrict__ tie_count,
@@ -1418,36 +1407,9 @@ __global__ void __launch_bounds__(128) k_resolve_ties_fast(
     {
         const int cell = tie_cells[t];
         const int x = cell % g.nx, y = cell % (g.nx * g.ny) / g.nx, z = cell / (g.nx * g.ny);
-        const int bxi = x / g.rx, byi = y / g.ry, bzi = z / g.rz;
-        // the 27 bins (z, y, x nested) as one list: the three bins along x lie one
-        // after another in bin_pts, so lane q < 9 holds run q's start and count,
-        // and the prefix sums give each run's offset in the list
-        int bs = 0, bc = 0;
-        if (lane < 9)
-        {
-            const int kk = bzi - 1 + lane / 3, jj = byi - 1 + lane % 3;
-            if (jj >= 0 && kk >= 0 && jj < g.by && kk < g.bz)
-            {
-                const int row = (kk * g.by + jj) * g.bx;
-                const int i0 = max(bxi - 1, 0), i1 = min(bxi + 1, g.bx - 1);
-                bs = bin_start[row + i0];
-                bc = bin_start[row + i1] + bin_cnt[row + i1] - bs;
-            }
-        }
-        int incl = bc;
-#pragma unroll
-        for (int o = 1; o < 16; o <<= 1)
-        {
-            const int tv = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += tv;
-        }
-        const int total = min(__shfl_sync(0xffffffffu, incl, 8), cap); // cap bounds every candidate list
         __syncwarp(); // the previous cell's reads are done
-        if (lane < 16)
-        {
-            pre[lane] = lane < 9 ? incl - bc : 0x7fffffff;
-            rst[lane] = bs;
-        }
+        const int total = min(candidate_runs(g, x / g.rx, y / g.ry, z / g.rz, bin_start, bin_cnt, lane, pre, rst),
+                              cap); // cap bounds every candidate list
         __syncwarp();
         // kTieChunks chunks of 32 list entries at a time: their three dependent
         // loads (point, coordinates, key) in flight together, then the chunks

@@ -20,4 +20,48 @@ __device__ __forceinline__ float4 surr_coords(const SurrDev &sd, int x, int y, i
                        fmaf(sd.T[5], fz, fmaf(sd.T[4], fy, sd.T[3] * fx)),
                        fmaf(sd.T[8], fz, fmaf(sd.T[7], fy, sd.T[6] * fx)), 0.0f);
 }
+
+// The candidates of the 27 bins around bin (bxi, byi, bzi), z, y and x nested, as
+// one list: the three bins along x lie one after another in bin_pts, so the list
+// is nine runs. Lanes 0 to 15 of a warp write the runs' offsets in the list (past
+// the ninth: past every place) and their starts in bin_pts; returns the length.
+__device__ __forceinline__ int candidate_runs(const Geom &g, int bxi, int byi, int bzi, const int *bin_start,
+                                              const int *bin_cnt, int lane, int *pre, int *start)
+{
+    int bs = 0, bc = 0;
+    if (lane < 9)
+    {
+        const int kk = bzi - 1 + lane / 3, jj = byi - 1 + lane % 3;
+        if (jj >= 0 && kk >= 0 && jj < g.by && kk < g.bz)
+        {
+            const int row = (kk * g.by + jj) * g.bx;
+            const int i0 = max(bxi - 1, 0), i1 = min(bxi + 1, g.bx - 1);
+            bs = bin_start[row + i0];
+            bc = bin_start[row + i1] + bin_cnt[row + i1] - bs;
+        }
+    }
+    int incl = bc;
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1)
+    {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane < 16)
+    {
+        pre[lane] = lane < 9 ? incl - bc : 0x7fffffff;
+        start[lane] = bs;
+    }
+    return __shfl_sync(0xffffffffu, incl, 8);
+}
+
+// the last of the nine runs whose offset in the list is <= i
+__device__ __forceinline__ int run_of(const int *pre, int i)
+{
+    int b = pre[8] <= i ? 8 : 0;
+#pragma unroll
+    for (int st = 4; st > 0; st >>= 1)
+        if (pre[b + st] <= i) b += st;
+    return b;
+}
 } // namespace hb

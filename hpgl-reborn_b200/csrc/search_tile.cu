@@ -99,44 +99,31 @@ __global__ void __launch_bounds__(256) k_search_tile(
     uint32_t *list = lists + threadIdx.x;
     uint16_t *sub = reinterpret_cast<uint16_t *>(lists + (size_t)cap * ld) + warp * tl.sub;
 
-    __shared__ int s_off[28];
+    // candidates of the 27 bins around, in the reference's order: every thread
+    // finds its own in the nine runs, so that their dependent loads (point,
+    // coordinates, value) are waited for together (a bin at a time, a block with
+    // few candidates waited 27 times)
+    __shared__ int s_pre[16], s_start[16], s_total;
     if (threadIdx.x < 32)
     {
-        // candidates of the 27 bins around, in the reference's order
-        const int q = threadIdx.x;
-        const int kk = bzi - 1 + q / 9, jj = byi - 1 + (q / 3) % 3, ii = bxi - 1 + q % 3;
-        const bool in = q < 27 && ii >= 0 && jj >= 0 && kk >= 0 && ii < g.bx && jj < g.by && kk < g.bz;
-        const int cnt = in ? bin_cnt[(kk * g.by + jj) * g.bx + ii] : 0;
-        int run = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-        {
-            const int v = __shfl_up_sync(FULL, run, o);
-            if (q >= o) run += v;
-        }
-        if (q < 28) s_off[q] = run - cnt;
+        const int c = candidate_runs(g, bxi, byi, bzi, bin_start, bin_cnt, threadIdx.x, s_pre, s_start);
+        if (threadIdx.x == 0) s_total = c;
     }
     __syncthreads();
-    const int C = s_off[27];
+    const int C = s_total;
     if (C <= tl.c_min || C > tl.c_max) return;
-    for (int q = 0; q < 27; ++q)
+#pragma unroll 2
+    for (int d = threadIdx.x; d < C; d += blockDim.x)
     {
-        const int cnt = s_off[q + 1] - s_off[q];
-        if (cnt == 0) continue;
-        const int kk = bzi - 1 + q / 9, jj = byi - 1 + (q / 3) % 3, ii = bxi - 1 + q % 3;
-        const int s = bin_start[(kk * g.by + jj) * g.bx + ii];
-        for (int i = threadIdx.x; i < cnt; i += blockDim.x)
-        {
-            const int p = bin_pts[s + i];
-            int px, py, pz;
-            unpack_xyz(pts_xyz[p], px, py, pz);
-            const int d = s_off[q] + i;
-            // float coordinates, and the offset into the key table from the bin corner
-            float4 c = surr_coords(sd, px - x0, py - y0, pz - z0);
-            c.w = __int_as_float(((pz - z0) * g.kny + (py - y0)) * g.knx + (px - x0));
-            ctp[d] = c;
-            crec[d] = make_int2(pair_lin(g, px - x0, py - y0, pz - z0), __float_as_int(pts_vf[p]));
-        }
+        const int q = run_of(s_pre, d);
+        const int p = bin_pts[s_start[q] + d - s_pre[q]];
+        int px, py, pz;
+        unpack_xyz(pts_xyz[p], px, py, pz);
+        // float coordinates, and the offset into the key table from the bin corner
+        float4 c = surr_coords(sd, px - x0, py - y0, pz - z0);
+        c.w = __int_as_float(((pz - z0) * g.kny + (py - y0)) * g.knx + (px - x0));
+        ctp[d] = c;
+        crec[d] = make_int2(pair_lin(g, px - x0, py - y0, pz - z0), __float_as_int(pts_vf[p]));
     }
     __syncthreads();
     const int kc0 = (g.khz * g.kny + g.khy) * g.knx + g.khx;
