@@ -702,13 +702,13 @@ static void run_solves(Engine &E, const Plan &pl, const DevPoints &P, const DevS
     if (!(tol > 0.0)) tol = 1e-9;
     (void)P;
     const Geom &g = pl.g;
-    int *bucket_cnt = E.buf<int>("bucket_cnt", kBuckets);
+    PrepareOut *prep = E.buf<PrepareOut>("prepare_out", 1);
+    int *bucket_cnt = prep->cnt;
     int *bucket_off = E.buf<int>("bucket_off", kBuckets + 1);
     const size_t n_tiles = (size_t)prepare_tiles(g.n_cells);
     int *tile_cnt = E.buf<int>("tile_cnt", n_tiles * kBuckets);
     unsigned long long *tile_mom = E.buf<unsigned long long>("tile_mom", n_tiles * kBuckets * 3);
     int2 *cells = E.buf<int2>("cells", (size_t)g.n_cells);
-    unsigned long long *moments = E.buf<unsigned long long>("moments", kBuckets * 3);
     // FP32-refined systems that fail the four-rows-per-lane kernel's check go
     // first to the two-rows-per-lane kernel (classic refinement), and what
     // that does not converge to the FP64 kernel
@@ -730,15 +730,15 @@ static void run_solves(Engine &E, const Plan &pl, const DevPoints &P, const DevS
                     tune_wanted(kBucketNP[b], pl.f.m.type, precision);
     if (any_quad) ref_cells = E.buf<int2>("ref_cells", (size_t)g.n_cells);
     launch_prepare(g, any_share ? solve_share_tile(g) : CellTile{0, 0, 0}, d_mask, all_cells, S.nb_n, d_status,
-                   bucket_cnt, bucket_off, tile_cnt, tile_mom, cells, moments, st);
+                   prep, bucket_off, tile_cnt, tile_mom, cells, st);
     HB_CK(cudaMemsetAsync(esc_cnt, 0, sizeof(int) * 3 * kBuckets, st));
     HB_CK(cudaGetLastError());
     E.stats.launches += 3;
-    int cnt[kBuckets];
-    unsigned long long mom[kBuckets * 3];
-    HB_CK(cudaMemcpyAsync(cnt, bucket_cnt, sizeof(cnt), cudaMemcpyDeviceToHost, st));
-    HB_CK(cudaMemcpyAsync(mom, moments, sizeof(mom), cudaMemcpyDeviceToHost, st));
+    PrepareOut host_prep;
+    HB_CK(cudaMemcpyAsync(&host_prep, prep, sizeof(host_prep), cudaMemcpyDeviceToHost, st));
     HB_CK(cudaStreamSynchronize(st));
+    const int *cnt = host_prep.cnt;
+    const unsigned long long *mom = host_prep.mom;
     E.mark(STAGE_PREPARE, st);
     // one list for every sharing bucket (they run one after another)
     int2 *left_cells = any_share ? E.buf<int2>("left_cells", (size_t)std::max(1, std::max(cnt[2], cnt[3]))) : nullptr;

@@ -191,9 +191,14 @@ void launch_build_pair(const Geom &g, const DevModel &m, int truncated, const do
 // tiles of the stable bucket partition; tile_cnt holds kBuckets ints and tile_mom
 // 3 kBuckets values per tile
 long long prepare_tiles(long long n_cells);
+struct PrepareOut
+{
+    unsigned long long mom[3 * kBuckets]; // sums of n, n^2 and n^3 over a bucket's cells
+    int cnt[kBuckets];                    // and their number
+};
 void launch_prepare(const Geom &g, const CellTile &order, const uint8_t *mask, int all_cells, const int *nb_n,
-                    signed char *status, int *bucket_cnt, int *bucket_off, int *tile_cnt, unsigned long long *tile_mom, int2 *cells,
-                    unsigned long long *moments, cudaStream_t st);
+                    signed char *status, PrepareOut *out, int *bucket_off, int *tile_cnt,
+                    unsigned long long *tile_mom, int2 *cells, cudaStream_t st);
 void launch_finalize_cont(const Geom &g, const float *in_data, signed char *status, int simple, float mean_f,
                           const float *cell_mean, float *out_data, uint8_t *out_mask, double *est64, double *var,
                           cudaStream_t st);

@@ -81,11 +81,27 @@ __device__ __forceinline__ int bucket_of(int n)
 // Per-cell status and the solve work lists, as a stable partition by bucket:
 // the list of every bucket holds its cells in the order `order` (tiles of a
 // few cells each), so the solver's blocks, which take contiguous runs of a
-// list, work on neighbouring cells. Three passes over tiles of kTile cells: counts (and the moments of n
-// per bucket, for the flop count), a one-block scan, and the ordered fill.
-constexpr int kTileThreads = 256, kTileIters = 8, kTile = kTileThreads * kTileIters;
+// list, work on neighbouring cells. Three passes over tiles of 256 to 2,048
+// cells: counts (and the moments of n per bucket, for the flop count), a one-block
+// scan, and the ordered fill. Each pass waits on memory, so a thread's cells are
+// loaded together, and small grids take small tiles (a block's cells more only
+// lengthen its chain of loads). The three, against eight rounds one after
+// another at every size and a scan of one barrier after another: 2,850 cells 11.6
+// against 49 us, 500,000 cells 24 against 60 us, 16.8M cells 339 against 476 us.
+constexpr int kTileThreads = 256, kTileWarps = kTileThreads / 32;
 
-long long prepare_tiles(long long n_cells) { return (n_cells + kTile - 1) / kTile; }
+// rounds of 256 cells a tile: the most that leave four tiles an SM
+static int tile_iters(long long n_cells)
+{
+    int it = 8;
+    while (it > 1 && n_cells < 4LL * 148 * kTileThreads * it) it /= 2;
+    return it;
+}
+long long prepare_tiles(long long n_cells)
+{
+    const long long tile = (long long)kTileThreads * tile_iters(n_cells);
+    return (n_cells + tile - 1) / tile;
+}
 
 __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
 {
@@ -96,57 +112,79 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
 
 // status: -1 informed (not kriged), 1 no neighbours, 3 queued for a solve.
 // tile_cnt[q * T + tile] = cells of bucket q in the tile; tile_mom[(3q + e) * T + tile]
-// = sum of n^(e+1) over them.
-__global__ void __launch_bounds__(kTileThreads) k_prepare(const Geom g, const CellTile order, const uint8_t *__restrict__ mask, int all_cells,
-                                                          const int *__restrict__ nb_n, signed char *__restrict__ status,
-                                                          int *__restrict__ tile_cnt,
+// = sum of n^(e+1) over them (below the last bucket n <= 64: 32 bits hold a tile's).
+template <int ITERS>
+__global__ void __launch_bounds__(kTileThreads) k_prepare(const Geom g, const CellTile order,
+                                                          const uint8_t *__restrict__ mask, int all_cells,
+                                                          const int *__restrict__ nb_n,
+                                                          signed char *__restrict__ status, int *__restrict__ tile_cnt,
                                                           unsigned long long *__restrict__ tile_mom)
 {
+    constexpr unsigned FULL = 0xffffffffu;
     const int T = gridDim.x;
-    const long long base = (long long)blockIdx.x * kTile;
+    const long long base = (long long)blockIdx.x * (kTileThreads * ITERS);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned c[ITERS];
+    int n[ITERS];
+    bool skip[ITERS];
+#pragma unroll
+    for (int it = 0; it < ITERS; ++it)
+    {
+        const long long t = base + it * kTileThreads + threadIdx.x;
+        const bool in = t < g.n_cells;
+        c[it] = in ? tile_cell(g, order, (unsigned)t) : 0u;
+        n[it] = in ? nb_n[c[it]] : -1;
+        skip[it] = in && !all_cells && mask[c[it]];
+    }
     int cnt[kBuckets];
-    unsigned long long mom[kBuckets * 3];
+    unsigned mom[3 * (kBuckets - 1)];
+    unsigned long long big[3] = {0, 0, 0};
 #pragma unroll
     for (int q = 0; q < kBuckets; ++q) cnt[q] = 0;
 #pragma unroll
-    for (int q = 0; q < kBuckets * 3; ++q) mom[q] = 0;
-    for (int it = 0; it < kTileIters; ++it)
-    {
-        const long long t = base + it * kTileThreads + threadIdx.x;
-        int b = -1, n = 0;
-        if (t < g.n_cells)
-        {
-            const unsigned c = tile_cell(g, order, (unsigned)t);
-            if (!all_cells && mask[c])
-                status[c] = -1;
-            else
-            {
-                n = nb_n[c];
-                b = bucket_of(n);
-                status[c] = b < 0 ? 1 : 3;
-            }
-        }
-        const unsigned long long nn = (unsigned long long)n;
+    for (int q = 0; q < 3 * (kBuckets - 1); ++q) mom[q] = 0;
 #pragma unroll
-        for (int q = 0; q < kBuckets; ++q)
+    for (int it = 0; it < ITERS; ++it)
+    {
+        int b = -1;
+        if (skip[it])
+            status[c[it]] = -1;
+        else if (n[it] >= 0)
         {
-            cnt[q] += __popc(__ballot_sync(0xffffffffu, b == q));
+            b = bucket_of(n[it]);
+            status[c[it]] = b < 0 ? 1 : 3;
+        }
+        const unsigned nn = (unsigned)n[it];
+#pragma unroll
+        for (int q = 0; q < kBuckets; ++q) cnt[q] += __popc(__ballot_sync(FULL, b == q));
+#pragma unroll
+        for (int q = 0; q < kBuckets - 1; ++q)
             if (b == q)
             {
                 mom[3 * q] += nn;
                 mom[3 * q + 1] += nn * nn;
                 mom[3 * q + 2] += nn * nn * nn;
             }
+        if (b == kBuckets - 1)
+        {
+            big[0] += nn;
+            big[1] += (unsigned long long)nn * nn;
+            big[2] += (unsigned long long)nn * nn * nn;
         }
     }
-    __shared__ int s_cnt[kTileThreads / 32][kBuckets];
-    __shared__ unsigned long long s_mom[kTileThreads / 32][kBuckets * 3];
+    __shared__ int s_cnt[kTileWarps][kBuckets];
+    __shared__ unsigned long long s_mom[kTileWarps][kBuckets * 3];
 #pragma unroll
-    for (int q = 0; q < kBuckets * 3; ++q)
+    for (int q = 0; q < 3 * (kBuckets - 1); ++q)
     {
-        const unsigned long long v = warp_sum_u64(mom[q]);
+        const unsigned v = __reduce_add_sync(FULL, mom[q]);
         if (lane == 0) s_mom[warp][q] = v;
+    }
+#pragma unroll
+    for (int e = 0; e < 3; ++e)
+    {
+        const unsigned long long v = cnt[kBuckets - 1] ? warp_sum_u64(big[e]) : 0ULL;
+        if (lane == 0) s_mom[warp][3 * (kBuckets - 1) + e] = v;
     }
     if (lane == 0)
     {
@@ -157,145 +195,184 @@ __global__ void __launch_bounds__(kTileThreads) k_prepare(const Geom g, const Ce
     if (threadIdx.x < kBuckets)
     {
         int v = 0;
-        for (int w = 0; w < kTileThreads / 32; ++w) v += s_cnt[w][threadIdx.x];
+        for (int w = 0; w < kTileWarps; ++w) v += s_cnt[w][threadIdx.x];
         tile_cnt[threadIdx.x * T + blockIdx.x] = v;
     }
     else if (threadIdx.x >= 32 && threadIdx.x < 32 + kBuckets * 3)
     {
         const int q = threadIdx.x - 32;
         unsigned long long v = 0;
-        for (int w = 0; w < kTileThreads / 32; ++w) v += s_mom[w][q];
+        for (int w = 0; w < kTileWarps; ++w) v += s_mom[w][q];
         tile_mom[q * T + blockIdx.x] = v;
     }
 }
 
-// One block: exclusive scan of every bucket's tile counts (in place, as offsets
-// into the whole list), bucket totals and offsets, and the moments.
-__global__ void __launch_bounds__(1024) k_prepare_scan(int T, int *__restrict__ tile_cnt,
-                                                       const unsigned long long *__restrict__ tile_mom,
-                                                       int *__restrict__ bucket_cnt, int *__restrict__ bucket_off,
-                                                       unsigned long long *__restrict__ moments)
+__device__ __forceinline__ int warp_scan(int v, int lane)
 {
-    __shared__ int s_part[1024];
-    __shared__ int s_total[kBuckets];
-    const int per = (T + blockDim.x - 1) / blockDim.x;
-    const int t0 = threadIdx.x * per, t1 = min(T, t0 + per);
-    for (int q = 0; q < kBuckets; ++q)
-    {
-        int *tc = tile_cnt + (long long)q * T;
-        int local = 0;
-        for (int t = t0; t < t1; ++t) local += tc[t];
-        s_part[threadIdx.x] = local;
-        __syncthreads();
-        // Hillis-Steele inclusive scan of the per-thread sums
-        for (int o = 1; o < (int)blockDim.x; o <<= 1)
-        {
-            const int v = threadIdx.x >= o ? s_part[threadIdx.x - o] : 0;
-            __syncthreads();
-            s_part[threadIdx.x] += v;
-            __syncthreads();
-        }
-        int run = s_part[threadIdx.x] - local;
-        for (int t = t0; t < t1; ++t)
-        {
-            const int c = tc[t];
-            tc[t] = run;
-            run += c;
-        }
-        if (threadIdx.x == blockDim.x - 1) s_total[q] = s_part[threadIdx.x];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-    {
-        int run = 0;
-        for (int q = 0; q < kBuckets; ++q)
-        {
-            bucket_cnt[q] = s_total[q];
-            bucket_off[q] = run;
-            run += s_total[q];
-        }
-        bucket_off[kBuckets] = run;
-    }
-    // moments: every thread sums a strided share of each of the 3 kBuckets rows
-    __shared__ unsigned long long s_m[32];
-    for (int q = 0; q < kBuckets * 3; ++q)
-    {
-        unsigned long long v = 0;
-        for (int t = threadIdx.x; t < T; t += blockDim.x) v += tile_mom[(long long)q * T + t];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if ((threadIdx.x & 31) == 0) s_m[threadIdx.x >> 5] = v;
-        __syncthreads();
-        if (threadIdx.x < 32)
-        {
-            unsigned long long w = threadIdx.x < (blockDim.x >> 5) ? s_m[threadIdx.x] : 0ULL;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-            if (threadIdx.x == 0) moments[q] = w;
-        }
-        __syncthreads();
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
     }
+    return v;
 }
 
-__global__ void __launch_bounds__(kTileThreads) k_bucket_fill(const Geom g, const CellTile order, const signed char *__restrict__ status,
+// One block: exclusive scan of every bucket's tile counts (in place, as offsets
+// into the whole list), bucket totals and offsets, and the moments. The buckets
+// are scanned together and the moments' rows take two warps each, so that a block
+// barrier is passed twice (a Hillis-Steele scan a bucket and a sum a row after
+// another: 17 us for two tiles, all barriers).
+__global__ void __launch_bounds__(1024) k_prepare_scan(int T, int *__restrict__ tile_cnt,
+                                                       const unsigned long long *__restrict__ tile_mom,
+                                                       PrepareOut *__restrict__ out, int *__restrict__ bucket_off)
+{
+    __shared__ int s_w[kBuckets][32];
+    __shared__ unsigned long long s_m[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int per = (T + blockDim.x - 1) / blockDim.x;
+    const int t0 = min(T, (int)threadIdx.x * per), t1 = min(T, t0 + per);
+    int local[kBuckets], incl[kBuckets];
+#pragma unroll
+    for (int q = 0; q < kBuckets; ++q) local[q] = 0;
+    for (int t = t0; t < t1; ++t)
+#pragma unroll
+        for (int q = 0; q < kBuckets; ++q) local[q] += tile_cnt[(long long)q * T + t];
+#pragma unroll
+    for (int q = 0; q < kBuckets; ++q)
+    {
+        incl[q] = warp_scan(local[q], lane);
+        if (lane == 31) s_w[q][warp] = incl[q];
+    }
+    if (warp < 2 * 3 * kBuckets)
+    {
+        const unsigned long long *row = tile_mom + (long long)(warp >> 1) * T;
+        unsigned long long v = 0;
+#pragma unroll 4
+        for (int t = (warp & 1) * 32 + lane; t < T; t += 64) v += row[t];
+        v = warp_sum_u64(v);
+        if (lane == 0) s_m[warp] = v;
+    }
+    __syncthreads();
+    int run[kBuckets], total[kBuckets];
+#pragma unroll
+    for (int q = 0; q < kBuckets; ++q)
+    {
+        const int v = s_w[q][lane], sc = warp_scan(v, lane);
+        run[q] = __shfl_sync(0xffffffffu, sc - v, warp) + incl[q] - local[q];
+        total[q] = __shfl_sync(0xffffffffu, sc, 31);
+    }
+    for (int t = t0; t < t1; ++t)
+#pragma unroll
+        for (int q = 0; q < kBuckets; ++q)
+        {
+            int *at = tile_cnt + (long long)q * T + t;
+            const int v = *at;
+            *at = run[q];
+            run[q] += v;
+        }
+    if (threadIdx.x == 0)
+    {
+        int sum = 0;
+#pragma unroll
+        for (int q = 0; q < kBuckets; ++q)
+        {
+            out->cnt[q] = total[q];
+            bucket_off[q] = sum;
+            sum += total[q];
+        }
+        bucket_off[kBuckets] = sum;
+    }
+    if (threadIdx.x < 3 * kBuckets) out->mom[threadIdx.x] = s_m[2 * threadIdx.x] + s_m[2 * threadIdx.x + 1];
+}
+
+template <int ITERS>
+__global__ void __launch_bounds__(kTileThreads) k_bucket_fill(const Geom g, const CellTile order,
+                                                              const signed char *__restrict__ status,
                                                               const int *__restrict__ nb_n,
                                                               const int *__restrict__ tile_off,
                                                               const int *__restrict__ bucket_off,
                                                               int2 *__restrict__ cells)
 {
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int R = ITERS * kTileWarps; // a bucket's counts: by round, then warp
     const int T = gridDim.x;
-    const long long base = (long long)blockIdx.x * kTile;
+    const long long base = (long long)blockIdx.x * (kTileThreads * ITERS);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    constexpr int W = kTileThreads / 32;
-    __shared__ int s_wc[W][kBuckets];
-    __shared__ int s_run[kBuckets];
-    if (threadIdx.x < kBuckets) s_run[threadIdx.x] = bucket_off[threadIdx.x] + tile_off[threadIdx.x * T + blockIdx.x];
+    __shared__ int s_wc[kBuckets][R];
     unsigned lt;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-    for (int it = 0; it < kTileIters; ++it)
+    unsigned c[ITERS];
+    int n[ITERS];
+    bool queued[ITERS];
+#pragma unroll
+    for (int it = 0; it < ITERS; ++it)
     {
         const long long t = base + it * kTileThreads + threadIdx.x;
-        const unsigned c = t < g.n_cells ? tile_cell(g, order, (unsigned)t) : 0u;
-        int b = -1, n = 0;
-        if (t < g.n_cells && status[c] == 3)
-        {
-            n = nb_n[c];
-            b = bucket_of(n);
-        }
-        unsigned my_bl = 0;
+        const bool in = t < g.n_cells;
+        c[it] = in ? tile_cell(g, order, (unsigned)t) : 0u;
+        n[it] = in ? nb_n[c[it]] : 0;
+        queued[it] = in && status[c[it]] == 3;
+    }
+    int at[ITERS]; // this thread's place among its warp's cells of its bucket
+#pragma unroll
+    for (int it = 0; it < ITERS; ++it)
+    {
+        const int b = queued[it] ? bucket_of(n[it]) : -1;
 #pragma unroll
         for (int q = 0; q < kBuckets; ++q)
         {
-            const unsigned bl = __ballot_sync(0xffffffffu, b == q);
-            if (b == q) my_bl = bl;
-            if (lane == 0) s_wc[warp][q] = __popc(bl);
+            const unsigned bl = __ballot_sync(FULL, b == q);
+            if (b == q) at[it] = __popc(bl & lt);
+            if (lane == 0) s_wc[q][it * kTileWarps + warp] = __popc(bl);
         }
-        __syncthreads();
-        if (b >= 0)
-        {
-            int off = s_run[b];
-            for (int w = 0; w < warp; ++w) off += s_wc[w][b];
-            cells[off + __popc(my_bl & lt)] = make_int2((int)c, n);
-        }
-        __syncthreads();
-        if (threadIdx.x < kBuckets)
-        {
-            int v = 0;
-            for (int w = 0; w < W; ++w) v += s_wc[w][threadIdx.x];
-            s_run[threadIdx.x] += v;
-        }
-        __syncthreads();
     }
+    __syncthreads();
+    if (warp < kBuckets) // the counts become places in the bucket's list
+    {
+        int run = bucket_off[warp] + tile_off[(long long)warp * T + blockIdx.x];
+#pragma unroll
+        for (int i = 0; i < R; i += 32)
+        {
+            const int v = i + lane < R ? s_wc[warp][i + lane] : 0;
+            const int sc = warp_scan(v, lane);
+            if (i + lane < R) s_wc[warp][i + lane] = run + sc - v;
+            run += __shfl_sync(FULL, sc, 31);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < ITERS; ++it)
+        if (queued[it])
+        {
+            const int b = bucket_of(n[it]);
+            if (b >= 0) cells[s_wc[b][it * kTileWarps + warp] + at[it]] = make_int2((int)c[it], n[it]);
+        }
+}
+
+template <int ITERS>
+static void prepare_passes(int T, const Geom &g, const CellTile &order, const uint8_t *mask, int all_cells,
+                           const int *nb_n, signed char *status, PrepareOut *out, int *bucket_off, int *tile_cnt,
+                           unsigned long long *tile_mom, int2 *cells, cudaStream_t st)
+{
+    k_prepare<ITERS><<<T, kTileThreads, 0, st>>>(g, order, mask, all_cells, nb_n, status, tile_cnt, tile_mom);
+    k_prepare_scan<<<1, 1024, 0, st>>>(T, tile_cnt, tile_mom, out, bucket_off);
+    k_bucket_fill<ITERS><<<T, kTileThreads, 0, st>>>(g, order, status, nb_n, tile_cnt, bucket_off, cells);
 }
 
 void launch_prepare(const Geom &g, const CellTile &order, const uint8_t *mask, int all_cells, const int *nb_n,
-                    signed char *status, int *bucket_cnt, int *bucket_off, int *tile_cnt, unsigned long long *tile_mom, int2 *cells,
-                    unsigned long long *moments, cudaStream_t st)
+                    signed char *status, PrepareOut *out, int *bucket_off, int *tile_cnt,
+                    unsigned long long *tile_mom, int2 *cells, cudaStream_t st)
 {
     const int T = (int)prepare_tiles(g.n_cells);
-    k_prepare<<<T, kTileThreads, 0, st>>>(g, order, mask, all_cells, nb_n, status, tile_cnt, tile_mom);
-    k_prepare_scan<<<1, 1024, 0, st>>>(T, tile_cnt, tile_mom, bucket_cnt, bucket_off, moments);
-    k_bucket_fill<<<T, kTileThreads, 0, st>>>(g, order, status, nb_n, tile_cnt, bucket_off, cells);
+    auto passes = prepare_passes<8>;
+    switch (tile_iters(g.n_cells))
+    {
+    case 1: passes = prepare_passes<1>; break;
+    case 2: passes = prepare_passes<2>; break;
+    case 4: passes = prepare_passes<4>; break;
+    }
+    passes(T, g, order, mask, all_cells, nb_n, status, out, bucket_off, tile_cnt, tile_mom, cells, st);
 }
 
 // ------------------------------------------------------------- finalize
