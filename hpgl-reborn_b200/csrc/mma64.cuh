@@ -95,46 +95,62 @@ constexpr int kMmaRowDoubles = 32;
 // fail[s] is set (on every lane) by a pivot that is not positive, or, with
 // EPS_PIVOT, below the machine epsilon. No step branches, so the chains of the S
 // systems overlap.
-template <int S, bool EPS_PIVOT = false>
+template <int S, bool EPS_PIVOT>
+__device__ __forceinline__ void mma_pivots(int j, Blk (&D)[S], double *row, int lane, bool (&fail)[S])
+{
+    const int r = lane >> 2, q = lane & 3;
+    double *buf = row + (j & 2) * 8;
+#pragma unroll
+    for (int s = 0; s < S; ++s)
+        if (r == j || r == j + 1)
+            reinterpret_cast<double2 *>(buf + s * kMmaRowDoubles + 8 * (r & 1))[q] = make_double2(D[s].x, D[s].y);
+    __syncwarp();
+#pragma unroll
+    for (int s = 0; s < S; ++s)
+    {
+        const double *b0 = buf + s * kMmaRowDoubles, *b1 = b0 + 8;
+        const double2 ab = reinterpret_cast<const double2 *>(b0)[j / 2]; // D(j, j), D(j, j + 1)
+        const double ia = pivot_inverse(ab.x);
+        const double t = ab.y * ia;
+        const double d = fma(-t, ab.y, b1[j + 1]); // the second pivot
+        fail[s] |= pivot_fails<EPS_PIVOT>(ab.x) || pivot_fails<EPS_PIVOT>(d);
+        if (j == 6)
+        {
+            // no later rows: row 7 alone
+            const double2 u0 = reinterpret_cast<const double2 *>(b0)[q];
+            const double n0 = r == 7 ? t : 0.0;
+            D[s].x = r == 7 && q == 3 ? -t : fma(-n0, u0.x, D[s].x);
+            D[s].y = fma(-n0, u0.y, D[s].y);
+            continue;
+        }
+        const double id = pivot_inverse(d);
+        const double2 u0 = reinterpret_cast<const double2 *>(b0)[q], u1 = reinterpret_cast<const double2 *>(b1)[q];
+        const double m0 = b0[r] * ia;
+        const double m1 = r > j + 1 ? fma(-m0, ab.y, b1[r]) * id : 0.0;
+        const double n0 = r > j + 1 ? fma(-m1, t, m0) : (r == j + 1 ? t : 0.0);
+        const bool own = q == j / 2;
+        D[s].x = own && r > j ? -n0 : fma(-m1, u1.x, fma(-n0, u0.x, D[s].x));
+        D[s].y = own && r > j + 1 ? -m1 : fma(-m1, u1.y, fma(-n0, u0.y, D[s].y));
+    }
+}
+
+// ROLL: the four steps as one copy of the code. For the sharing kernel, which is
+// longer than the instruction cache likes (9.5M systems of up to 64: 62.3 -> 58.7 ms,
+// 19.7M of up to 32: 21.9 -> 20.4 ms); the simulation's weights, a short loop, lose
+// by it (8.3M systems: 23 -> 27 ms).
+template <int S, bool EPS_PIVOT = false, bool ROLL = false>
 __device__ __forceinline__ void mma_diag(Blk (&D)[S], double *row, int lane, bool (&fail)[S])
 {
     const int r = lane >> 2, q = lane & 3;
-#pragma unroll
-    for (int j = 0; j < 8; j += 2)
+    if constexpr (ROLL)
     {
-        double *buf = row + (j & 2) * 8;
+#pragma unroll 1
+        for (int j = 0; j < 8; j += 2) mma_pivots<S, EPS_PIVOT>(j, D, row, lane, fail);
+    }
+    else
+    {
 #pragma unroll
-        for (int s = 0; s < S; ++s)
-            if (r == j || r == j + 1)
-                reinterpret_cast<double2 *>(buf + s * kMmaRowDoubles + 8 * (r & 1))[q] = make_double2(D[s].x, D[s].y);
-        __syncwarp();
-#pragma unroll
-        for (int s = 0; s < S; ++s)
-        {
-            const double *b0 = buf + s * kMmaRowDoubles, *b1 = b0 + 8;
-            const double2 ab = reinterpret_cast<const double2 *>(b0)[j / 2]; // D(j, j), D(j, j + 1)
-            const double ia = pivot_inverse(ab.x);
-            const double t = ab.y * ia;
-            const double d = fma(-t, ab.y, b1[j + 1]); // the second pivot
-            fail[s] |= pivot_fails<EPS_PIVOT>(ab.x) || pivot_fails<EPS_PIVOT>(d);
-            if (j == 6)
-            {
-                // no later rows: row 7 alone
-                const double2 u0 = reinterpret_cast<const double2 *>(b0)[q];
-                const double n0 = r == 7 ? t : 0.0;
-                D[s].x = r == 7 && q == 3 ? -t : fma(-n0, u0.x, D[s].x);
-                D[s].y = fma(-n0, u0.y, D[s].y);
-                continue;
-            }
-            const double id = pivot_inverse(d);
-            const double2 u0 = reinterpret_cast<const double2 *>(b0)[q], u1 = reinterpret_cast<const double2 *>(b1)[q];
-            const double m0 = b0[r] * ia;
-            const double m1 = r > j + 1 ? fma(-m0, ab.y, b1[r]) * id : 0.0;
-            const double n0 = r > j + 1 ? fma(-m1, t, m0) : (r == j + 1 ? t : 0.0);
-            const bool own = q == j / 2;
-            D[s].x = own && r > j ? -n0 : fma(-m1, u1.x, fma(-n0, u0.x, D[s].x));
-            D[s].y = own && r > j + 1 ? -m1 : fma(-m1, u1.y, fma(-n0, u0.y, D[s].y));
-        }
+        for (int j = 0; j < 8; j += 2) mma_pivots<S, EPS_PIVOT>(j, D, row, lane, fail);
     }
 #pragma unroll
     for (int s = 0; s < S; ++s)
@@ -212,7 +228,7 @@ __device__ __forceinline__ void mma_factor(Blk (&A)[S][NB * (NB + 1) / 2], int n
         Blk D[S];
 #pragma unroll
         for (int s = 0; s < S; ++s) D[s] = A[s][blk_at(k, k)];
-        mma_diag<S>(D, row, lane, fail);
+        mma_diag<S, false, true>(D, row, lane, fail);
 #pragma unroll
         for (int s = 0; s < S; ++s) A[s][blk_at(k, k)] = D[s];
 #pragma unroll

@@ -117,46 +117,71 @@ __global__ void __launch_bounds__(TH, 1)
         __syncwarp();
         // ---- which cells have which neighbour: open addressing
         bool over = false;
-        for (int c0 = 0; c0 < w; c0 += 4)
-        {
-            int2 rec[4][RPL];
+        auto load = [&](int c, int2 (&rec)[RPL]) { // the lane's records of cell c, none from w on
+            const int cell = __shfl_sync(FULL, my.x, c), n = __shfl_sync(FULL, my.y, c);
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
+            for (int e = 0; e < RPL; ++e)
             {
-                const int cell = __shfl_sync(FULL, my.x, c0 + u), n = __shfl_sync(FULL, my.y, c0 + u);
+                const int i = lane + 32 * e;
+                rec[e] = c < w && i < n ? nb_rec[(long long)cell * g.k + i] : make_int2(kShareEmpty, 0);
+            }
+        };
+        auto insert = [&](int c, const int2 (&rec)[RPL]) {
+            const int off = __shfl_sync(FULL, my_off, c);
+#pragma unroll
+            for (int e = 0; e < RPL; ++e)
+                if (rec[e].x != kShareEmpty)
+                {
+                    const int key = rec[e].x + off;
+                    int s = (int)(((unsigned)key * 0x9E3779B1u) >> 16) & (T - 1);
+                    int tries = 0;
+                    for (; tries < 32; ++tries)
+                    {
+                        const int old = atomicCAS(&sh.key[s], kShareEmpty, key);
+                        if (old == kShareEmpty || old == key) break;
+                        s = (s + 1) & (T - 1);
+                    }
+                    if (tries == 32) over = true;
+                    else
+                    {
+                        const float v = __int_as_float(rec[e].y);
+                        sh.val[s] = (ind_value >= 0 ? (v == (float)ind_value ? 1.0f : 0.0f) : v) - P.mf;
+                        atomicOr(&sh.mask[s], 1 << c);
+                    }
+                    sh.slot[c][lane + 32 * e] = (unsigned char)s;
+                }
+        };
+        if constexpr (RPL == 1)
+        {
+            for (int c0 = 0; c0 < w; c0 += 4)
+            {
+                int2 rec[4][RPL];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) load(c0 + u, rec[u]);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) insert(c0 + u, rec[u]);
+            }
+        }
+        else
+        {
+            // one copy of the code, the loads three cells ahead: with up to 64 neighbours
+            // the kernel's eight warps wait for its instructions more than for anything
+            // else (9.5M systems of clustered data: 58.7 -> 54.5 ms; with up to 32 the
+            // four copies above are 2 to 10 % faster)
+            int2 rec[3][RPL];
+#pragma unroll
+            for (int u = 0; u < 3; ++u) load(u, rec[u]);
+#pragma unroll 1
+            for (int c = 0; c < w; ++c)
+            {
+                insert(c, rec[0]);
 #pragma unroll
                 for (int e = 0; e < RPL; ++e)
                 {
-                    const int i = lane + 32 * e;
-                    rec[u][e] = c0 + u < w && i < n ? nb_rec[(long long)cell * g.k + i] : make_int2(kShareEmpty, 0);
+                    rec[0][e] = rec[1][e];
+                    rec[1][e] = rec[2][e];
                 }
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-            {
-                const int off = __shfl_sync(FULL, my_off, c0 + u);
-#pragma unroll
-                for (int e = 0; e < RPL; ++e)
-                    if (rec[u][e].x != kShareEmpty)
-                    {
-                        const int key = rec[u][e].x + off;
-                        int s = (int)(((unsigned)key * 0x9E3779B1u) >> 16) & (T - 1);
-                        int tries = 0;
-                        for (; tries < 32; ++tries)
-                        {
-                            const int old = atomicCAS(&sh.key[s], kShareEmpty, key);
-                            if (old == kShareEmpty || old == key) break;
-                            s = (s + 1) & (T - 1);
-                        }
-                        if (tries == 32) over = true;
-                        else
-                        {
-                            const float v = __int_as_float(rec[u][e].y);
-                            sh.val[s] = (ind_value >= 0 ? (v == (float)ind_value ? 1.0f : 0.0f) : v) - P.mf;
-                            atomicOr(&sh.mask[s], 1 << (c0 + u));
-                        }
-                        sh.slot[c0 + u][lane + 32 * e] = (unsigned char)s;
-                    }
+                load(c + 3, rec[2]);
             }
         }
         over = __any_sync(FULL, over);
