@@ -1317,10 +1317,12 @@ static void run_sim_levels(Engine &E, const std::vector<SisCat> &cats, int kmax,
         E.stats.launches += 1;
         if (p0 == 0) before_levels();
         const int p1 = a.first + a.count;
+        bool beside = false; // the chunk's first level waits for its weights and, once, for the draws
         for (; l < n_levels && offs[l] < p1; ++l)
         {
             const int from = std::max(offs[l], a.first), to = std::min(offs[l + 1], p1);
-            HB_CK(level(a, from - a.first, to - from));
+            HB_CK(level(a, from - a.first, to - from, beside));
+            beside = beside || to > from;
             E.stats.launches += 1;
             if (offs[l + 1] > p1) break; // the rest of this level in the next chunk
         }
@@ -1550,8 +1552,8 @@ int sgs_simulation(const int *dims, float *data, unsigned char *mask, const unsi
             const std::vector<SisCat> one{
                 SisCat{pair64, nb, nb_lin, nb_cnt, nullptr, g.pair_center, g.pnx, g.pny, k, 0.0f}};
             run_sim_levels(E, one, k, sim_cells, order, offs, n_levels, n_sim, true, ordinary, false, st,
-                           draws_in, [&](const SimWeights &w, int first, int count) {
-                               return launch_sgs_level(w, first, count, d_data, d_means, d_u, st_rank, st);
+                           draws_in, [&](const SimWeights &w, int first, int count, bool beside) {
+                               return launch_sgs_level(w, first, count, beside, d_data, d_means, d_u, st_rank, st);
                            });
         }
         else
@@ -1871,8 +1873,8 @@ int sis_simulation(const int *dims, unsigned char *data, unsigned char *mask, co
         for (int c = 0; c < kcat; ++c) kmax = std::max(kmax, cats[c].max_nb);
         if (n_sim > 0)
             run_sim_levels(E, hc, kmax, sim_cells, order, offs, n_levels, n_sim, false, false,
-                           correlogram && means, st, draws_in, [&](const SimWeights &w, int first, int count) {
-                               return launch_sis_level(w, first, count, ncat, d_data, d_u, st_rank, st);
+                           correlogram && means, st, draws_in, [&](const SimWeights &w, int first, int count, bool beside) {
+                               return launch_sis_level(w, first, count, beside, ncat, d_data, d_u, st_rank, st);
                            });
         else
             draws_in();

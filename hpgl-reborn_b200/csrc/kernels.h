@@ -262,9 +262,9 @@ struct SimWeights
 cudaError_t launch_sim_weights(const SimWeights &a, bool sgs, bool ordinary, bool correlogram, int n_sm,
                                cudaStream_t st);
 // positions first .. first + count of the chunk, all of one level
-cudaError_t launch_sgs_level(const SimWeights &a, int first, int count, float *data, const float *means,
+cudaError_t launch_sgs_level(const SimWeights &a, int first, int count, bool beside, float *data, const float *means,
                              const double *uniforms, signed char *st_rank, cudaStream_t st);
-cudaError_t launch_sis_level(const SimWeights &a, int first, int count, int ncat, uint8_t *data,
+cudaError_t launch_sis_level(const SimWeights &a, int first, int count, bool beside, int ncat, uint8_t *data,
                              const double *uniforms, signed char *st_rank, cudaStream_t st);
 void launch_sgs_levels(const int *nb_rank, const int *nb_cnt, int k, int n_sim, int *levp1, int *ticket,
                        int *level_count, int level_cap, int *max_level, int *err, int n_sm, cudaStream_t st);

@@ -159,7 +159,19 @@ __global__ void __launch_bounds__(kWeightThreads, 1) k_sim_weights(const SimWeig
 // (values of lower levels are final). The rows of a node are stored together:
 // position-major rows of one neighbour each, which one thread a node would read
 // coalesced, lie megabytes apart and took 33 us a level in TLB misses.
-constexpr int kLevelRows = 32, kLevelWarps = 8;
+//
+// A level is a few thousand nodes: what it takes is the chain of its loads (order,
+// neighbours, values, then the sums and the draw) and the launch. All but the
+// values are there before the level below is done, so a level is launched as soon
+// as the blocks of the one below have started (programmatic dependent launch),
+// reads what is there, and waits for the values (read past L1, which blocks of the
+// level below share). Every thread waits, so a level ends after the one below.
+// 364 levels of 8.3M nodes: 4.5 -> 2.1 ms; 426 levels of 4M nodes with five
+// categories: 2.1 ms less.
+constexpr int kLevelRows = 32, kLevelWarps = 8, kLevelPer = kLevelRows / kLevelWarps;
+
+__device__ __forceinline__ void level_started() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void level_below_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __global__ void __launch_bounds__(32 * kLevelWarps) k_sgs_level(
     const SimWeights a, int first, int count, float *__restrict__ data, const float *__restrict__ means,
@@ -168,25 +180,47 @@ __global__ void __launch_bounds__(32 * kLevelWarps) k_sgs_level(
     __shared__ float term[kLevelRows][33];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int row0 = blockIdx.x * kLevelRows;
+    level_started();
+    int q[kLevelPer];
+    double w[kLevelPer];
 #pragma unroll
-    for (int j = warp; j < kLevelRows; j += kLevelWarps)
+    for (int e = 0; e < kLevelPer; ++e)
     {
-        const int pos = first + row0 + j;
-        float t = 0.0f;
+        const int j = warp + e * kLevelWarps, pos = first + row0 + j;
+        q[e] = -1;
         if (row0 + j < count && lane < a.n[pos])
         {
-            const int q = a.cats[0].nb[(long long)a.order[a.first + pos] * a.kmax + lane];
-            const float v = means ? __fsub_rn(data[q], means[q]) : data[q];
-            t = __double2float_rn(__dmul_rn(a.W[(long long)pos * a.kmax + lane], (double)v));
+            q[e] = a.cats[0].nb[(long long)a.order[a.first + pos] * a.kmax + lane];
+            w[e] = a.W[(long long)pos * a.kmax + lane];
         }
-        term[j][lane] = t;
+    }
+    const bool mine = warp == 0 && row0 + lane < count;
+    int r = 0, cell = 0, n = 0, status = 0;
+    double u = 0.0, var = 0.0;
+    if (mine)
+    {
+        const int pos = first + row0 + lane;
+        r = a.order[a.first + pos];
+        cell = a.sim_cells[r];
+        n = a.n[pos];
+        status = a.st[pos];
+        u = uniforms[r];
+        var = a.var[pos];
+    }
+    level_below_done();
+#pragma unroll
+    for (int e = 0; e < kLevelPer; ++e)
+    {
+        float t = 0.0f;
+        if (q[e] >= 0)
+        {
+            const float d = __ldcg(data + q[e]), v = means ? __fsub_rn(d, means[q[e]]) : d;
+            t = __double2float_rn(__dmul_rn(w[e], (double)v));
+        }
+        term[warp + e * kLevelWarps][lane] = t;
     }
     __syncthreads();
-    if (warp != 0 || row0 + lane >= count) return;
-    const int pos = first + row0 + lane;
-    const int r = a.order[a.first + pos], cell = a.sim_cells[r];
-    const int n = a.n[pos], status = a.st[pos];
-    const double u = uniforms[r], var = a.var[pos];
+    if (!mine) return;
     float est = means ? means[cell] : 0.0f;
 #pragma unroll 8
     for (int i = 0; i < n; ++i) est = __fadd_rn(est, term[lane][i]);
@@ -205,19 +239,33 @@ __global__ void __launch_bounds__(32 * kLevelWarps) k_sis_level(
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nodes = kLevelRows / a.kcat, rows = nodes * a.kcat;
     const int node0 = blockIdx.x * nodes;
-    for (int j = warp; j < rows; j += kLevelWarps)
+    level_started();
+    int q[kLevelPer];
+    double w[kLevelPer];
+    float mean[kLevelPer];
+#pragma unroll
+    for (int e = 0; e < kLevelPer; ++e)
     {
-        const int cat = j % a.kcat, node = node0 + j / a.kcat;
+        const int j = warp + e * kLevelWarps, cat = j % a.kcat, node = node0 + j / a.kcat;
         const long long row = (long long)(first + node) * a.kcat + cat;
-        double t = 0.0;
-        if (node < count && lane < a.n[row])
+        q[e] = -1;
+        if (j < rows && node < count && lane < a.n[row])
         {
             const SisCat &C = a.cats[cat];
-            const int q = C.nb[(long long)a.order[a.first + first + node] * C.k + lane];
-            // indicator - mean, in float
-            const float d = __fsub_rn(data[q] == cat ? 1.0f : 0.0f, C.means ? C.means[q] : C.marginal);
-            t = __dmul_rn(a.W[row * a.kmax + lane], (double)d);
+            q[e] = C.nb[(long long)a.order[a.first + first + node] * C.k + lane];
+            w[e] = a.W[row * a.kmax + lane];
+            mean[e] = C.means ? C.means[q[e]] : C.marginal;
         }
+    }
+    level_below_done();
+#pragma unroll
+    for (int e = 0; e < kLevelPer; ++e)
+    {
+        const int j = warp + e * kLevelWarps;
+        if (j >= rows) break;
+        double t = 0.0;
+        // indicator - mean, in float
+        if (q[e] >= 0) t = __dmul_rn(w[e], (double)__fsub_rn(__ldcg(data + q[e]) == j % a.kcat ? 1.0f : 0.0f, mean[e]));
         term[j][lane] = t;
     }
     __syncthreads();
@@ -288,20 +336,36 @@ cudaError_t launch_sim_weights(const SimWeights &a, bool sgs, bool ordinary, boo
     return correlogram ? launch_weights<kSimCorr>(a, n_sm, st) : launch_weights<kSimIK>(a, n_sm, st);
 }
 
-cudaError_t launch_sgs_level(const SimWeights &a, int first, int count, float *data, const float *means,
+// beside: the launch before this one in the stream is the level below
+template <typename... P, typename... A>
+static cudaError_t launch_level(void (*kern)(P...), int blocks, bool beside, cudaStream_t st, A... args)
+{
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(32 * kLevelWarps);
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = beside ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
+cudaError_t launch_sgs_level(const SimWeights &a, int first, int count, bool beside, float *data, const float *means,
                              const double *uniforms, signed char *st_rank, cudaStream_t st)
 {
     if (count <= 0) return cudaSuccess;
-    k_sgs_level<<<(count + kLevelRows - 1) / kLevelRows, 32 * kLevelWarps, 0, st>>>(a, first, count, data, means, uniforms, st_rank);
-    return cudaGetLastError();
+    return launch_level(k_sgs_level, (count + kLevelRows - 1) / kLevelRows, beside, st, a, first, count, data, means,
+                        uniforms, st_rank);
 }
 
-cudaError_t launch_sis_level(const SimWeights &a, int first, int count, int ncat, uint8_t *data,
+cudaError_t launch_sis_level(const SimWeights &a, int first, int count, bool beside, int ncat, uint8_t *data,
                              const double *uniforms, signed char *st_rank, cudaStream_t st)
 {
     if (count <= 0) return cudaSuccess;
     const int nodes = kLevelRows / a.kcat;
-    k_sis_level<<<(count + nodes - 1) / nodes, 32 * kLevelWarps, 0, st>>>(a, first, count, ncat, data, uniforms, st_rank);
-    return cudaGetLastError();
+    return launch_level(k_sis_level, (count + nodes - 1) / nodes, beside, st, a, first, count, ncat, data, uniforms,
+                        st_rank);
 }
 } // namespace hb
