@@ -1234,10 +1234,13 @@ def main():
     achieved = b_flops / (b_ms / 1e3) / 1e12
     tpc = traffic_per_cell()
     kname = bucket_kernel(W, b, wl.cov.cov_type, 1, kind == 0 and not lvm)
-    roofline = {"bound": "fp32", "kernel": kname,
-                "achieved": achieved, "peak": pk["fp32"], "unit": "TFLOP/s", "frac": achieved / pk["fp32"],
+    np_ = [8, 16, 32, 64, 65][b]
+    in64 = b == 4 or shared_solve(W, np_, W.solve_variant(np_, wl.cov.cov_type, 1), 1)
+    bound = "fp64" if in64 else "fp32"
+    roofline = {"bound": bound, "kernel": kname,
+                "achieved": achieved, "peak": pk[bound], "unit": "TFLOP/s", "frac": achieved / pk[bound],
                 "traffic": (tpc * last[f"bucket_items_{b}"]) if tpc else None,
-                "peak_source": f"CUDA-core FP32 peak 148 SM x 128 lanes x 2 x {pk['source']}",
+                "peak_source": f"{bound.upper()} peak 148 SM x {64 if in64 else 128} lanes x 2 x {pk['source']}",
                 "algorithmic_flops_per_launch": b_flops, "kernel_ms": b_ms}
     s64b = s64[-1]
     b64 = int(np.argmax([s64b[f"bucket_ms_{i}"] for i in range(5)]))
@@ -1325,7 +1328,7 @@ def main():
         line = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms32, "higher_is_better": True, "scaling": "weak",
-            "vs_baseline": None, "dtype": "f32 (FP64-refined residuals)", "data": "synthetic (seeded, geo_bsd.workloads)",
+            "vs_baseline": None, "dtype": "f64" if in64 else "f32 (FP64-refined residuals)", "data": "synthetic (seeded, geo_bsd.workloads)",
             "config": {"workload": f"{KIND_NAMES[args.kind]} {wl.dims[0]}x{wl.dims[1]}x"
                                    f"{wl.dims[2]}, 1% lognormal conditioning, exponential (30,15,6) az 30, "
                                    f"k={wl.max_neighbours}", "precision": "fp32_refined",

@@ -725,8 +725,17 @@ static void run_solves(Engine &E, const Plan &pl, const DevPoints &P, const DevS
         any_quad = any_quad || (precision && b < 4 && kBucketNP[b] <= 32 &&
                                 (is_quad_variant(variant[b]) || tune_wanted(kBucketNP[b], pl.f.m.type, precision)));
     }
-    for (int b = 0; b < 4 && g.n_cells >= 64 * E.n_sm(); ++b)
-        any_share = any_share || is_share_variant(kBucketNP[b], precision, variant[b]) ||
+    // A warp of the sharing solve takes eight cells in a row, 20 to 30 us of dependent
+    // steps; until every warp has two such groups (one with up to 64 neighbours, whose
+    // solves are longer), the one-system kernel, one cell a warp, is through sooner. At
+    // 1 % and 2 % of the cells informed, us shared / alone: up to 32 neighbours,
+    // 11,400 systems 54 60 / 44 44, 25,300 84 98 / 81 80, 48,700 121 131 / 141 138,
+    // 519,000 736 891 / 1230 1211; up to 64, 11,400 142 180 / 140 140, 25,300 190 288 /
+    // 293 291, 81,000 704 857 / 889 876.
+    auto share_from = [&](int b) { return (kBucketNP[b] <= 32 ? 256 : 128) * E.n_sm(); };
+    for (int b = 0; b < 4; ++b)
+        if (g.n_cells >= share_from(b))
+            any_share = any_share || is_share_variant(kBucketNP[b], precision, variant[b]) ||
                     tune_wanted(kBucketNP[b], pl.f.m.type, precision);
     if (any_quad) ref_cells = E.buf<int2>("ref_cells", (size_t)g.n_cells);
     launch_prepare(g, any_share ? solve_share_tile(g) : CellTile{0, 0, 0}, d_mask, all_cells, S.nb_n, d_status,
@@ -794,11 +803,8 @@ static void run_solves(Engine &E, const Plan &pl, const DevPoints &P, const DevS
             if (b < 4)
             {
                 int2 *first_esc = quad ? ref_cells + off : (esc_cells ? esc_cells + off : nullptr);
-                // A warp of the sharing solve takes eight cells in a row, about 20 us of
-                // dependent steps; below 64 cells an SM the one-system kernel, one cell a
-                // warp, is through sooner (9,472 systems of 32: 24 us against 25).
                 const bool share =
-                    is_share_variant(kBucketNP[b], precision, variant[b]) && cnt[b] >= 64 * E.n_sm();
+                    is_share_variant(kBucketNP[b], precision, variant[b]) && cnt[b] >= share_from(b);
                 HB_CK(launch_solve_bucket(kBucketNP[b], precision, variant[b], ordinary, g, bcells, bucket_cnt + b,
                                           cnt[b], S.nb_rec, S.nb_n, ind_value, S.pair64, S.pair32, mean, c0, steps,
                                           tol, out, first_esc, quad ? ref_cnt + b : esc_cnt + b,

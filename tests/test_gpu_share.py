@@ -91,3 +91,23 @@ def test_refined_option_runs_the_shared_solve(np_, k):
         W.solve_variant(np_, wl.cov.cov_type, W.FP32_REFINED, prev)
     with pytest.raises(ValueError):
         W.solve_variant(16, 1, W.FP32_REFINED, W.VARIANT_SHARE)
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("k", [17, 24, 25, 31, 32, 33, 40, 41, 48, 56, 57, 64])
+def test_neighbour_limits_shared(kind, k):
+    """Enough systems for the sharing kernel whatever k (fewer go one by one)."""
+    s = _check(_wl((53, 47, 19), 2400, EXP, (12, 9, 7), k), kind)
+    assert s["bucket_items_%d" % (2 if k <= 32 else 3)] >= 256 * 148
+
+
+@pytest.mark.parametrize("dims,points,rad", [
+    ((45001, 1, 1), 4500, (200, 3, 3)), ((1, 45001, 1), 4500, (3, 200, 3)), ((1, 1, 45001), 4500, (3, 3, 200)),
+    ((3, 7003, 2), 2900, (4, 60, 2)), ((4501, 3, 3), 2900, (60, 3, 3)), ((9, 7, 701), 2900, (6, 6, 12)),
+    ((47, 40, 23), 40000, (1, 1, 1)), ((47, 43, 23), 44000, (2, 1, 3)),
+])
+@pytest.mark.parametrize("kind", [0, 1])
+def test_thin_and_ragged_grids_shared(kind, dims, points, rad):
+    cov = WL.CovSpec(WL.EXPONENTIAL, tuple(10.0 * v for v in rad), (0.0, 0.0, 0.0), 1.0, 0.05)
+    for k in (19, 32, 50):
+        _check(_wl(dims, min(points, dims[0] * dims[1] * dims[2] // 10), cov, rad, k), kind)
