@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(kCokThreads, 1) k_cok_solve_warp(const CokArgs
         __syncwarp();
         const int nb = (n + 7) >> 3;
         nn = it + stride < a.n_targets ? a.nb_n[ncell] : 0;
-        const bool fail = warp_factor<2, true, false>(T, lane, n, nb, pair_c);
+        const bool fail = warp_factor<2, true, false, true>(T, lane, n, nb, pair_c);
         rec = load(ncell, nn);
         warp_back<2>(T, lane, nb);
         const double x = lane < n ? T.y[0][lane] : 0.0, y = lane < n ? T.y[1][lane] : 0.0;

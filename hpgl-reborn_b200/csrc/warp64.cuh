@@ -66,14 +66,14 @@ __device__ __forceinline__ bool warp_eliminate(WarpSmem<Q, SCALE> &T, int lane, 
 
 // The same for the system of n unknowns read from a pair table (nb = ceil(n / 8));
 // T.lin (and T.sig) must be visible too.
-template <int Q, bool EPS_PIVOT, bool SCALE>
+template <int Q, bool EPS_PIVOT, bool SCALE, bool UPPER = false>
 __device__ __forceinline__ bool warp_factor(WarpSmem<Q, SCALE> &T, int lane, int n, int nb,
                                             const double *__restrict__ pair_c)
 {
     constexpr int NB = kWarpNB;
     const int r = lane >> 2, q = lane & 3;
     Blk A[1][kWarpBlocks];
-    mma_load<NB>(A[0], pair_c, T.lin, n, nb, lane);
+    mma_load<NB, UPPER>(A[0], pair_c, T.lin, n, nb, lane);
     if constexpr (SCALE)
     {
         // A[i][c] = pair * (sig_i * sig_c) for live entries (padding rows: sig 1)
