@@ -349,7 +349,15 @@ static cudaError_t launch_level(void (*kern)(P...), int blocks, bool beside, cud
     cfg.stream = st;
     cfg.attrs = &attr;
     cfg.numAttrs = beside ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+    if (e == cudaErrorNotSupported && beside)
+    {
+        // a stream that does not take the attribute: one level after another
+        cudaGetLastError();
+        cfg.numAttrs = 0;
+        e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+    }
+    return e;
 }
 
 cudaError_t launch_sgs_level(const SimWeights &a, int first, int count, bool beside, float *data, const float *means,
