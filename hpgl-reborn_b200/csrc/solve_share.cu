@@ -216,7 +216,11 @@ __global__ void __launch_bounds__(TH, 1)
                 }
                 nc += __popc(b);
             }
-            if (cb < 1 || nc < 8 * cb) continue;
+            if (cb < 1 || nc < 8 * cb)
+            {
+                __syncwarp(); // the next size writes clin, cval and id from other lanes
+                continue;
+            }
             // the distinct extras, each numbered by its first cell, and the
             // extras of every cell as rows of R
             ur = 0;
