@@ -105,12 +105,13 @@ def loo_geometry(prop, grid, radiuses: Sequence[int], max_neighbours: int, cov_m
 def _loo_call(name: str, geom: LooGeometry, M, r0: float, sill, nugget, values, stream, outputs):
     """hpgl_b200_<name> on `stream`. A variogram that lies on the values' device is
     read there by the kernel (reading it here would wait for the device three times
-    a call); any other is passed as host numbers."""
+    a call); any other, one of other sizes among them, is passed as host numbers."""
     points = (geom.pts_xyz.data_ptr(), values.data_ptr(), int(values.numel()), geom.targets.data_ptr(),
               geom.nb_idx.data_ptr(), geom.nb_cnt.data_ptr(), int(geom.targets.numel()), geom.k, geom.cov_type)
     tail = [t.data_ptr() for t in outputs] + [stream.cuda_stream]
     par = (M, sill, nugget)
-    if all(torch.is_tensor(t) and t.device == values.device and t.dtype == torch.float64 for t in par):
+    if all(torch.is_tensor(t) and t.device == values.device and t.dtype == torch.float64 and t.numel() == size
+           for t, size in zip(par, (9, 1, 1))):
         par = tuple(t.detach().contiguous() for t in par)
         for t in par:
             t.record_stream(stream)
