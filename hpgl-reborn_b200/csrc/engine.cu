@@ -427,7 +427,8 @@ static double root_up(double h2) { return std::sqrt(h2) * (1.0 + 1e-15); }
 // uninformed ones. Table slots are suffixed with `tag` so several flavours can
 // coexist (IK categories run one after another and reuse them).
 static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const uint8_t *d_mask, int all_cells,
-                            cudaStream_t st, bool want_pids = false, bool exact_search = false, bool ordered = false)
+                            cudaStream_t st, bool want_pids = false, bool exact_search = false,
+                            bool warp_per_cell = false)
 {
     const Geom &g = pl.g;
     DevSearch S;
@@ -511,9 +512,9 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
     int max_cand = host_scal[1];
     const int n_tmpl_bins = host_scal[2];
     const int max_cand_tmpl = host_scal[6];
-    // neighbours in candidate order serve where only the set matters, and where that
-    // order is the points' own (a bin left unsorted has none that repeats)
-    ordered = ordered || want_pids || host_scal[7] > 0;
+    // one cell a lane writes no point ids; and equal ranks stand in the points' order,
+    // which a bin left unsorted does not have
+    warp_per_cell = warp_per_cell || want_pids || host_scal[7] > 0;
     // Template-path bins (sugarbox_neighbour_lookup.h:171-197: the first k informed
     // cells of the sorted template, in its order) as a selection: the informed
     // cells of the 27 bins around a cell keyed by their offset's position in the
@@ -522,7 +523,6 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
     int n_tmpl = 0;
     int4 *tmpl = E.buf<int4>("tmpl", std::max<long>(pl.tmpl_count, 1));
     bool tmpl_select = false, tmpl_tile = false, tmpl_scan = false, rank_keys = false;
-    // one cell a lane where the order of the neighbours is free
     const int tile_limit = search_tile_limit(g.k, E.max_smem() - 1024);
     uint16_t *keypos16 = nullptr;
     SurrDev sdp = {};
@@ -536,7 +536,7 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
         // and the cells whose k-th slot a tie straddles by the template scan (on the
         // clustered 512x512x64 grid, 111,537 offsets: 49 ms for every template-path
         // cell's scan)
-        rank_keys = tv.size() > 0xFFFE && use_sd && !ordered && tile_limit > 0;
+        rank_keys = tv.size() > 0xFFFE && use_sd && !warp_per_cell && tile_limit > 0;
         if (rank_keys)
         {
             tmpl_tile = true;
@@ -547,7 +547,7 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
             build_surrogate_template(pl.f, tv, sgp);
             sdp.on = sgp.ok && !exact_search ? 1 : 0;
             cand_cap_t = std::max(4, (max_cand_tmpl + 3) / 4 * 4);
-            tmpl_tile = sdp.on && !ordered && tile_limit > 0;
+            tmpl_tile = sdp.on && !warp_per_cell && tile_limit > 0;
             if (!tmpl_tile)
             {
                 while (warps_t > 1 && search_fast_smem_bytes(cand_cap_t, g.k, warps_t) > (size_t)E.max_smem()) --warps_t;
@@ -614,14 +614,14 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
     int *tie_cells = E.buf<int>("tie_cells", (size_t)g.n_cells);
     HB_CK(cudaMemsetAsync(S.nb_n, 0, sizeof(int) * g.n_cells, st));
     HB_CK(cudaEventRecord(E.ev_[8], st));
-    const bool tile = fast && sd.on && !ordered && cand_cap <= tile_limit;
+    const bool tile = fast && sd.on && !warp_per_cell && cand_cap <= tile_limit;
     if (tile)
         HB_CK(launch_search_tile(g, d_mask, all_cells, bin_start, bin_cnt, S.bin_flag, bin_pts, P.pts_xyz, P.pts_val,
                                  keytab16, sd, 0, g.n_bins, cand_cap, E.max_smem() - 1024, S.nb_rec, S.nb_n, tie_cells, scal + 3,
                                  scal + 4, scal + 5, st));
     else if (fast)
         HB_CK(launch_search_fast(g, d_mask, all_cells, bin_start, bin_cnt, S.bin_flag, bin_pts, P.pts_xyz, P.pts_val,
-                                 keytab16, sd, 0, ordered, P.pid_of_node, cand_cap, warps, S.nb_pid,
+                                 keytab16, sd, 0, P.pid_of_node, cand_cap, warps, S.nb_pid,
                                  S.nb_rec, S.nb_n, tie_cells, scal + 3, scal + 4, scal + 5, st));
     else
         HB_CK(launch_search(g, d_mask, all_cells, bin_start, bin_cnt, S.bin_flag, bin_pts, P.pts_xyz, P.pts_val,
@@ -642,7 +642,7 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
     }
     else if (tmpl_select)
         HB_CK(launch_search_fast(g, d_mask, all_cells, bin_start, bin_cnt, S.bin_flag, bin_pts, P.pts_xyz, P.pts_val,
-                                 keypos16, sdp, 1, ordered, P.pid_of_node, cand_cap_t, warps_t, S.nb_pid, S.nb_rec, S.nb_n,
+                                 keypos16, sdp, 1, P.pid_of_node, cand_cap_t, warps_t, S.nb_pid, S.nb_rec, S.nb_n,
                                  tie_cells, scal + 3, scal + 4, scal + 5, st));
     if (tmpl_scan)
         HB_CK(launch_search_template(g, d_mask, bits, all_cells, tmpl_bins, n_tmpl_bins, bin_cnt, tmpl_tile ? tile_limit : -1, P.pts_val, tmpl,
@@ -2049,7 +2049,7 @@ int cokriging(const int *dims, const float *pdata, const unsigned char *pmask, c
             pl.g.limit = INT_MAX; // no bin takes the template path
             try
             {
-                // cokriging's float sums run in the neighbours' order
+                // (measured with the warp-per-cell search alone)
                 DevSearch S = run_search(E, pl, P, d_pm, 0, st, false, false, true);
                 if (S.ties != 0) throw CudaFail{-2, "cokriging search: equal template keys"};
                 nb_rec = S.nb_rec;

@@ -90,18 +90,16 @@ struct SurrDev
 
 size_t search_fast_smem_bytes(int cand_cap, int k, int warps);
 // exact_cells (may be null) counts cells the float prefilter left to the exact
-// path. `ordered` writes each cell's neighbours in key order; without it they
-// stand in candidate order (the same set, cheaper). template_bins = 0 searches the cluster-path bins; 1 the template-path
-// bins, keytab16 then holding template positions (n_template_cells counts them)
+// path. Each cell's neighbours are written in key order, equal keys in candidate
+// order. template_bins = 0 searches the cluster-path bins; 1 the template-path bins, keytab16 then holding template positions (n_template_cells counts them)
 cudaError_t launch_search_fast(const Geom &g, const uint8_t *mask, int all_cells, const int *bin_start,
                                const int *bin_cnt, const uint8_t *bin_flag, const int *bin_pts,
                                const unsigned long long *pts_xyz, const float *pts_vf, const uint16_t *keytab16,
-                               const SurrDev &sd, int template_bins, bool ordered, const int *pid_of_node,
+                               const SurrDev &sd, int template_bins, const int *pid_of_node,
                                int cand_cap, int warps, int *nb_pid, int2 *nb_rec, int *nb_n, int *tie_cells, int *tie_count,
                                int *n_template_cells, int *exact_cells, cudaStream_t st);
-// The same selection with the prefilter on, one cell a lane, neighbours in
-// candidate order (search_tile.cu): the bins with at most search_tile_limit
-// candidates. n_bins: how many bins there are of the kind searched.
+// The same with the prefilter on, one cell a lane (search_tile.cu): the bins with at
+// most search_tile_limit candidates. n_bins: how many bins there are of the kind searched.
 int search_tile_limit(int k, int max_smem);
 cudaError_t launch_search_tile(const Geom &g, const uint8_t *mask, int all_cells, const int *bin_start,
                                const int *bin_cnt, const uint8_t *bin_flag, const int *bin_pts,

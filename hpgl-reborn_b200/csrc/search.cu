@@ -655,93 +655,47 @@ __device__ __forceinline__ int warp_count_le(const uint32_t *keys, int C, uint32
     return c;
 }
 
-// Writes the kept candidates of a cell. With ORDERED, v is sorted ascending
-// (element i in v[i / 32] of lane i % 32) and the first n_sel go out in that
-// order; else v holds them anywhere (0 elsewhere) and they go out as they stand,
-// in candidate order.
-template <int E, bool ORDERED>
+// Writes the first n_sel of a cell's kept candidates, v sorted ascending (element i
+// in v[i / 32] of lane i % 32).
+template <int E>
 __device__ __forceinline__ void emit_selected(const uint32_t (&v)[E], int n_sel, int lane, const int *cplin,
                                               const int *cpid, const float *cval, int plin_c, int *out_pid,
                                               int2 *out_rec)
 {
-    int done = 0;
 #pragma unroll
     for (int e = 0; e < E; ++e)
     {
-        int i = e * 32 + lane;
-        bool in = i < n_sel;
-        if (!ORDERED)
+        const int i = e * 32 + lane;
+        if (i < n_sel)
         {
-            in = v[e] != 0u;
-            const unsigned bl = __ballot_sync(0xffffffffu, in);
-            i = done + __popc(bl & lanemask_lt());
-            done += __popc(bl);
-        }
-        if (in)
-        {
-            const int pos = (int)((v[e] - 1u) & 0xFFFFu);
+            const int pos = (int)(v[e] & 0xFFFFu);
             if (out_pid) out_pid[i] = cpid[pos];
             if (out_rec) out_rec[i] = make_int2(cplin[pos] - plin_c, __float_as_int(cval[pos]));
         }
     }
 }
 
-// The k smallest of the warp's nk non-zero keys in v (unique; 0 is no key, a
-// key is its rank << 16 | position, plus one): kth and nxt receive the k-th and
-// the (k+1)-th smallest (nxt 0 when nk <= k; kth the largest when nk < k). v
-// keeps the k smallest in place, or, with ORDERED, sorted. In place, the few keys
-// above the k-th are taken out one by one, largest first, each by a warp maximum
-// (a step on the benchmark keeps 37 keys for 32); from kSelectSteps surplus keys
-// on, and with ORDERED, the whole set is sorted (21 exchange stages for 64 keys).
-constexpr int kSelectSteps = 20;
-template <int E, bool ORDERED>
+// Sorts the warp's nk keys in v (rank << 16 | position; kNoKey elsewhere); kth and
+// nxt receive the k-th and the (k+1)-th smallest (kNoKey where there is none; kth the
+// largest when nk < k).
+constexpr uint32_t kNoKey = 0xFFFFFFFFu;
+template <int E>
 __device__ __forceinline__ void select_smallest(uint32_t (&v)[E], int nk, int k, int lane, uint32_t &kth,
                                                 uint32_t &nxt)
 {
-    nxt = 0u;
-    kth = 0u;
+    kth = nxt = kNoKey;
     if (nk == 0) return;
-    if (!ORDERED && nk - k < kSelectSteps)
-    {
-        uint32_t top = 0u;
-        for (int it = nk; it >= k; --it)
-        {
-            uint32_t m = v[0];
-#pragma unroll
-            for (int e = 1; e < E; ++e) m = max(m, v[e]);
-            top = __reduce_max_sync(0xffffffffu, m);
-            if (it <= k) break;
-            nxt = top;
-#pragma unroll
-            for (int e = 0; e < E; ++e)
-                if (v[e] == top) v[e] = 0u;
-        }
-        if (nk < k)
-        {
-            uint32_t m = v[0];
-#pragma unroll
-            for (int e = 1; e < E; ++e) m = max(m, v[e]);
-            top = __reduce_max_sync(0xffffffffu, m);
-        }
-        kth = top;
-        return;
-    }
-    uint32_t t[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) t[e] = v[e] - 1u; // no key: the largest
-    warp_bitonic_sort<E>(t, lane);
+    warp_bitonic_sort<E>(v, lane);
     const int i = min(nk, k) - 1;
 #pragma unroll
     for (int e = 0; e < E; ++e)
     {
-        if (e == (i >> 5)) kth = __shfl_sync(0xffffffffu, t[e], i & 31) + 1u;
-        if (nk > k && e == (k >> 5)) nxt = __shfl_sync(0xffffffffu, t[e], k & 31) + 1u;
+        if (e == (i >> 5)) kth = __shfl_sync(0xffffffffu, v[e], i & 31);
+        if (nk > k && e == (k >> 5)) nxt = __shfl_sync(0xffffffffu, v[e], k & 31);
     }
-#pragma unroll
-    for (int e = 0; e < E; ++e) v[e] = ORDERED ? t[e] + 1u : (v[e] <= kth ? v[e] : 0u);
 }
 
-template <int E, bool ORDERED>
+template <int E>
 __device__ __forceinline__ int select_fast(const Geom &g, int C, const int *cklin, const int *cplin, const int *cpid,
                            const float *cval, int kc0, int klin_c, int plin_c,
                            const uint16_t *__restrict__ keytab, uint32_t *keys, uint32_t *sel, int lane,
@@ -820,15 +774,15 @@ __device__ __forceinline__ int select_fast(const Geom &g, int C, const int *ckli
     for (int e = 0; e < E; ++e)
     {
         const int i = e * 32 + lane;
-        v[e] = i < cnt ? sel[i] + 1u : 0u;
+        v[e] = i < cnt ? sel[i] : kNoKey;
     }
     const int n_sel = cnt < k ? cnt : k;
     if (n_sel <= 0) return 0;
     uint32_t kth, nxt;
-    select_smallest<E, ORDERED>(v, cnt, k, lane, kth, nxt);
-    kguess = (int)((kth - 1u) >> 16);
-    if (cnt > k && (int)((nxt - 1u) >> 16) == kguess) return -1;
-    emit_selected<E, ORDERED>(v, n_sel, lane, cplin, cpid, cval, plin_c, out_pid, out_rec);
+    select_smallest<E>(v, cnt, k, lane, kth, nxt);
+    kguess = (int)(kth >> 16);
+    if (cnt > k && (int)(nxt >> 16) == kguess) return -1;
+    emit_selected<E>(v, n_sel, lane, cplin, cpid, cval, plin_c, out_pid, out_rec);
     return n_sel;
 }
 
@@ -846,7 +800,7 @@ __device__ __forceinline__ int select_fast(const Geom &g, int C, const int *ckli
 // candidate within r_sub of the cell. Returns n_sel, -1 for a tie group
 // straddling the k-th slot, or -2 when the prefilter cannot decide (the caller
 // then runs select_fast). On success or -1, H receives that largest distance.
-template <int E, bool ORDERED>
+template <int E>
 __device__ __forceinline__ int select_surr(const Geom &g, const SurrDev &sd, int C, const float4 *ctp, const int *cklin,
                            const int *cplin, const int *cpid, const float *cval, int kc0, int klin_c, int plin_c,
                            const uint16_t *__restrict__ keytab, uint32_t *sel, int lane, float tcx, float tcy,
@@ -905,14 +859,14 @@ __device__ __forceinline__ int select_surr(const Geom &g, const SurrDev &sd, int
         for (int e = 0; e < E; ++e)
         {
             const int i = e * 32 + lane;
-            v[e] = 0u;
+            v[e] = kNoKey;
             if (i < cnt)
             {
                 const uint32_t pos = sel[i];
                 const uint32_t r16 = keytab[kc0 + cklin[pos] - klin_c];
-                if (r16 != 0xFFFFu) v[e] = ((r16 << 16) | pos) + 1u;
+                if (r16 != 0xFFFFu) v[e] = (r16 << 16) | pos;
             }
-            nk += __popc(__ballot_sync(0xffffffffu, v[e] != 0u));
+            nk += __popc(__ballot_sync(0xffffffffu, v[e] != kNoKey));
         }
         if (nk < k && rt < r_all)
         {
@@ -921,8 +875,8 @@ __device__ __forceinline__ int select_surr(const Geom &g, const SurrDev &sd, int
             continue;
         }
         uint32_t kth, nxt;
-        select_smallest<E, ORDERED>(v, nk, k, lane, kth, nxt);
-        H = nk >= k ? sd.h_rank[(kth - 1u) >> 16] : sd.h_cut;
+        select_smallest<E>(v, nk, k, lane, kth, nxt);
+        H = nk >= k ? sd.h_rank[kth >> 16] : sd.h_cut;
         if (!((rt - sd.e3) * (1.0 - 1e-12) > H))
         {
             lo = rf;
@@ -930,15 +884,15 @@ __device__ __forceinline__ int select_surr(const Geom &g, const SurrDev &sd, int
             continue;
         }
         const int n_sel = nk < k ? nk : k;
-        if (n_sel > 0) kguess = (int)((kth - 1u) >> 16);
-        if (nk > k && (int)((nxt - 1u) >> 16) == kguess) return -1;
-        emit_selected<E, ORDERED>(v, n_sel, lane, cplin, cpid, cval, plin_c, out_pid, out_rec);
+        if (n_sel > 0) kguess = (int)(kth >> 16);
+        if (nk > k && (int)(nxt >> 16) == kguess) return -1;
+        emit_selected<E>(v, n_sel, lane, cplin, cpid, cval, plin_c, out_pid, out_rec);
         return n_sel;
     }
     return -2;
 }
 
-template <int E, bool ORDERED>
+template <int E>
 __global__ void __launch_bounds__(256, E == 2 ? 4 : 2) k_search_fast(
     const Geom g, const uint8_t *__restrict__ mask, int all_cells, const int *__restrict__ bin_start,
     const int *__restrict__ bin_cnt, const uint8_t *__restrict__ bin_flag, const int *__restrict__ bin_pts,
@@ -1156,13 +1110,13 @@ __global__ void __launch_bounds__(256, E == 2 ? 4 : 2) k_search_fast(
                 const float dc = sqrtf(fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
                 r_sub = Rcov * (1.0f - 1e-5f) - dc * (1.0f + 1e-6f) - slack;
             }
-            n = select_surr<E, ORDERED>(g, sd, C, ctp, cklin, cplin, cpid, cval, kc0, klin_c, plin_c, keytab16, sel,
+            n = select_surr<E>(g, sd, C, ctp, cklin, cplin, cpid, cval, kc0, klin_c, plin_c, keytab16, sel,
                                         lane, tc.x, tc.y, tc.z, rt + 2.0 * sd.e3, keys, n_sub, r_sub, h, kguess, o_pid,
                                         o_rec);
         }
         if (n == -2)
         {
-            n = select_fast<E, ORDERED>(g, C, cklin, cplin, cpid, cval, kc0, klin_c, plin_c, keytab16, keys, sel, lane,
+            n = select_fast<E>(g, C, cklin, cplin, cpid, cval, kc0, klin_c, plin_c, keytab16, keys, sel, lane,
                                         kguess, o_pid, o_rec);
             sl_ok = false; // keys[] now holds select_fast's keys
             n_exact += sd.on;
@@ -1195,7 +1149,7 @@ size_t search_fast_smem_bytes(int cand_cap, int k, int warps)
 cudaError_t launch_search_fast(const Geom &g, const uint8_t *mask, int all_cells, const int *bin_start,
                                const int *bin_cnt, const uint8_t *bin_flag, const int *bin_pts,
                                const unsigned long long *pts_xyz, const float *pts_vf, const uint16_t *keytab16,
-                               const SurrDev &sd, int template_bins, bool ordered, const int *pid_of_node,
+                               const SurrDev &sd, int template_bins, const int *pid_of_node,
                                int cand_cap, int warps, int *nb_pid, int2 *nb_rec, int *nb_n, int *tie_cells, int *tie_count,
                                int *n_template_cells, int *exact_cells, cudaStream_t st)
 {
@@ -1208,8 +1162,7 @@ cudaError_t launch_search_fast(const Geom &g, const uint8_t *mask, int all_cells
                                                  nb_rec, nb_n, tie_cells, tie_count, n_template_cells, exact_cells);
         return cudaGetLastError();
     };
-    if (g.k <= 32) return ordered ? launch(k_search_fast<2, true>) : launch(k_search_fast<2, false>);
-    return ordered ? launch(k_search_fast<4, true>) : launch(k_search_fast<4, false>);
+    return g.k <= 32 ? launch(k_search_fast<2>) : launch(k_search_fast<4>);
 }
 
 // One thread per tie-straddling cell: rebuild the threshold-filtered candidate

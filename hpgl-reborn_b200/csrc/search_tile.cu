@@ -1,5 +1,5 @@
-// Neighbour selection, one cell a lane (the set of the reference's lookups; see
-// search.cu for the warp-per-cell forms, which order the neighbours by key).
+// Neighbour selection, one cell a lane (the reference's lookups; see search.cu for
+// the warp-per-cell forms).
 #include "engine.cuh"
 #include "kernels.h"
 #include "search_common.cuh"
@@ -11,15 +11,17 @@
 namespace hb
 {
 // One cell by exact ranks over all C candidates, without scratch: the smallest
-// rank with k candidates up to it by bisection, then those candidates in their
-// order. Returns the neighbour count, or -1 for a tie group across the k-th slot.
-__device__ int exact_select(const Geom &g, int C, const float4 *ctp, const int2 *crec, int kofs, int plin_c,
-                            const uint16_t *__restrict__ keytab, int lane, int2 *out_rec)
+// rank with k candidates up to it by bisection, then those candidates' keys (rank
+// << 16 | place) to out, ld apart. Returns the neighbour count, or -1 for a tie
+// group across the k-th slot.
+__device__ int exact_select(const Geom &g, int C, const float4 *ctp, int kofs, const uint16_t *__restrict__ keytab,
+                            int lane, uint32_t *out, int ld)
 {
     const int k = g.k;
+    auto rank = [&](int i) { return (int)keytab[kofs + __float_as_int(ctp[i].w)]; };
     auto count = [&](int top) {
         int c = 0;
-        for (int i = lane; i < C; i += 32) c += (int)keytab[kofs + __float_as_int(ctp[i].w)] <= top;
+        for (int i = lane; i < C; i += 32) c += rank(i) <= top;
         return __reduce_add_sync(0xffffffffu, c);
     };
     int lo = -1, hi = 0xFFFE; // kept ranks stay below 0xFFFF
@@ -42,13 +44,125 @@ __device__ int exact_select(const Geom &g, int C, const float4 *ctp, const int2 
     int done = 0;
     for (int base = 0; base < C; base += 32)
     {
-        const int i = base + lane;
-        const bool in = i < C && (int)keytab[kofs + __float_as_int(ctp[i < C ? i : 0].w)] <= hi;
-        const unsigned bl = __ballot_sync(0xffffffffu, in);
-        if (in) out_rec[done + __popc(bl & lanemask_lt())] = make_int2(crec[i].x - plin_c, crec[i].y);
+        const int i = base + lane, r = i < C ? rank(i) : 0xFFFF;
+        const unsigned bl = __ballot_sync(0xffffffffu, r <= hi);
+        if (r <= hi) out[(done + __popc(bl & lanemask_lt())) * ld] = ((uint32_t)r << 16) | (uint32_t)i;
         done += __popc(bl);
     }
     return done;
+}
+
+// ---- ascending order of a lane's own keys: Batcher's odd-even merge sort (K. E.
+// Batcher, Sorting networks and their applications, 1968) on registers. A lane has
+// its list to itself, so 32 cells' lists of 32 take 191 comparators, about 14 warp
+// instructions a cell; sorted across the warp a cell at a time, 60.
+template <int A, int B, int N>
+__device__ __forceinline__ void compare_exchange(uint32_t (&v)[N])
+{
+    const uint32_t lo = min(v[A], v[B]);
+    v[B] = max(v[A], v[B]);
+    v[A] = lo;
+}
+template <int FIRST, int LEN, int STEP, int I, int N>
+__device__ __forceinline__ void merge_pairs(uint32_t (&v)[N])
+{
+    if constexpr (I + STEP < FIRST + LEN)
+    {
+        compare_exchange<I, I + STEP>(v);
+        merge_pairs<FIRST, LEN, STEP, I + 2 * STEP>(v);
+    }
+}
+template <int FIRST, int LEN, int STEP, int N>
+__device__ __forceinline__ void odd_even_merge(uint32_t (&v)[N])
+{
+    if constexpr (2 * STEP < LEN)
+    {
+        odd_even_merge<FIRST, LEN, 2 * STEP>(v);
+        odd_even_merge<FIRST + STEP, LEN, 2 * STEP>(v);
+        merge_pairs<FIRST, LEN, STEP, FIRST + STEP>(v);
+    }
+    else
+        compare_exchange<FIRST, FIRST + STEP>(v);
+}
+template <int FIRST, int LEN, int N>
+__device__ __forceinline__ void merge_sort(uint32_t (&v)[N])
+{
+    if constexpr (LEN > 1)
+    {
+        merge_sort<FIRST, LEN / 2>(v);
+        merge_sort<FIRST + LEN / 2, LEN / 2>(v);
+        odd_even_merge<FIRST, LEN, 1>(v);
+    }
+}
+
+constexpr uint32_t kNoKey = 0xFFFFFFFFu; // past every key
+
+// the N keys from `first` on of a lane's list of n, ld apart
+template <int N, int P>
+__device__ __forceinline__ void load_keys(uint32_t (&v)[P], const uint32_t *list, int ld, int first, int n)
+{
+#pragma unroll
+    for (int e = 0; e < N; ++e) v[e] = first + e < n ? list[(first + e) * ld] : kNoKey;
+}
+template <int N, int P>
+__device__ __forceinline__ void store_keys(const uint32_t (&v)[P], uint32_t *list, int ld, int first, int n)
+{
+#pragma unroll
+    for (int e = 0; e < N; ++e)
+        if (first + e < n) list[(first + e) * ld] = v[e];
+}
+// (a function of its own: inlined, its registers drove the search's to local memory,
+// 4.3 -> 7.3 ms; 4.75 so)
+template <int N>
+__device__ __noinline__ void order_keys(uint32_t *list, int ld, int first, int n)
+{
+    constexpr int P = N <= 8 ? 8 : (N <= 16 ? 16 : 32);
+    uint32_t v[P];
+    load_keys<N>(v, list, ld, first, n);
+#pragma unroll
+    for (int e = N; e < P; ++e) v[e] = kNoKey; // the compiler drops their comparators
+    merge_sort<0, P>(v);
+    store_keys<N>(v, list, ld, first, n);
+}
+// a bitonic run of 32 put in order
+__device__ __forceinline__ void order_bitonic(uint32_t (&v)[32])
+{
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1)
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+            if (!(i & s))
+            {
+                const uint32_t lo = min(v[i], v[i + s]);
+                v[i + s] = max(v[i], v[i + s]);
+                v[i] = lo;
+            }
+}
+// 33 to 64 keys: two sorted halves, the i-th of the first against the (31 - i)-th of
+// the second, then two bitonic runs (64 registers would not fit beside the search's)
+__device__ __noinline__ void order_keys64(uint32_t *list, int ld, int n)
+{
+#pragma unroll 1
+    for (int h = 0; h < 64; h += 32) order_keys<32>(list, ld, h, n);
+    uint32_t v[32];
+    load_keys<32>(v, list, ld, 0, n);
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+    {
+        const int at = 63 - i;
+        if (at < n)
+        {
+            const uint32_t x = list[at * ld];
+            list[at * ld] = max(v[i], x);
+            v[i] = min(v[i], x);
+        }
+    }
+    order_bitonic(v);
+    store_keys<32>(v, list, ld, 0, n);
+    // the upper half: bitonic with kNoKey from n on
+    load_keys<32>(v, list, ld, 32, n);
+    order_bitonic(v);
+    store_keys<32>(v, list, ld, 32, n);
 }
 
 // ---- the same selection, one cell a lane
@@ -61,7 +175,11 @@ __device__ int exact_select(const Geom &g, int C, const float4 *ctp, const int2 
 // is about a tenth of the warp-per-cell form's (whose every step costs a warp
 // instruction for one cell). Lanes whose radius was a bad guess repeat the scan
 // with another; what is undecided after kTileTries goes through exact_select.
-// Neighbours are written in candidate order.
+// Neighbours are written in key order, equal ranks in candidate order: the nearest
+// first is also what keeps the solves' rounding low (12 neighbours, Gaussian, nugget
+// 0.05, simple kriging: in candidate order 2.2 times the estimates' error and 1.5 times
+// the variances'). The sort of each lane's list costs 0.5 of 4.8 ms at 8.3M cells of 32,
+// 2 of 48 ms at 16.8M clustered cells of 64, 0.8 of 13.2 ms at 20M indicator cells of 24.
 //
 // What bounds it: instructions (on a grid of 32 neighbours about half the issue
 // slots, on clustered data of 64 a third, where the lists leave room for 14 warps
@@ -411,9 +529,32 @@ __global__ void __launch_bounds__(256, 3) k_search_tile(
             const float h = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(n != -2 ? H : 0.0f)));
             if (h > 0.0f) guess = h * 1.02f + e3;
         }
-        // ---- write the decided cells' neighbours, a cell at a time
+        // ---- undecided cells: by exact ranks over every candidate
         __syncwarp();
-        for (unsigned todo = __ballot_sync(FULL, mine && n >= 0); todo; todo &= todo - 1)
+        for (unsigned todo = __ballot_sync(FULL, open); todo; todo &= todo - 1)
+        {
+            const int src = __ffs(todo) - 1;
+            const int r = exact_select(g, C, ctp, kc0 - __shfl_sync(FULL, klin_c, src), keytab, lane,
+                                       lists + warp * 32 + src, ld);
+            if (lane == src) n = r;
+            ++n_exact;
+        }
+        __syncwarp();
+        // ---- the lists in key order
+        const int own = mine ? max(n, 0) : 0, longest = __reduce_max_sync(FULL, own);
+        if (longest > 32)
+            order_keys64(list, ld, own);
+        else if (longest > 24)
+            order_keys<32>(list, ld, 0, own);
+        else if (longest > 16)
+            order_keys<24>(list, ld, 0, own);
+        else if (longest > 8)
+            order_keys<16>(list, ld, 0, own);
+        else if (longest > 1)
+            order_keys<8>(list, ld, 0, own);
+        // ---- written a cell at a time
+        __syncwarp();
+        for (unsigned todo = __ballot_sync(FULL, own > 0); todo; todo &= todo - 1)
         {
             const int src = __ffs(todo) - 1;
             const int ns = __shfl_sync(FULL, n, src);
@@ -425,17 +566,7 @@ __global__ void __launch_bounds__(256, 3) k_search_tile(
                 nb_rec[cs * k + e] = make_int2(rec.x - pl, rec.y);
             }
         }
-        // ---- undecided cells: by exact ranks over every candidate
         __syncwarp();
-        for (unsigned todo = __ballot_sync(FULL, open); todo; todo &= todo - 1)
-        {
-            const int src = __ffs(todo) - 1;
-            const int r = exact_select(g, C, ctp, crec, kc0 - __shfl_sync(FULL, klin_c, src),
-                                       __shfl_sync(FULL, pair_lin(g, cxr, cyr, czr), src), keytab, lane,
-                                       nb_rec + __shfl_sync(FULL, cell, src) * k);
-            if (lane == src) n = r;
-            ++n_exact;
-        }
         if (mine)
         {
             nb_n[cell] = n < 0 ? k : n;
