@@ -162,7 +162,8 @@ struct LooSolve
 {
     int n;
     bool ok;
-    int pid;        // this lane's neighbour (row) point id, -1 for padding rows
+    int pid;        // this lane's neighbour, -1 for padding rows
+    int at;         // its place among the unknowns
     int px, py, pz; // its coordinates
     int tx, ty, tz; // the target's
     double lambda;  // OK weight
@@ -170,7 +171,7 @@ struct LooSolve
     double zhat;
 };
 
-// Assemble, factor and solve the target's system; lane r holds unknown r.
+// Assemble, factor and solve the target's system; lane r holds neighbour r.
 __device__ LooSolve loo_solve(const LooParams &P, const LooModel &m, int t, LooSmem &W)
 {
     const int lane = threadIdx.x & 31;
@@ -188,11 +189,12 @@ __device__ LooSolve loo_solve(const LooParams &P, const LooModel &m, int t, LooS
     S.pz = live ? P.pts_xyz[3 * S.pid + 2] : 0;
     const double z = live ? P.values[S.pid] : 0.0;
     const double b = live ? cov_d(m, P.cov_type, S.px - S.tx, S.py - S.ty, S.pz - S.tz).c : 0.0;
+    S.at = mma_slot(lane, n, nb);
     __syncwarp(); // the previous target's reads are done
-    W.pt[lane] = make_int4(S.px, S.py, S.pz, 0);
-    W.T.y[0][lane] = b;
-    W.T.y[1][lane] = live ? 1.0 : 0.0;
-    W.T.y[2][lane] = z;
+    W.pt[S.at] = make_int4(S.px, S.py, S.pz, 0);
+    W.T.y[0][S.at] = b;
+    W.T.y[1][S.at] = live ? 1.0 : 0.0;
+    W.T.y[2][S.at] = z;
     __syncwarp();
 
     // the lower triangle's blocks (the diagonal ones whole), padding rows identity
@@ -232,9 +234,9 @@ __device__ LooSolve loo_solve(const LooParams &P, const LooModel &m, int t, LooS
         }
     }
     // L y = [b, 1, z], then L^T x = y
-    const bool fail = warp_eliminate<3, false, false>(W.T, lane, nb, A);
+    const bool fail = warp_eliminate<3, false, false, true>(W.T, lane, nb, A);
     warp_back<3>(W.T, lane, nb);
-    const double x0 = live ? W.T.y[0][lane] : 0.0, x1 = live ? W.T.y[1][lane] : 0.0, x2 = live ? W.T.y[2][lane] : 0.0;
+    const double x0 = live ? W.T.y[0][S.at] : 0.0, x1 = live ? W.T.y[1][S.at] : 0.0, x2 = live ? W.T.y[2][S.at] : 0.0;
     const double sx = warp_sum(x0), sy = warp_sum(x1), sz = warp_sum(x2);
     const double mu = (sx - 1.0) / sy, beta = sz / sy;
     S.lambda = live ? x0 - mu * x1 : 0.0;
@@ -303,8 +305,8 @@ __global__ void __launch_bounds__(32 * kLooWarps, kAdjointBlocks) k_loo_adjoint(
         if (live) atomicAdd(&grad_values[S.pid], g * S.lambda);
         const double ga = g * S.alpha; // 0 beyond n
         __syncwarp();
-        W.T.y[0][lane] = S.lambda;
-        W.T.y[1][lane] = ga;
+        W.T.y[0][S.at] = S.lambda;
+        W.T.y[1][S.at] = ga;
         __syncwarp();
         // alpha_r dC(b_r) - alpha_r sum_c lambda_c dC(A_rc), A_rc and A_cr together
         if (live) add(S.px - S.tx, S.py - S.ty, S.pz - S.tz, ga);

@@ -1058,6 +1058,10 @@ int cont_kriging(int kind, const int *dims, const float *in_data, const unsigned
         SolveOut so{};
         so.out_data = d_out;
         so.out_mask = d_omask;
+        // the slower form of the shared factors where its smaller error shows (mma64.cuh):
+        // in FP64 results (a float's rounding is above 10^5 times either form's error) of
+        // Gaussian and spherical models
+        so.by_halves = (d_est || d_var) && pl.f.m.type != 1;
         so.est64 = d_est;
         so.var = d_var;
         so.status = d_status;

@@ -29,6 +29,7 @@ struct SolveOut
     int prob_stride;     // distance between cells in `prob` (the category count)
     int write_cont;      // write out_data / out_mask
     const float *cell_mean; // LVM: per-cell mean, added at the centre instead of the SK mean
+    bool by_halves; // the shared factors' diagonal blocks are applied by halves (mma64.cuh)
 };
 
 // scan / points / bins (search.cu)

@@ -54,38 +54,37 @@ __global__ void __launch_bounds__(TH, 1)
     load_rec(w_cur);
     for (; it < run_end; it += nwarps)
     {
-        const int cell = w_cur.x, n = w_cur.y;
+        const int cell = w_cur.x, n = w_cur.y, nb = (n + 7) >> 3;
 #pragma unroll
         for (int e = 0; e < RPL; ++e)
         {
-            const int i = lane + 32 * e;
+            const int i = lane + 32 * e, at = mma_slot(i, n, nb);
             const bool live = i < n;
-            lin[i] = rec[e].x;
-            xs[i] = live ? __ldg(pair_c + abs(rec[e].x)) : 0.0;
-            if (ORDINARY) xs[N + i] = live ? 1.0 : 0.0;
-            xs[2 * N + i] = centred_value(live, __int_as_float(rec[e].y), ind_value, P.mf);
+            lin[at] = rec[e].x;
+            xs[at] = live ? __ldg(pair_c + abs(rec[e].x)) : 0.0;
+            if (ORDINARY) xs[N + at] = live ? 1.0 : 0.0;
+            xs[2 * N + at] = centred_value(live, __int_as_float(rec[e].y), ind_value, P.mf);
         }
         __syncwarp();
-        const int nb = (n + 7) >> 3;
-        Blk A[1][NB * (NB + 1) / 2], X[1][NB];
-        bool fail[1] = {false};
-        mma_load<NB>(A[0], pair_c, lin, n, nb, lane);
+        Blk A[NB * (NB + 1) / 2], X[NB];
+        bool fail = false;
+        mma_load<NB>(A, pair_c, lin, n, nb, lane);
         const bool used = ORDINARY ? r < 3 : (r == 0 || r == 2);
 #pragma unroll
         for (int k = 0; k < NB; ++k)
         {
             double2 v = make_double2(0.0, 0.0);
             if (used) v = reinterpret_cast<const double2 *>(xs + r * N + 8 * k)[q];
-            X[0][k] = Blk{v.x, v.y};
+            X[k] = Blk{v.x, v.y};
         }
         load_rec(w_nxt);
         w_cur = w_nxt;
         w_nxt = it + 2 * nwarps < run_end ? cells[it + 2 * nwarps] : make_int2(0, 0);
-        mma_factor<NB, 1>(A, X, nb, row, lane, fail);
+        half_factor<NB, true, false, false>(A, X, nb, row, lane, fail);
         Blk G{0.0, 0.0};
 #pragma unroll
         for (int k = 0; k < NB; ++k)
-            if (k < nb) blk_mul_t(G, X[0][k], X[0][k]);
+            if (k < nb) blk_mul_t(G, X[k], X[k]);
         // rows 0 = b, 1 = ones, 2 = v - mean: lane 0 has (0,0) and (0,1)
         const double s_vb = __shfl_sync(0xffffffffu, G.x, 1);
         double s_11 = 0.0, s_v1 = 0.0;
@@ -94,7 +93,7 @@ __global__ void __launch_bounds__(TH, 1)
             s_11 = __shfl_sync(0xffffffffu, G.y, 4);
             s_v1 = __shfl_sync(0xffffffffu, G.x, 5);
         }
-        if (lane == 0) write_solution<ORDINARY>(P, cell, fail[0], s_vb, G.x, G.y, s_v1, s_11);
+        if (lane == 0) write_solution<ORDINARY>(P, cell, fail, s_vb, G.x, G.y, s_v1, s_11);
         __syncwarp();
     }
 }

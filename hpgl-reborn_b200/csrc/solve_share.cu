@@ -17,8 +17,8 @@
 // Groups come from tiles of eight cells (the list is in tile order), the
 // largest of 8, 4, 2 following cells with 8 cb common neighbours; cells that
 // share with no other go to a queue (left_cells) for
-// the one-system-per-warp kernel, and so does a cell with a failing pivot,
-// which decides its status in the neighbours' own order.
+// the one-system-per-warp kernel, and so does a cell with a failing pivot (which the
+// cell's own order of unknowns may not have).
 #include "engine.cuh"
 #include "kernels.h"
 #include "mma64.cuh"
@@ -72,7 +72,7 @@ struct __align__(16) ShareWarp
     unsigned char eid[kShareCells][8];            // extra -> row of R
 };
 
-template <int CB, bool ORDINARY, int TH>
+template <int CB, bool ORDINARY, int TH, bool HALVES>
 __global__ void __launch_bounds__(TH, 1)
     k_solve_share(const Geom g, const int2 *__restrict__ cells, const int *__restrict__ n_items_ptr,
                   const int2 *__restrict__ nb_rec, int ind_value, SolveParams P, CellTile tile,
@@ -209,8 +209,9 @@ __global__ void __launch_bounds__(TH, 1)
                 const int rank = nc + __popc(b & below);
                 if (com && rank < 8 * cb)
                 {
-                    sh.clin[rank] = sh.key[sl];
-                    sh.cval[rank] = sh.val[sl];
+                    const int at = HALVES ? mma_slot(rank, 8 * cb, cb) : rank;
+                    sh.clin[at] = sh.key[sl];
+                    sh.cval[at] = sh.val[sl];
                     sh.id[sl] = 255;
                     shared |= 1u << e;
                 }
@@ -275,10 +276,13 @@ __global__ void __launch_bounds__(TH, 1)
         __syncwarp();
         {
             // ---- the common block, factored once
-            Blk A[1][CB * (CB + 1) / 2];
+            Blk A[1][CB * (CB + 1) / 2], none[1];
             bool fail[1] = {false};
             mma_load<CB>(A[0], pair_c, sh.clin, 8 * cb, cb, lane);
-            mma_factor<CB, 1>(A, cb, sh.row, lane, fail);
+            if constexpr (HALVES)
+                half_factor<CB, false, false, true>(A[0], none, cb, sh.row, lane, fail[0]);
+            else
+                mma_factor<CB, 1>(A, cb, sh.row, lane, fail);
 
             // ---- the rows of R, eight at a time
             const int rows = ur + gn + Q - 1;
@@ -312,7 +316,8 @@ __global__ void __launch_bounds__(TH, 1)
                 for (int k = 0; k < CB; ++k)
                 {
                     if (k >= cb) break;
-                    Blk t = blk_prod_t(R[k], A[0][blk_at(k, k)]);
+                    const Blk &D = A[0][blk_at(k, k)];
+                    Blk t = HALVES ? blk_solve_t(R[k], D) : blk_prod_t(R[k], D);
                     reinterpret_cast<double2 *>(&sh.R[rho * LD + 8 * k])[q] = make_double2(t.x, t.y);
                     t = blk_neg(t);
 #pragma unroll
@@ -473,13 +478,13 @@ __global__ void __launch_bounds__(TH, 1)
     }
 }
 
-template <int CB, bool ORD, int TH>
+template <int CB, bool ORD, int TH, bool HALVES>
 static cudaError_t launch_share(const Geom &g, const int2 *cells, const int *n_items, int max_items, const int2 *nb_rec,
                                 int ind_value, const SolveParams &P, const CellTile &tile, int2 *left_cells, int *left_count,
                                 int n_sm, cudaStream_t st)
 {
     const size_t smem = sizeof(ShareWarp<CB>) * (TH / 32);
-    auto kern = k_solve_share<CB, ORD, TH>;
+    auto kern = k_solve_share<CB, ORD, TH, HALVES>;
     int blocks = 0;
     cudaError_t e = launch_kernel(kern, TH, smem, max_items, TH / 32 * kShareCells, n_sm, blocks);
     if (e != cudaSuccess) return e;
@@ -525,9 +530,13 @@ cudaError_t launch_solve_share(int np, bool ordinary, const Geom &g, const int2 
                                int2 *left_cells, int *left_count, int n_sm, cudaStream_t st)
 {
 #define HB_ARGS g, cells, n_items, max_items, nb_rec, ind_value, P, tile, left_cells, left_count, n_sm, st
-    if (np == 32) return ordinary ? launch_share<3, true, 512>(HB_ARGS) : launch_share<3, false, 512>(HB_ARGS);
-    if (np == 64) return ordinary ? launch_share<7, true, 256>(HB_ARGS) : launch_share<7, false, 256>(HB_ARGS);
+#define HB_SHARE(CB, TH)                                                                         \
+    (P.out.by_halves ? (ordinary ? launch_share<CB, true, TH, true>(HB_ARGS) : launch_share<CB, false, TH, true>(HB_ARGS)) \
+              : (ordinary ? launch_share<CB, true, TH, false>(HB_ARGS) : launch_share<CB, false, TH, false>(HB_ARGS)))
+    if (np == 32) return HB_SHARE(3, 512);
+    if (np == 64) return HB_SHARE(7, 256);
     return cudaErrorInvalidValue;
+#undef HB_SHARE
 #undef HB_ARGS
 }
 } // namespace hb

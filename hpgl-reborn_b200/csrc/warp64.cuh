@@ -29,8 +29,8 @@ __device__ __forceinline__ int blk_chunk(int r, int q) { return 4 * r + (q ^ ((r
 
 // The factorisation of the warp's system A of nb block rows with the forward
 // substitution of its Q right-hand sides, T.y in place (it must be visible).
-// Returns whether a pivot failed.
-template <int Q, bool EPS_PIVOT, bool SCALE>
+// Returns whether a pivot failed. HALVES: for users that return FP64 numbers.
+template <int Q, bool EPS_PIVOT, bool SCALE, bool HALVES = false>
 __device__ __forceinline__ bool warp_eliminate(WarpSmem<Q, SCALE> &T, int lane, int nb, Blk (&A)[1][kWarpBlocks])
 {
     constexpr int NB = kWarpNB;
@@ -47,7 +47,10 @@ __device__ __forceinline__ bool warp_eliminate(WarpSmem<Q, SCALE> &T, int lane, 
         }
     }
     bool fail[1] = {false};
-    mma_factor<NB, 1, EPS_PIVOT>(A, X, nb, T.row, lane, fail);
+    if constexpr (HALVES)
+        half_factor<NB, true, true, false>(A[0], X[0], nb, T.row, lane, fail[0]);
+    else
+        mma_factor<NB, 1, EPS_PIVOT>(A, X, nb, T.row, lane, fail);
     double2 *LM = reinterpret_cast<double2 *>(T.LM);
     const int at = blk_chunk(r, q);
     __syncwarp(); // the previous system's reads of LM are done
@@ -65,7 +68,8 @@ __device__ __forceinline__ bool warp_eliminate(WarpSmem<Q, SCALE> &T, int lane, 
 }
 
 // The same for the system of n unknowns read from a pair table (nb = ceil(n / 8));
-// T.lin (and T.sig) must be visible too.
+// T.lin (and T.sig) must be visible too. Its users return floats and categories,
+// whose rounding hides the whole inverses' error (by halves, 8.3M systems 26.2 -> 30.4 ms).
 template <int Q, bool EPS_PIVOT, bool SCALE, bool UPPER = false>
 __device__ __forceinline__ bool warp_factor(WarpSmem<Q, SCALE> &T, int lane, int n, int nb,
                                             const double *__restrict__ pair_c)

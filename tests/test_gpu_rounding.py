@@ -24,6 +24,10 @@ def _rms(a, b):
 
 @pytest.mark.parametrize("cov_type,ranges,azimuth,nugget,density,k", [
     (WL.GAUSSIAN, (20, 15, 6), 30.0, 0.05, 0.01, 12), (WL.GAUSSIAN, (20, 15, 6), 30.0, 0.01, 0.01, 16),
+    # beyond 16 neighbours: the sharing solves
+    (WL.GAUSSIAN, (20, 15, 6), 30.0, 0.05, 0.01, 32), (WL.GAUSSIAN, (18, 18, 6), 0.0, 0.05, 0.015, 24),
+    (WL.GAUSSIAN, (20, 15, 6), 30.0, 0.2, 0.02, 40), (WL.SPHERICAL, (18, 18, 6), 0.0, 0.0, 0.015, 24),
+    (WL.EXPONENTIAL, (30, 15, 6), 30.0, 0.0, 0.01, 32),
 ])
 def test_error_is_that_of_a_substitution(cov_type, ranges, azimuth, nugget, density, k):
     dims = (72, 64, 48)
