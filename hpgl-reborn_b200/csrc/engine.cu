@@ -1763,7 +1763,9 @@ int sis_simulation(const int *dims, unsigned char *data, unsigned char *mask, co
         HB_CK(cudaMemsetAsync(nb_rank, 0xFF, ns * ktot * 4, st)); // -1: no neighbour
         std::vector<double *> pair64(kcat);
         std::vector<int *> nb(kcat), nb_lin(kcat), nb_cnt(kcat);
+        // the host tables live until the synchronisation behind the last copy of them
         std::vector<SisPlan> plans;
+        std::vector<std::vector<int4>> templates(kcat);
         for (int c = 0; c < kcat; ++c)
         {
             plans.push_back(plan_p[c].get_future().get());
@@ -1778,7 +1780,8 @@ int sis_simulation(const int *dims, unsigned char *data, unsigned char *mask, co
             pair64[c] = E.buf<double>(("sis_pair64_" + sfx).c_str(), (size_t)pn);
             float *p32 = E.buf<float>(("sis_pair32_" + sfx).c_str(), (size_t)pn);
             launch_build_pair(g, dev_model(pl.f.m), 1, sv, pair64[c], p32, st);
-            std::vector<int4> t4(tv.size());
+            std::vector<int4> &t4 = templates[c];
+            t4.resize(tv.size());
             for (size_t i = 0; i < tv.size(); ++i) t4[i] = make_int4(tv[i].dx, tv[i].dy, tv[i].dz, pair_lin(g, tv[i].dx, tv[i].dy, tv[i].dz));
             int4 *tmpl = E.buf<int4>(("sis_tmpl_" + sfx).c_str(), std::max<size_t>(t4.size(), 1));
             if (!t4.empty())
