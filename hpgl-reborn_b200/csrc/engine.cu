@@ -1295,11 +1295,13 @@ static bool sgs_walk(long long size, long long seed, SgsWalk &w)
 // before_levels runs once, after the first chunk's solves are queued.
 constexpr size_t kSimChunkBytes = (size_t)256 << 20;
 template <typename B, typename L>
-static void run_sim_levels(Engine &E, const std::vector<SisCat> &cats, int kmax, const int *sim_cells,
+static void run_sim_levels(Engine &E, const int *dims, const std::vector<SisCat> &cats, int kmax, const int *sim_cells,
                            const int *order, const std::vector<int> &offs, int n_levels, int n_sim, bool sgs,
                            bool ordinary, bool correlogram, cudaStream_t st, B before_levels, L level)
 {
     SimWeights a{};
+    a.nx = FastDiv::of(dims[0]);
+    a.ny = FastDiv::of(dims[1]);
     a.kcat = (int)cats.size();
     a.kmax = kmax;
     a.sim_cells = sim_cells;
@@ -1471,7 +1473,7 @@ int sgs_simulation(const int *dims, float *data, unsigned char *mask, const unsi
         launch_build_pair(g, dev_model(pl.f.m), 1, search_vals, pair64, pair32, st);
         E.stats.launches += 1 + ((use_cdf || lvm) ? 1 : 0) + (n_sim > 0 ? 4 : 0); // + search, moments, levels x2
         std::vector<int4> t4(tv.size());
-        for (size_t i = 0; i < tv.size(); ++i) t4[i] = make_int4(tv[i].dx, tv[i].dy, tv[i].dz, pair_lin(g, tv[i].dx, tv[i].dy, tv[i].dz));
+        for (size_t i = 0; i < tv.size(); ++i) t4[i] = make_int4(tv[i].dx, tv[i].dy, tv[i].dz, 0);
         int4 *tmpl = E.buf<int4>("sgs_tmpl", std::max<size_t>(t4.size(), 1));
         if (!t4.empty())
             HB_CK(cudaMemcpyAsync(tmpl, t4.data(), t4.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
@@ -1485,12 +1487,10 @@ int sgs_simulation(const int *dims, float *data, unsigned char *mask, const unsi
         // neighbours of every simulated node
         const int k = a.max_nb;
         int *nb = E.buf<int>("sgs_nb", (size_t)std::max(n_sim, 1) * k);
-        int *nb_lin = k <= 32 ? E.buf<int>("sgs_nb_lin", (size_t)std::max(n_sim, 1) * k) : nullptr;
         int *nb_rank = E.buf<int>("sgs_nb_rank", (size_t)std::max(n_sim, 1) * k);
         int *nb_cnt = E.buf<int>("sgs_nb_cnt", (size_t)std::max(n_sim, 1));
         if (n_sim > 0)
-            launch_sgs_search(g, tmpl, (int)t4.size(), sim_cells, n_sim, rank_of, k, nb, nb_lin, nb_rank, nb_cnt, E.n_sm(),
-                              st);
+            launch_sgs_search(g, tmpl, (int)t4.size(), sim_cells, n_sim, rank_of, k, nb, nb_rank, nb_cnt, E.n_sm(), st);
         HB_CK(cudaGetLastError());
         E.mark(STAGE_SEARCH, st);
 
@@ -1560,8 +1560,8 @@ int sgs_simulation(const int *dims, float *data, unsigned char *mask, const unsi
         if (k <= 32 && n_sim > 0)
         {
             const std::vector<SisCat> one{
-                SisCat{pair64, nb, nb_lin, nb_cnt, nullptr, g.pair_center, g.pnx, g.pny, k, 0.0f}};
-            run_sim_levels(E, one, k, sim_cells, order, offs, n_levels, n_sim, true, ordinary, false, st,
+                SisCat{pair64, nb, nb_cnt, nullptr, g.pair_center, g.pnx, g.pny, k, 0.0f}};
+            run_sim_levels(E, dims, one, k, sim_cells, order, offs, n_levels, n_sim, true, ordinary, false, st,
                            draws_in, [&](const SimWeights &w, int first, int count, bool beside) {
                                return launch_sgs_level(w, first, count, beside, d_data, d_means, d_u, st_rank, st);
                            });
@@ -1762,7 +1762,7 @@ int sis_simulation(const int *dims, unsigned char *data, unsigned char *mask, co
         int *nb_rank = E.buf<int>("sis_nb_rank", ns * ktot);
         HB_CK(cudaMemsetAsync(nb_rank, 0xFF, ns * ktot * 4, st)); // -1: no neighbour
         std::vector<double *> pair64(kcat);
-        std::vector<int *> nb(kcat), nb_lin(kcat), nb_cnt(kcat);
+        std::vector<int *> nb(kcat), nb_cnt(kcat);
         // the host tables live until the synchronisation behind the last copy of them
         std::vector<SisPlan> plans;
         std::vector<std::vector<int4>> templates(kcat);
@@ -1782,15 +1782,14 @@ int sis_simulation(const int *dims, unsigned char *data, unsigned char *mask, co
             launch_build_pair(g, dev_model(pl.f.m), 1, sv, pair64[c], p32, st);
             std::vector<int4> &t4 = templates[c];
             t4.resize(tv.size());
-            for (size_t i = 0; i < tv.size(); ++i) t4[i] = make_int4(tv[i].dx, tv[i].dy, tv[i].dz, pair_lin(g, tv[i].dx, tv[i].dy, tv[i].dz));
+            for (size_t i = 0; i < tv.size(); ++i) t4[i] = make_int4(tv[i].dx, tv[i].dy, tv[i].dz, 0);
             int4 *tmpl = E.buf<int4>(("sis_tmpl_" + sfx).c_str(), std::max<size_t>(t4.size(), 1));
             if (!t4.empty())
                 HB_CK(cudaMemcpyAsync(tmpl, t4.data(), t4.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
             nb[c] = E.buf<int>(("sis_nb_" + sfx).c_str(), ns * cats[c].max_nb);
-            nb_lin[c] = E.buf<int>(("sis_nb_lin_" + sfx).c_str(), ns * cats[c].max_nb);
             nb_cnt[c] = E.buf<int>(("sis_nb_cnt_" + sfx).c_str(), ns);
             if (n_sim > 0)
-                launch_sgs_search(g, tmpl, (int)t4.size(), sim_cells, n_sim, rank_of, cats[c].max_nb, nb[c], nb_lin[c],
+                launch_sgs_search(g, tmpl, (int)t4.size(), sim_cells, n_sim, rank_of, cats[c].max_nb, nb[c],
                                   nb_rank + koff[c], nb_cnt[c], E.n_sm(), st, -1, ktot);
             HB_CK(cudaGetLastError());
             if (c + 1 < kcat) HB_CK(cudaStreamSynchronize(st)); // the host tables of this category
@@ -1879,13 +1878,13 @@ int sis_simulation(const int *dims, unsigned char *data, unsigned char *mask, co
         for (int c = 0; c < kcat; ++c)
         {
             const Geom &g = plans[c].first.g;
-            hc[c] = SisCat{pair64[c], nb[c], nb_lin[c], nb_cnt[c], d_means[c], g.pair_center, g.pnx, g.pny, cats[c].max_nb,
+            hc[c] = SisCat{pair64[c], nb[c], nb_cnt[c], d_means[c], g.pair_center, g.pnx, g.pny, cats[c].max_nb,
                            (float)cats[c].marginal};
         }
         int kmax = 0;
         for (int c = 0; c < kcat; ++c) kmax = std::max(kmax, cats[c].max_nb);
         if (n_sim > 0)
-            run_sim_levels(E, hc, kmax, sim_cells, order, offs, n_levels, n_sim, false, false,
+            run_sim_levels(E, dims, hc, kmax, sim_cells, order, offs, n_levels, n_sim, false, false,
                            correlogram && means, st, draws_in, [&](const SimWeights &w, int first, int count, bool beside) {
                                return launch_sis_level(w, first, count, beside, ncat, d_data, d_u, st_rank, st);
                            });

@@ -226,10 +226,9 @@ void launch_sgs_path(const SgsWalk &w, const uint8_t *mask, const uint8_t *sim_m
 void launch_sgs_index(long long n, const int *path_cell, const int *flag, const int *scan, const uint8_t *mask,
                       int *rank_of, int *sim_cells, cudaStream_t st);
 // Template scan with the rank predicate rank_of[q] < rank (or < fixed_rank when
-// fixed_rank >= 0); nb_rank may be null, and so may nb_lin, which
-// gets the neighbours' pair-table offsets (the template's .w).
+// fixed_rank >= 0); nb_rank may be null.
 void launch_sgs_search(const Geom &g, const int4 *tmpl, int n_tmpl, const int *sim_cells, int n_sim,
-                       const int *rank_of, int k, int *nb, int *nb_lin, int *nb_rank, int *nb_cnt, int n_sm, cudaStream_t st,
+                       const int *rank_of, int k, int *nb, int *nb_rank, int *nb_cnt, int n_sm, cudaStream_t st,
                        int fixed_rank = -1, int rank_stride = 0);
 // Weights of the simulated nodes, solved ahead of the levels (sim_weights.cu)
 constexpr int kSisMaxCat = 16;
@@ -237,7 +236,6 @@ struct SisCat
 {
     const double *pair64; // the category's pair table
     const int *nb;        // its neighbour cells, k per rank
-    const int *nb_lin;    // and their pair-table offsets from the node
     const int *nb_cnt;
     const float *means;   // LVM: the category's mean per cell, or null
     long long pair_center;
@@ -245,8 +243,23 @@ struct SisCat
     int k;
     float marginal;       // the category's mean (float, as the reference stores it)
 };
+// x / d for x < 2^31 by a multiplication: x m >> 31 + s, m = ceil(2^(31 + s) / d),
+// 2^s >= d (T. Granlund and P. Montgomery, Division by invariant integers using
+// multiplication, 1994: m d - 2^(31 + s) < d <= 2^s, so the quotient is exact)
+struct FastDiv
+{
+    unsigned d, m;
+    int s;
+    static FastDiv of(int d)
+    {
+        int s = 0;
+        while ((1ll << s) < d) ++s;
+        return FastDiv{(unsigned)d, (unsigned)(((1ull << (31 + s)) + d - 1) / d), s};
+    }
+};
 struct SimWeights
 {
+    FastDiv nx, ny;      // the grid's rows and row counts
     const SisCat *cats;  // kcat entries (device); SGS: one
     int kcat, kmax;      // kmax: the largest k of the categories (at most 32)
     const int *sim_cells;

@@ -197,8 +197,7 @@ __global__ void k_sgs_index(long long n, const int *__restrict__ path_cell, cons
 __global__ void __launch_bounds__(256) k_sgs_search(const Geom g, const int4 *__restrict__ tmpl, int n_tmpl,
                                                     const int *__restrict__ sim_cells, int n_sim,
                                                     const int *__restrict__ rank_of, int k, int fixed_rank,
-                                                    int *__restrict__ nb, int *__restrict__ nb_lin,
-                                                    int *__restrict__ nb_rank, int rank_stride,
+                                                    int *__restrict__ nb, int *__restrict__ nb_rank, int rank_stride,
                                                     int *__restrict__ nb_cnt)
 {
     const int lane = threadIdx.x & 31;
@@ -215,7 +214,7 @@ __global__ void __launch_bounds__(256) k_sgs_search(const Geom g, const int4 *__
         {
             const int t = base + lane;
             bool hit = false;
-            int q = 0, rq = 0, lin = 0;
+            int q = 0, rq = 0;
             if (t < n_tmpl)
             {
                 const int4 o = tmpl[t];
@@ -224,7 +223,6 @@ __global__ void __launch_bounds__(256) k_sgs_search(const Geom g, const int4 *__
                 {
                     q = (int)(((long long)Z * g.ny + Y) * g.nx + X);
                     rq = rank_of[q];
-                    lin = o.w;
                     hit = rq < thr;
                 }
             }
@@ -233,7 +231,6 @@ __global__ void __launch_bounds__(256) k_sgs_search(const Geom g, const int4 *__
             if (hit && slot < k)
             {
                 out[slot] = q;
-                if (nb_lin) nb_lin[r * (long long)k + slot] = lin;
                 if (out_rank) out_rank[slot] = rq;
             }
             found += __popc(m);
@@ -576,10 +573,10 @@ void launch_sgs_index(long long n, const int *path_cell, const int *flag, const 
     k_sgs_index<<<1184, 256, 0, st>>>(n, path_cell, flag, scan, mask, rank_of, sim_cells);
 }
 void launch_sgs_search(const Geom &g, const int4 *tmpl, int n_tmpl, const int *sim_cells, int n_sim,
-                       const int *rank_of, int k, int *nb, int *nb_lin, int *nb_rank, int *nb_cnt, int n_sm, cudaStream_t st,
+                       const int *rank_of, int k, int *nb, int *nb_rank, int *nb_cnt, int n_sm, cudaStream_t st,
                        int fixed_rank, int rank_stride)
 {
-    k_sgs_search<<<n_sm * 8, 256, 0, st>>>(g, tmpl, n_tmpl, sim_cells, n_sim, rank_of, k, fixed_rank, nb, nb_lin, nb_rank,
+    k_sgs_search<<<n_sm * 8, 256, 0, st>>>(g, tmpl, n_tmpl, sim_cells, n_sim, rank_of, k, fixed_rank, nb, nb_rank,
                                            rank_stride > 0 ? rank_stride : k, nb_cnt);
 }
 void launch_sgs_levels(const int *nb_rank, const int *nb_cnt, int k, int n_sim, int *levp1, int *ticket,

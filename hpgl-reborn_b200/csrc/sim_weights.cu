@@ -23,6 +23,11 @@ namespace hb
 // 20 warps of 96 registers (the chain of pivots is what a warp waits for)
 constexpr int kWeightThreads = 640;
 
+__device__ __forceinline__ int fast_div(int x, const FastDiv &f)
+{
+    return f.s ? (int)(__umulhi((unsigned)x, f.m) >> (f.s - 1)) : x;
+}
+
 enum SimMode
 {
     kSimSK = 0,  // SGS, simple kriging
@@ -46,7 +51,7 @@ __global__ void __launch_bounds__(kWeightThreads, 1) k_sim_weights(const SimWeig
     // is issued a stage at a time during the current solve
     struct Item
     {
-        int cat, pos, r, n, lin;
+        int cat, pos, r, n, cell, q; // q: the lane's neighbour (the node itself beyond n)
     };
     auto stage_a = [&](int it, Item &s) {
         s.cat = 0;
@@ -61,10 +66,11 @@ __global__ void __launch_bounds__(kWeightThreads, 1) k_sim_weights(const SimWeig
     };
     auto stage_b = [&](Item &s) {
         s.n = s.r >= 0 ? __ldg(a.cats[s.cat].nb_cnt + s.r) : 0;
+        s.cell = s.r >= 0 ? __ldg(a.sim_cells + s.r) : 0;
     };
     auto stage_c = [&](Item &s) {
         const SisCat &C = a.cats[s.cat];
-        s.lin = lane < s.n ? __ldg(C.nb_lin + (long long)s.r * C.k + lane) : 0;
+        s.q = lane < s.n ? __ldg(C.nb + (long long)s.r * C.k + lane) : s.cell;
     };
     int it = blockIdx.x * (kWeightThreads / 32) + (threadIdx.x >> 5);
     Item cur, nxt;
@@ -77,21 +83,26 @@ __global__ void __launch_bounds__(kWeightThreads, 1) k_sim_weights(const SimWeig
         const SisCat &C = a.cats[cur.cat];
         const double *pair_c = C.pair64 + C.pair_center;
         const int n = cur.n;
-        // ---- this warp's system
+        // ---- this warp's system. The neighbours' pair-table offsets are formed here:
+        // stored by the search they took four bytes more a neighbour
+        const int rows_q = fast_div(cur.q, a.nx), rows_c = fast_div(cur.cell, a.nx);
+        const int z_q = fast_div(rows_q, a.ny), z_c = fast_div(rows_c, a.ny);
+        const int dz = z_q - z_c, dy = rows_q - rows_c - (int)a.ny.d * dz;
+        const int dx = cur.q - cur.cell - (int)a.nx.d * (rows_q - rows_c);
+        const int lin = dx + C.pnx * (dy + C.pny * dz);
         double bi = 0.0;
         {
             double s = 1.0;
             if (lane < n)
             {
-                bi = __ldg(pair_c + abs(cur.lin));
+                bi = __ldg(pair_c + abs(lin));
                 if (CORR)
                 {
-                    const int q = C.nb[(long long)cur.r * C.k + lane], c = a.sim_cells[cur.r];
-                    s = sis_sigma(C.means ? C.means[q] : C.marginal);
-                    bi = __dmul_rn(bi, __dmul_rn(s, sis_sigma(C.means ? C.means[c] : C.marginal)));
+                    s = sis_sigma(C.means ? C.means[cur.q] : C.marginal);
+                    bi = __dmul_rn(bi, __dmul_rn(s, sis_sigma(C.means ? C.means[cur.cell] : C.marginal)));
                 }
             }
-            T.lin[lane] = cur.lin;
+            T.lin[lane] = lin;
             T.y[0][lane] = bi;
             if (Q == 2) T.y[Q - 1][lane] = lane < n ? 1.0 : 0.0;
             if (CORR) T.sig[lane] = s;
