@@ -500,7 +500,8 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
     launch_bin_count(P.pts_xyz, P.n_pts, g, bin_cnt, st);
     HB_CK(cudaMemcpyAsync(bin_start, bin_cnt, sizeof(int) * g.n_bins, cudaMemcpyDeviceToDevice, st));
     exclusive_scan(bin_start, g.n_bins, tmp, scal + 0, st);
-    int *bin_tmp = E.buf<int>("bin_tmp", std::max(P.m, 1));
+    int *tie_cells = E.buf<int>("tie_cells", (size_t)g.n_cells);
+    int *bin_tmp = tie_cells; // (the searches write tie_cells later on the stream)
     launch_bin_fill(P.pts_xyz, P.n_pts, g, bin_start, bin_fill, bin_tmp, st);
     launch_bin_sort(g, bin_start, bin_cnt, bin_tmp, bin_pts, S.bin_flag, st);
     launch_bin_region(g, S.bin_flag, bin_cnt, scal + 1, scal + 2, tmpl_bins, scal + 6, scal + 7, st);
@@ -611,7 +612,6 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
     S.nb_rec = E.buf<int2>("nb_rec", (size_t)g.n_cells * g.k);
     S.nb_pid = want_pids ? E.buf<int>("nb_pid", (size_t)g.n_cells * g.k) : nullptr;
     S.nb_n = E.buf<int>("nb_n", (size_t)g.n_cells);
-    int *tie_cells = E.buf<int>("tie_cells", (size_t)g.n_cells);
     HB_CK(cudaMemsetAsync(S.nb_n, 0, sizeof(int) * g.n_cells, st));
     HB_CK(cudaEventRecord(E.ev_[8], st));
     const bool tile = fast && sd.on && !warp_per_cell && cand_cap <= tile_limit;
@@ -632,7 +632,8 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
                          : nullptr;
     if (tmpl_tile)
     {
-        int *ties_t = rank_keys ? E.buf<int>("tmpl_ties", (size_t)g.n_cells) : tie_cells;
+        // the solves' work list, which is written after the search
+        int *ties_t = rank_keys ? reinterpret_cast<int *>(E.buf<int2>("cells", (size_t)g.n_cells)) : tie_cells;
         HB_CK(launch_search_tile(g, d_mask, all_cells, bin_start, bin_cnt, S.bin_flag, bin_pts, P.pts_xyz, P.pts_val,
                                  keypos16, sdp, 1, n_tmpl_bins, cand_cap_t, E.max_smem() - 1024, S.nb_rec, S.nb_n, ties_t,
                                  scal + (rank_keys ? 8 : 3), scal + 4, scal + 5, st));
@@ -749,8 +750,10 @@ static void run_solves(Engine &E, const Plan &pl, const DevPoints &P, const DevS
     const int *cnt = host_prep.cnt;
     const unsigned long long *mom = host_prep.mom;
     E.mark(STAGE_PREPARE, st);
-    // one list for every sharing bucket (they run one after another)
-    int2 *left_cells = any_share ? E.buf<int2>("left_cells", (size_t)std::max(1, std::max(cnt[2], cnt[3]))) : nullptr;
+    // one list for every sharing bucket (they run one after another); where the device
+    // has no room for it, every cell goes to the one-system kernel
+    int2 *left_cells =
+        any_share ? E.try_buf<int2>("left_cells", (size_t)std::max(1, std::max(cnt[2], cnt[3]))) : nullptr;
     int off = 0;
     const double c0 = pl.f.c0();
     const double rhs = ordinary ? 2.0 : 1.0;
@@ -804,7 +807,7 @@ static void run_solves(Engine &E, const Plan &pl, const DevPoints &P, const DevS
             {
                 int2 *first_esc = quad ? ref_cells + off : (esc_cells ? esc_cells + off : nullptr);
                 const bool share =
-                    is_share_variant(kBucketNP[b], precision, variant[b]) && cnt[b] >= share_from(b);
+                    left_cells && is_share_variant(kBucketNP[b], precision, variant[b]) && cnt[b] >= share_from(b);
                 HB_CK(launch_solve_bucket(kBucketNP[b], precision, variant[b], ordinary, g, bcells, bucket_cnt + b,
                                           cnt[b], S.nb_rec, S.nb_n, ind_value, S.pair64, S.pair32, mean, c0, steps,
                                           tol, out, first_esc, quad ? ref_cnt + b : esc_cnt + b,
