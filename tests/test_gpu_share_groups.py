@@ -11,6 +11,7 @@ import torch
 
 import helpers as H
 import oracle as O
+from geo_bsd import hpgl_wrap as W
 from geo_bsd import workloads as WL
 
 pytestmark = pytest.mark.gpu
@@ -77,3 +78,66 @@ def test_groups_that_fail_and_are_halved(kind):
     assert sum(not whole and half for whole, half in groups) >= 10
     assert sum(not half for _, half in groups) >= 10
     _shares(_check(wl, kind), 2)
+
+
+@pytest.mark.parametrize("dims,rad", [((96, 80, 60), (1, 1, 1)), ((60, 60, 40), (2, 1, 3))])
+@pytest.mark.parametrize("kind", [0, 1])
+def test_small_radiuses_shared(kind, dims, rad):
+    """The pair table of a small radius limits how far apart grouped cells may be: two
+    thirds of the cells informed, so that its few cells hold 17 neighbours."""
+    cov = WL.CovSpec(WL.EXPONENTIAL, (30.0, 30.0, 30.0), (0.0, 0.0, 0.0), 1.0, 0.05)
+    _shares(_check(_wl(dims, 0.66, cov, rad, 27), kind), 2)
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("k", [19, 32, 50])
+def test_long_thin_grid_shared(kind, k):
+    cov = WL.CovSpec(WL.EXPONENTIAL, (600.0, 30.0, 30.0), (0.0, 0.0, 0.0), 1.0, 0.05)
+    _shares(_check(_wl((5301, 3, 3), 0.07, cov, (60, 3, 3), k), kind), 2 if k <= 32 else 3)
+
+
+@pytest.mark.parametrize("np_,k,informed", [(32, 32, 0.05), (64, 50, 0.05)])
+@pytest.mark.parametrize("kind", [0, 1])
+def test_refined_option_shared(kind, np_, k, informed):
+    """FP32-refined keys set to SHARE: the FP64 solves, nothing escalated."""
+    cov = WL.CovSpec(WL.EXPONENTIAL, (12.0, 9.0, 7.0), (30.0, 0.0, 0.0), 1.0, 0.05)
+    wl = _wl((53, 47, 19), informed, cov, (12, 9, 7), k)
+    prev = W.solve_variant(np_, cov.cov_type, W.FP32_REFINED, W.VARIANT_SHARE)
+    try:
+        s = _check(wl, kind, precision=W.FP32_REFINED)
+    finally:
+        W.solve_variant(np_, cov.cov_type, W.FP32_REFINED, prev)
+    _shares(s, 2 if np_ == 32 else 3)
+    assert s["escalated_cells"] == 0
+
+
+@pytest.mark.parametrize("k,bucket,nugget", [(30, 2, 0.75), (52, 3, 0.82)])
+def test_indefinite_systems_shared(k, bucket, nugget):
+    """Simple kriging whose box cuts the covariance off at a fifth of its range: some
+    systems are indefinite, and fail in any order of elimination; the others' solves
+    go through. Cells whose smallest eigenvalue is within 1e-6 of zero are left out."""
+    rad = (6, 6, 6)
+    cov = WL.CovSpec(WL.GAUSSIAN, (30.0, 30.0, 30.0), (0.0, 0.0, 0.0), 1.0, nugget)
+    wl = _wl((50, 46, 24), 0.05, cov, rad, k)
+    nx, ny, _ = wl.dims
+    nodes = np.flatnonzero(wl.mask == 0).astype(np.int32)
+    r = O.krige_nodes("port", 1, wl.dims, wl.data, wl.mask, cov, rad, k, mean=0.0, nodes=nodes)
+    e = H.engine_cont(1, wl, precision=0, mean=0.0)
+    _shares(e["stats"], bucket)
+    clear = np.zeros(len(nodes), bool)
+    for n in np.unique(r["count"]):
+        at = np.flatnonzero(r["count"] == n)
+        if n == 0:
+            clear[at] = True
+            continue
+        p = r["idx"][at, :n]
+        xyz = np.stack([p % nx, p // nx % ny, p // (nx * ny)], -1)
+        d = xyz[:, :, None, :] - xyz[:, None, :, :]
+        A = (1 - nugget) * np.exp(-3 * (d * d).sum(-1) / 900.0) * (np.abs(d) <= np.array(rad)).all(-1)
+        A += nugget * np.eye(n)
+        clear[at] = np.abs(np.linalg.eigvalsh(A)).min(-1) > 1e-6
+    failed = r["status"] == 2
+    assert clear.mean() > 0.9 and (failed & clear).sum() > 1000 and (~failed & clear).sum() > 1000
+    np.testing.assert_array_equal(e["status"][nodes][clear], r["status"][clear].astype(np.int8))
+    ok = clear & (r["status"] == 0)
+    assert H.rel_err(e["est"][nodes][ok], r["est"][ok]) <= 1e-8  # condition numbers below 10^8
