@@ -143,6 +143,18 @@ def z_slab(wl, z0, nz):
     return (nx, ny, nz), np.ascontiguousarray(wl.data[a:b]), np.ascontiguousarray(wl.mask[a:b])
 
 
+def reference_missing(kind):
+    """Why the reference's own code cannot run here, or None where it can: its
+    library (LVM: the harness around its per-node code) is built from its sources
+    and is absent where they were."""
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import oracle as O
+    path = O.REF_PATH if kind == "lvm" else O.REF_API_PATH
+    if os.path.exists(path):
+        return None
+    return f"{os.path.relpath(path, ROOT)} is not here (it is built from the reference's sources)"
+
+
 def ref_api_slab(wl, kind, nz, threads):
     """One whole call of the reference library's own public entry point
     (hpgl_ordinary_kriging / hpgl_simple_kriging from oracle/_ref/libhpgl.so,
@@ -211,8 +223,20 @@ def cpu_reference(wl, kind, target_seconds, threads):
     rate = len(probe) / t_probe
     n = int(min(len(unk), max(len(probe), rate * target_seconds)))
     sample = np.sort(rng.choice(unk, n, replace=False)).astype(np.int32)
-    t = timed(sample) - setup
+    t = max(timed(sample) - setup, 1e-3)
     return n / t, {"which": which, "sample_cells": n, "seconds": t, "setup_seconds": setup, "threads": threads}
+
+
+def cpu_baseline_nodes(wl, kind, target_seconds):
+    """cpu_baseline of the reference's per-node code (without it, of its CPU
+    restatement) on sampled cells, all host threads."""
+    threads = os.cpu_count() or 1
+    v, info = cpu_reference(wl, kind, target_seconds, threads)
+    code = "the reference's own per-node code (kriging_interpolation)" if info["which"] == "ref" else \
+        "the CPU restatement of the reference's per-node code"
+    return {"value": v, "unit": UNIT, "cores": threads, "kind": "reference" if info["which"] == "ref" else "port",
+            "sample": f"{info['sample_cells']} random uninformed cells of the same grid; {code} over OpenMP, lookup "
+                      f"construction excluded ({info['setup_seconds']:.2f}s)", "cpu_model": cpu_model()}
 
 
 # ---------------------------------------------------------------- clocks
@@ -450,7 +474,7 @@ def bench_sgs(args, rank, world, local):
     lib.hpgl_b200_host_free(h_data)
     lib.hpgl_b200_host_free(h_mask)
     cpu = None
-    if rank == 0 and not args.skip_cpu_baseline:
+    if rank == 0 and not args.skip_cpu_baseline and not reference_missing(args.kind):
         v, info = sgs_reference(args.cpu_seconds)
         d = "x".join(str(x) for x in info["dims"])
         cpu = {"value": v, "unit": UNIT, "cores": 1, "kind": "reference",
@@ -649,7 +673,7 @@ def bench_sis(args, rank, world, local):
     lib.hpgl_b200_host_free(h_data)
     lib.hpgl_b200_host_free(h_mask)
     cpu = None
-    if rank == 0 and not args.skip_cpu_baseline:
+    if rank == 0 and not args.skip_cpu_baseline and not reference_missing(args.kind):
         v, info = sis_reference(args.cpu_seconds)
         d = "x".join(str(x) for x in info["dims"])
         cpu = {"value": v, "unit": UNIT, "cores": 1, "kind": "reference",
@@ -823,7 +847,7 @@ def bench_cok(args, rank, world, local):
     for ptr in h:
         lib.hpgl_b200_host_free(ptr)
     cpu = None
-    if rank == 0 and not args.skip_cpu_baseline:
+    if rank == 0 and not args.skip_cpu_baseline and not reference_missing(args.kind):
         v, info = cok_reference(args.cpu_seconds)
         d = "x".join(str(x) for x in info["dims"])
         cpu = {"value": v, "unit": UNIT, "cores": 1, "kind": "reference",
@@ -1071,6 +1095,12 @@ def bench_other_configs(args, W, dev, stream, pk):
 def main():
     args = parse()
     rank, world, local = dist_env()
+    if args.impl == "reference":
+        why = reference_missing(args.kind)
+        if why:
+            if rank == 0:
+                print(json.dumps({"impl": "reference", "unavailable": why}), flush=True)
+            return
     if args.kind == "sgs":
         bench_sgs(args, rank, world, local)
         return
@@ -1314,15 +1344,10 @@ def main():
 
     cpu = None
     if rank == 0 and world == 1 and not args.skip_cpu_baseline:
-        if args.kind in ("ok", "sk"):
+        if args.kind in ("ok", "sk") and not reference_missing(args.kind):
             cpu = cpu_baseline_api(wl, args.kind, args.cpu_seconds)
         else:
-            threads = os.cpu_count() or 1
-            v, info = cpu_reference(wl, args.kind, args.cpu_seconds, threads)
-            cpu = {"value": v, "unit": UNIT, "cores": threads, "kind": "reference" if info["which"] == "ref" else "port",
-                   "sample": f"{info['sample_cells']} random uninformed cells of the same grid; the reference's own "
-                             f"per-node code (kriging_interpolation) over OpenMP, lookup construction excluded "
-                             f"({info['setup_seconds']:.2f}s)", "cpu_model": cpu_model()}
+            cpu = cpu_baseline_nodes(wl, args.kind, args.cpu_seconds)
 
     if rank == 0:
         line = {
