@@ -877,20 +877,35 @@ def bench_cok(args, rank, world, local):
 
 
 def shared_solve(W, np_, v, precision):
-    """Whether variant v of a key runs the FP64 solves that share factorisations."""
+    """Whether variant v of a key runs the FP64 tensor solves (which share
+    factorisations between neighbouring cells)."""
     if precision:
         return v == getattr(W, "VARIANT_SHARE", -1)
     return (np_ == 32 and v == W.VARIANT_FOLD) or (np_ == 64 and v in (getattr(W, "VARIANT_WIDE", -1), W.VARIANT_DEFAULT))
 
 
-def bucket_kernel(W, b, cov_type, precision, ordinary):
-    """Name of the solve kernel that ran bucket b (0..4) for this key."""
+def sm_count():
+    import torch
+    return torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+
+
+def shares_from(np_, sms):
+    """Systems in a bucket from which it shares (run_solves: share_from)."""
+    return (256 if np_ <= 32 else 128) * sms
+
+
+def bucket_kernel(W, b, cov_type, precision, ordinary, items, sms):
+    """Name of the solve kernel that ran the `items` systems of bucket b (0..4) for
+    this key on `sms` multiprocessors."""
     if b == 4:
         return "k_solve_large (n > 64, one block per system, FP64)"
     np_ = [8, 16, 32, 64][b]
     v = W.solve_variant(np_, cov_type, precision) if hasattr(W, "solve_variant") else 1
     kind = "ordinary" if ordinary else "simple"
     if shared_solve(W, np_, v, precision):
+        if items < shares_from(np_, sms):
+            nb, th = (4, 640) if np_ == 32 else (8, 256)
+            return f"k_solve_mma<NB={nb}, {kind}, {th}> (FP64 tensor, one system per warp)"
         cb, th = (3, 512) if np_ == 32 else (7, 256)
         return f"k_solve_share<CB={cb}, {kind}, {th}> (FP64 tensor, factorisations shared by neighbouring cells)"
     if np_ == 64 and v in (getattr(W, "VARIANT_WIDE", -1), W.VARIANT_DEFAULT):
@@ -919,7 +934,8 @@ def solve_roofline(W, stats_list, cov_type, precision, ordinary, pk):
     np_ = [8, 16, 32, 64, 65][b]
     fp32 = precision and not (b < 4 and shared_solve(W, np_, W.solve_variant(np_, cov_type, precision), precision))
     peak = pk["fp32"] if fp32 else pk["fp64"]
-    return {"kernel": bucket_kernel(W, b, cov_type, precision, ordinary), "kernel_ms": ms,
+    return {"kernel": bucket_kernel(W, b, cov_type, precision, ordinary, last[f"bucket_items_{b}"], sm_count()),
+            "kernel_ms": ms,
             "algorithmic_flops": flops, "achieved_tflops": tf, "peak_tflops": peak, "frac": tf / peak,
             "bound": "fp32" if fp32 else "fp64"}
 
@@ -1263,7 +1279,7 @@ def main():
     b_flops = last[f"bucket_flops_{b}"]
     achieved = b_flops / (b_ms / 1e3) / 1e12
     tpc = traffic_per_cell()
-    kname = bucket_kernel(W, b, wl.cov.cov_type, 1, kind == 0 and not lvm)
+    kname = bucket_kernel(W, b, wl.cov.cov_type, 1, kind == 0 and not lvm, last[f"bucket_items_{b}"], sm_count())
     np_ = [8, 16, 32, 64, 65][b]
     in64 = b == 4 or shared_solve(W, np_, W.solve_variant(np_, wl.cov.cov_type, 1), 1)
     bound = "fp64" if in64 else "fp32"
