@@ -490,8 +490,9 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
     int *bin_pts = E.buf<int>("bin_pts", std::max(P.m, 1));
     int *tmpl_bins = E.buf<int>("tmpl_bins", g.n_bins);
     // 0 total, 1 max_cand, 2 tmpl bins, 3 ties, 4 tmpl cells, 5 exact cells, 6 max_cand of the template
-    // bins, 7 the largest bin above kBinSortMax, 8 ties of template-path cells selected by rank
-    constexpr int kScalars = 9;
+    // bins, 7 the largest bin above kBinSortMax, 8 ties of template-path cells selected by rank,
+    // 9 whether template bins are better scanned (1), and others not (2)
+    constexpr int kScalars = 10;
     int *scal = E.buf<int>("scalars", kScalars);
     int *tmp = E.buf<int>("scan_tmp2", (size_t)scan_tmp_ints(g.n_bins) + 4);
     HB_CK(cudaMemsetAsync(bin_cnt, 0, sizeof(int) * g.n_bins, st));
@@ -504,7 +505,7 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
     int *bin_tmp = tie_cells; // (the searches write tie_cells later on the stream)
     launch_bin_fill(P.pts_xyz, P.n_pts, g, bin_start, bin_fill, bin_tmp, st);
     launch_bin_sort(g, bin_start, bin_cnt, bin_tmp, bin_pts, S.bin_flag, st);
-    launch_bin_region(g, S.bin_flag, bin_cnt, scal + 1, scal + 2, tmpl_bins, scal + 6, scal + 7, st);
+    launch_bin_region(g, S.bin_flag, bin_cnt, scal + 1, scal + 2, tmpl_bins, scal + 6, scal + 7, scal + 9, st);
     HB_CK(cudaGetLastError());
     int host_scal[kScalars];
     HB_CK(cudaMemcpyAsync(host_scal, scal, sizeof(host_scal), cudaMemcpyDeviceToHost, st));
@@ -524,7 +525,17 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
     int n_tmpl = 0;
     int4 *tmpl = E.buf<int4>("tmpl", std::max<long>(pl.tmpl_count, 1));
     bool tmpl_select = false, tmpl_tile = false, tmpl_scan = false, rank_keys = false;
-    const int tile_limit = search_tile_limit(g.k, E.max_smem() - 1024);
+    // The template scan probes a bitmap of the grid padded by the radiuses, by linear
+    // offsets of 32 bits.
+    const long long pad_x = g.nx + 2LL * g.rx, pad_y = g.ny + 2LL * g.ry;
+    const bool scannable = (long long)g.rz * pad_y * pad_x + (long long)g.ry * pad_x + g.rx <= 2147483647LL;
+    // The lane-a-cell search takes cluster-path bins while a warp of it fits, since what is
+    // left is slower still; of the template-path bins, where they can be scanned, those whose
+    // candidates leave room for eight warps (500,000 cells, radius 10, 40 % informed, 16
+    // neighbours: with one warp 5.6 ms, with eight 1.75, scanned 0.62)
+    const int tile_limit = search_tile_limit(g.k, E.max_smem() - 1024, 1);
+    const int tile_limit_t = search_tile_limit(g.k, E.max_smem() - 1024, scannable ? 8 : 1);
+    const bool leave_scans = scannable && (host_scal[9] & 1), scan_all = leave_scans && !(host_scal[9] & 2);
     uint16_t *keypos16 = nullptr;
     SurrDev sdp = {};
     int cand_cap_t = 0, warps_t = 8;
@@ -537,18 +548,18 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
         // and the cells whose k-th slot a tie straddles by the template scan (on the
         // clustered 512x512x64 grid, 111,537 offsets: 49 ms for every template-path
         // cell's scan)
-        rank_keys = tv.size() > 0xFFFE && use_sd && !warp_per_cell && tile_limit > 0;
+        rank_keys = tv.size() > 0xFFFE && use_sd && !warp_per_cell && !scan_all && tile_limit_t > 0;
         if (rank_keys)
         {
             tmpl_tile = true;
             cand_cap_t = std::max(4, (max_cand_tmpl + 3) / 4 * 4);
         }
-        else if (g.k <= 64 && tv.size() <= 0xFFFE)
+        else if (g.k <= 64 && tv.size() <= 0xFFFE && !(scan_all && !warp_per_cell))
         {
             build_surrogate_template(pl.f, tv, sgp);
             sdp.on = sgp.ok && !exact_search ? 1 : 0;
             cand_cap_t = std::max(4, (max_cand_tmpl + 3) / 4 * 4);
-            tmpl_tile = sdp.on && !warp_per_cell && tile_limit > 0;
+            tmpl_tile = sdp.on && !warp_per_cell && tile_limit_t > 0;
             if (!tmpl_tile)
             {
                 while (warps_t > 1 && search_fast_smem_bytes(cand_cap_t, g.k, warps_t) > (size_t)E.max_smem()) --warps_t;
@@ -581,14 +592,10 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
             }
         }
         std::vector<int4> t4;
-        tmpl_scan = !tmpl_select && (!tmpl_tile || max_cand_tmpl > tile_limit);
+        tmpl_scan = !tmpl_select && (!tmpl_tile || max_cand_tmpl > tile_limit_t || leave_scans);
         if (tmpl_scan || rank_keys)
         {
-            // the template probes a bitmap of the grid padded by the radiuses; its
-            // linear offsets are 32-bit
-            const long long PX = g.nx + 2LL * g.rx, PY = g.ny + 2LL * g.ry;
-            if ((long long)g.rz * PY * PX + (long long)g.ry * PX + g.rx > 2147483647LL)
-                throw CudaFail{-4, "grid too large for the template search path at these radiuses"};
+            if (!scannable) throw CudaFail{-4, "grid too large for the template search path at these radiuses"};
             t4.resize(tv.size());
             for (size_t i = 0; i < tv.size(); ++i)
                 t4[i] = make_int4(tv[i].dx, tv[i].dy, tv[i].dz, template_padded_offset(g, tv[i].dx, tv[i].dy, tv[i].dz));
@@ -617,7 +624,7 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
     const bool tile = fast && sd.on && !warp_per_cell && cand_cap <= tile_limit;
     if (tile)
         HB_CK(launch_search_tile(g, d_mask, all_cells, bin_start, bin_cnt, S.bin_flag, bin_pts, P.pts_xyz, P.pts_val,
-                                 keytab16, sd, 0, g.n_bins, cand_cap, E.max_smem() - 1024, S.nb_rec, S.nb_n, tie_cells, scal + 3,
+                                 keytab16, sd, 0, g.n_bins, cand_cap, tile_limit, false, E.max_smem() - 1024, S.nb_rec, S.nb_n, tie_cells, scal + 3,
                                  scal + 4, scal + 5, st));
     else if (fast)
         HB_CK(launch_search_fast(g, d_mask, all_cells, bin_start, bin_cnt, S.bin_flag, bin_pts, P.pts_xyz, P.pts_val,
@@ -635,7 +642,7 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
         // the solves' work list, which is written after the search
         int *ties_t = rank_keys ? reinterpret_cast<int *>(E.buf<int2>("cells", (size_t)g.n_cells)) : tie_cells;
         HB_CK(launch_search_tile(g, d_mask, all_cells, bin_start, bin_cnt, S.bin_flag, bin_pts, P.pts_xyz, P.pts_val,
-                                 keypos16, sdp, 1, n_tmpl_bins, cand_cap_t, E.max_smem() - 1024, S.nb_rec, S.nb_n, ties_t,
+                                 keypos16, sdp, 1, n_tmpl_bins, cand_cap_t, tile_limit_t, leave_scans, E.max_smem() - 1024, S.nb_rec, S.nb_n, ties_t,
                                  scal + (rank_keys ? 8 : 3), scal + 4, scal + 5, st));
         if (rank_keys)
             HB_CK(launch_search_template_list(g, d_mask, bits, ties_t, scal + 8, P.pts_val, tmpl, n_tmpl,
@@ -646,7 +653,7 @@ static DevSearch run_search(Engine &E, const Plan &pl, const DevPoints &P, const
                                  keypos16, sdp, 1, P.pid_of_node, cand_cap_t, warps_t, S.nb_pid, S.nb_rec, S.nb_n,
                                  tie_cells, scal + 3, scal + 4, scal + 5, st));
     if (tmpl_scan)
-        HB_CK(launch_search_template(g, d_mask, bits, all_cells, tmpl_bins, n_tmpl_bins, bin_cnt, tmpl_tile ? tile_limit : -1, P.pts_val, tmpl,
+        HB_CK(launch_search_template(g, d_mask, bits, all_cells, tmpl_bins, n_tmpl_bins, bin_cnt, tmpl_tile ? tile_limit_t : -1, P.pts_val, tmpl,
                                      n_tmpl, P.pid_of_node, S.nb_pid, S.nb_rec, S.nb_n, scal + 4, E.n_sm(), st));
     HB_CK(cudaEventRecord(E.ev_[9], st));
     HB_CK(cudaMemcpyAsync(host_scal, scal, sizeof(host_scal), cudaMemcpyDeviceToHost, st));

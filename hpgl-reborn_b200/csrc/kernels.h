@@ -51,13 +51,14 @@ constexpr int kBinSortMax = 1024;
 void launch_bin_sort(const Geom &g, const int *bin_start, const int *bin_cnt, const int *bin_tmp, int *bin_pts,
                      uint8_t *bin_flag, cudaStream_t st);
 // max_cand / max_cand_tmpl: the largest 27-bin candidate count of the cluster-
-// path / template-path bins; max_bin: the largest bin when above kBinSortMax
+// path / template-path bins; max_bin: the largest bin when above kBinSortMax; scans: 1 for
+// template-path bins that are better scanned (scan_is_shorter, search_common.cuh), 2 for others
 void launch_bin_region(const Geom &g, uint8_t *bin_flag, const int *bin_cnt, int *max_cand, int *n_tmpl_bins,
-                       int *tmpl_bins, int *max_cand_tmpl, int *max_bin, cudaStream_t st);
+                       int *tmpl_bins, int *max_cand_tmpl, int *max_bin, int *scans, cudaStream_t st);
 // Template-path search over a bitmap of the grid padded by the radiuses:
 // `bits` is scratch of (template_padded_cells + 31) / 32 words; template entries
-// carry template_padded_offset(dx, dy, dz) in .w. With min_cand >= 0 only bins of
-// more candidates than that are searched.
+// carry template_padded_offset(dx, dy, dz) in .w. With min_cand >= 0 only the bins
+// that launch_search_tile leaves at that limit are searched.
 long long template_padded_cells(const Geom &g);
 int template_padded_offset(const Geom &g, int dx, int dy, int dz);
 cudaError_t launch_search_template(const Geom &g, const uint8_t *mask, uint32_t *bits, int all_cells,
@@ -100,12 +101,15 @@ cudaError_t launch_search_fast(const Geom &g, const uint8_t *mask, int all_cells
                                int cand_cap, int warps, int *nb_pid, int2 *nb_rec, int *nb_n, int *tie_cells, int *tie_count,
                                int *n_template_cells, int *exact_cells, cudaStream_t st);
 // The same with the prefilter on, one cell a lane (search_tile.cu): the bins with at
-// most search_tile_limit candidates. n_bins: how many bins there are of the kind searched.
-int search_tile_limit(int k, int max_smem);
+// most `limit` candidates; with leave_scans, of the template-path ones, those that are
+// not better scanned. n_bins: how many bins there are of the kind searched.
+// search_tile_limit: the candidates that leave room for `warps` warps a block.
+int search_tile_limit(int k, int max_smem, int warps);
 cudaError_t launch_search_tile(const Geom &g, const uint8_t *mask, int all_cells, const int *bin_start,
                                const int *bin_cnt, const uint8_t *bin_flag, const int *bin_pts,
                                const unsigned long long *pts_xyz, const float *pts_vf, const uint16_t *keytab16,
-                               const SurrDev &sd, int template_bins, int n_bins, int cand_cap, int max_smem, int2 *nb_rec,
+                               const SurrDev &sd, int template_bins, int n_bins, int cand_cap, int limit, bool leave_scans,
+                               int max_smem, int2 *nb_rec,
                                int *nb_n, int *tie_cells, int *tie_count, int *n_template_cells, int *exact_cells,
                                cudaStream_t st);
 void launch_resolve_ties(const Geom &g, const int *tie_cells, const int *tie_count, int first, int chunk,

@@ -235,7 +235,7 @@ __global__ void __launch_bounds__(256) k_bin_sort(Geom g, const int *__restrict_
 __global__ void k_bin_region(Geom g, uint8_t *__restrict__ bin_flag, const int *__restrict__ bin_cnt,
                              int *__restrict__ max_cand, int *__restrict__ n_template_bins,
                              int *__restrict__ template_bins, int *__restrict__ max_cand_tmpl,
-                             int *__restrict__ max_bin)
+                             int *__restrict__ max_bin, int *__restrict__ scans)
 {
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < g.n_bins; b += gridDim.x * blockDim.x)
     {
@@ -257,6 +257,8 @@ __global__ void k_bin_region(Geom g, uint8_t *__restrict__ bin_flag, const int *
             bin_flag[b] |= 2;
             template_bins[atomicAdd(n_template_bins, 1)] = b;
             atomicMax(max_cand_tmpl, cand);
+            if (cx * g.rx < g.nx && cy * g.ry < g.ny && cz * g.rz < g.nz)
+                atomicOr(scans, scan_is_shorter(g, cx, cy, cz, cand, bin_cnt[b]) ? 1 : 2);
         }
         else
             atomicMax(max_cand, cand);
@@ -1508,10 +1510,11 @@ void launch_bin_sort(const Geom &g, const int *bin_start, const int *bin_cnt, co
     k_bin_sort<<<blocks, 256, 0, st>>>(g, bin_start, bin_cnt, bin_tmp, bin_pts, bin_flag);
 }
 void launch_bin_region(const Geom &g, uint8_t *bin_flag, const int *bin_cnt, int *max_cand, int *n_tmpl_bins,
-                       int *tmpl_bins, int *max_cand_tmpl, int *max_bin, cudaStream_t st)
+                       int *tmpl_bins, int *max_cand_tmpl, int *max_bin, int *scans, cudaStream_t st)
 {
     int blocks = (g.n_bins + 255) / 256;
-    k_bin_region<<<blocks, 256, 0, st>>>(g, bin_flag, bin_cnt, max_cand, n_tmpl_bins, tmpl_bins, max_cand_tmpl, max_bin);
+    k_bin_region<<<blocks, 256, 0, st>>>(g, bin_flag, bin_cnt, max_cand, n_tmpl_bins, tmpl_bins, max_cand_tmpl, max_bin,
+                                         scans);
 }
 
 // Template-path cells (k_search and k_search_fast leave their bins alone): a
@@ -1534,7 +1537,8 @@ __global__ void __launch_bounds__(256) k_search_template(
         const int q = threadIdx.x & 31, kk = bzi - 1 + q / 9, jj = byi - 1 + (q / 3) % 3, ii = bxi - 1 + q % 3;
         if (q < 27 && ii >= 0 && jj >= 0 && kk >= 0 && ii < g.bx && jj < g.by && kk < g.bz)
             cand = bin_cnt[(kk * g.by + jj) * g.bx + ii];
-        if (__reduce_add_sync(0xffffffffu, cand) <= min_cand) return;
+        cand = __reduce_add_sync(0xffffffffu, cand);
+        if (cand <= min_cand && !scan_is_shorter(g, bxi, byi, bzi, cand, bin_cnt[b])) return;
     }
     const int wx = min(x0 + g.rx, g.nx) - x0, wy = min(y0 + g.ry, g.ny) - y0, wz = min(z0 + g.rz, g.nz) - z0;
     const int lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;

@@ -203,6 +203,7 @@ struct SearchTile
     int sub;     // candidates near a tile, at most (beyond: all are scanned)
     int slices;  // blocks per bin
     int c_min, c_max; // the bins of this launch: c_min < candidates <= c_max
+    bool leave_scans; // and not those that are better scanned
 };
 
 __global__ void __launch_bounds__(256, 3) k_search_tile(
@@ -243,6 +244,7 @@ __global__ void __launch_bounds__(256, 3) k_search_tile(
     __syncthreads();
     const int C = s_total;
     if (C <= tl.c_min || C > tl.c_max) return;
+    if (tl.leave_scans && scan_is_shorter(g, bxi, byi, bzi, C, bin_cnt[b])) return;
 #pragma unroll 2
     for (int d = threadIdx.x; d < C; d += blockDim.x)
     {
@@ -593,7 +595,7 @@ static size_t tile_smem(int cand_cap, int cap, int sub, int warps)
 static SearchTile search_tile_shape(const Geom &g, const SurrDev &sd, int n_bins, int cand_cap, int max_smem, int &warps,
                                     size_t &smem)
 {
-    SearchTile t{1, 1, tile_cap(g.k), cand_cap <= kManyCandidates ? 256 : 1024, 1, 0, cand_cap};
+    SearchTile t{1, 1, tile_cap(g.k), cand_cap <= kManyCandidates ? 256 : 1024, 1, 0, cand_cap, false};
     const int bx = std::min(g.rx, g.nx), by = std::min(g.ry, g.ny), bz = std::min(g.rz, g.nz);
     float best = 3.4e38f;
     int cells = 0;
@@ -636,21 +638,22 @@ static SearchTile search_tile_shape(const Geom &g, const SurrDev &sd, int n_bins
     return t;
 }
 
-// Candidates per bin that k_search_tile takes at most, at k neighbours.
-int search_tile_limit(int k, int max_smem)
+// Candidates of a bin that leave room for `warps` warps a block, at k neighbours.
+int search_tile_limit(int k, int max_smem, int warps)
 {
-    const long long room = (long long)max_smem - (long long)tile_smem(0, tile_cap(k), 1024, 1);
+    const long long room = (long long)max_smem - (long long)tile_smem(0, tile_cap(k), 1024, warps);
     return (int)std::max(0LL, std::min(room / 24 / 4 * 4, 65536LL));
 }
 
 cudaError_t launch_search_tile(const Geom &g, const uint8_t *mask, int all_cells, const int *bin_start,
                                const int *bin_cnt, const uint8_t *bin_flag, const int *bin_pts,
                                const unsigned long long *pts_xyz, const float *pts_vf, const uint16_t *keytab16,
-                               const SurrDev &sd, int template_bins, int n_bins, int cand_cap, int max_smem, int2 *nb_rec,
+                               const SurrDev &sd, int template_bins, int n_bins, int cand_cap, int limit, bool leave_scans,
+                               int max_smem, int2 *nb_rec,
                                int *nb_n, int *tie_cells, int *tie_count, int *n_template_cells, int *exact_cells,
                                cudaStream_t st)
 {
-    cand_cap = std::min(cand_cap, search_tile_limit(g.k, max_smem));
+    cand_cap = std::min(cand_cap, limit);
     if (cand_cap <= 0) return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(k_search_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
     if (e != cudaSuccess) return e;
@@ -664,6 +667,7 @@ cudaError_t launch_search_tile(const Geom &g, const uint8_t *mask, int all_cells
         if (warps <= 0) return cudaErrorInvalidValue;
         tl.c_min = c_min;
         tl.c_max = c_max;
+        tl.leave_scans = leave_scans;
         k_search_tile<<<(unsigned)((long long)g.n_bins * tl.slices), warps * 32, smem, st>>>(
             g, mask, all_cells, bin_start, bin_cnt, bin_flag, bin_pts, pts_xyz, pts_vf, keytab16, sd, tl, template_bins,
             c_max, nb_rec, nb_n, tie_cells, tie_count, n_template_cells, exact_cells);
