@@ -10,10 +10,10 @@
 // a product X Y^T. So the factorisation
 //     L_ik = A_ik L_kk^-T,   A_ij -= L_ik L_jk^T
 // needs no data movement between its steps: every product it makes is of the
-// form X Y^T. How L_kk^-1 is applied is a choice (HALVES, below): as one explicit
-// 8x8 inverse M, or by halves. Right-hand sides are carried as rows of one more
-// block row X (rows 0..2 in use), which leaves X_k = (L^-1 rhs)^T and the forms
-// rhs_i^T A^-1 rhs_j as the entries of sum_k X_k X_k^T.
+// form X Y^T. How L_kk^-1 is applied is a choice: as one explicit 8x8 inverse M
+// (mma_factor), or by halves (half_factor). Right-hand sides are carried as rows of
+// one more block row X (rows 0..2 in use), which leaves X_k = (L^-1 rhs)^T and the
+// forms rhs_i^T A^-1 rhs_j as the entries of sum_k X_k X_k^T.
 //
 // Rounding. With M the error is that of a substitution times the condition of L_kk.
 // Root mean square errors against 128 bits of the sharing solves (estimate and
@@ -296,7 +296,7 @@ __device__ __forceinline__ int mma_slot(int i, int n, int nb)
 // the error of a substitution. The elimination is mma_diag's with the pivots
 // p0 and p1 = p0 + 2: (0, 2) and (4, 6), then, ODD, (1, 3) and (5, 7) (h = 0 and 1).
 // The sharing solves of 8.3M systems of 32 take 11.6 ms in place of 10.9, of 9.5M of
-// up to 64 62.5 in place of 54.5.
+// up to 64 62.7 in place of 55.8.
 struct Halves
 {
     Blk half; // E^-1 in the even rows' x, -F in the odd rows' x, O^-1 in the odd rows' y, zero elsewhere
